@@ -107,10 +107,17 @@ cudaError_t ensure_device(void** ptr, size_t* cap, size_t bytes) {
   return e;
 }
 
-gtd_status ensure_flags(gtd_handle h, size_t tiles) {
-  if (h->flags_cap >= tiles && h->d_flags)
+void release_byte_table(gtd_handle h) {
+  cudaFree(h->d_bytes);
+  h->d_bytes = nullptr;
+  h->bytes_cap = 0;
+  h->bytes_valid = false;
+}
+
+gtd_status ensure_flags(gtd_handle h, size_t groups) {
+  if (h->flags_cap >= groups && h->d_flags)
     return GTD_OK;
-  GTD_CUDA(h, ensure_field(&h->d_flags, &h->flags_cap, tiles));
+  GTD_CUDA(h, ensure_field(&h->d_flags, &h->flags_cap, groups));
   GTD_CUDA(h, cudaMemsetAsync(h->d_flags, 0, h->flags_cap * sizeof(uint32_t), h->stream));
   h->epoch = 0;
   return GTD_OK;
@@ -127,9 +134,12 @@ gtd_status next_epoch(gtd_handle h, uint32_t* epoch) {
 
 namespace {
 
-// Tile bits measured best on GB300 (1 KB tiles up to n = 25, 2 KB above:
-// n = 30 3.51 ms with 11 bits vs 3.76 ms with 10 and 4.72 ms with 12).
-int default_tile_bits(int n) { return n >= 26 ? 11 : 10; }
+// Tile bits measured best on GB300: one tile up to n = 12 (n = 12: 16 us with
+// 12 bits against 30 with 10); few classes per tile while the levels are too
+// narrow to fill the GPU (n = 20: 108 us with 8 bits, 132 with 10; n = 25: 200
+// against 259); 11 bits from there (n = 28: 352 us against 355 with 10 and 348
+// with 8; n = 30: 718 against 743 and 958; n = 33: 4.68 ms against 5.14 and 7.5).
+int default_tile_bits(int n) { return n <= kDpMaxTileBits ? n : n <= 25 ? 8 : 11; }
 
 // Allocates (or grows) the table and flag buffers and enqueues the
 // validation, DP and tree kernels for one graph. Outputs go to
@@ -138,27 +148,33 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, int n, const gtd_dp_o
                       int32_t* d_td, int32_t* d_parent, int32_t* d_order) {
   const int tile_bits = (opts && opts->tile_bits > 0) ? opts->tile_bits : default_tile_bits(n);
   const DpLayout L = make_dp_layout(n, tile_bits);
+  const int lb = L.lb < kDpMinTileBits ? kDpMinTileBits : L.lb;  // n < 8: one padded tile
   const size_t table_bytes = size_t(1) << n;
-  if (h->table_cap < table_bytes)
+  const size_t plane_bytes = size_t(L.ntiles) * dp_tile_bytes(lb);
+  const uint32_t groups = dp_groups(L.binom, L.nh, lb);
+  h->bytes_valid = false;
+  if (h->table_cap < plane_bytes) {
     h->have_table = false;
-  GTD_CUDA(h, ensure_field(&h->d_table, &h->table_cap, table_bytes));
-  gtd_status s = ensure_flags(h, L.ntiles);
+    release_byte_table(h);
+  }
+  GTD_CUDA(h, ensure_field(&h->d_table, &h->table_cap, plane_bytes));
+  gtd_status s = ensure_flags(h, groups);
   if (s != GTD_OK)
     return s;
 
   DpBatchParams p;
   dp_fill_binom(p);
   p.single.table_off = 0;
-  p.single.tile_base = 0;
+  p.single.flag_base = 0;
   p.single.ntiles = L.ntiles;
   p.single.adj_off = 0;
   p.single.n = n;
   p.single.nh = L.nh;
-  p.single.lb = L.lb;
+  p.single.lb = lb;
   p.single.out_idx = 0;
   p.num_graphs = 1;
-  p.lb = L.lb;
-  p.total_tiles = L.ntiles;
+  p.lb = lb;
+  p.total_groups = groups;
   p.table = h->d_table;
   p.flags = h->d_flags;
   p.ticket = reinterpret_cast<uint32_t*>(h->d_io + kIoTicket);
@@ -172,21 +188,23 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, int n, const gtd_dp_o
   p.parent_out = d_parent;
   p.order_out = d_order;
 
-  if (h->dp_occ[p.lb] <= 0)
-    h->dp_occ[p.lb] = dp_tile_occupancy(p.lb);
-  int occ = h->dp_occ[p.lb];
+  p.kid_rows = L.nh;
+  int& dp_occ = h->dp_occ[p.lb][L.nh];
+  if (dp_occ <= 0)
+    dp_occ = dp_tile_occupancy(p.lb, L.nh);
+  int occ = dp_occ;
   if (opts && opts->ctas_per_sm > 0 && opts->ctas_per_sm < occ)
     occ = opts->ctas_per_sm;
   if (occ < 1)
     occ = 1;
   long long ctas = static_cast<long long>(h->num_sms) * occ;
-  if (ctas > p.total_tiles)
-    ctas = p.total_tiles;
+  if (ctas > p.total_groups)
+    ctas = p.total_groups;
 
   GTD_CUDA(h, cudaMemsetAsync(h->d_io, 0, 4 * sizeof(int32_t), h->stream));
   if (take_poison_fault())  // test injection: every byte must be written before it is read
     GTD_CUDA(h, cudaMemsetAsync(h->d_table, 0xFF, h->table_cap, h->stream));
-  if (take_stall_fault())  // test injection: ticket 0 (the level-0 tile) is never taken
+  if (take_stall_fault())  // test injection: ticket 0 (the level-0 group) is never taken
     GTD_CUDA(h, cudaMemsetAsync(h->d_io + kIoTicket, 1, 1, h->stream));
   GTD_CUDA(h, dp_launch_validate(p, h->stream));
   GTD_CUDA(h, cudaEventRecord(h->ev[0], h->stream));
@@ -202,9 +220,21 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, int n, const gtd_dp_o
   st = gtd_dp_stats{};
   st.table_bytes = table_bytes;
   st.alg_bytes = table_bytes + static_cast<uint64_t>(n) * (table_bytes / 2);
-  st.tile_bits = p.lb;
-  st.tiles = static_cast<int>(p.total_tiles);
+  h->last_tile_bits = L.lb;
+  st.tile_bits = L.lb;
+  st.tiles = static_cast<int>(L.ntiles);
   st.ctas = static_cast<int>(ctas);
+  return GTD_OK;
+}
+
+// The last solve's byte table in h->d_bytes (enqueued on the stream).
+gtd_status make_byte_table(gtd_handle h) {
+  if (h->bytes_valid)
+    return GTD_OK;
+  const size_t bytes = size_t(1) << h->last_params.single.n;
+  GTD_CUDA(h, ensure_field(&h->d_bytes, &h->bytes_cap, bytes));
+  GTD_CUDA(h, dp_launch_expand(h->last_params, h->d_bytes, bytes, h->stream));
+  h->bytes_valid = true;
   return GTD_OK;
 }
 
@@ -298,6 +328,7 @@ gtd_status gtd_destroy(gtd_handle h) {
       cudaGraphExecDestroy(h->bgraph);
     gtd_bnb_release(h);
     cudaFree(h->d_table);
+    cudaFree(h->d_bytes);
     cudaFree(h->d_flags);
     cudaFree(h->d_io);
     cudaFree(h->d_adj);
@@ -443,14 +474,20 @@ gtd_status gtd_dp_table(gtd_handle h, const uint8_t** d_table, uint64_t* bytes, 
     return GTD_INVALID_ARG;
   if (!h->have_table)
     return fail(h, GTD_NO_RESULT, "no DP table: solve a graph first");
-  if (d_table)
-    *d_table = h->d_table;
+  if (d_table) {
+    DeviceGuard g(h->device);
+    const gtd_status s = make_byte_table(h);
+    if (s != GTD_OK)
+      return s;
+    GTD_CUDA(h, cudaStreamSynchronize(h->stream));
+    *d_table = h->d_bytes;
+  }
   if (bytes)
     *bytes = uint64_t(1) << h->last_params.single.n;
   if (n)
     *n = h->last_params.single.n;
   if (tile_bits)
-    *tile_bits = h->last_params.lb;
+    *tile_bits = h->last_tile_bits;
   return GTD_OK;
 }
 
@@ -463,7 +500,10 @@ gtd_status gtd_dp_read_table(gtd_handle h, uint8_t* out, uint64_t bytes) {
   if (!out || bytes < need)
     return fail(h, GTD_INVALID_ARG, "output buffer smaller than the table");
   DeviceGuard g(h->device);
-  GTD_CUDA(h, cudaMemcpyAsync(out, h->d_table, need, cudaMemcpyDeviceToHost, h->stream));
+  const gtd_status s = make_byte_table(h);
+  if (s != GTD_OK)
+    return s;
+  GTD_CUDA(h, cudaMemcpyAsync(out, h->d_bytes, need, cudaMemcpyDeviceToHost, h->stream));
   GTD_CUDA(h, cudaStreamSynchronize(h->stream));
   return GTD_OK;
 }

@@ -33,6 +33,9 @@ struct Plan {
   std::vector<DpGraph> graphs;  // processing order
   uint64_t table_bytes = 0;
   uint32_t total_tiles = 0;
+  uint32_t total_groups = 0;    // tickets
+  int kid_rows = 0;             // largest nh
+  uint64_t plane_bytes = 0;     // the pool itself; table_bytes counts one byte per padded subset
   uint64_t subsets = 0;
   uint64_t alg_bytes = 0;
   std::vector<uint32_t> level_base;  // [graph][level]: first ticket of that level
@@ -91,11 +94,18 @@ void pick_tile_bits(gtd_handle h, const gtd_graph_desc* descs, int count, const 
       uniform(lb);
     }
   }
+  // high vertices of the batch's largest graph at lb bits
+  auto high_at = [&](int lb) {
+    int n = GTD_DP_MAX_N;
+    while (n > 0 && !count_by_n[n])
+      --n;
+    return std::min(std::max(0, n - lb), kDpMaxHigh);
+  };
   int occ_one[kTuneLbMax + 1] = {};
   for (int lb = kTuneLbMin; lb <= kTuneLbMax; ++lb)
-    occ_one[lb] = std::max(1, dp_tile_occupancy(lb));
+    occ_one[lb] = std::max(1, dp_tile_occupancy(lb, high_at(lb)));
   for (int c = kTuneLbMin; c <= kTuneLbMax; ++c) {
-    const int occ_mixed = dp_mixed_occupancy(c);
+    const int occ_mixed = dp_mixed_occupancy(c, high_at(kTuneLbMin));
     const float eff = h->tune_mixed_eff[c];
     if (eff <= 0 || occ_mixed < 1)
       continue;  // unmeasured: never mix at this cap
@@ -135,8 +145,14 @@ void make_plan(Plan& P, const gtd_graph_desc* descs, int count) {
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return descs[a].n > descs[b].n; });
   P.graphs.resize(count);
+  uint32_t binom[kDpMaxHigh + 1][kDpMaxHigh + 1] = {};
+  for (int a = 0; a <= kDpMaxHigh; ++a) {
+    binom[a][0] = 1;
+    for (int b = 1; b <= a; ++b)
+      binom[a][b] = binom[a - 1][b - 1] + (b <= a - 1 ? binom[a - 1][b] : 0u);
+  }
   uint64_t off = 0;
-  uint32_t tile = 0;
+  uint32_t tile = 0, group = 0;
   for (int k = 0; k < count; ++k) {
     const gtd_graph_desc& d = descs[order[k]];
     DpGraph& G = P.graphs[k];
@@ -146,32 +162,30 @@ void make_plan(Plan& P, const gtd_graph_desc* descs, int count) {
     G.nh = d.n > lb ? d.n - lb : 0;
     G.ntiles = 1u << G.nh;
     G.table_off = off;
-    G.tile_base = tile;
+    G.flag_base = group;
     G.adj_off = static_cast<uint32_t>(d.offset);
     G.out_idx = order[k];
-    off += uint64_t(G.ntiles) << lb;
+    off += uint64_t(G.ntiles) * dp_tile_bytes(lb);
+    P.table_bytes += uint64_t(G.ntiles) << lb;
     tile += G.ntiles;
+    group += dp_groups(binom, G.nh, lb);
+    P.kid_rows = std::max(P.kid_rows, G.nh);
     const uint64_t sub = uint64_t(1) << d.n;
     P.subsets += sub;
     P.alg_bytes += sub + uint64_t(d.n) * (sub / 2);
   }
-  P.table_bytes = off;
+  P.plane_bytes = off;
   P.total_tiles = tile;
+  P.total_groups = group;
   // Tickets level-major across graphs: level 0 of every graph, then level 1...
   P.level_base.assign(size_t(count) * kLevelSlots, 0);
-  uint32_t binom[kDpMaxHigh + 1][kDpMaxHigh + 1] = {};
-  for (int a = 0; a <= kDpMaxHigh; ++a) {
-    binom[a][0] = 1;
-    for (int b = 1; b <= a; ++b)
-      binom[a][b] = binom[a - 1][b - 1] + (b <= a - 1 ? binom[a - 1][b] : 0u);
-  }
   uint32_t ticket = 0;
   for (int j = 0; j <= kDpMaxHigh; ++j)
     for (int k = 0; k < count; ++k) {
       const DpGraph& G = P.graphs[k];
       if (j <= G.nh) {
         P.level_base[size_t(k) * kLevelSlots + j] = ticket;
-        ticket += binom[G.nh][j];
+        ticket += (binom[G.nh][j] + dp_group_tiles(G.lb) - 1) / dp_group_tiles(G.lb);
       }
     }
 }
@@ -221,14 +235,14 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
   make_plan(P, descs, count);
   const int lb = P.lb;
   const uint64_t timeout = (opts && opts->timeout_ns) ? opts->timeout_ns : 10ull * 1000 * 1000 * 1000;
-  int occ = P.mixed ? dp_mixed_occupancy(lb) : dp_tile_occupancy(lb);
+  int occ = P.mixed ? dp_mixed_occupancy(lb, P.kid_rows) : dp_tile_occupancy(lb, P.kid_rows);
   if (opts && opts->ctas_per_sm > 0 && opts->ctas_per_sm < occ)
     occ = opts->ctas_per_sm;
   if (occ < 1)
     occ = 1;
   long long ctas = static_cast<long long>(h->num_sms) * occ;
-  if (ctas > P.total_tiles)
-    ctas = P.total_tiles;
+  if (ctas > P.total_groups)
+    ctas = P.total_groups;
   const bool use_graph = !opts || opts->use_cuda_graph;
   const uint64_t key = fingerprint(P, d_adj, d_td, d_parent, static_cast<int>(ctas), timeout);
 
@@ -252,7 +266,7 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
   if (use_graph && h->bgraph_valid && h->bgraph_key == key && same_buffers) {
     st.graph_replayed = 1;
     if (poison)
-      GTD_CUDA(h, cudaMemsetAsync(h->d_table, 0xFF, P.table_bytes, h->stream));
+      GTD_CUDA(h, cudaMemsetAsync(h->d_table, 0xFF, P.plane_bytes, h->stream));
     GTD_CUDA(h, cudaEventRecord(h->ev[0], h->stream));
     GTD_CUDA(h, cudaGraphLaunch(h->bgraph, h->stream));
     GTD_CUDA(h, cudaEventRecord(h->ev[1], h->stream));
@@ -263,11 +277,13 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
   // Device state for this shape.
   h->have_table = false;
   h->bgraph_valid = false;
-  GTD_CUDA(h, ensure_field(&h->d_table, &h->table_cap, P.table_bytes));
-  gtd_status s = ensure_flags(h, P.total_tiles);
+  if (h->table_cap < P.plane_bytes)
+    release_byte_table(h);
+  GTD_CUDA(h, ensure_field(&h->d_table, &h->table_cap, P.plane_bytes));
+  gtd_status s = ensure_flags(h, P.total_groups);
   if (s != GTD_OK)
     return s;
-  GTD_CUDA(h, ensure_field(&h->d_tile_map, &h->tile_map_cap, P.total_tiles));
+  GTD_CUDA(h, ensure_field(&h->d_tile_map, &h->tile_map_cap, P.total_groups));
   GTD_CUDA(h, ensure_field(&h->d_level_base, &h->level_base_cap, P.level_base.size()));
   GTD_CUDA(h, ensure_field(&h->d_bgraphs, &h->bgraphs_cap, size_t(count)));
   // Descriptors and level bases go up through pinned staging (synchronised
@@ -295,7 +311,8 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
   bp.num_graphs = count;
   bp.lb = lb;
   bp.mixed = P.mixed ? 1 : 0;
-  bp.total_tiles = P.total_tiles;
+  bp.kid_rows = P.kid_rows;
+  bp.total_groups = P.total_groups;
   bp.table = h->d_table;
   bp.flags = h->d_flags;
   bp.ticket = reinterpret_cast<uint32_t*>(h->d_io + kIoTicket);
@@ -306,7 +323,7 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
   bp.parent_out = d_parent;
   GTD_CUDA(h, dp_launch_fill_tile_map(bp, h->stream));
   if (poison)
-    GTD_CUDA(h, cudaMemsetAsync(h->d_table, 0xFF, P.table_bytes, h->stream));
+    GTD_CUDA(h, cudaMemsetAsync(h->d_table, 0xFF, P.plane_bytes, h->stream));
 
   if (use_graph) {
     if (h->bgraph) {
@@ -316,7 +333,7 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
     bp.epoch = kGraphEpoch;
     cudaGraph_t graph = nullptr;
     GTD_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t ce = cudaMemsetAsync(h->d_flags, 0, size_t(P.total_tiles) * sizeof(uint32_t), h->stream);
+    cudaError_t ce = cudaMemsetAsync(h->d_flags, 0, size_t(P.total_groups) * sizeof(uint32_t), h->stream);
     if (ce == cudaSuccess)
       ce = cudaMemsetAsync(h->d_io, 0, 4 * sizeof(int32_t), h->stream);
     if (ce == cudaSuccess)

@@ -3,8 +3,8 @@
 // Reference: DynamicGPU (Treedepth/src/dynamic_gpu/dynamic_gpu.cu:40-201),
 // which runs one thread per k-subset per level, labels components by repeated
 // CSR sweeps, re-encodes S - v with 64-bit divides and gathers 8-byte
-// {td, root} entries at random. This kernel computes the same table values
-// with a different schedule and layout:
+// {td, root} entries at random. This kernel computes the same values with a
+// different schedule and layout:
 //
 //  * Recurrence. For |S| >= 3, S is connected iff at least two v in S leave
 //    S - v connected (a connected graph has >= 2 non-cut vertices, and if
@@ -15,33 +15,32 @@
 //      T[S] = 1 + min_v T[S - v]   (connected; dynamic_gpu.cu:68-89)
 //      T[S] = max_v T[S - v]       (disconnected; = max over components,
 //                                   dynamic_gpu.cu:90-111)
-//    with each table byte holding td << 1 | connected. No per-subset BFS, no
-//    ranking per child.
-//  * Reduction. Deleting a vertex lowers treedepth by at most one, so the
-//    children's treedepths are td(S) - 1 or td(S): two consecutive values at
-//    most. Their OR plus their AND is then 2a + 1 when both a and a + 1
-//    occur (td(S) = a + 1, connected or not) and 2v when all equal v
-//    (td(S) = v + connected(S)), so with s = OR + AND,
-//      td(S) = (s >> 1) + ((s & 1) | connected(S)).
-//    OR and AND of the raw bytes are plain 32-bit logic over 4 subsets at
-//    once; a third word collects "at least two connected children" in bit 0.
-//  * Layout (gtd_dp_layout.h). Tiles of 2^lb subsets share a high part H;
-//    a tile's cross-tile children are the whole tiles H - h one level down,
-//    read as contiguous 2^lb-byte blocks (16-byte vector loads through L2);
-//    the in-tile children are resolved in shared memory, 4 subsets per
-//    32-bit word, words in popcount order of the word index, one unrolled
-//    pass per popcount class (its size and child count compile-time).
-//  * Schedule. One persistent launch; every warp is an independent tile
-//    worker (no CTA barriers in the loop). A warp takes a tile by ticket
-//    (atomicAdd) in level-major order and decodes it with ballots over a
-//    shared-memory binomial table; lane v in H ranks child tile H - v by a
-//    prefix and a suffix sum and waits on its ready flag (each wait bounded
-//    by a deadline). The warp reduces the cross-tile children with OR / AND /
-//    majority logic on 16-byte loads, keeps that summary as two virtual
-//    children in shared memory, resolves the tile there, stores it and
-//    publishes its flag with a release store. A tile only waits on tiles
-//    with smaller tickets, and a ticket is only taken by a running warp, so
-//    the smallest unfinished ticket can always proceed.
+//    No per-subset BFS, no ranking per child.
+//  * Bit slicing. Deleting a vertex lowers treedepth by at most one, so the
+//    children's treedepths are a or a + 1 with a = td(S) - 1 or td(S), and
+//    residues modulo 3 tell which: the table keeps three bits per subset
+//    (planes "td = 0 mod 3", "td = 1 mod 3", "connected"), 32 subsets per
+//    word. Children are reduced by OR per residue and a two-bit saturating
+//    count of connected ones: 3.5 logic operations per child and 32 subsets,
+//    where one byte per subset took 2 per child and 4 subsets (2.67 times
+//    the bytes from L2 and DRAM too). Full treedepths are read back along a
+//    chain of deletions (TreeCtx::td_of).
+//  * Layout (gtd_dp_layout.h). Tiles of 2^lb subsets share a high part H; a
+//    tile is its three planes, 2^(lb-5) words each. The cross-tile children
+//    are whole tiles H - h one level down, read as 16-byte vectors; the
+//    in-tile children are other words of the tile, resolved in popcount order
+//    of the word index; the five lowest vertices live inside the word. There
+//    the children of a subset are shifts of the word itself, one round per
+//    subset size; four tiles are resolved together (resolve_quad), their
+//    words transposed by bytes so that only three vertices are left inside.
+//  * Schedule. One persistent launch; a CTA takes a group of consecutive
+//    tiles of one level by ticket (atomicAdd, level-major), unranks them one
+//    per thread, checks the ready flags of their children's groups, reduces
+//    the cross-tile children, resolves the tiles in shared memory, stores
+//    them and publishes the group's flag with a release store. A group only
+//    waits on groups with smaller tickets, and tickets are only taken by
+//    running CTAs, so the smallest unfinished ticket can always proceed; each
+//    wait is bounded by a deadline.
 //
 // Reconstruction (dp_tree_kernel): one warp, one lane per vertex, rebuilds
 // the reference's tree (first-argmin root per component, dynamic_gpu.cu:84-87,
@@ -55,176 +54,191 @@
 
 namespace gtd {
 
-// One warp resolves one tile; a CTA holds kDpWarps independent tile workers
-// that share only the adjacency and the word order table.
-constexpr int kDpWarps = 4;
-
+// A group of tiles of LB bits in shared memory: five planes of kWords x
+// kGroup words (the cross-tile children's summary: residues 0, 1, 2 present,
+// at least one and at least two connected; the first three then receive the
+// tiles).
 template <int LB>
 struct TileShape {
-  static constexpr int kEntries = 1 << LB;
-  static constexpr int kWords = kEntries / 4;   // 4 subsets per 32-bit word
-  static constexpr int kWordBits = LB - 2;
-  // dynamic shared memory: per warp T and U (kWords words each), then, for
-  // the CTA, the word order (kWords uint16) and a copy of the binomial
-  // table, then per warp the child-tile list (32 words). Between the two
-  // phases T and U hold the cross-tile children's summary as two virtual
-  // children (see the in-tile loop); T then receives the tile.
-  static constexpr size_t kPerWarp = size_t(2) * kWords * 4;
-  static constexpr size_t kOrderOff = size_t(kDpWarps) * kPerWarp;
-  static constexpr size_t kBinomOff = (kOrderOff + kWords * 2 + 15) & ~size_t(15);
-  static constexpr size_t kKidsOff = (kBinomOff + sizeof(uint32_t) * (kDpMaxHigh + 1) * (kDpMaxHigh + 1) + 15) &
-                                     ~size_t(15);
-  static constexpr size_t kSmem = kKidsOff + size_t(kDpWarps) * 32 * 4;
+  static constexpr uint32_t kWords = 1u << (LB - 5);         // words of a plane of a tile
+  static constexpr uint32_t kGroup = dp_group_tiles(LB);     // tiles of a group
+  static constexpr uint32_t kQuads = kGroup / 4;             // sets of four tiles resolved together
+  static constexpr uint32_t kPlane = kWords * kGroup;
+  static constexpr uint32_t kChunks = kWords / 4;            // 16-byte parts of a plane of a tile
+  static constexpr uint32_t kTileBytes = dp_tile_bytes(LB);
 };
 
 using Binom = uint32_t[kDpMaxHigh + 1][kDpMaxHigh + 1];
 
-// Per word (4 subsets, one per byte): o = OR and a = AND of the children's
-// bytes, d = "at least two connected children" in bit 0 of each byte.
+// Offset of word w of tile q in a shared-memory plane. The four tiles of a
+// quad are adjacent (one 16-byte access in the in-tile phase, a warp on one w
+// covers a row); the quads of a row are permuted by the word's chunk so that
+// the chunk-wise accesses of the other phases spread over the banks.
+template <int LB>
+__device__ __forceinline__ uint32_t plane_at(uint32_t q, uint32_t w) {
+  using Shape = TileShape<LB>;
+  constexpr uint32_t kStep = Shape::kChunks >= 8 ? 4u : 32u / Shape::kChunks;
+  return (w * Shape::kGroup + q) ^ (((w >> 2) * kStep) & 28u);
+}
+
+// What the children of 32 subsets have: residue k of their treedepths
+// present (o0, o1, o2), at least one (c1) and two (c2) connected.
 struct Acc {
-  uint32_t o, a, d;
+  uint32_t o0 = 0u, o1 = 0u, o2 = 0u, c1 = 0u, c2 = 0u;
 };
 
-__device__ __forceinline__ void acc_init(Acc& c) {
-  c.o = 0u;
-  c.a = 0xFFFFFFFFu;
-  c.d = 0u;
+__device__ __forceinline__ void acc_add1(Acc& a, uint32_t p0, uint32_t p1, uint32_t c) {
+  a.o0 |= p0;
+  a.o1 |= p1;
+  a.o2 |= ~(p0 | p1);
+  a.c2 |= a.c1 & c;
+  a.c1 |= c;
 }
 
-__device__ __forceinline__ void acc_add2(Acc& c, uint32_t x, uint32_t y) {
-  c.d |= (c.o & (x | y)) | (x & y);  // majority of (any before, x, y)
-  c.o |= x | y;
-  c.a &= x & y;
+__device__ __forceinline__ void acc_add2(Acc& a, uint32_t p0, uint32_t p1, uint32_t c, uint32_t q0, uint32_t q1,
+                                         uint32_t d) {
+  a.o0 |= p0 | q0;
+  a.o1 |= p1 | q1;
+  a.o2 |= ~(p0 | p1);
+  a.o2 |= ~(q0 | q1);
+  a.c2 |= (a.c1 & (c | d)) | (c & d);
+  a.c1 |= c | d;
 }
 
-__device__ __forceinline__ void acc_add3(Acc& c, uint32_t x, uint32_t y, uint32_t z) {
-  const uint32_t any = x | y | z;
-  c.d |= (c.o & any) | (x & y) | (x & z) | (y & z);  // at least two of (any before, x, y, z)
-  c.o |= any;
-  c.a &= x & y & z;
+struct Planes {
+  uint32_t p0, p1, c;
+};
+
+// Connectivity of the subsets of size <= 2 of a word (the count of connected
+// children only decides it from size 3 on): conn = (count & keep) | set.
+struct SmallSets {
+  uint32_t keep = 0xFFFFFFFFu, set = 0u, zero = 0u;  // zero: the empty set's position (td 0)
+};
+
+// Residues of the subsets: 1 + min over the children when connected, else
+// the max; the children hold a and possibly a + 1, so residue k is the result
+// iff k + 1 is absent and (connected) k - 1 or (disconnected) k is present.
+__device__ __forceinline__ Planes finish(const Acc& a, const SmallSets& s) {
+  Planes r;
+  r.c = (a.c2 & s.keep) | s.set;
+  r.p0 = (~a.o1 & ((r.c & a.o2) | (~r.c & a.o0))) | s.zero;
+  r.p1 = ~a.o2 & ((r.c & a.o0) | (~r.c & a.o1));
+  return r;
 }
 
-__device__ __forceinline__ void acc_add1(Acc& c, uint32_t x) {
-  c.d |= c.o & x;
-  c.o |= x;
-  c.a &= x;
-}
+// Four sets of 8 subsets, one per byte, each over the three lowest vertices
+// (position x in the byte = the subset x), from the summary of their other
+// children, by size of x: position 0; its broadcast to positions 1, 2, 4;
+// 3, 5, 6 from those by one shift per vertex; 7 from 3, 5, 6.
+__device__ __forceinline__ Planes resolve_octets(const Acc& ext, const SmallSets& s) {
+  Planes r = finish(ext, s);
+  Acc a = ext;
+  a.o0 |= (r.p0 & 0x01010101u) * 0x16u;
+  a.o1 |= (r.p1 & 0x01010101u) * 0x16u;
+  a.o2 |= (~(r.p0 | r.p1) & 0x01010101u) * 0x16u;
+  a.c2 |= a.c1 & ((r.c & 0x01010101u) * 0x16u);
+  r = finish(a, s);
 
-// Four subsets with |S| >= 3 (connected <=> >= 2 connected children) and at
-// least one child each: per byte s = OR(td) + AND(td) <= 126, so no carries;
-// td = (s >> 1) + ((s & 1) | connected), stored as td << 1 | connected.
-__device__ __forceinline__ uint32_t resolve4(uint32_t o, uint32_t a, uint32_t d) {
-  const uint32_t s = ((o & 0xFEFEFEFEu) + (a & 0xFEFEFEFEu)) >> 1;
-  const uint32_t half = (s & 0xFEFEFEFEu) | (d & 0x01010101u);  // 2 (s >> 1) | connected
-  return half + (((s | d) & 0x01010101u) << 1);
-}
-
-__device__ __forceinline__ bool adjacent_in(const uint64_t* adj, int n, uint64_t s2) {
-  const int u = __ffsll(static_cast<long long>(s2)) - 1;
-  const int v = 63 - __clzll(static_cast<long long>(s2));
-  return u < n && v < n && ((__ldg(adj + u) >> v) & 1ull);
-}
-
-// One subset of size k from its children's OR o, AND a and count flag d;
-// `adjacent` gives connectivity when k == 2.
-__device__ __forceinline__ uint32_t resolve1(uint32_t o, uint32_t a, uint32_t d, int k, bool adjacent) {
-  if (k == 0)
-    return 0u;  // empty set: td 0
-  const uint32_t cn = k == 1 ? 1u : k == 2 ? (adjacent ? 1u : 0u) : (d & 1u);
-  const uint32_t s = ((o & 0xFEu) + (a & 0xFEu)) >> 1;
-  return ((s & 0xFEu) + (((s | cn) & 1u) << 1)) | cn;
-}
-
-__device__ __forceinline__ void fold1(uint32_t& o, uint32_t& a, uint32_t& d, uint32_t v) {
-  d |= o & v;
-  o |= v;
-  a &= v;
-}
-
-__device__ __forceinline__ void fold2(uint32_t& o, uint32_t& a, uint32_t& d, uint32_t x, uint32_t y) {
-  d |= (o & (x | y)) | (x & y);  // majority of (any before, x, y)
-  o |= x | y;
-  a &= x & y;
-}
-
-// The word's four subsets (low bits 00, 01, 10, 11), all of size >= 3, from
-// the summary (o, a, d) of their children outside the word: subset 00 is
-// final first and is folded into 01 and 10, which are then final and are
-// folded into 11.
-__device__ __forceinline__ uint32_t resolve_word(uint32_t o, uint32_t a, uint32_t d) {
-  uint32_t v = resolve4(o, a, d);
-  const uint32_t x = __byte_perm(v, 0u, 0x4004u);  // byte 0 into bytes 1 and 2
-  d |= o & x;
-  o |= x;
-  a &= x | 0xFF0000FFu;
-  v = resolve4(o, a, d);
-  const uint32_t y1 = __byte_perm(v, 0u, 0x1444u), y2 = __byte_perm(v, 0u, 0x2444u);  // bytes 1, 2 into 3
-  d |= (o & (y1 | y2)) | (y1 & y2);
-  o |= y1 | y2;
-  a &= (y1 & y2) | 0x00FFFFFFu;
-  return resolve4(o, a, d);
-}
-
-// The same for a word that may hold subsets of size <= 2 (k = |S| of its
-// subset 00; S0 the subset 00 itself): one byte at a time, connectivity of a
-// pair from the adjacency.
-__device__ __forceinline__ uint32_t resolve_word_small(uint32_t go, uint32_t ga, uint32_t gd, int k,
-                                                       const uint64_t* adj, int n, uint64_t S0) {
-  uint32_t o[4], a[4], d[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    o[q] = (go >> (8 * q)) & 0xFFu;
-    a[q] = (ga >> (8 * q)) & 0xFFu;
-    d[q] = (gd >> (8 * q)) & 0xFFu;
+  constexpr uint32_t kHas0 = 0xAAAAAAAAu, kHas1 = 0xCCCCCCCCu, kHas2 = 0xF0F0F0F0u;
+  uint32_t p2 = ~(r.p0 | r.p1);
+  a = ext;
+  a.o0 |= (r.p0 << 1) & kHas0;
+  a.o1 |= (r.p1 << 1) & kHas0;
+  a.o2 |= (p2 << 1) & kHas0;
+  a.o0 |= (r.p0 << 2) & kHas1;
+  a.o1 |= (r.p1 << 2) & kHas1;
+  a.o2 |= (p2 << 2) & kHas1;
+  a.o0 |= (r.p0 << 4) & kHas2;
+  a.o1 |= (r.p1 << 4) & kHas2;
+  a.o2 |= (p2 << 4) & kHas2;
+  {
+    const uint32_t x = (r.c << 1) & kHas0, y = (r.c << 2) & kHas1, z = (r.c << 4) & kHas2;
+    a.c2 |= ((x & y) | (x & z) | (y & z)) | (a.c1 & (x | y | z));
   }
-  const uint32_t v0 = resolve1(o[0], a[0], d[0], k, k == 2 && adjacent_in(adj, n, S0));
-  fold1(o[1], a[1], d[1], v0);
-  fold1(o[2], a[2], d[2], v0);
-  const uint32_t v1 = resolve1(o[1], a[1], d[1], k + 1, k + 1 == 2 && adjacent_in(adj, n, S0 | 1u));
-  const uint32_t v2 = resolve1(o[2], a[2], d[2], k + 1, k + 1 == 2 && adjacent_in(adj, n, S0 | 2u));
-  fold1(o[3], a[3], d[3], v1);
-  fold1(o[3], a[3], d[3], v2);
-  const uint32_t v3 = resolve1(o[3], a[3], d[3], k + 2, k + 2 == 2 && adjacent_in(adj, n, S0 | 3u));
-  return v0 | (v1 << 8) | (v2 << 16) | (v3 << 24);
+  r = finish(a, s);
+
+  // bits 3, 5, 6 of a byte plus 0x78 carry into its bit 7 iff one is set
+  constexpr uint32_t kPairs = 0x68686868u, kCarry = 0x78787878u, kTop = 0x80808080u;
+  p2 = ~(r.p0 | r.p1);
+  a = ext;
+  a.o0 |= ((r.p0 & kPairs) + kCarry) & kTop;
+  a.o1 |= ((r.p1 & kPairs) + kCarry) & kTop;
+  a.o2 |= ((p2 & kPairs) + kCarry) & kTop;
+  {
+    const uint32_t x = r.c << 4, y = r.c << 2, z = r.c << 1;
+    a.c2 |= (((x & y) | (x & z) | (y & z)) | (a.c1 & (x | y | z))) & kTop;
+  }
+  const Planes t = finish(a, s);
+  r.p0 = (r.p0 & ~kTop) | (t.p0 & kTop);
+  r.p1 = (r.p1 & ~kTop) | (t.p1 & kTop);
+  r.c = (r.c & ~kTop) | (t.c & kTop);
+  return r;
 }
 
-// A word's summary (o, a, d) of at least one child is reproduced by two
-// virtual children: o itself and a with bit 0 replaced by d. Their OR is o
-// (a's bits lie inside o's, d implies o's bit 0), their AND carries a's
-// treedepth bits, and both have bit 0 set exactly when d is: at least two
-// connected children.
-__device__ __forceinline__ uint32_t second_child(const Acc& c) {
-  return (c.a & 0xFEFEFEFEu) | (c.d & 0x01010101u);
+// Byte t of x[b] to byte b of x[t].
+__device__ __forceinline__ void transpose_bytes(uint32_t& x0, uint32_t& x1, uint32_t& x2, uint32_t& x3) {
+  const uint32_t a = __byte_perm(x0, x1, 0x5140u), b = __byte_perm(x2, x3, 0x5140u);
+  const uint32_t c = __byte_perm(x0, x1, 0x7362u), d = __byte_perm(x2, x3, 0x7362u);
+  x0 = __byte_perm(a, b, 0x5410u);
+  x1 = __byte_perm(a, b, 0x7632u);
+  x2 = __byte_perm(c, d, 0x5410u);
+  x3 = __byte_perm(c, d, 0x7632u);
 }
 
-// Level j, high part H and start of level j - 1 of local tile t of a graph
-// with nh high vertices (level-major order, colex rank inside a level),
-// computed by the whole warp: lane i <= nh holds the running level total
-// sum_{k <= i} C(nh, k) and a ballot counts the levels that end at or before
-// t; each element of H is then the largest a < nh with C(a, k) <= r (colex
-// unranking, one ballot per element, k = j .. 1).
-__device__ __forceinline__ void decode_tile(const Binom& binom, int nh, uint32_t t, int& j, uint32_t& H,
-                                                 uint32_t& off_prev) {
-  const int lane = threadIdx.x & 31;
-  uint32_t cum = lane <= nh ? binom[nh][lane] : 0u;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t x = __shfl_up_sync(0xffffffffu, cum, d);
-    if (lane >= d)
-      cum += x;
+// The word of four tiles (32 subsets each, the five lowest vertices inside
+// the word) from the summary a[b] of tile b's children outside the word.
+// Byte t of a word holds the subsets whose vertices 3 and 4 are the bits of
+// t: after a byte transpose a[t] holds them for all four tiles, t = 0 is a
+// child of t = 1 and 2, and those are of 3. Resolving the words one by one
+// with all five vertices inside takes three rounds of five shifts instead of
+// this one round of three per octet: 210 operations a word against 120.
+__device__ __forceinline__ void resolve_quad(Acc (&a)[4], SmallSets (&s)[4], Planes (&r)[4]) {
+  transpose_bytes(a[0].o0, a[1].o0, a[2].o0, a[3].o0);
+  transpose_bytes(a[0].o1, a[1].o1, a[2].o1, a[3].o1);
+  transpose_bytes(a[0].o2, a[1].o2, a[2].o2, a[3].o2);
+  transpose_bytes(a[0].c1, a[1].c1, a[2].c1, a[3].c1);
+  transpose_bytes(a[0].c2, a[1].c2, a[2].c2, a[3].c2);
+  transpose_bytes(s[0].keep, s[1].keep, s[2].keep, s[3].keep);
+  transpose_bytes(s[0].set, s[1].set, s[2].set, s[3].set);
+  transpose_bytes(s[0].zero, s[1].zero, s[2].zero, s[3].zero);
+  r[0] = resolve_octets(a[0], s[0]);
+  acc_add1(a[1], r[0].p0, r[0].p1, r[0].c);
+  r[1] = resolve_octets(a[1], s[1]);
+  acc_add1(a[2], r[0].p0, r[0].p1, r[0].c);
+  r[2] = resolve_octets(a[2], s[2]);
+  acc_add2(a[3], r[1].p0, r[1].p1, r[1].c, r[2].p0, r[2].p1, r[2].c);
+  r[3] = resolve_octets(a[3], s[3]);
+  transpose_bytes(r[0].p0, r[1].p0, r[2].p0, r[3].p0);
+  transpose_bytes(r[0].p1, r[1].p1, r[2].p1, r[3].p1);
+  transpose_bytes(r[0].c, r[1].c, r[2].c, r[3].c);
+}
+
+// Bits 0..4 to the positions of the singles.
+__device__ __forceinline__ uint32_t spread5(uint32_t a) {
+  return (a & 1u) << 1 | (a & 2u) << 1 | (a & 4u) << 2 | (a & 8u) << 5 | (a & 16u) << 12;
+}
+
+// SmallSets of the word whose position 0 is the set S0 of k <= 2 vertices
+// >= 5 (vertices >= n are padding, isolated).
+__device__ __noinline__ SmallSets small_sets(uint64_t S0, int k, const uint64_t* adj, int n) {
+  auto at = [&](int v) -> uint64_t { return v < n ? __ldg(adj + v) : 0ull; };
+  constexpr uint32_t kSingles = 0x00010116u, kPairs = 0x01161668u;  // |x| = 1, 2
+  SmallSets s;
+  if (k == 2) {
+    const int u = __ffsll(static_cast<long long>(S0)) - 1, v = 63 - __clzll(static_cast<long long>(S0));
+    s.keep = ~1u;
+    s.set = static_cast<uint32_t>(at(u) >> v) & 1u;
+  } else if (k == 1) {
+    s.keep = ~(1u | kSingles);
+    s.set = 1u | spread5(static_cast<uint32_t>(at(__ffsll(static_cast<long long>(S0)) - 1)));
+  } else {
+    s.keep = ~(1u | kSingles | kPairs);
+    s.set = kSingles;
+    for (int i = 1; i < 5; ++i)
+      s.set |= spread5(static_cast<uint32_t>(at(i)) & ((1u << i) - 1u)) << (1u << i);
+    s.zero = 1u;
   }
-  j = __popc(__ballot_sync(0xffffffffu, lane <= nh && cum <= t));
-  const uint32_t off = __shfl_sync(0xffffffffu, cum, (j + 31) & 31);       // lane j - 1
-  const uint32_t prev = __shfl_sync(0xffffffffu, cum, (j + 30) & 31);      // lane j - 2
-  off_prev = j >= 2 ? prev : 0u;
-  uint32_t r = t - (j >= 1 ? off : 0u);
-  H = 0;
-  for (int k = j; k > 0; --k) {
-    const uint32_t c = lane < nh ? binom[lane][k] : 0xFFFFFFFFu;
-    const int a = 31 - __clz(__ballot_sync(0xffffffffu, c <= r));
-    H |= 1u << a;
-    r -= binom[a][k];
-  }
+  return s;
 }
 
 __device__ __forceinline__ uint32_t rank_colex(const Binom& binom, uint32_t H) {
@@ -260,14 +274,15 @@ __global__ void dp_validate_kernel(const __grid_constant__ DpBatchParams p) {
 }
 
 // Batches issue tickets level-major across graphs (every graph's level-0
-// tiles, then every level-1 tile, ...), so that a tile's children lie far
+// groups, then every level-1 group, ...), so that a tile's children lie far
 // back in the ticket stream; tables and flags stay graph-major.
 __global__ void dp_fill_tile_map_kernel(const __grid_constant__ DpBatchParams p) {
   for (int g = blockIdx.x; g < p.num_graphs; g += gridDim.x) {
     const DpGraph G = p.graphs[g];
+    const uint32_t per = dp_group_tiles(G.lb);
     uint32_t local = 0;
     for (int j = 0; j <= G.nh; ++j) {
-      const uint32_t count = p.binom[G.nh][j];
+      const uint32_t count = (p.binom[G.nh][j] + per - 1u) / per;
       const uint32_t base = p.level_base[size_t(g) * (kDpMaxHigh + 2) + j];
       for (uint32_t i = threadIdx.x; i < count; i += blockDim.x)
         p.tile_map[base + i] = make_uint2(static_cast<uint32_t>(g), local + i);
@@ -280,367 +295,341 @@ __global__ void dp_fill_tile_map_kernel(const __grid_constant__ DpBatchParams p)
 // popcount class. For a tile of fewer word bits the words of class s are the
 // first C(wb, s) entries of the class (colex order lists the subsets of the
 // lower positions first), so one table serves every smaller tile size.
-__device__ void build_word_order(uint16_t* sOrder, const Binom& binom, int bits) {
+__device__ void build_word_order(uint8_t* sOrder, const Binom& binom, int bits) {
   for (int w = threadIdx.x; w < (1 << bits); w += blockDim.x) {
     const int i = __popc(w);
     uint32_t pos = 0;
     for (int q = 0; q < i; ++q)
       pos += binom[bits][q];
     pos += rank_colex(binom, static_cast<uint32_t>(w));
-    sOrder[pos] = static_cast<uint16_t>(w);
+    sOrder[pos] = static_cast<uint8_t>(w);
   }
 }
 
-__device__ __forceinline__ uint32_t smem_u32(const void* ptr) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(ptr));
+__device__ __forceinline__ uint4 ldcg128(const uint8_t* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
+
+// Dynamic shared memory of a launch: the planes of a group, the child lists
+// (kid_rows children of every tile of a group, the launch's largest number of
+// high vertices), the tiles' high parts, the binomial table, the word order.
+struct SmemLayout {
+  uint32_t kids_off, high_off, binom_off, order_off, bytes;
+};
+
+__host__ __device__ constexpr SmemLayout smem_layout(uint32_t plane_words, uint32_t tiles, int kid_rows,
+                                                     int order_bits) {
+  SmemLayout s{};
+  s.kids_off = 5u * 4u * plane_words;
+  s.high_off = s.kids_off + 4u * tiles * static_cast<uint32_t>(kid_rows);
+  s.binom_off = s.high_off + 4u * tiles;
+  s.order_off = s.binom_off + static_cast<uint32_t>(sizeof(Binom));
+  s.bytes = s.order_off + (1u << order_bits);
+  return s;
 }
 
-__device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-  return v;
-}
-
-__device__ __forceinline__ void sts_u32(uint32_t addr, uint32_t v) {
-  asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
-
-__host__ __device__ constexpr uint32_t cbinom(int n, int k) {
-  if (k < 0 || k > n)
-    return 0u;
-  uint64_t r = 1;
-  for (int i = 1; i <= k; ++i)
-    r = r * static_cast<uint64_t>(n - k + i) / static_cast<uint64_t>(i);
-  return static_cast<uint32_t>(r);
-}
-
-// In-tile phase, popcount class S of the word index and every class above
-// it: each lane resolves whole words of the class (listed in sOrder), whose
-// in-tile children are the S words w - b (b a bit of w) of class S - 1,
-// already final in T (shared address tbase); T and U (u_off bytes further)
-// at w hold the cross-tile children's summary as two virtual children. The
-// class size and the number of children are compile-time, so the child loop
-// is unrolled and child w - b is read at A - 4b, A = tbase + 4w, the bits
-// taken lowest first (r4 & (r4 - 4) drops the lowest).
-template <int LB, int S>
-__device__ __forceinline__ void intile_class(const DpBatchParams& p, const DpGraph& G, uint64_t Hfull, int j,
-                                             uint32_t tbase, uint32_t u_off, const uint16_t* sOrder,
-                                             int order_bits) {
-  constexpr int kWordBits = LB - 2;
-  constexpr uint32_t kCount = cbinom(kWordBits, S);
-  const int lane = threadIdx.x & 31;
-#pragma unroll 1
-  for (uint32_t e = lane; e < kCount; e += 32) {
-    const uint32_t w = sOrder[e];
-    const uint32_t A = tbase + (w << 2);
-    uint32_t o = 0u, a = 0xFFFFFFFFu, d = 0u;
-    if (j > 0) {  // the level-0 tile has no cross-tile children
-      const uint32_t x = lds_u32(A), y = lds_u32(A + u_off);
-      o = x | y;
-      a = x & y;
-      d = a;
-    }
-    uint32_t r4 = w << 2;
-#pragma unroll
-    for (int i = 0; i + 2 <= S; i += 2) {
-      const uint32_t n1 = r4 & (r4 - 4u), n2 = n1 & (n1 - 4u);
-      fold2(o, a, d, lds_u32(A + n1 - r4), lds_u32(A + n2 - n1));
-      r4 = n2;
-    }
-    if constexpr ((S & 1) != 0)
-      fold1(o, a, d, lds_u32(A - r4));
-    uint32_t out;
-    if constexpr (S >= 3) {
-      out = resolve_word(o, a, d);
-    } else {
-      if (j + S >= 3)
-        out = resolve_word(o, a, d);
-      else
-        out = resolve_word_small(o, a, d, j + S, p.adj + G.adj_off, G.n, Hfull | (uint64_t(w) << 2));
-    }
-    sts_u32(A, out);
+// Tiles of up to lb bits (min_lb = lb: the launch's only size).
+__host__ __device__ constexpr SmemLayout smem_layout_for(int min_lb, int lb, int kid_rows) {
+  uint32_t planes = 0, tiles = 0;
+  for (int b = min_lb; b <= lb; ++b) {
+    const uint32_t t = dp_group_tiles(b);
+    tiles = t > tiles ? t : tiles;
+    planes = (t << (b - 5)) > planes ? (t << (b - 5)) : planes;
   }
-  __syncwarp();
-  if constexpr (S < kWordBits)  // the order table's class sizes (order_bits >= kWordBits)
-    intile_class<LB, S + 1>(p, G, Hfull, j, tbase, u_off, sOrder + p.binom[order_bits][S], order_bits);
+  return smem_layout(planes, tiles, kid_rows, lb - 5);
 }
 
-constexpr uint32_t kNoPending = 0xFFFFFFFFu;
+struct Workspace {
+  uint32_t* planes;
+  uint32_t* kids;
+  uint32_t* high;
+  const Binom& binom;
+  const uint8_t* order;  // word order table of order_bits bits
+  int order_bits;
+};
 
-// Publishes the ready flag p.flags[pending] of the tile this warp stored
-// last. The tile's stores are warp-wide instructions of every lane; the
-// warp barrier orders them before lane 0's store, and that store is a
-// gpu-scope release, which is cumulative: a reader that acquires the flag
-// sees every byte of the tile. (No separate fence: the release is the
-// fence.) The tile loops call this right after tile_work returns, before
-// the next ticket, so the flag is not delayed; keeping the release out of
-// tile_work's body lets the one-size kernel fit in 43 registers, 10 CTAs
-// per SM, against 55 with it inside.
-__device__ __forceinline__ void publish_pending(const DpBatchParams& p, uint32_t& pending) {
-  if (pending == kNoPending)
-    return;
-  __syncwarp();
-  if ((threadIdx.x & 31) == 0)
-    st_release_u32(p.flags + pending, p.epoch);
-  pending = kNoPending;
+__device__ __forceinline__ Workspace make_workspace(const DpBatchParams& p, const SmemLayout& L, int order_bits) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  Binom& sBinom = *reinterpret_cast<Binom*>(smem + L.binom_off);
+  for (int i = threadIdx.x; i < (kDpMaxHigh + 1) * (kDpMaxHigh + 1); i += blockDim.x)
+    (&sBinom[0][0])[i] = (&p.binom[0][0])[i];
+  build_word_order(smem + L.order_off, p.binom, order_bits);
+  return Workspace{reinterpret_cast<uint32_t*>(smem), reinterpret_cast<uint32_t*>(smem + L.kids_off),
+                   reinterpret_cast<uint32_t*>(smem + L.high_off), sBinom, smem + L.order_off, order_bits};
 }
 
-// One warp resolves local tile tl of graph G (tiles of LB bits): waits for
-// its child tiles, reduces them, resolves the tile in T / U (shared memory,
-// 2^LB / 4 words each) and stores it; `pending` then names its flag for
-// publish_pending. sOrder is a word order table of order_bits >= LB - 2
-// bits. False if a wait gave up.
+// The CTA resolves group `group` of graph G (tiles of LB bits, level-major
+// group numbers): waits for its child tiles' groups, reduces them, resolves
+// the tiles in shared memory and stores them; the caller publishes the group
+// after a CTA barrier. False (for every thread) if a wait gave up.
+//
+// Bound by latency: 34 % of issue slots at n = 30 (16 warps per SM, as many as
+// shared memory and registers take), a group's time going to unranking and
+// flags (15 %), the gathers (27 %), the classes of the in-tile phase (33 %)
+// and waits at the narrow levels (16 %). 8.5 warp instructions per word of 32
+// subsets; n = 30 takes 0.69 ms, n = 33 4.7 ms (at one byte per subset and one
+// warp per tile, 1.52 warp instructions per subset: 1.92 and 14.9 ms). Tried
+// and not kept: a warp per group (0.91 ms), 64 threads per CTA (0.79), the next
+// group unranked by an idle warp beside the in-tile phase (0.72 and 5.2).
 template <int LB>
-__device__ __forceinline__ bool tile_work(const DpBatchParams& p, const DpGraph& G, uint32_t tl, uint32_t* T,
-                                          uint32_t* U, const uint16_t* sOrder, int order_bits, const Binom& sBinom,
-                                          uint32_t* kids, uint32_t& pending) {
-  constexpr int kWords = TileShape<LB>::kWords;
-  const int lane = threadIdx.x & 31;
+__device__ __forceinline__ bool group_work(const DpBatchParams& p, const DpGraph& G, uint32_t group,
+                                           const Workspace& ws) {
+  using Shape = TileShape<LB>;
+  constexpr uint32_t kQ = Shape::kGroup, kW = Shape::kWords, kPlane = Shape::kPlane, kChunks = Shape::kChunks;
+  constexpr int kWordBits = LB - 5;
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
   uint8_t* const table = p.table + G.table_off;
-  uint32_t* const flags = p.flags + G.tile_base;
+  const uint32_t* const flags = p.flags + G.flag_base;
+  const Binom& binom = ws.binom;
+  const int nh = G.nh;
 
-  int j;
-  uint32_t H, off_prev;
-  decode_tile(sBinom, G.nh, tl, j, H, off_prev);
-
-  // Lane v (a high vertex, v < nh <= 26) with v in H owns child tile
-  // H - v. Its colex rank keeps the terms C(u, i + 1) of the bits u < v and
-  // shifts the bits u > v down one place, C(u, i): a prefix sum and a
-  // suffix sum over the lanes. The child goes to kids[index of v in H].
-  const bool inH = (H >> lane) & 1u;
-  const uint32_t q = __popc(H & ((1u << lane) - 1u));
-  const uint32_t t1 = inH ? sBinom[lane][q + 1] : 0u, t0 = inH ? sBinom[lane][q] : 0u;
-  uint32_t pre = t1, suf = t0;
+  // Level j of the group: running totals over the levels, lane i holding the
+  // tiles (cumT) and groups (cumG) of levels 0..i (every warp alike).
+  const uint32_t level_tiles = static_cast<int>(lane) <= nh ? binom[nh][lane] : 0u;
+  uint32_t cumT = level_tiles, cumG = (level_tiles + kQ - 1u) / kQ;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t x = __shfl_up_sync(0xffffffffu, pre, d);
-    const uint32_t y = __shfl_down_sync(0xffffffffu, suf, d);
-    if (lane >= d)
-      pre += x;
-    if (lane + d < 32)
-      suf += y;
+    const uint32_t x = __shfl_up_sync(0xffffffffu, cumT, d);
+    const uint32_t y = __shfl_up_sync(0xffffffffu, cumG, d);
+    if (static_cast<int>(lane) >= d) {
+      cumT += x;
+      cumG += y;
+    }
   }
+  const int j = __popc(__ballot_sync(0xffffffffu, static_cast<int>(lane) <= nh && cumG <= group));
+  const uint32_t tiles_j = __shfl_sync(0xffffffffu, level_tiles, j);
+  uint32_t off_j = __shfl_sync(0xffffffffu, cumT, (j + 31) & 31);        // first tile of level j
+  uint32_t groups_j = __shfl_sync(0xffffffffu, cumG, (j + 31) & 31);     // first group of level j
+  uint32_t off_prev = __shfl_sync(0xffffffffu, cumT, (j + 30) & 31);     // ... of level j - 1
+  uint32_t groups_prev = __shfl_sync(0xffffffffu, cumG, (j + 30) & 31);
+  if (j < 1)
+    off_j = groups_j = 0u;
+  if (j < 2)
+    off_prev = groups_prev = 0u;
+  const uint32_t r0 = (group - groups_j) * kQ;          // rank of the first tile in its level
+  const uint32_t count = min(kQ, tiles_j - r0);
+
+  // Thread q unranks tile r0 + q (colex, descending) and ranks its children
+  // on the way: deleting element a keeps the terms below it (`rest`) and
+  // shifts those above down one place (`shifted`). Child i of tile q:
+  // kids[i * kQ + q].
+  if (tid < count) {
+    uint32_t rest = r0 + tid, kid = off_prev, at = tid, H = 0;  // kid: off_prev + `shifted`
+    int k = j;
+    for (int a = nh - 1; a >= 0; --a) {  // k = 0: C(a, 0) = 1 > rest = 0
+      const uint32_t c = binom[a][k], d = binom[a][max(k - 1, 0)];
+      if (rest >= c) {
+        rest -= c;
+        H |= 1u << a;
+        ws.kids[at] = kid + rest;
+        at += kQ;
+        kid += d;
+        --k;
+      }
+    }
+    ws.high[tid] = H;
+  }
+  __syncthreads();
+
+  // The children's groups: every thread looks at some (tile, child) pairs,
+  // four loads in flight. Relaxed flag loads followed by a gpu-scope fence
+  // acquire the groups whose flags they read; the barrier hands that to every
+  // thread.
+  const uint32_t pairs = static_cast<uint32_t>(j) * kQ;
+  auto flag_of = [&](uint32_t i) { return flags + groups_prev + (ws.kids[i] - off_prev) / kQ; };
   bool ok = true;
-  if (inH) {
-    const uint32_t child = off_prev + (pre - t1) + (suf - t0);
-    kids[q] = child;
-    ok = wait_flag(flags + child, p.epoch, p.timeout_ns, p.error);
-  }
-  if (__any_sync(0xffffffffu, !ok))
-    return false;
-  __syncwarp();  // kids[] written above, read by every lane below
-
-  // Cross-tile children: j whole tiles, 4 subsets per word, children three
-  // at a time from 10-bit tiles up (three 16-byte loads in flight per
-  // lane), else two at a time.
-  if constexpr (kWords >= 128) {
-#pragma unroll 1
-    for (int c0 = 0; c0 < kWords; c0 += 128) {
-      Acc g[4];
+  for (uint32_t i0 = tid; i0 < pairs; i0 += 4 * kDpThreads) {
+    uint32_t seen[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        acc_init(g[q]);
-      int m = 0;
-      for (; LB >= 10 && m + 3 <= j; m += 3) {  // three loads in flight
-        const uint4 a = __ldcg(reinterpret_cast<const uint4*>(table + (size_t(kids[m]) << LB)) + (c0 >> 2) + lane);
-        const uint4 b =
-            __ldcg(reinterpret_cast<const uint4*>(table + (size_t(kids[m + 1]) << LB)) + (c0 >> 2) + lane);
-        const uint4 c =
-            __ldcg(reinterpret_cast<const uint4*>(table + (size_t(kids[m + 2]) << LB)) + (c0 >> 2) + lane);
-        acc_add3(g[0], a.x, b.x, c.x);
-        acc_add3(g[1], a.y, b.y, c.y);
-        acc_add3(g[2], a.z, b.z, c.z);
-        acc_add3(g[3], a.w, b.w, c.w);
-      }
-      for (; m + 2 <= j; m += 2) {  // pairs: the remainder, or every child below 10 bits
-        const uint32_t c_a = kids[m];
-        const uint32_t c_b = kids[m + 1];
-        const uint4 a = __ldcg(reinterpret_cast<const uint4*>(table + (size_t(c_a) << LB)) + (c0 >> 2) + lane);
-        const uint4 b = __ldcg(reinterpret_cast<const uint4*>(table + (size_t(c_b) << LB)) + (c0 >> 2) + lane);
-        acc_add2(g[0], a.x, b.x);
-        acc_add2(g[1], a.y, b.y);
-        acc_add2(g[2], a.z, b.z);
-        acc_add2(g[3], a.w, b.w);
-      }
-      if (m < j) {
-        const uint32_t c_a = kids[m];
-        const uint4 a = __ldcg(reinterpret_cast<const uint4*>(table + (size_t(c_a) << LB)) + (c0 >> 2) + lane);
-        acc_add1(g[0], a.x);
-        acc_add1(g[1], a.y);
-        acc_add1(g[2], a.z);
-        acc_add1(g[3], a.w);
-      }
-      reinterpret_cast<uint4*>(T + c0)[lane] = make_uint4(g[0].o, g[1].o, g[2].o, g[3].o);
-      reinterpret_cast<uint4*>(U + c0)[lane] =
-          make_uint4(second_child(g[0]), second_child(g[1]), second_child(g[2]), second_child(g[3]));
+    for (uint32_t u = 0; u < 4; ++u) {
+      const uint32_t i = i0 + u * kDpThreads;
+      seen[u] = i < pairs && i % kQ < count ? ld_relaxed_u32(flag_of(i)) : p.epoch;
     }
-  } else {
-    for (int w = lane; w < kWords; w += 32) {
-      Acc g;
-      acc_init(g);
-      for (int m = 0; m < j; ++m) {
-        const uint32_t c_a = kids[m];
-        acc_add1(g, __ldcg(reinterpret_cast<const uint32_t*>(table + (size_t(c_a) << LB)) + w));
-      }
-      T[w] = g.o;
-      U[w] = second_child(g);
+#pragma unroll
+    for (uint32_t u = 0; u < 4; ++u)
+      ok &= seen[u] == p.epoch;
+  }
+  fence_acq_rel_gpu();
+  if (!__syncthreads_and(ok)) {  // some child is still being resolved
+    ok = true;
+    for (uint32_t i = tid; i < pairs && ok; i += kDpThreads)
+      if (i % kQ < count)
+        ok = wait_flag(flag_of(i), p.epoch, p.timeout_ns, p.error);
+    if (!__syncthreads_and(ok))
+      return false;
+  }
+
+  // Cross-tile children, 16 bytes (4 words) of a plane per thread and load.
+#pragma unroll 1
+  for (uint32_t ci = tid; ci < count * kChunks; ci += kDpThreads) {
+    const uint32_t q = ci / kChunks, k = ci % kChunks;
+    Acc a[4];
+    const uint8_t* const base = table + k * 16u;
+    const uint32_t* kid = ws.kids + q;
+    int m = 0;
+#pragma unroll 2
+    for (; m + 2 <= j; m += 2) {
+      const uint8_t* s = base + size_t(kid[0]) * Shape::kTileBytes;
+      const uint8_t* t = base + size_t(kid[kQ]) * Shape::kTileBytes;
+      kid += 2 * kQ;
+      const uint4 s0 = ldcg128(s), s1 = ldcg128(s + 4 * kW), sc = ldcg128(s + 8 * kW);
+      const uint4 t0 = ldcg128(t), t1 = ldcg128(t + 4 * kW), tc = ldcg128(t + 8 * kW);
+      acc_add2(a[0], s0.x, s1.x, sc.x, t0.x, t1.x, tc.x);
+      acc_add2(a[1], s0.y, s1.y, sc.y, t0.y, t1.y, tc.y);
+      acc_add2(a[2], s0.z, s1.z, sc.z, t0.z, t1.z, tc.z);
+      acc_add2(a[3], s0.w, s1.w, sc.w, t0.w, t1.w, tc.w);
+    }
+    if (m < j) {
+      const uint8_t* s = base + size_t(kid[0]) * Shape::kTileBytes;
+      const uint4 s0 = ldcg128(s), s1 = ldcg128(s + 4 * kW), sc = ldcg128(s + 8 * kW);
+      acc_add1(a[0], s0.x, s1.x, sc.x);
+      acc_add1(a[1], s0.y, s1.y, sc.y);
+      acc_add1(a[2], s0.z, s1.z, sc.z);
+      acc_add1(a[3], s0.w, s1.w, sc.w);
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i) {
+      uint32_t* const at = ws.planes + plane_at<LB>(q, 4 * k + i);
+      at[0] = a[i].o0;
+      at[kPlane] = a[i].o1;
+      at[2 * kPlane] = a[i].o2;
+      at[3 * kPlane] = a[i].c1;
+      at[4 * kPlane] = a[i].c2;
     }
   }
-  __syncwarp();
+  __syncthreads();
 
-  // In-tile children: words in popcount order of the word index, one
-  // unrolled pass per popcount class; inside a word the subsets with low
-  // bits 00, then 01 and 10, then 11.
-  // U lies u_off bytes after T: 2^LB in the one-size kernel, the largest
-  // tile's 2^lb in the mixed one.
-  const uint32_t u_off =
-      static_cast<uint32_t>(reinterpret_cast<const uint8_t*>(U) - reinterpret_cast<const uint8_t*>(T));
-  intile_class<LB, 0>(p, G, static_cast<uint64_t>(H) << LB, j, smem_u32(T), u_off, sOrder, order_bits);
-
-  // Store the tile; the caller publishes it (publish_pending).
-  uint32_t* dst = reinterpret_cast<uint32_t*>(table + (size_t(tl) << LB));
-  if constexpr (kWords >= 128) {
-    for (int w4 = lane; w4 < kWords / 4; w4 += 32)
-      reinterpret_cast<uint4*>(dst)[w4] = reinterpret_cast<const uint4*>(T)[w4];
-  } else {
-    for (int w = lane; w < kWords; w += 32)
-      dst[w] = T[w];
+  // In-tile children: words in popcount order of the word index, a thread per
+  // word and quad of tiles (from 32 quads on a warp is on one word). Tiles
+  // past `count` in the last quad come along and are not stored.
+  const uint32_t quads = (count + 3u) / 4u;
+  const uint8_t* order = ws.order;
+#pragma unroll 1
+  for (int s = 0; s <= kWordBits; ++s) {
+    const uint32_t items = binom[kWordBits][s] * Shape::kQuads;
+#pragma unroll 1
+    for (uint32_t e = tid; e < items; e += kDpThreads) {
+      const uint32_t q = (e % Shape::kQuads) * 4u, w = order[e / Shape::kQuads];
+      if (q >= quads * 4u)
+        continue;
+      uint32_t* const at = ws.planes + plane_at<LB>(q, w);
+      auto load = [](const uint32_t* from) { return *reinterpret_cast<const uint4*>(from); };
+      const uint4 o0 = load(at), o1 = load(at + kPlane), o2 = load(at + 2 * kPlane), c1 = load(at + 3 * kPlane),
+                  c2 = load(at + 4 * kPlane);
+      Acc a[4] = {{o0.x, o1.x, o2.x, c1.x, c2.x},
+                  {o0.y, o1.y, o2.y, c1.y, c2.y},
+                  {o0.z, o1.z, o2.z, c1.z, c2.z},
+                  {o0.w, o1.w, o2.w, c1.w, c2.w}};
+#pragma unroll 1
+      for (uint32_t bits = w; bits; bits &= bits - 1u) {
+        const uint32_t* const child = ws.planes + plane_at<LB>(q, w ^ (bits & (0u - bits)));
+        const uint4 p0 = load(child), p1 = load(child + kPlane), c = load(child + 2 * kPlane);
+        acc_add1(a[0], p0.x, p1.x, c.x);
+        acc_add1(a[1], p0.y, p1.y, c.y);
+        acc_add1(a[2], p0.z, p1.z, c.z);
+        acc_add1(a[3], p0.w, p1.w, c.w);
+      }
+      SmallSets small[4];
+      Planes r[4];
+      if (j + s > 2) {
+        resolve_quad(a, small, r);
+      } else {
+        for (uint32_t b = 0; b < 4; ++b)
+          if (q + b < count)
+            small[b] = small_sets((uint64_t(ws.high[q + b]) << LB) | (uint64_t(w) << 5), j + s, p.adj + G.adj_off, G.n);
+        resolve_quad(a, small, r);
+      }
+      *reinterpret_cast<uint4*>(at) = make_uint4(r[0].p0, r[1].p0, r[2].p0, r[3].p0);
+      *reinterpret_cast<uint4*>(at + kPlane) = make_uint4(r[0].p1, r[1].p1, r[2].p1, r[3].p1);
+      *reinterpret_cast<uint4*>(at + 2 * kPlane) = make_uint4(r[0].c, r[1].c, r[2].c, r[3].c);
+    }
+    order += binom[ws.order_bits][s];
+    __syncthreads();
   }
-  pending = G.tile_base + tl;
+
+  // Store the tiles.
+  uint8_t* const dst = table + size_t(off_j + r0) * Shape::kTileBytes;
+#pragma unroll 1
+  for (uint32_t ci = tid; ci < count * kChunks; ci += kDpThreads) {
+    const uint32_t q = ci / kChunks, k = ci % kChunks;
+    uint8_t* const out = dst + q * Shape::kTileBytes + k * 16u;
+#pragma unroll
+    for (uint32_t plane = 0; plane < 3; ++plane) {
+      const uint32_t* const from = ws.planes + plane * kPlane;
+      *reinterpret_cast<uint4*>(out + plane * 4 * kW) =
+          make_uint4(from[plane_at<LB>(q, 4 * k)], from[plane_at<LB>(q, 4 * k + 1)], from[plane_at<LB>(q, 4 * k + 2)],
+                     from[plane_at<LB>(q, 4 * k + 3)]);
+    }
+  }
   return true;
 }
 
-// Takes the next ticket (lane 0) and maps it to (graph, local tile);
-// false when the tickets are used up or an error was raised.
-__device__ __forceinline__ bool next_tile(const DpBatchParams& p, uint32_t& gi, uint32_t& tl) {
-  const int lane = threadIdx.x & 31;
-  uint32_t t = 0;
-  gi = 0;
-  tl = 0;
-  if (lane == 0) {
-    t = ld_relaxed_s32(p.error) != 0 ? 0xffffffffu : atomicAdd(p.ticket, 1u);
-    tl = t;
-    if (t < p.total_tiles && p.graphs) {
-      const uint2 m = __ldg(p.tile_map + t);
-      gi = m.x;
-      tl = m.y;
+constexpr uint32_t kNone = 0xFFFFFFFFu;
+
+// The launch's loop: the ticket of the next group (and the error word) is on
+// its way while `work` resolves a group; a CTA works its tickets in order, so
+// taking one early holds nothing up that the ticket before it does not.
+//
+// Publication: the group's stores are ordered before thread 0's flag store by
+// the CTA barrier, and that store is a gpu-scope release, which is cumulative:
+// a reader that acquires the flag sees every byte of the group's tiles.
+template <typename Work>
+__device__ __forceinline__ void group_loop(const DpBatchParams& p, Work work) {
+  __shared__ uint2 sNext;  // (graph, group); graph kNone: no more
+  uint32_t pending = kNone, ticket = 0;
+  int32_t error = 0;
+  if (threadIdx.x == 0) {
+    error = ld_relaxed_s32(p.error);
+    ticket = atomicAdd(p.ticket, 1u);
+  }
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0)
+      sNext = error != 0 || ticket >= p.total_groups ? make_uint2(kNone, 0u)
+              : p.graphs                             ? __ldg(p.tile_map + ticket)
+                                                     : make_uint2(0u, ticket);
+    if (threadIdx.x == 32 && pending != kNone)
+      st_release_u32(p.flags + pending, p.epoch);
+    __syncthreads();
+    const uint2 next = sNext;
+    if (next.x == kNone)
+      return;
+    if (threadIdx.x == 0) {
+      error = ld_relaxed_s32(p.error);
+      ticket = atomicAdd(p.ticket, 1u);
     }
+    const DpGraph G = p.graphs ? p.graphs[next.x] : p.single;
+    if (!work(G, next.x, next.y))
+      return;
+    pending = G.flag_base + next.y;
   }
-  t = __shfl_sync(0xffffffffu, t, 0);
-  gi = __shfl_sync(0xffffffffu, gi, 0);
-  tl = __shfl_sync(0xffffffffu, tl, 0);
-  return t < p.total_tiles;
 }
 
-// Every tile of the launch has LB bits (single-graph solves, and batches
-// that use one tile size).
+// Tiles of one size (single-graph solves, and batches that use one).
 template <int LB>
-__device__ __forceinline__ void dp_tile_body(const DpBatchParams& p) {
-  using Shape = TileShape<LB>;
-  extern __shared__ __align__(16) uint8_t smem[];
-  const int warp = threadIdx.x >> 5;
-  uint32_t* T = reinterpret_cast<uint32_t*>(smem + size_t(warp) * Shape::kPerWarp);
-  uint32_t* U = T + Shape::kWords;
-  uint16_t* sOrder = reinterpret_cast<uint16_t*>(smem + Shape::kOrderOff);
-  Binom& sBinom = *reinterpret_cast<Binom*>(smem + Shape::kBinomOff);
-  uint32_t* kids = reinterpret_cast<uint32_t*>(smem + Shape::kKidsOff) + warp * 32;
-
-  for (int i = threadIdx.x; i < (kDpMaxHigh + 1) * (kDpMaxHigh + 1); i += blockDim.x)
-    (&sBinom[0][0])[i] = (&p.binom[0][0])[i];
-  build_word_order(sOrder, p.binom, Shape::kWordBits);
-  __syncthreads();
-
-  uint32_t gi, tl, pending = kNoPending;
-  while (publish_pending(p, pending), next_tile(p, gi, tl)) {
-    const DpGraph G = p.graphs ? p.graphs[gi] : p.single;
-    if (!tile_work<LB>(p, G, tl, T, U, sOrder, Shape::kWordBits, sBinom, kids, pending))
-      break;
-  }
-  publish_pending(p, pending);
-}
-
-// Tiles of 10 to 12 bits (three cross-tile loads in flight): the launch
-// bound holds the registers to the CTAs per SM that shared memory allows, 10
-// at 10 and 11 bits, 6 at 12.
-template <int LB>
-constexpr int kDpMinCtas = LB >= 12 ? 6 : 10;
-
-template <int LB>
-__global__ void __launch_bounds__(32 * kDpWarps, kDpMinCtas<LB>)
-    dp_tile_kernel(const __grid_constant__ DpBatchParams p) {
-  dp_tile_body<LB>(p);
-}
-
-// Smaller tiles (pairs of cross-tile loads): registers left to the compiler.
-template <int LB>
-__global__ void __launch_bounds__(32 * kDpWarps) dp_tile_kernel_small(const __grid_constant__ DpBatchParams p) {
-  dp_tile_body<LB>(p);
-}
-
-template <int LB>
-constexpr auto tile_kernel_for() {
-  if constexpr (LB >= 10)
-    return &dp_tile_kernel<LB>;
-  else
-    return &dp_tile_kernel_small<LB>;
+__global__ void __launch_bounds__(kDpThreads, 4) dp_tile_kernel(const __grid_constant__ DpBatchParams p) {
+  const Workspace ws = make_workspace(p, smem_layout_for(LB, LB, p.kid_rows), LB - 5);
+  group_loop(p, [&](const DpGraph& G, uint32_t, uint32_t group) { return group_work<LB>(p, G, group, ws); });
 }
 
 // Batches whose graphs use different tile sizes (DpGraph::lb, 8 .. p.lb):
-// shared memory is laid out for the largest (p.lb, a runtime value, so the
-// launch's occupancy follows it) and each tile dispatches on its graph's lb.
-// The five inlined tile sizes raise the register count (64 against 47 for
-// one size), so this kernel holds fewer CTAs than the one-size kernel; the
-// autotuner measures that cost and the planner only mixes sizes when the
+// shared memory is laid out for the largest (p.lb, a runtime value) and each
+// group dispatches on its graph's lb. The autotuner measures what the
+// dispatch costs against one size and the planner only mixes sizes when the
 // per-size gains outweigh it.
-__global__ void __launch_bounds__(32 * kDpWarps)
-    dp_tile_kernel_mixed(const __grid_constant__ DpBatchParams p) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  const int warp = threadIdx.x >> 5;
-  const int words = (1 << p.lb) / 4, bits = p.lb - 2;
-  const size_t per_warp = size_t(2) * words * 4;
-  const size_t order_off = kDpWarps * per_warp;
-  const size_t binom_off = (order_off + size_t(words) * 2 + 15) & ~size_t(15);
-  const size_t kids_off = (binom_off + sizeof(Binom) + 15) & ~size_t(15);
-  uint32_t* T = reinterpret_cast<uint32_t*>(smem + size_t(warp) * per_warp);
-  uint32_t* U = T + words;
-  uint16_t* sOrder = reinterpret_cast<uint16_t*>(smem + order_off);
-  Binom& sBinom = *reinterpret_cast<Binom*>(smem + binom_off);
-  uint32_t* kids = reinterpret_cast<uint32_t*>(smem + kids_off) + warp * 32;
-
-  for (int i = threadIdx.x; i < (kDpMaxHigh + 1) * (kDpMaxHigh + 1); i += blockDim.x)
-    (&sBinom[0][0])[i] = (&p.binom[0][0])[i];
-  build_word_order(sOrder, p.binom, bits);
-  __syncthreads();
-
-  uint32_t gi, tl, pending = kNoPending;
-  while (publish_pending(p, pending), next_tile(p, gi, tl)) {
-    const DpGraph G = p.graphs[gi];
-    bool ok = false;
-    if (G.lb > p.lb) {  // the planner never does this: the tile would not fit
-      raise_error(p.error, kDevInvalidInput, static_cast<int32_t>(gi));
-      break;
+__global__ void __launch_bounds__(kDpThreads, 4) dp_tile_kernel_mixed(const __grid_constant__ DpBatchParams p) {
+  const Workspace ws = make_workspace(p, smem_layout_for(kDpMinTileBits, p.lb, p.kid_rows), p.lb - 5);
+  group_loop(p, [&](const DpGraph& G, uint32_t graph, uint32_t group) {
+    switch (G.lb <= p.lb ? G.lb : 0) {
+      case 8: return group_work<8>(p, G, group, ws);
+      case 9: return group_work<9>(p, G, group, ws);
+      case 10: return group_work<10>(p, G, group, ws);
+      case 11: return group_work<11>(p, G, group, ws);
+      case 12: return group_work<12>(p, G, group, ws);
+      default:  // the planner never does this: the tile would not fit
+        if (threadIdx.x == 0)
+          raise_error(p.error, kDevInvalidInput, static_cast<int32_t>(graph));
+        return false;
     }
-    switch (G.lb) {
-      case 8: ok = tile_work<8>(p, G, tl, T, U, sOrder, bits, sBinom, kids, pending); break;
-      case 9: ok = tile_work<9>(p, G, tl, T, U, sOrder, bits, sBinom, kids, pending); break;
-      case 10: ok = tile_work<10>(p, G, tl, T, U, sOrder, bits, sBinom, kids, pending); break;
-      case 11: ok = tile_work<11>(p, G, tl, T, U, sOrder, bits, sBinom, kids, pending); break;
-      case 12: ok = tile_work<12>(p, G, tl, T, U, sOrder, bits, sBinom, kids, pending); break;
-      default: raise_error(p.error, kDevInvalidInput, static_cast<int32_t>(gi)); break;
-    }
-    if (!ok)
-      break;
-  }
-  publish_pending(p, pending);
-}
-
-// Dynamic shared memory of the mixed kernel for tiles of up to lb bits.
-size_t dp_mixed_smem(int lb) {
-  const size_t words = (size_t(1) << lb) / 4;
-  const size_t order_off = kDpWarps * 2 * words * 4;
-  const size_t binom_off = (order_off + words * 2 + 15) & ~size_t(15);
-  const size_t kids_off = (binom_off + sizeof(Binom) + 15) & ~size_t(15);
-  return kids_off + size_t(kDpWarps) * 32 * 4;
+  });
 }
 
 // ---------------------------------------------------------------------------
@@ -680,29 +669,55 @@ struct TreeCtx {
   const Binom& binom;
   const uint8_t* table;
   int lb, nh, n;
-  __device__ uint32_t td_of(uint64_t S) const {
+  // td(S) mod 3 (one lane).
+  __device__ uint32_t residue(uint64_t S) const {
     const uint32_t H = static_cast<uint32_t>(S >> lb);
     const int j = __popc(H);
     uint32_t off = 0;
     for (int i = 0; i < j; ++i)
       off += binom[nh][i];
-    const uint64_t tile = off + rank_colex(binom, H);
-    return table[(tile << lb) | (S & ((1ull << lb) - 1))] >> 1;
+    const uint32_t words = 1u << (lb - 5);
+    const uint32_t* t = reinterpret_cast<const uint32_t*>(table + size_t(off + rank_colex(binom, H)) * (12u * words)) +
+                        ((static_cast<uint32_t>(S) >> 5) & (words - 1u));
+    const uint32_t bit = static_cast<uint32_t>(S) & 31u;
+    const uint32_t p0 = (t[0] >> bit) & 1u, p1 = (t[words] >> bit) & 1u;
+    return p0 ? 0u : 2u - p1;
+  }
+  // td(S) (whole warp): along the chain S & {v, v + 1, ...}, v = 0 .. n, each
+  // deletion lowers the treedepth by 0 or 1, which the residues tell.
+  __device__ uint32_t td_of(uint64_t S) const {
+    const int lane = threadIdx.x & 31;
+    const uint64_t above_lo = S & (~0ull << lane), above_hi = S & (~0ull << (lane + 32));
+    const uint32_t lo = lane <= n ? residue(above_lo) : 0u;
+    const uint32_t hi = lane + 32 <= n ? residue(above_hi) : 0u;
+    uint32_t next_lo = __shfl_down_sync(0xffffffffu, lo, 1);
+    const uint32_t first_hi = __shfl_sync(0xffffffffu, hi, 0), next_hi = __shfl_down_sync(0xffffffffu, hi, 1);
+    if (lane == 31)
+      next_lo = first_hi;
+    uint32_t drop = 0;
+    if (lane < n)
+      drop += lo == (next_lo == 2u ? 0u : next_lo + 1u) ? 1u : 0u;
+    if (lane + 32 < n)
+      drop += hi == (next_hi == 2u ? 0u : next_hi + 1u) ? 1u : 0u;
+    return __reduce_add_sync(0xffffffffu, drop);
   }
   // First vertex v of the connected set C with td(C - v) = td(C) - 1, i.e.
   // the first argmin of td(C - v) (td(C) = 1 + min_v td(C - v) for a
-  // connected C): one round of table reads, no read of td(C) itself.
+  // connected C): one round of table reads, no read of td(C) itself. The
+  // values are a and possibly a + 1, so residue a is the one present whose
+  // predecessor is absent. -1 on three residues (a corrupt table).
   __device__ int root(uint64_t C) const {
     if (__popcll(C) == 1)
       return __ffsll(static_cast<long long>(C)) - 1;
     const int lane = threadIdx.x & 31;
     const bool in_lo = (C >> lane) & 1ull;
     const bool in_hi = lane + 32 < n && ((C >> (lane + 32)) & 1ull);
-    const uint32_t t_lo = in_lo ? td_of(C & ~(1ull << lane)) : 0xFFFFFFFFu;
-    const uint32_t t_hi = in_hi ? td_of(C & ~(1ull << (lane + 32))) : 0xFFFFFFFFu;
-    const uint32_t m = __reduce_min_sync(0xffffffffu, min(t_lo, t_hi));
+    const uint32_t t_lo = in_lo ? residue(C & ~(1ull << lane)) : 3u;
+    const uint32_t t_hi = in_hi ? residue(C & ~(1ull << (lane + 32))) : 3u;
+    const uint32_t have = __reduce_or_sync(0xffffffffu, (1u << t_lo) | (1u << t_hi)) & 7u;
+    const uint32_t m = (have & 5u) == 5u ? 2u : (have & 1u) ? 0u : (have & 2u) ? 1u : 2u;
     const uint64_t hits = ballot64(in_lo && t_lo == m, in_hi && t_hi == m);
-    return hits ? __ffsll(static_cast<long long>(hits)) - 1 : -1;
+    return have != 7u && hits ? __ffsll(static_cast<long long>(hits)) - 1 : -1;
   }
 };
 
@@ -872,28 +887,26 @@ void dp_fill_binom(DpBatchParams& p) {
 
 template <int LB>
 static cudaError_t launch_tiles(const DpBatchParams& p, int ctas, cudaStream_t s) {
-  tile_kernel_for<LB>()<<<ctas, 32 * kDpWarps, TileShape<LB>::kSmem, s>>>(p);
+  dp_tile_kernel<LB><<<ctas, kDpThreads, smem_layout_for(LB, LB, p.kid_rows).bytes, s>>>(p);
   return cudaGetLastError();
 }
 
-template <int LB>
-static int occupancy_tiles() {
-  if (cudaFuncSetAttribute(tile_kernel_for<LB>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(TileShape<LB>::kSmem)) != cudaSuccess)
+template <typename Kernel>
+static int occupancy_of(Kernel kernel, const SmemLayout& at, const SmemLayout& most) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most.bytes)) !=
+      cudaSuccess)
     return 0;
   int blocks = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, tile_kernel_for<LB>(), 32 * kDpWarps,
-                                                TileShape<LB>::kSmem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, kDpThreads, at.bytes);
   return blocks;
 }
 
-int dp_tile_occupancy(int lb) {
+int dp_tile_occupancy(int lb, int kid_rows) {
   switch (lb) {
 #define GTD_CASE(X) \
   case X:           \
-    return occupancy_tiles<X>();
-    GTD_CASE(2) GTD_CASE(3) GTD_CASE(4) GTD_CASE(5) GTD_CASE(6)
-    GTD_CASE(7) GTD_CASE(8) GTD_CASE(9) GTD_CASE(10) GTD_CASE(11) GTD_CASE(12)
+    return occupancy_of(dp_tile_kernel<X>, smem_layout_for(X, X, kid_rows), smem_layout_for(X, X, kDpMaxHigh));
+    GTD_CASE(8) GTD_CASE(9) GTD_CASE(10) GTD_CASE(11) GTD_CASE(12)
 #undef GTD_CASE
     default:
       return 0;
@@ -911,29 +924,23 @@ cudaError_t dp_launch_fill_tile_map(const DpBatchParams& p, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-int dp_mixed_occupancy(int lb) {
-  const size_t smem = dp_mixed_smem(lb);
-  if (cudaFuncSetAttribute(dp_tile_kernel_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(dp_mixed_smem(kDpMaxTileBits))) != cudaSuccess)
-    return 0;
-  int blocks = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, dp_tile_kernel_mixed, 32 * kDpWarps, smem);
-  return blocks;
+int dp_mixed_occupancy(int lb, int kid_rows) {
+  return occupancy_of(dp_tile_kernel_mixed, smem_layout_for(kDpMinTileBits, lb, kid_rows),
+                      smem_layout_for(kDpMinTileBits, kDpMaxTileBits, kDpMaxHigh));
 }
 
 cudaError_t dp_launch_tiles(const DpBatchParams& p, int ctas, cudaStream_t s) {
   if (p.mixed) {
     if (p.lb < kDpMinTileBits || p.lb > kDpMaxTileBits)
       return cudaErrorInvalidValue;
-    dp_tile_kernel_mixed<<<ctas, 32 * kDpWarps, dp_mixed_smem(p.lb), s>>>(p);
+    dp_tile_kernel_mixed<<<ctas, kDpThreads, smem_layout_for(kDpMinTileBits, p.lb, p.kid_rows).bytes, s>>>(p);
     return cudaGetLastError();
   }
   switch (p.lb) {
 #define GTD_CASE(X) \
   case X:           \
     return launch_tiles<X>(p, ctas, s);
-    GTD_CASE(2) GTD_CASE(3) GTD_CASE(4) GTD_CASE(5) GTD_CASE(6)
-    GTD_CASE(7) GTD_CASE(8) GTD_CASE(9) GTD_CASE(10) GTD_CASE(11) GTD_CASE(12)
+    GTD_CASE(8) GTD_CASE(9) GTD_CASE(10) GTD_CASE(11) GTD_CASE(12)
 #undef GTD_CASE
     default:
       return cudaErrorInvalidValue;
@@ -970,12 +977,12 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
       }
       continue;
     }
-    const uint32_t td = ctx.td_of(S);
+    const uint32_t td = ctx.td_of(S), below = (td + 2u) % 3u;  // residue of td - 1
     bool lo = false, hi = false;
     if ((S >> lane) & 1ull)
-      lo = ctx.td_of(S & ~(1ull << lane)) + 1u == td;
+      lo = ctx.residue(S & ~(1ull << lane)) == below;
     if (lane + 32 < G.n && ((S >> (lane + 32)) & 1ull))
-      hi = ctx.td_of(S & ~(1ull << (lane + 32))) + 1u == td;
+      hi = ctx.residue(S & ~(1ull << (lane + 32))) == below;
     const uint64_t roots = ballot64(lo, hi);
     if (lane == 0) {
       td_out[i] = static_cast<int32_t>(td);
@@ -992,6 +999,69 @@ cudaError_t dp_launch_labels(const DpBatchParams& p, const uint64_t* subsets, in
   if (blocks < 1)
     blocks = 1;
   dp_labels_kernel<<<blocks, 32 * kTreeWarps, 0, s>>>(p, subsets, count, td_out, roots_out);
+  return cudaGetLastError();
+}
+
+// The byte table of gtd_dp_table (td << 1 | connected per subset, tiles of
+// 2^lb bytes in tile order) from the planes, one warp per tile: td(H) from
+// the warp's chain, each word's first subset along the chain of its bits, the
+// word's subsets from one another.
+__global__ void __launch_bounds__(32 * kTreeWarps)
+    dp_expand_kernel(const __grid_constant__ DpBatchParams p, uint8_t* out, uint64_t bytes) {
+  __shared__ Binom sBinom;
+  for (int i = threadIdx.x; i < (kDpMaxHigh + 1) * (kDpMaxHigh + 1); i += blockDim.x)
+    (&sBinom[0][0])[i] = (&p.binom[0][0])[i];
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const DpGraph G = p.single;
+  const TreeCtx ctx{sBinom, p.table + G.table_off, G.lb, G.nh, G.n};
+  const uint32_t words = 1u << (G.lb - 5);
+  for (uint32_t t = blockIdx.x * kTreeWarps + warp; t < G.ntiles; t += gridDim.x * kTreeWarps) {
+    uint32_t r = t, H = 0;
+    int j = 0;
+    while (r >= sBinom[G.nh][j])
+      r -= sBinom[G.nh][j++];
+    for (int a = G.nh - 1, k = j; k > 0; --a)
+      if (r >= sBinom[a][k]) {
+        r -= sBinom[a][k--];
+        H |= 1u << a;
+      }
+    const uint32_t base = ctx.td_of(static_cast<uint64_t>(H) << G.lb);
+    const uint32_t* tile = reinterpret_cast<const uint32_t*>(ctx.table + size_t(t) * (12u * words));
+    auto first = [&](uint32_t w) { return (tile[w] & 1u) ? 0u : 2u - (tile[words + w] & 1u); };
+    for (uint32_t w = lane; w < words; w += 32) {
+      uint32_t td[32];
+      td[0] = base;
+      uint32_t here = first(w);
+      for (uint32_t x = w; x; x &= x - 1) {
+        const uint32_t next = first(x & (x - 1));
+        td[0] += here != next;
+        here = next;
+      }
+      const uint32_t p0 = tile[w], p1 = tile[words + w], c = tile[2 * words + w];
+      // residue changes between x and x without its lowest bit: treedepth + 1
+#pragma unroll
+      for (int x = 1; x < 32; ++x) {
+        const int y = x & (x - 1);
+        td[x] = td[y] + ((((p0 >> x) ^ (p0 >> y)) | ((p1 >> x) ^ (p1 >> y))) & 1u);
+      }
+      const uint64_t at = (static_cast<uint64_t>(t) << G.lb) + w * 32u;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        uint32_t v = 0;
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+          v |= (td[4 * i + b] << 1 | ((c >> (4 * i + b)) & 1u)) << (8 * b);
+        if (at + 4 * i + 4 <= bytes)
+          *reinterpret_cast<uint32_t*>(out + at + 4 * i) = v;
+      }
+    }
+  }
+}
+
+cudaError_t dp_launch_expand(const DpBatchParams& p, uint8_t* out, uint64_t bytes, cudaStream_t s) {
+  const uint32_t ctas = (p.single.ntiles + kTreeWarps - 1) / kTreeWarps;
+  dp_expand_kernel<<<ctas < 16384u ? ctas : 16384u, 32 * kTreeWarps, 0, s>>>(p, out, bytes);
   return cudaGetLastError();
 }
 

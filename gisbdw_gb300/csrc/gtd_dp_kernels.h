@@ -9,12 +9,12 @@
 
 namespace gtd {
 
-// One graph of a DP launch (40 bytes). A graph with n < lb is padded with
+// One graph of a DP launch (48 bytes). A graph with n < lb is padded with
 // isolated vertices up to lb (one tile); padding changes no treedepth of a
 // real subset and the reconstruction never touches padded vertices.
 struct DpGraph {
   uint64_t table_off = 0;  // byte offset of the graph's table in the table pool
-  uint32_t tile_base = 0;  // first flag of the graph (graph-major tile count)
+  uint32_t flag_base = 0;  // first flag of the graph (graph-major count of tile groups)
   uint32_t ntiles = 0;     // 2^nh
   uint32_t adj_off = 0;    // first adjacency mask; also the first output slot
   int32_t n = 0;           // real vertices
@@ -29,14 +29,15 @@ struct DpBatchParams {
   uint32_t binom[kDpMaxHigh + 1][kDpMaxHigh + 1] = {};  // C(a, b)
   const DpGraph* graphs = nullptr;  // device descriptors; nullptr: only `single`
   DpGraph single;
-  uint2* tile_map = nullptr;        // ticket -> (graph, local tile) (batches)
+  uint2* tile_map = nullptr;        // ticket -> (graph, its tile group) (batches)
   const uint32_t* level_base = nullptr;  // [graph][level] first ticket (batches)
   int num_graphs = 1;
   int lb = 0;                       // tile bits of this launch (mixed batches: the largest)
+  int kid_rows = 0;                 // largest nh of the launch's graphs
   int mixed = 0;                    // 1: graphs carry their own tile bits (DpGraph::lb)
-  uint32_t total_tiles = 0;
-  uint8_t* table = nullptr;         // table pool
-  uint32_t* flags = nullptr;        // one ready stamp per global tile
+  uint32_t total_groups = 0;        // tickets: groups of tiles of one level
+  uint8_t* table = nullptr;         // table pool: tiles of three bit planes
+  uint32_t* flags = nullptr;        // one ready stamp per tile group
   uint32_t* ticket = nullptr;       // work counter, zeroed before each launch
   int32_t* error = nullptr;         // [0] code, [1] info
   const uint64_t* adj = nullptr;    // adjacency pool (device)
@@ -51,14 +52,18 @@ struct DpBatchParams {
 };
 
 void dp_fill_binom(DpBatchParams& p);
-int dp_tile_occupancy(int lb);
-// CTAs per SM of the mixed-tile-size kernel with tiles of up to lb bits.
-int dp_mixed_occupancy(int lb);
+// CTAs per SM with tiles of lb bits and up to kid_rows high vertices, and of
+// the mixed-tile-size kernel with tiles of up to lb bits.
+int dp_tile_occupancy(int lb, int kid_rows);
+int dp_mixed_occupancy(int lb, int kid_rows);
 cudaError_t dp_launch_validate(const DpBatchParams& p, cudaStream_t s);
 cudaError_t dp_launch_fill_tile_map(const DpBatchParams& p, cudaStream_t s);
 cudaError_t dp_launch_tiles(const DpBatchParams& p, int ctas, cudaStream_t s);
 cudaError_t dp_launch_tree(const DpBatchParams& p, cudaStream_t s);
 cudaError_t dp_launch_labels(const DpBatchParams& p, const uint64_t* subsets, int count, int32_t* td_out,
                              uint64_t* roots_out, cudaStream_t s);
+// The byte table (td << 1 | connected, 2^n bytes in tile order) of a solved
+// single graph.
+cudaError_t dp_launch_expand(const DpBatchParams& p, uint8_t* out, uint64_t bytes, cudaStream_t s);
 
 }  // namespace gtd

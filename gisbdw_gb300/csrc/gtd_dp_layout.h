@@ -1,16 +1,18 @@
 // Layout of the subset-DP table in device memory (host and device code).
 //
-// Every subset S of the n vertices owns one byte, td(G[S]) << 1 | c, where
-// c = 1 iff G[S] is connected. Vertices 0..lb-1 are the tile's "low"
-// vertices and vertices lb..n-1 its "high" ones (nh = n - lb of them). The
-// 2^lb subsets that share the same high part H form one tile of 2^lb
-// contiguous bytes, indexed inside the tile by the low part's bit mask.
-// Tiles are stored level by level in |H| order and, inside a level, in the
-// combinatorial-number-system rank of H (colex order, the ranking of
+// Vertices 0..lb-1 are the tile's "low" vertices and vertices lb..n-1 its
+// "high" ones (nh = n - lb of them). The 2^lb subsets that share the same
+// high part H form one tile, indexed inside the tile by the low part's bit
+// mask. Tiles are stored level by level in |H| order and, inside a level, in
+// the combinatorial-number-system rank of H (colex order, the ranking of
 // set_encoder.hpp:40-46 in the reference), so
 //   index(S) = (level_off[|H|] + rank(H)) * 2^lb + (S & (2^lb - 1)).
-// A tile's |H| children H \ h are whole tiles one level down: every
-// cross-tile gather of the DP reads 2^lb contiguous bytes.
+// The solve keeps three bits per subset: a tile is three planes of 2^(lb-5)
+// words (td mod 3 == 0, td mod 3 == 1, connected), bit S & 31 of word
+// (S >> 5) & (2^(lb-5) - 1). The byte table handed out on request has one
+// byte td(G[S]) << 1 | c per subset (c = 1 iff G[S] is connected) at
+// index(S). A tile's |H| children H \ h are whole tiles one level down:
+// every cross-tile gather of the DP reads contiguous words of them.
 #pragma once
 
 #include <cstdint>
@@ -27,6 +29,18 @@ constexpr int kDpMaxN = 36;          // 2^36 B = 64 GiB table
 constexpr int kDpMaxHigh = 26;       // nh <= 26: C(26, 13) < 2^32, 2^26 tiles
 constexpr int kDpMinTileBits = 8;
 constexpr int kDpMaxTileBits = 12;
+
+// Threads of a CTA of the tile kernel.
+constexpr int kDpThreads = 128;
+
+// Tiles per group (a power of two), the unit of work of one CTA: 16 words of a
+// plane per thread, at most one tile per thread.
+GTD_HD constexpr int dp_group_shift(int lb) { return lb <= 9 ? 7 : 16 - lb; }
+GTD_HD constexpr int dp_group_tiles(int lb) { return 1 << dp_group_shift(lb); }
+static_assert(dp_group_tiles(9) == kDpThreads && (dp_group_tiles(11) << (11 - 5)) == 16 * kDpThreads, "group size");
+
+// Bytes of a tile of the solve's table.
+GTD_HD constexpr uint32_t dp_tile_bytes(int lb) { return 12u << (lb - 5); }
 
 struct DpLayout {
   int n = 0;
@@ -72,6 +86,16 @@ struct DpLayout {
 #endif
   }
 };
+
+// Groups of tiles of a graph with nh high vertices and tiles of lb bits: no
+// group spans two levels.
+inline uint32_t dp_groups(const uint32_t (&binom)[kDpMaxHigh + 1][kDpMaxHigh + 1], int nh, int lb) {
+  const uint32_t per = dp_group_tiles(lb);
+  uint32_t groups = 0;
+  for (int j = 0; j <= nh; ++j)
+    groups += (binom[nh][j] + per - 1) / per;
+  return groups;
+}
 
 // Fills a layout for n vertices and the requested tile bits (clamped so
 // that lb <= n and nh <= kDpMaxHigh). Host only.

@@ -44,10 +44,13 @@ struct gtd_handle_s {
   std::string last_error;
 
   // Subset DP buffers (shared by single and batched solves).
-  uint8_t* d_table = nullptr;
+  uint8_t* d_table = nullptr;  // bit planes (gtd_dp_layout.h)
   size_t table_cap = 0;
+  uint8_t* d_bytes = nullptr;  // byte table of the last solve, made on request (gtd_dp_table)
+  size_t bytes_cap = 0;
+  bool bytes_valid = false;
   uint32_t* d_flags = nullptr;
-  size_t flags_cap = 0;  // number of tiles
+  size_t flags_cap = 0;  // number of tile groups
   uint32_t epoch = 0;
   int32_t* d_io = nullptr;   // control/IO block
   uint64_t* d_adj = nullptr; // kDpMaxN masks
@@ -80,9 +83,10 @@ struct gtd_handle_s {
   // Mixed-size kernel throughput over the one-size kernel's, per largest tile
   // size (0 = unmeasured), from the autotuner.
   float tune_mixed_eff[gtd::kTuneLbMax + 1] = {};
-  // CTAs per SM of the one-size DP kernel per tile size (0 = not asked yet):
+  // CTAs per SM of the one-size DP kernel per tile size and number of high
+  // vertices (0 = not asked yet):
   // a property of the kernel and the device, looked up once per handle.
-  int dp_occ[gtd::kDpMaxTileBits + 1] = {};
+  int dp_occ[gtd::kDpMaxTileBits + 1][gtd::kDpMaxHigh + 1] = {};
 
   gtd_bnb_state* bnb = nullptr;
   void* d_scratch = nullptr;  // general device scratch (labels, GNN batches)
@@ -93,6 +97,7 @@ struct gtd_handle_s {
   // Last DP solve (for gtd_dp_query / gtd_sync).
   bool have_table = false;
   bool pending_stats = false;
+  int last_tile_bits = 0;  // of the byte table's layout (n < 8: n, the planes pad to 8)
   gtd::DpBatchParams last_params;
   gtd_dp_stats last_stats = {};
 };
@@ -127,8 +132,10 @@ cudaError_t ensure_field(T** field, size_t* cap_elems, size_t count) {
 bool take_alloc_fault();
 bool take_stall_fault();
 bool take_poison_fault();
+// Frees the byte table (gtd_dp_table), if one was made.
+void release_byte_table(gtd_handle h);
 // Grows the flag array; fresh flags are zeroed and the epoch restarts.
-gtd_status ensure_flags(gtd_handle h, size_t tiles);
+gtd_status ensure_flags(gtd_handle h, size_t groups);
 // Next epoch for a direct (non-graph) launch.
 gtd_status next_epoch(gtd_handle h, uint32_t* epoch);
 

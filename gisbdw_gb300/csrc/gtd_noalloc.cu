@@ -42,7 +42,7 @@ namespace gtd {
 namespace {
 
 constexpr int kNoallocTileBits = 10;
-constexpr size_t kNoallocTableBytes = size_t(1) << GTD_DP_NOALLOC_MAX_N;
+constexpr size_t kNoallocTableBytes = size_t(1) << GTD_DP_NOALLOC_MAX_N;  // the planes take 3/8 of it
 // Tiles of the largest accepted graph: make_dp_layout(n, 10) keeps 10 tile
 // bits for 10 <= n <= 24 (2^(n - 10) tiles) and one tile below that.
 constexpr size_t kNoallocMaxTiles = size_t(1) << (GTD_DP_NOALLOC_MAX_N - kNoallocTileBits);
@@ -99,10 +99,10 @@ extern "C" gtd_status gtd_dp_solve_noalloc(const uint64_t* d_adj, int n, int32_t
   p.single.ntiles = L.ntiles;
   p.single.n = n;
   p.single.nh = L.nh;
-  p.single.lb = L.lb;
+  p.single.lb = L.lb < kDpMinTileBits ? kDpMinTileBits : L.lb;  // n < 8: one padded tile
   p.num_graphs = 1;
-  p.lb = L.lb;
-  p.total_tiles = L.ntiles;
+  p.lb = p.single.lb;
+  p.total_groups = dp_groups(L.binom, L.nh, p.lb);
   p.table = base;
   p.flags = reinterpret_cast<uint32_t*>(base + kNoallocFlagsOffset);
   int32_t* ctrl = reinterpret_cast<int32_t*>(base + kNoallocCtrlOffset);
@@ -122,12 +122,13 @@ extern "C" gtd_status gtd_dp_solve_noalloc(const uint64_t* d_adj, int n, int32_t
   if (clear_flags && cudaMemsetAsync(p.flags, 0, kNoallocMaxTiles * sizeof(uint32_t), s) != cudaSuccess)
     return GTD_CUDA_ERROR;  // wrapped: no stale stamp may match the new epoch
 
-  int occ = dp_tile_occupancy(p.lb);
+  p.kid_rows = L.nh;
+  int occ = dp_tile_occupancy(p.lb, L.nh);
   if (occ < 1)
     occ = 1;
   long long ctas = static_cast<long long>(sms) * occ;
-  if (ctas > p.total_tiles)
-    ctas = p.total_tiles;
+  if (ctas > p.total_groups)
+    ctas = p.total_groups;
   if (cudaMemsetAsync(ctrl, 0, 4 * sizeof(int32_t), s) != cudaSuccess)
     return GTD_CUDA_ERROR;
   if (dp_launch_validate(p, s) != cudaSuccess)

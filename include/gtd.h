@@ -89,7 +89,7 @@ typedef struct {
   float dp_ms;          /* DP kernel time, CUDA events on the handle's stream */
   float tree_ms;        /* tree reconstruction kernel */
   float total_ms;       /* whole call including copies */
-  uint64_t table_bytes; /* 2^n */
+  uint64_t table_bytes; /* 2^n, the byte table of gtd_dp_table */
   uint64_t alg_bytes;   /* 2^n + n 2^(n-1): one write + |S| one-byte gathers per subset */
   int tile_bits;
   int tiles;
@@ -130,7 +130,10 @@ gtd_status gtd_dp_query(gtd_handle h, uint64_t subset_mask, int32_t* td_out,
 /* Device pointer and size of the last solve's table (for inspection in
  * tests): entry of subset S lives at gtd_dp_table_index(n, tile_bits, S).
  * Each byte holds td << 1 | connected (td in bits 1-6, bit 0 set iff the
- * induced subgraph is connected). */
+ * induced subgraph is connected). The solve keeps three bits per subset; the
+ * bytes are written from them by the first of gtd_dp_table and
+ * gtd_dp_read_table after a solve, into a buffer of 2^n bytes that the handle
+ * keeps until a larger solve (GTD_OOM if it cannot be had). */
 gtd_status gtd_dp_table(gtd_handle h, const uint8_t** d_table, uint64_t* bytes,
                         int* n, int* tile_bits);
 uint64_t gtd_dp_table_index(int n, int tile_bits, uint64_t subset_mask);
@@ -163,7 +166,8 @@ typedef struct {
   float total_ms;       /* whole call including copies */
   uint64_t subsets;     /* sum of 2^n over the batch */
   uint64_t alg_bytes;   /* sum of 2^n + n 2^(n-1) */
-  uint64_t table_bytes; /* table pool (graphs with n < tile bits padded) */
+  uint64_t table_bytes; /* subsets in the table pool, graphs with n < tile bits
+                           padded (the pool takes three bits for each) */
   int tile_bits;        /* the launch's largest tile size */
   int tiles;
   int ctas;
