@@ -134,12 +134,15 @@ gtd_status next_epoch(gtd_handle h, uint32_t* epoch) {
 
 namespace {
 
-// Tile bits measured best on GB300: one tile up to n = 12 (n = 12: 16 us with
-// 12 bits against 30 with 10); few classes per tile while the levels are too
-// narrow to fill the GPU (n = 20: 108 us with 8 bits, 132 with 10; n = 25: 200
-// against 259); 11 bits from there (n = 28: 352 us against 355 with 10 and 348
-// with 8; n = 30: 718 against 743 and 958; n = 33: 4.68 ms against 5.14 and 7.5).
-int default_tile_bits(int n) { return n <= kDpMaxTileBits ? n : n <= 25 ? 8 : 11; }
+// Tile bits of the table's layout unless the caller gives them; the tile
+// kernel's best from n = 26 on (n = 30: 718 us with 11 bits against 743 with 10
+// and 803 with 12; n = 33: 4.68 ms against 5.14 and 5.23).
+int default_tile_bits(int n) { return n >= 26 ? 11 : 10; }
+
+// Up to this n the level kernel solves a graph, unless the caller gives tile
+// bits (level / 11-bit tile kernel: n = 12 20 / 24 us, 16 31 / 56, 20 45 / 117,
+// 25 112 / 234, 27 176 / 299, 28 264 / 344, 29 436 / 436, 30 806 / 690).
+constexpr int kLevelMaxN = 28;
 
 // Allocates (or grows) the table and flag buffers and enqueues the
 // validation, DP and tree kernels for one graph. Outputs go to
@@ -148,10 +151,14 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, int n, const gtd_dp_o
                       int32_t* d_td, int32_t* d_parent, int32_t* d_order) {
   const int tile_bits = (opts && opts->tile_bits > 0) ? opts->tile_bits : default_tile_bits(n);
   const DpLayout L = make_dp_layout(n, tile_bits);
-  const int lb = L.lb < kDpMinTileBits ? kDpMinTileBits : L.lb;  // n < 8: one padded tile
+  const bool by_level = !(opts && opts->tile_bits > 0) && n <= kLevelMaxN;
+  // the planes' tiles: n < lb is padded to one tile
+  const int lb = by_level ? kDpLevelTileBits : L.lb < kDpMinTileBits ? kDpMinTileBits : L.lb;
+  const int nh = n > lb ? n - lb : 0;
+  const uint32_t ntiles = 1u << nh;
   const size_t table_bytes = size_t(1) << n;
-  const size_t plane_bytes = size_t(L.ntiles) * dp_tile_bytes(lb);
-  const uint32_t groups = dp_groups(L.binom, L.nh, lb);
+  const size_t plane_bytes = size_t(ntiles) * dp_tile_bytes(lb);
+  const uint32_t groups = dp_groups(L.binom, nh, by_level ? kDpLevelChunk : dp_group_tiles(lb));
   h->bytes_valid = false;
   if (h->table_cap < plane_bytes) {
     h->have_table = false;
@@ -166,10 +173,10 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, int n, const gtd_dp_o
   dp_fill_binom(p);
   p.single.table_off = 0;
   p.single.flag_base = 0;
-  p.single.ntiles = L.ntiles;
+  p.single.ntiles = ntiles;
   p.single.adj_off = 0;
   p.single.n = n;
-  p.single.nh = L.nh;
+  p.single.nh = nh;
   p.single.lb = lb;
   p.single.out_idx = 0;
   p.num_graphs = 1;
@@ -178,6 +185,7 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, int n, const gtd_dp_o
   p.table = h->d_table;
   p.flags = h->d_flags;
   p.ticket = reinterpret_cast<uint32_t*>(h->d_io + kIoTicket);
+  p.level_done = reinterpret_cast<uint32_t*>(h->d_io + kIoLevels);
   p.error = h->d_io + kIoError;
   p.adj = d_adj;
   s = next_epoch(h, &p.epoch);
@@ -188,10 +196,10 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, int n, const gtd_dp_o
   p.parent_out = d_parent;
   p.order_out = d_order;
 
-  p.kid_rows = L.nh;
-  int& dp_occ = h->dp_occ[p.lb][L.nh];
+  p.kid_rows = nh;
+  int& dp_occ = h->dp_occ[by_level ? 0 : p.lb][nh];
   if (dp_occ <= 0)
-    dp_occ = dp_tile_occupancy(p.lb, L.nh);
+    dp_occ = by_level ? dp_level_occupancy(nh) : dp_tile_occupancy(p.lb, nh);
   int occ = dp_occ;
   if (opts && opts->ctas_per_sm > 0 && opts->ctas_per_sm < occ)
     occ = opts->ctas_per_sm;
@@ -201,14 +209,15 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, int n, const gtd_dp_o
   if (ctas > p.total_groups)
     ctas = p.total_groups;
 
-  GTD_CUDA(h, cudaMemsetAsync(h->d_io, 0, 4 * sizeof(int32_t), h->stream));
+  GTD_CUDA(h, cudaMemsetAsync(h->d_io, 0, kIoWords * sizeof(int32_t), h->stream));
   if (take_poison_fault())  // test injection: every byte must be written before it is read
     GTD_CUDA(h, cudaMemsetAsync(h->d_table, 0xFF, h->table_cap, h->stream));
   if (take_stall_fault())  // test injection: ticket 0 (the level-0 group) is never taken
     GTD_CUDA(h, cudaMemsetAsync(h->d_io + kIoTicket, 1, 1, h->stream));
   GTD_CUDA(h, dp_launch_validate(p, h->stream));
   GTD_CUDA(h, cudaEventRecord(h->ev[0], h->stream));
-  GTD_CUDA(h, dp_launch_tiles(p, static_cast<int>(ctas), h->stream));
+  GTD_CUDA(h, by_level ? dp_launch_levels(p, static_cast<int>(ctas), h->stream)
+                       : dp_launch_tiles(p, static_cast<int>(ctas), h->stream));
   GTD_CUDA(h, cudaEventRecord(h->ev[1], h->stream));
   GTD_CUDA(h, dp_launch_tree(p, h->stream));
   GTD_CUDA(h, cudaEventRecord(h->ev[2], h->stream));
@@ -221,6 +230,7 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, int n, const gtd_dp_o
   st.table_bytes = table_bytes;
   st.alg_bytes = table_bytes + static_cast<uint64_t>(n) * (table_bytes / 2);
   h->last_tile_bits = L.lb;
+  h->last_tiles = L.ntiles;
   st.tile_bits = L.lb;
   st.tiles = static_cast<int>(L.ntiles);
   st.ctas = static_cast<int>(ctas);
@@ -233,7 +243,7 @@ gtd_status make_byte_table(gtd_handle h) {
     return GTD_OK;
   const size_t bytes = size_t(1) << h->last_params.single.n;
   GTD_CUDA(h, ensure_field(&h->d_bytes, &h->bytes_cap, bytes));
-  GTD_CUDA(h, dp_launch_expand(h->last_params, h->d_bytes, bytes, h->stream));
+  GTD_CUDA(h, dp_launch_expand(h->last_params, h->last_tile_bits, h->last_tiles, h->d_bytes, bytes, h->stream));
   h->bytes_valid = true;
   return GTD_OK;
 }

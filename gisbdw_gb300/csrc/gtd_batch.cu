@@ -168,7 +168,7 @@ void make_plan(Plan& P, const gtd_graph_desc* descs, int count) {
     off += uint64_t(G.ntiles) * dp_tile_bytes(lb);
     P.table_bytes += uint64_t(G.ntiles) << lb;
     tile += G.ntiles;
-    group += dp_groups(binom, G.nh, lb);
+    group += dp_groups(binom, G.nh, dp_group_tiles(lb));
     P.kid_rows = std::max(P.kid_rows, G.nh);
     const uint64_t sub = uint64_t(1) << d.n;
     P.subsets += sub;

@@ -42,6 +42,10 @@ __device__ __forceinline__ void st_release_u32(uint32_t* p, uint32_t v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+__device__ __forceinline__ void red_release_add_u32(uint32_t* p, uint32_t v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
 __device__ __forceinline__ uint64_t global_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -74,6 +78,25 @@ __device__ __forceinline__ bool wait_flag(const uint32_t* flag, uint32_t want,
     __nanosleep(sleep_ns);
     if (sleep_ns < 2048)
       sleep_ns *= 2;
+  }
+}
+
+// Waits until *count == want, polling without a pause (the count is expected
+// within microseconds). Gives up as wait_flag does.
+__device__ __forceinline__ bool wait_count(const uint32_t* count, uint32_t want, uint64_t timeout_ns, int32_t* err) {
+  if (ld_acquire_u32(count) == want)
+    return true;
+  const uint64_t deadline = global_ns() + timeout_ns;
+  for (;;) {
+    for (int i = 0; i < 16; ++i)
+      if (ld_acquire_u32(count) == want)
+        return true;
+    if (ld_relaxed_s32(err) != 0)
+      return false;
+    if (global_ns() > deadline) {
+      raise_error(err, kDevWaitTimeout, 0);
+      return false;
+    }
   }
 }
 

@@ -633,6 +633,205 @@ __global__ void __launch_bounds__(kDpThreads, 4) dp_tile_kernel_mixed(const __gr
 }
 
 // ---------------------------------------------------------------------------
+// Narrow levels: a thread per tile of 7 bits, level by level.
+// ---------------------------------------------------------------------------
+
+// A word's 32 subsets (bit x = the subset x of the five lowest vertices) from
+// the summary of their children outside the word, by size of x: position 0,
+// its broadcast to the singles, three rounds over the five vertices (round r
+// settles size r; smaller sizes come out as before, larger ones are not
+// final), then position 31 from its five children.
+__device__ __forceinline__ Planes resolve_word(const Acc& ext, const SmallSets& s) {
+  constexpr uint32_t kSingles = 0x00010116u, kFours = 0x68808000u, kTop = 0x80000000u;  // |x| = 1, 4, 5
+  Planes r = finish(ext, s);
+  Acc a = ext;
+  a.o0 |= (r.p0 & 1u) * kSingles;
+  a.o1 |= (r.p1 & 1u) * kSingles;
+  a.o2 |= (~(r.p0 | r.p1) & 1u) * kSingles;
+  a.c2 |= a.c1 & ((r.c & 1u) * kSingles);
+  r = finish(a, s);
+#pragma unroll
+  for (int round = 2; round <= 4; ++round) {
+    constexpr uint32_t kHas[5] = {0xAAAAAAAAu, 0xCCCCCCCCu, 0xF0F0F0F0u, 0xFF00FF00u, 0xFFFF0000u};
+    const uint32_t p2 = ~(r.p0 | r.p1);
+    a = ext;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const int sh = 1 << i;
+      a.o0 |= (r.p0 << sh) & kHas[i];
+      a.o1 |= (r.p1 << sh) & kHas[i];
+      a.o2 |= (p2 << sh) & kHas[i];
+      const uint32_t x = (r.c << sh) & kHas[i];
+      a.c2 |= a.c1 & x;
+      a.c1 |= x;
+    }
+    r = finish(a, s);
+  }
+  const uint32_t p2 = ~(r.p0 | r.p1), k = r.c & kFours;
+  a = ext;
+  a.o0 |= (r.p0 & kFours) ? kTop : 0u;
+  a.o1 |= (r.p1 & kFours) ? kTop : 0u;
+  a.o2 |= (p2 & kFours) ? kTop : 0u;
+  a.c2 |= (k ? a.c1 & kTop : 0u) | ((k & (k - 1u)) ? kTop : 0u);
+  const Planes t = finish(a, s);
+  r.p0 = (r.p0 & ~kTop) | (t.p0 & kTop);
+  r.p1 = (r.p1 & ~kTop) | (t.p1 & kTop);
+  r.c = (r.c & ~kTop) | (t.c & kTop);
+  return r;
+}
+
+constexpr int kLevelThreads = kDpLevelChunk;
+
+// Thread r of a chunk resolves the tile of rank r: unranks it, gathers its
+// child tiles (48 bytes each), resolves its four words in order 00, 01 and
+// 10, 11 of vertices 5 and 6. A chunk of level j waits until every chunk of
+// level j - 1 is done (one counter per level, acquired by one thread), after
+// unranking: no flags to look up per child. Tickets as in the tile kernel.
+//
+// For levels too narrow to fill the GPU, where the latency of the tile
+// kernel's groups (15 us a level at 11 bits) leaves most SMs idle: a level costs
+// 2.5 to 3 us here (n = 20: 45 us), most of it the count, the gathers and the
+// chain through three words. A tile of 48 bytes is also the widest load that
+// the gathers can use, so tables beyond the L2 (n >= 29) go to the tile kernel.
+__global__ void __launch_bounds__(kLevelThreads, 4) dp_level_kernel(const __grid_constant__ DpBatchParams p) {
+  constexpr int LB = kDpLevelTileBits;
+  constexpr uint32_t kTileBytes = dp_tile_bytes(LB);
+  extern __shared__ __align__(16) uint8_t smem[];
+  uint32_t* const kids = reinterpret_cast<uint32_t*>(smem) + threadIdx.x;  // kids[i * kLevelThreads]
+  __shared__ Binom binom;
+  __shared__ uint32_t sTicket;
+  __shared__ int sStop;
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  for (int i = tid; i < (kDpMaxHigh + 1) * (kDpMaxHigh + 1); i += kLevelThreads)
+    (&binom[0][0])[i] = (&p.binom[0][0])[i];
+  uint32_t ticket = 0;
+  if (tid == 0)
+    ticket = atomicAdd(p.ticket, 1u);
+  const DpGraph G = p.single;
+  uint8_t* const table = p.table + G.table_off;
+  const int nh = G.nh;
+  for (;;) {
+    if (tid == 0)
+      sTicket = ticket;
+    __syncthreads();
+    const uint32_t chunk = sTicket;
+    if (chunk >= p.total_groups)
+      return;
+    if (tid == 0)
+      ticket = atomicAdd(p.ticket, 1u);
+    // Level j of the chunk: lane i holds the tiles and chunks of levels 0..i.
+    const uint32_t level_tiles = static_cast<int>(lane) <= nh ? binom[nh][lane] : 0u;
+    const uint32_t level_chunks = (level_tiles + kLevelThreads - 1u) / kLevelThreads;
+    uint32_t cumT = level_tiles, cumG = level_chunks;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xffffffffu, cumT, d);
+      const uint32_t y = __shfl_up_sync(0xffffffffu, cumG, d);
+      if (static_cast<int>(lane) >= d) {
+        cumT += x;
+        cumG += y;
+      }
+    }
+    const int j = __popc(__ballot_sync(0xffffffffu, static_cast<int>(lane) <= nh && cumG <= chunk));
+    const uint32_t tiles_j = __shfl_sync(0xffffffffu, level_tiles, j);
+    const uint32_t off_j = __shfl_sync(0xffffffffu, cumT, j) - tiles_j;
+    const uint32_t first = __shfl_sync(0xffffffffu, cumG - level_chunks, j);
+    const uint32_t off_prev = off_j - __shfl_sync(0xffffffffu, level_tiles, (j + 31) & 31);
+    const uint32_t chunks_prev = __shfl_sync(0xffffffffu, level_chunks, (j + 31) & 31);
+    const uint32_t rank = (chunk - first) * kLevelThreads + tid;
+    const bool mine = rank < tiles_j;
+    uint32_t H = 0;
+    if (mine) {
+      uint32_t rest = rank, kid = off_prev;
+      uint32_t* at = kids;
+      int k = j;
+      for (int a = nh - 1; a >= 0; --a) {  // as in the tile kernel
+        const uint32_t c = binom[a][k], d = binom[a][max(k - 1, 0)];
+        if (rest >= c) {
+          rest -= c;
+          H |= 1u << a;
+          *at = kid + rest;
+          at += kLevelThreads;
+          kid += d;
+          --k;
+        }
+      }
+    }
+    if (j > 0) {
+      if (tid == 0)
+        sStop = wait_count(p.level_done + (j - 1), chunks_prev, p.timeout_ns, p.error) ? 0 : 1;
+      __syncthreads();
+      if (sStop)
+        return;
+    }
+    if (mine) {
+      Acc a[4];
+      const uint32_t* kid = kids;
+      auto child = [&](uint32_t t, uint4& p0, uint4& p1, uint4& c) {
+        const uint8_t* from = table + size_t(t) * kTileBytes;
+        p0 = ldcg128(from);
+        p1 = ldcg128(from + 16);
+        c = ldcg128(from + 32);
+      };
+      int m = 0;
+#pragma unroll 2
+      for (; m + 2 <= j; m += 2) {
+        uint4 s0, s1, sc, t0, t1, tc;
+        child(kid[0], s0, s1, sc);
+        child(kid[kLevelThreads], t0, t1, tc);
+        kid += 2 * kLevelThreads;
+        acc_add2(a[0], s0.x, s1.x, sc.x, t0.x, t1.x, tc.x);
+        acc_add2(a[1], s0.y, s1.y, sc.y, t0.y, t1.y, tc.y);
+        acc_add2(a[2], s0.z, s1.z, sc.z, t0.z, t1.z, tc.z);
+        acc_add2(a[3], s0.w, s1.w, sc.w, t0.w, t1.w, tc.w);
+      }
+      if (m < j) {
+        uint4 s0, s1, sc;
+        child(kid[0], s0, s1, sc);
+        acc_add1(a[0], s0.x, s1.x, sc.x);
+        acc_add1(a[1], s0.y, s1.y, sc.y);
+        acc_add1(a[2], s0.z, s1.z, sc.z);
+        acc_add1(a[3], s0.w, s1.w, sc.w);
+      }
+      Planes r[4];
+      if (j > 2) {
+        const SmallSets any;
+        r[0] = resolve_word(a[0], any);
+        acc_add1(a[1], r[0].p0, r[0].p1, r[0].c);
+        acc_add1(a[2], r[0].p0, r[0].p1, r[0].c);
+        r[1] = resolve_word(a[1], any);
+        r[2] = resolve_word(a[2], any);
+        acc_add2(a[3], r[1].p0, r[1].p1, r[1].c, r[2].p0, r[2].p1, r[2].c);
+        r[3] = resolve_word(a[3], any);
+      } else {
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          if (w == 3) {
+            acc_add2(a[3], r[1].p0, r[1].p1, r[1].c, r[2].p0, r[2].p1, r[2].c);
+          } else if (w > 0) {
+            acc_add1(a[w], r[0].p0, r[0].p1, r[0].c);
+          }
+          const int size = j + __popc(w);
+          r[w] = resolve_word(a[w], size <= 2 ? small_sets((uint64_t(H) << LB) | (uint64_t(w) << 5), size,
+                                                           p.adj + G.adj_off, G.n)
+                                              : SmallSets{});
+        }
+      }
+      uint4* const out = reinterpret_cast<uint4*>(table + size_t(off_j + rank) * kTileBytes);
+      out[0] = make_uint4(r[0].p0, r[1].p0, r[2].p0, r[3].p0);
+      out[1] = make_uint4(r[0].p1, r[1].p1, r[2].p1, r[3].p1);
+      out[2] = make_uint4(r[0].c, r[1].c, r[2].c, r[3].c);
+    }
+    // The chunk's stores are ordered before the count by the barrier; the
+    // count is a gpu-scope release, and a chain of such additions hands every
+    // chunk's stores to the thread that acquires the final value.
+    __syncthreads();
+    if (tid == 0)
+      red_release_add_u32(p.level_done + j, 1u);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Reconstruction: one warp per graph; lanes cover vertices lane, lane + 32.
 // ---------------------------------------------------------------------------
 
@@ -669,18 +868,21 @@ struct TreeCtx {
   const Binom& binom;
   const uint8_t* table;
   int lb, nh, n;
-  // td(S) mod 3 (one lane).
-  __device__ uint32_t residue(uint64_t S) const {
+  // The first plane's word that holds S (the other planes: 2^(lb-5) words on).
+  __device__ const uint32_t* word(uint64_t S) const {
     const uint32_t H = static_cast<uint32_t>(S >> lb);
     const int j = __popc(H);
     uint32_t off = 0;
     for (int i = 0; i < j; ++i)
       off += binom[nh][i];
-    const uint32_t words = 1u << (lb - 5);
-    const uint32_t* t = reinterpret_cast<const uint32_t*>(table + size_t(off + rank_colex(binom, H)) * (12u * words)) +
-                        ((static_cast<uint32_t>(S) >> 5) & (words - 1u));
+    return reinterpret_cast<const uint32_t*>(table + size_t(off + rank_colex(binom, H)) * dp_tile_bytes(lb)) +
+           ((static_cast<uint32_t>(S) >> 5) & ((1u << (lb - 5)) - 1u));
+  }
+  // td(S) mod 3 (one lane).
+  __device__ uint32_t residue(uint64_t S) const {
+    const uint32_t* t = word(S);
     const uint32_t bit = static_cast<uint32_t>(S) & 31u;
-    const uint32_t p0 = (t[0] >> bit) & 1u, p1 = (t[words] >> bit) & 1u;
+    const uint32_t p0 = (t[0] >> bit) & 1u, p1 = (t[1u << (lb - 5)] >> bit) & 1u;
     return p0 ? 0u : 2u - p1;
   }
   // td(S) (whole warp): along the chain S & {v, v + 1, ...}, v = 0 .. n, each
@@ -929,6 +1131,18 @@ int dp_mixed_occupancy(int lb, int kid_rows) {
                       smem_layout_for(kDpMinTileBits, kDpMaxTileBits, kDpMaxHigh));
 }
 
+int dp_level_occupancy(int kid_rows) {
+  const int smem = static_cast<int>(sizeof(uint32_t)) * kLevelThreads * kid_rows;
+  int blocks = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, dp_level_kernel, kLevelThreads, smem);
+  return blocks;
+}
+
+cudaError_t dp_launch_levels(const DpBatchParams& p, int ctas, cudaStream_t s) {
+  dp_level_kernel<<<ctas, kLevelThreads, sizeof(uint32_t) * kLevelThreads * p.kid_rows, s>>>(p);
+  return cudaGetLastError();
+}
+
 cudaError_t dp_launch_tiles(const DpBatchParams& p, int ctas, cudaStream_t s) {
   if (p.mixed) {
     if (p.lb < kDpMinTileBits || p.lb > kDpMaxTileBits)
@@ -1003,11 +1217,11 @@ cudaError_t dp_launch_labels(const DpBatchParams& p, const uint64_t* subsets, in
 }
 
 // The byte table of gtd_dp_table (td << 1 | connected per subset, tiles of
-// 2^lb bytes in tile order) from the planes, one warp per tile: td(H) from
-// the warp's chain, each word's first subset along the chain of its bits, the
-// word's subsets from one another.
+// 2^lb bytes in tile order; the planes may have tiles of another size), one
+// warp per tile: td(H) from the warp's chain, each word's first subset along
+// the chain of its bits, the word's subsets from one another.
 __global__ void __launch_bounds__(32 * kTreeWarps)
-    dp_expand_kernel(const __grid_constant__ DpBatchParams p, uint8_t* out, uint64_t bytes) {
+    dp_expand_kernel(const __grid_constant__ DpBatchParams p, int lb, uint32_t tiles, uint8_t* out, uint64_t bytes) {
   __shared__ Binom sBinom;
   for (int i = threadIdx.x; i < (kDpMaxHigh + 1) * (kDpMaxHigh + 1); i += blockDim.x)
     (&sBinom[0][0])[i] = (&p.binom[0][0])[i];
@@ -1015,20 +1229,21 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const DpGraph G = p.single;
   const TreeCtx ctx{sBinom, p.table + G.table_off, G.lb, G.nh, G.n};
-  const uint32_t words = 1u << (G.lb - 5);
-  for (uint32_t t = blockIdx.x * kTreeWarps + warp; t < G.ntiles; t += gridDim.x * kTreeWarps) {
+  const int nh = G.n > lb ? G.n - lb : 0;
+  const uint32_t words = lb > 5 ? 1u << (lb - 5) : 1u;
+  for (uint32_t t = blockIdx.x * kTreeWarps + warp; t < tiles; t += gridDim.x * kTreeWarps) {
     uint32_t r = t, H = 0;
     int j = 0;
-    while (r >= sBinom[G.nh][j])
-      r -= sBinom[G.nh][j++];
-    for (int a = G.nh - 1, k = j; k > 0; --a)
+    while (r >= sBinom[nh][j])
+      r -= sBinom[nh][j++];
+    for (int a = nh - 1, k = j; k > 0; --a)
       if (r >= sBinom[a][k]) {
         r -= sBinom[a][k--];
         H |= 1u << a;
       }
-    const uint32_t base = ctx.td_of(static_cast<uint64_t>(H) << G.lb);
-    const uint32_t* tile = reinterpret_cast<const uint32_t*>(ctx.table + size_t(t) * (12u * words));
-    auto first = [&](uint32_t w) { return (tile[w] & 1u) ? 0u : 2u - (tile[words + w] & 1u); };
+    const uint64_t high = static_cast<uint64_t>(H) << lb;
+    const uint32_t base = ctx.td_of(high);
+    auto first = [&](uint32_t w) { return ctx.residue(high | (static_cast<uint64_t>(w) << 5)); };
     for (uint32_t w = lane; w < words; w += 32) {
       uint32_t td[32];
       td[0] = base;
@@ -1038,14 +1253,15 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
         td[0] += here != next;
         here = next;
       }
-      const uint32_t p0 = tile[w], p1 = tile[words + w], c = tile[2 * words + w];
+      const uint32_t* word = ctx.word(high | (static_cast<uint64_t>(w) << 5));
+      const uint32_t stride = 1u << (G.lb - 5), p0 = word[0], p1 = word[stride], c = word[2 * stride];
       // residue changes between x and x without its lowest bit: treedepth + 1
 #pragma unroll
       for (int x = 1; x < 32; ++x) {
         const int y = x & (x - 1);
         td[x] = td[y] + ((((p0 >> x) ^ (p0 >> y)) | ((p1 >> x) ^ (p1 >> y))) & 1u);
       }
-      const uint64_t at = (static_cast<uint64_t>(t) << G.lb) + w * 32u;
+      const uint64_t at = (static_cast<uint64_t>(t) << lb) + w * 32u;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         uint32_t v = 0;
@@ -1059,9 +1275,10 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
   }
 }
 
-cudaError_t dp_launch_expand(const DpBatchParams& p, uint8_t* out, uint64_t bytes, cudaStream_t s) {
-  const uint32_t ctas = (p.single.ntiles + kTreeWarps - 1) / kTreeWarps;
-  dp_expand_kernel<<<ctas < 16384u ? ctas : 16384u, 32 * kTreeWarps, 0, s>>>(p, out, bytes);
+cudaError_t dp_launch_expand(const DpBatchParams& p, int lb, uint32_t tiles, uint8_t* out, uint64_t bytes,
+                             cudaStream_t s) {
+  const uint32_t ctas = (tiles + kTreeWarps - 1) / kTreeWarps;
+  dp_expand_kernel<<<ctas < 16384u ? ctas : 16384u, 32 * kTreeWarps, 0, s>>>(p, lb, tiles, out, bytes);
   return cudaGetLastError();
 }
 

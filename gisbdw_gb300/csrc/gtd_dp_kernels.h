@@ -39,6 +39,7 @@ struct DpBatchParams {
   uint8_t* table = nullptr;         // table pool: tiles of three bit planes
   uint32_t* flags = nullptr;        // one ready stamp per tile group
   uint32_t* ticket = nullptr;       // work counter, zeroed before each launch
+  uint32_t* level_done = nullptr;   // chunks done per level (level kernel), zeroed before each launch
   int32_t* error = nullptr;         // [0] code, [1] info
   const uint64_t* adj = nullptr;    // adjacency pool (device)
   uint32_t epoch = 0;               // flags equal to epoch are ready
@@ -59,11 +60,16 @@ int dp_mixed_occupancy(int lb, int kid_rows);
 cudaError_t dp_launch_validate(const DpBatchParams& p, cudaStream_t s);
 cudaError_t dp_launch_fill_tile_map(const DpBatchParams& p, cudaStream_t s);
 cudaError_t dp_launch_tiles(const DpBatchParams& p, int ctas, cudaStream_t s);
+// The level kernel (single graph, tiles of kDpLevelTileBits): total_groups
+// counts chunks of kDpLevelChunk tiles of one level.
+int dp_level_occupancy(int kid_rows);
+cudaError_t dp_launch_levels(const DpBatchParams& p, int ctas, cudaStream_t s);
 cudaError_t dp_launch_tree(const DpBatchParams& p, cudaStream_t s);
 cudaError_t dp_launch_labels(const DpBatchParams& p, const uint64_t* subsets, int count, int32_t* td_out,
                              uint64_t* roots_out, cudaStream_t s);
-// The byte table (td << 1 | connected, 2^n bytes in tile order) of a solved
-// single graph.
-cudaError_t dp_launch_expand(const DpBatchParams& p, uint8_t* out, uint64_t bytes, cudaStream_t s);
+// The byte table (td << 1 | connected, 2^n bytes) of a solved single graph,
+// in `tiles` tiles of 2^lb bytes.
+cudaError_t dp_launch_expand(const DpBatchParams& p, int lb, uint32_t tiles, uint8_t* out, uint64_t bytes,
+                             cudaStream_t s);
 
 }  // namespace gtd

@@ -39,6 +39,10 @@ GTD_HD constexpr int dp_group_shift(int lb) { return lb <= 9 ? 7 : 16 - lb; }
 GTD_HD constexpr int dp_group_tiles(int lb) { return 1 << dp_group_shift(lb); }
 static_assert(dp_group_tiles(9) == kDpThreads && (dp_group_tiles(11) << (11 - 5)) == 16 * kDpThreads, "group size");
 
+// The level kernel's tiles (a thread per tile) and tiles per chunk.
+constexpr int kDpLevelTileBits = 7;
+constexpr int kDpLevelChunk = 128;
+
 // Bytes of a tile of the solve's table.
 GTD_HD constexpr uint32_t dp_tile_bytes(int lb) { return 12u << (lb - 5); }
 
@@ -87,10 +91,9 @@ struct DpLayout {
   }
 };
 
-// Groups of tiles of a graph with nh high vertices and tiles of lb bits: no
-// group spans two levels.
-inline uint32_t dp_groups(const uint32_t (&binom)[kDpMaxHigh + 1][kDpMaxHigh + 1], int nh, int lb) {
-  const uint32_t per = dp_group_tiles(lb);
+// Groups of `per` tiles of a graph with nh high vertices: no group spans two
+// levels.
+inline uint32_t dp_groups(const uint32_t (&binom)[kDpMaxHigh + 1][kDpMaxHigh + 1], int nh, uint32_t per) {
   uint32_t groups = 0;
   for (int j = 0; j <= nh; ++j)
     groups += (binom[nh][j] + per - 1) / per;

@@ -20,6 +20,7 @@ constexpr int kIoError = 1;
 constexpr int kIoTd = 4;
 constexpr int kIoParent = 8;
 constexpr int kIoOrder = 72;
+constexpr int kIoLevels = 208;  // chunks done per level (level kernel), 32 words
 constexpr int kIoWords = 256;
 // Byte offsets inside the handle's 4096-byte pinned staging block.
 constexpr size_t kPinnedIo = 1024;     // IO block copies (kIoOrder + 64 words)
@@ -84,7 +85,7 @@ struct gtd_handle_s {
   // size (0 = unmeasured), from the autotuner.
   float tune_mixed_eff[gtd::kTuneLbMax + 1] = {};
   // CTAs per SM of the one-size DP kernel per tile size and number of high
-  // vertices (0 = not asked yet):
+  // vertices, row 0 the level kernel's (0 = not asked yet):
   // a property of the kernel and the device, looked up once per handle.
   int dp_occ[gtd::kDpMaxTileBits + 1][gtd::kDpMaxHigh + 1] = {};
 
@@ -97,7 +98,8 @@ struct gtd_handle_s {
   // Last DP solve (for gtd_dp_query / gtd_sync).
   bool have_table = false;
   bool pending_stats = false;
-  int last_tile_bits = 0;  // of the byte table's layout (n < 8: n, the planes pad to 8)
+  int last_tile_bits = 0;  // of the byte table's layout (the planes' tiles may differ)
+  uint32_t last_tiles = 0;
   gtd::DpBatchParams last_params;
   gtd_dp_stats last_stats = {};
 };

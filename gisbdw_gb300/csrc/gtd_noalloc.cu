@@ -102,7 +102,7 @@ extern "C" gtd_status gtd_dp_solve_noalloc(const uint64_t* d_adj, int n, int32_t
   p.single.lb = L.lb < kDpMinTileBits ? kDpMinTileBits : L.lb;  // n < 8: one padded tile
   p.num_graphs = 1;
   p.lb = p.single.lb;
-  p.total_groups = dp_groups(L.binom, L.nh, p.lb);
+  p.total_groups = dp_groups(L.binom, L.nh, dp_group_tiles(p.lb));
   p.table = base;
   p.flags = reinterpret_cast<uint32_t*>(base + kNoallocFlagsOffset);
   int32_t* ctrl = reinterpret_cast<int32_t*>(base + kNoallocCtrlOffset);

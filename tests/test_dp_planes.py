@@ -202,11 +202,12 @@ def test_child_ranks_while_unranking():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("tile_bits", [8, 9, 10, 11, 12])
+@pytest.mark.parametrize("tile_bits", [0, 8, 9, 10, 11, 12])  # 0: the level kernel
 @pytest.mark.parametrize("n", [2, 4, 7, 8, 9, 12, 13, 16, 18])
 def test_kernel_at_tile_edges_matches_oracle(handle, port, tile_bits, n):
     """Padded tiles (n < 8), one tile, one to a few tiles per level, levels of
-    just under and over a group: every byte of the table, tree and order."""
+    just under and over a group or chunk: every byte of the table, the tree,
+    the order."""
     from gisbdw_gb300 import _lib
     for g in (G.gnp(n, 0.35, 40 + n), G.path(n), G.complete(n)):
         td, parent, order, _ = handle.dp_solve(g.adj64(), n, tile_bits=tile_bits)
@@ -215,7 +216,7 @@ def test_kernel_at_tile_edges_matches_oracle(handle, port, tile_bits, n):
         assert (td, parent.tolist()) == (otd, opar.tolist()), g.name
         assert sorted(order.tolist()) == list(range(n))
         raw, tn, lb = handle.dp_read_table()
-        assert tn == n and lb == min(n, tile_bits)
+        assert tn == n and lb == min(n, tile_bits or 10)
         S = np.arange(1 << n, dtype=np.int64)
         tile = np.array([_lib.table_index(n, lb, int(h) << lb) >> lb for h in range(1 << (n - lb))], dtype=np.int64)
         tab = raw[(tile[S >> lb] << lb) | (S & ((1 << lb) - 1))]
