@@ -170,7 +170,6 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, int n, const gtd_dp_o
     return s;
 
   DpBatchParams p;
-  dp_fill_binom(p);
   p.single.table_off = 0;
   p.single.flag_base = 0;
   p.single.ntiles = ntiles;

@@ -304,7 +304,6 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
 
   DpBatchParams& bp = h->bparams;
   bp = DpBatchParams{};
-  dp_fill_binom(bp);
   bp.graphs = h->d_bgraphs;
   bp.tile_map = h->d_tile_map;
   bp.level_base = h->d_level_base;

@@ -24,7 +24,7 @@
 //    count of connected ones: 3.5 logic operations per child and 32 subsets,
 //    where one byte per subset took 2 per child and 4 subsets (2.67 times
 //    the bytes from L2 and DRAM too). Full treedepths are read back along a
-//    chain of deletions (TreeCtx::td_of).
+//    chain of deletions (chain_td).
 //  * Layout (gtd_dp_layout.h). Tiles of 2^lb subsets share a high part H; a
 //    tile is its three planes, 2^(lb-5) words each. The cross-tile children
 //    are whole tiles H - h one level down, read as 16-byte vectors; the
@@ -108,6 +108,21 @@ __device__ __forceinline__ void acc_add2(Acc& a, uint32_t p0, uint32_t p1, uint3
 struct Planes {
   uint32_t p0, p1, c;
 };
+
+// The binomial table (C(a, b) = 0 for b > a), row by row by the first warp; a
+// CTA barrier must follow.
+__device__ __forceinline__ void fill_binom(Binom& binom) {
+  if (threadIdx.x < 32) {
+    uint32_t c = threadIdx.x == 0 ? 1u : 0u;
+    for (int a = 0; a <= kDpMaxHigh; ++a) {
+      if (threadIdx.x <= kDpMaxHigh)
+        binom[a][threadIdx.x] = c;
+      const uint32_t left = __shfl_up_sync(0xffffffffu, c, 1);
+      if (threadIdx.x > 0)
+        c += left;
+    }
+  }
+}
 
 // Connectivity of the subsets of size <= 2 of a word (the count of connected
 // children only decides it from size 3 on): conn = (count & keep) | set.
@@ -277,12 +292,15 @@ __global__ void dp_validate_kernel(const __grid_constant__ DpBatchParams p) {
 // groups, then every level-1 group, ...), so that a tile's children lie far
 // back in the ticket stream; tables and flags stay graph-major.
 __global__ void dp_fill_tile_map_kernel(const __grid_constant__ DpBatchParams p) {
+  __shared__ Binom binom;
+  fill_binom(binom);
+  __syncthreads();
   for (int g = blockIdx.x; g < p.num_graphs; g += gridDim.x) {
     const DpGraph G = p.graphs[g];
     const uint32_t per = dp_group_tiles(G.lb);
     uint32_t local = 0;
     for (int j = 0; j <= G.nh; ++j) {
-      const uint32_t count = (p.binom[G.nh][j] + per - 1u) / per;
+      const uint32_t count = (binom[G.nh][j] + per - 1u) / per;
       const uint32_t base = p.level_base[size_t(g) * (kDpMaxHigh + 2) + j];
       for (uint32_t i = threadIdx.x; i < count; i += blockDim.x)
         p.tile_map[base + i] = make_uint2(static_cast<uint32_t>(g), local + i);
@@ -349,9 +367,9 @@ struct Workspace {
 __device__ __forceinline__ Workspace make_workspace(const DpBatchParams& p, const SmemLayout& L, int order_bits) {
   extern __shared__ __align__(16) uint8_t smem[];
   Binom& sBinom = *reinterpret_cast<Binom*>(smem + L.binom_off);
-  for (int i = threadIdx.x; i < (kDpMaxHigh + 1) * (kDpMaxHigh + 1); i += blockDim.x)
-    (&sBinom[0][0])[i] = (&p.binom[0][0])[i];
-  build_word_order(smem + L.order_off, p.binom, order_bits);
+  fill_binom(sBinom);
+  __syncthreads();
+  build_word_order(smem + L.order_off, sBinom, order_bits);
   return Workspace{reinterpret_cast<uint32_t*>(smem), reinterpret_cast<uint32_t*>(smem + L.kids_off),
                    reinterpret_cast<uint32_t*>(smem + L.high_off), sBinom, smem + L.order_off, order_bits};
 }
@@ -702,8 +720,7 @@ __global__ void __launch_bounds__(kLevelThreads, 4) dp_level_kernel(const __grid
   __shared__ uint32_t sTicket;
   __shared__ int sStop;
   const uint32_t tid = threadIdx.x, lane = tid & 31;
-  for (int i = tid; i < (kDpMaxHigh + 1) * (kDpMaxHigh + 1); i += kLevelThreads)
-    (&binom[0][0])[i] = (&p.binom[0][0])[i];
+  fill_binom(binom);
   uint32_t ticket = 0;
   if (tid == 0)
     ticket = atomicAdd(p.ticket, 1u);
@@ -849,33 +866,20 @@ __device__ __forceinline__ uint64_t warp_or64(uint64_t x) {
   return (static_cast<uint64_t>(hi) << 32) | lo;
 }
 
-__device__ uint64_t warp_component(uint64_t S, int v, const uint64_t* adj, int n) {
-  const int lane = threadIdx.x & 31;
-  uint64_t reach = 1ull << v, frontier = reach;
-  while (frontier) {
-    uint64_t nb = 0;
-    for (int u = lane; u < n; u += 32)
-      if ((frontier >> u) & 1ull)
-        nb |= adj[u];
-    nb = warp_or64(nb) & S & ~reach;
-    reach |= nb;
-    frontier = nb;
-  }
-  return reach;
-}
-
+// Subsets of a table in global memory.
 struct TreeCtx {
   const Binom& binom;
+  const uint32_t* off;  // first tile of every level
   const uint8_t* table;
-  int lb, nh, n;
+  int lb, n;
   // The first plane's word that holds S (the other planes: 2^(lb-5) words on).
   __device__ const uint32_t* word(uint64_t S) const {
-    const uint32_t H = static_cast<uint32_t>(S >> lb);
-    const int j = __popc(H);
-    uint32_t off = 0;
-    for (int i = 0; i < j; ++i)
-      off += binom[nh][i];
-    return reinterpret_cast<const uint32_t*>(table + size_t(off + rank_colex(binom, H)) * dp_tile_bytes(lb)) +
+    uint32_t H = static_cast<uint32_t>(S >> lb), rank = off[__popc(H)];
+    const uint32_t* col = &binom[0][1];
+#pragma unroll 4
+    for (; H; H &= H - 1, ++col)
+      rank += col[(__ffs(H) - 1) * (kDpMaxHigh + 1)];
+    return reinterpret_cast<const uint32_t*>(table + size_t(rank) * dp_tile_bytes(lb)) +
            ((static_cast<uint32_t>(S) >> 5) & ((1u << (lb - 5)) - 1u));
   }
   // td(S) mod 3 (one lane).
@@ -885,189 +889,233 @@ struct TreeCtx {
     const uint32_t p0 = (t[0] >> bit) & 1u, p1 = (t[1u << (lb - 5)] >> bit) & 1u;
     return p0 ? 0u : 2u - p1;
   }
-  // td(S) (whole warp): along the chain S & {v, v + 1, ...}, v = 0 .. n, each
-  // deletion lowers the treedepth by 0 or 1, which the residues tell.
-  __device__ uint32_t td_of(uint64_t S) const {
-    const int lane = threadIdx.x & 31;
-    const uint64_t above_lo = S & (~0ull << lane), above_hi = S & (~0ull << (lane + 32));
-    const uint32_t lo = lane <= n ? residue(above_lo) : 0u;
-    const uint32_t hi = lane + 32 <= n ? residue(above_hi) : 0u;
-    uint32_t next_lo = __shfl_down_sync(0xffffffffu, lo, 1);
-    const uint32_t first_hi = __shfl_sync(0xffffffffu, hi, 0), next_hi = __shfl_down_sync(0xffffffffu, hi, 1);
-    if (lane == 31)
-      next_lo = first_hi;
-    uint32_t drop = 0;
-    if (lane < n)
-      drop += lo == (next_lo == 2u ? 0u : next_lo + 1u) ? 1u : 0u;
-    if (lane + 32 < n)
-      drop += hi == (next_hi == 2u ? 0u : next_hi + 1u) ? 1u : 0u;
-    return __reduce_add_sync(0xffffffffu, drop);
-  }
-  // First vertex v of the connected set C with td(C - v) = td(C) - 1, i.e.
-  // the first argmin of td(C - v) (td(C) = 1 + min_v td(C - v) for a
-  // connected C): one round of table reads, no read of td(C) itself. The
-  // values are a and possibly a + 1, so residue a is the one present whose
-  // predecessor is absent. -1 on three residues (a corrupt table).
-  __device__ int root(uint64_t C) const {
-    if (__popcll(C) == 1)
-      return __ffsll(static_cast<long long>(C)) - 1;
-    const int lane = threadIdx.x & 31;
-    const bool in_lo = (C >> lane) & 1ull;
-    const bool in_hi = lane + 32 < n && ((C >> (lane + 32)) & 1ull);
-    const uint32_t t_lo = in_lo ? residue(C & ~(1ull << lane)) : 3u;
-    const uint32_t t_hi = in_hi ? residue(C & ~(1ull << (lane + 32))) : 3u;
-    const uint32_t have = __reduce_or_sync(0xffffffffu, (1u << t_lo) | (1u << t_hi)) & 7u;
-    const uint32_t m = (have & 5u) == 5u ? 2u : (have & 1u) ? 0u : (have & 2u) ? 1u : 2u;
-    const uint64_t hits = ballot64(in_lo && t_lo == m, in_hi && t_hi == m);
-    return have != 7u && hits ? __ffsll(static_cast<long long>(hits)) - 1 : -1;
-  }
 };
+
+// First tiles of the levels of a graph with nh high vertices (whole warp).
+__device__ __forceinline__ void level_offsets(const Binom& binom, int nh, uint32_t* off) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t own = lane <= nh ? binom[nh][lane] : 0u;
+  uint32_t cum = own;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t x = __shfl_up_sync(0xffffffffu, cum, d);
+    if (lane >= d)
+      cum += x;
+  }
+  off[lane] = cum - own;
+  __syncwarp();
+}
+
+// Residues of the chain S & {v, v + 1, ...}, v = lane and lane + 32 (0 .. n),
+// and from them td(S): each deletion lowers the treedepth by 0 or 1, which the
+// residues tell. (Two parts, so that the loads can be on their way meanwhile.)
+struct Chain {
+  uint32_t lo, hi;
+};
+template <class Ctx>
+__device__ __forceinline__ Chain load_chain(const Ctx& ctx, uint64_t S) {
+  const int lane = threadIdx.x & 31;
+  return Chain{lane <= ctx.n ? ctx.residue(S & (~0ull << lane)) : 0u,
+               lane + 32 <= ctx.n ? ctx.residue(S & (~0ull << (lane + 32))) : 0u};
+}
+__device__ __forceinline__ uint32_t chain_td(const Chain& c, int n) {
+  const int lane = threadIdx.x & 31;
+  uint32_t next_lo = __shfl_down_sync(0xffffffffu, c.lo, 1);
+  const uint32_t first_hi = __shfl_sync(0xffffffffu, c.hi, 0), next_hi = __shfl_down_sync(0xffffffffu, c.hi, 1);
+  if (lane == 31)
+    next_lo = first_hi;
+  return __reduce_add_sync(0xffffffffu, (lane < n && c.lo != next_lo ? 1u : 0u) +
+                                            (lane + 32 < n && c.hi != next_hi ? 1u : 0u));
+}
+
+// Shared memory of one warp's reconstruction.
+struct TreeMem {
+  uint64_t set[2][kDpMaxN];       // components of the depth in work and of the next
+  unsigned long long kids[kDpMaxN];  // children of each vertex
+  int32_t owner[2][kDpMaxN];
+  int32_t par[kDpMaxN];           // the canonical tree
+  int32_t dep[kDpMaxN];           // depth of each vertex in it
+  uint32_t hgt[kDpMaxN];          // subtree height (in vertices)
+  uint32_t low[kDpMaxN];          // 255 - the subtree's lowest vertex
+  uint8_t comp[64];               // component of each vertex, of the depth in work
+  uint32_t off[32];
+};
+
+// The canonical tree of `query` and what p asks of it (whole warp): every
+// component is rooted at the first vertex v with td(C - v) = td(C) - 1 and its
+// sub-components hang below that root (dynamic_cpu.hpp:59-81). All components
+// of a depth are taken together: their vertices are disjoint, so one round of
+// loads, lane v reading C(v) - v, finds every root of the depth. The time is
+// the depth of the tree times one load's latency and the component searches
+// (n = 30: 61 us when each component took a round of its own).
+template <class Ctx>
+__device__ bool build_tree(const DpBatchParams& p, const DpGraph& G, const Ctx& ctx, TreeMem& m, uint64_t query) {
+  const int lane = threadIdx.x & 31, n = G.n;
+  const uint64_t adj_lo = lane < n ? __ldg(p.adj + G.adj_off + lane) : 0ull;
+  const uint64_t adj_hi = lane + 32 < n ? __ldg(p.adj + G.adj_off + lane + 32) : 0ull;
+  const Chain chain = load_chain(ctx, query);
+  int height = 0, count = 0;      // count: components of the next depth
+  uint64_t in_next = 0;           // their union
+  // The components of `rest`, below `owner` at depth d: single vertices are
+  // done, the others join list `to`.
+  const bool wide = n > 32;
+  auto split = [&](uint64_t rest, int owner, int d, int to) {
+    if (rest)
+      height = max(height, d);
+    // the vertices without a neighbour left, all at once
+    const bool one_lo = ((rest >> lane) & 1ull) && (adj_lo & rest) == 0ull;
+    const bool one_hi = ((rest >> (lane + 32)) & 1ull) && (adj_hi & rest) == 0ull;
+    if (one_lo) {
+      m.par[lane] = owner;
+      m.dep[lane] = d;
+    }
+    if (one_hi) {
+      m.par[lane + 32] = owner;
+      m.dep[lane + 32] = d;
+    }
+    rest &= ~ballot64(one_lo, one_hi);
+    while (rest) {
+      uint64_t reach = rest & (0ull - rest), frontier = reach;
+      if (!wide) {
+        uint32_t r32 = static_cast<uint32_t>(reach), f32 = r32;
+        while (f32) {
+          const uint32_t nb = ((f32 >> lane) & 1u) ? static_cast<uint32_t>(adj_lo) : 0u;
+          f32 = __reduce_or_sync(0xffffffffu, nb) & static_cast<uint32_t>(rest) & ~r32;
+          r32 |= f32;
+        }
+        reach = r32;
+        frontier = 0ull;
+      }
+      while (frontier) {
+        const uint64_t nb = (((frontier >> lane) & 1ull) ? adj_lo : 0ull) |
+                            (((frontier >> (lane + 32)) & 1ull) ? adj_hi : 0ull);
+        frontier = warp_or64(nb) & rest & ~reach;
+        reach |= frontier;
+      }
+      rest &= ~reach;
+      if (lane == 0) {
+        m.set[to][count] = reach;
+        m.owner[to][count] = owner;
+      }
+      if ((reach >> lane) & 1ull)
+        m.comp[lane] = static_cast<uint8_t>(count);
+      if ((reach >> (lane + 32)) & 1ull)
+        m.comp[lane + 32] = static_cast<uint8_t>(count);
+      in_next |= reach;
+      ++count;
+    }
+  };
+  split(query, -1, 1, 0);
+  for (int depth = 1, cur = 0; count > 0; ++depth, cur ^= 1) {
+    __syncwarp();
+    const bool in_lo = (in_next >> lane) & 1ull, in_hi = (in_next >> (lane + 32)) & 1ull;
+    const uint32_t t_lo = in_lo ? ctx.residue(m.set[cur][m.comp[lane]] & ~(1ull << lane)) : 0u;
+    const uint32_t t_hi = in_hi ? ctx.residue(m.set[cur][m.comp[lane + 32]] & ~(1ull << (lane + 32))) : 0u;
+    const int here = count;
+    count = 0;
+    in_next = 0;
+    __syncwarp();  // comp[] read above, rewritten by split
+    for (int i = 0; i < here; ++i) {
+      const uint64_t C = m.set[cur][i];
+      const bool c_lo = (C >> lane) & 1ull, c_hi = (C >> (lane + 32)) & 1ull;
+      // td(C - v) over v in C is a and possibly a + 1: residue a is the one
+      // present whose predecessor is absent (three: a corrupt table)
+      const uint32_t have = __reduce_or_sync(0xffffffffu, (c_lo ? 1u << t_lo : 0u) | (c_hi ? 1u << t_hi : 0u));
+      const uint32_t a = (have & 5u) == 5u ? 2u : (have & 1u) ? 0u : (have & 2u) ? 1u : 2u;
+      const uint64_t hits = ballot64(c_lo && t_lo == a, c_hi && t_hi == a);
+      if (have == 7u || hits == 0ull)
+        return false;
+      const int root = __ffsll(static_cast<long long>(hits)) - 1, owner = m.owner[cur][i];
+      if (lane == 0) {
+        m.par[root] = owner;
+        m.dep[root] = depth;
+      }
+      split(C & ~(1ull << root), root, depth + 1, cur ^ 1);
+    }
+  }
+  __syncwarp();
+  const uint32_t td = chain_td(chain, n);
+  if (lane == 0 && p.td_out)
+    p.td_out[G.out_idx] = static_cast<int32_t>(td);
+  if (static_cast<uint32_t>(height) != td)
+    return false;
+  if (p.parent_out) {
+    int32_t* parent = p.parent_out + G.adj_off;
+    for (int v = lane; v < n; v += 32)
+      if ((query >> v) & 1ull)
+        parent[v] = m.par[v];
+  }
+
+  if (p.order_out) {
+    // GetElimination (dynamic_gpu.hpp:58-63): repeatedly remove the stored
+    // root of the remaining set; for a disconnected set that is the root of
+    // its first deepest component, components taken in order of their
+    // lowest vertex (dynamic_gpu.cu:92-103). The components of the
+    // remaining set are subtrees of the canonical tree and a component's
+    // treedepth is its subtree's height, so the order is read off the tree:
+    // the active subtree of greatest height, ties to the lowest vertex,
+    // gives its root and is replaced by its children's subtrees.
+    for (int v = lane; v < n; v += 32) {
+      m.hgt[v] = 0u;  // the tallest child so far
+      m.low[v] = 255u - static_cast<uint32_t>(v);
+      m.kids[v] = 0ull;
+    }
+    __syncwarp();
+    for (int d = height; d >= 1; --d) {  // deepest first: children before parents
+      for (int v = lane; v < n; v += 32) {
+        if (((query >> v) & 1ull) && m.dep[v] == d) {
+          const uint32_t h = m.hgt[v] + 1u;  // own height = tallest child + 1
+          m.hgt[v] = h;
+          const int pv = m.par[v];
+          if (pv >= 0) {
+            atomicMax(&m.hgt[pv], h);
+            atomicMax(&m.low[pv], m.low[v]);
+            atomicOr(&m.kids[pv], 1ull << v);
+          }
+        }
+      }
+      __syncwarp();
+    }
+    int32_t* order = p.order_out + G.adj_off;
+    uint64_t active = 0;
+    for (int v = lane; v < n; v += 32)
+      if (((query >> v) & 1ull) && m.par[v] < 0)
+        active |= 1ull << v;
+    active = warp_or64(active);
+    // key: height << 8 | 255 - lowest vertex (unique: the subtrees are disjoint)
+    const uint32_t key_lo = lane < n ? m.hgt[lane] << 8 | m.low[lane] : 0u;
+    const uint32_t key_hi = lane + 32 < n ? m.hgt[lane + 32] << 8 | m.low[lane + 32] : 0u;
+    for (int step = 0; active; ++step) {
+      const uint32_t k_lo = ((active >> lane) & 1ull) ? key_lo : 0u;
+      const uint32_t k_hi = ((active >> (lane + 32)) & 1ull) ? key_hi : 0u;
+      const uint32_t best = __reduce_max_sync(0xffffffffu, max(k_lo, k_hi));
+      const uint64_t hit = ballot64(k_lo == best && k_lo != 0u, k_hi == best && k_hi != 0u);
+      const int v = __ffsll(static_cast<long long>(hit)) - 1;
+      if (lane == 0)
+        order[step] = v;
+      active = (active & ~(1ull << v)) | m.kids[v];
+    }
+  }
+  return true;
+}
 
 __global__ void __launch_bounds__(32 * kTreeWarps)
     dp_tree_kernel(const __grid_constant__ DpBatchParams p) {
-  __shared__ uint64_t sAdjAll[kTreeWarps][kDpMaxN];
-  __shared__ uint64_t stMaskAll[kTreeWarps][kDpMaxN];
-  __shared__ int32_t stOwnerAll[kTreeWarps][kDpMaxN];
-  __shared__ int32_t stDepthAll[kTreeWarps][kDpMaxN];
-  __shared__ int32_t sParAll[kTreeWarps][kDpMaxN];     // the canonical tree
-  __shared__ int32_t sDepAll[kTreeWarps][kDpMaxN];     // depth of each vertex in it
-  __shared__ uint32_t sHgtAll[kTreeWarps][kDpMaxN];    // subtree height (in vertices)
-  __shared__ uint32_t sLowAll[kTreeWarps][kDpMaxN];    // 255 - the subtree's lowest vertex
-  __shared__ unsigned long long sKidsAll[kTreeWarps][kDpMaxN];  // children of each vertex
-  // The binomial table in shared memory: every lane ranks a different subset,
-  // which the parameter bank would serve one address at a time.
   __shared__ Binom sBinom;
-  for (int i = threadIdx.x; i < (kDpMaxHigh + 1) * (kDpMaxHigh + 1); i += blockDim.x)
-    (&sBinom[0][0])[i] = (&p.binom[0][0])[i];
+  __shared__ TreeMem mem[kTreeWarps];
+  fill_binom(sBinom);
   __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint64_t* sAdj = sAdjAll[warp];
-  uint64_t* stMask = stMaskAll[warp];
-  int32_t* stOwner = stOwnerAll[warp];
-  int32_t* stDepth = stDepthAll[warp];
+  const int warp = threadIdx.x >> 5;
   if (ld_relaxed_s32(p.error) != 0)
     return;
-
   for (int g = blockIdx.x * kTreeWarps + warp; g < p.num_graphs; g += gridDim.x * kTreeWarps) {
     const DpGraph G = p.graphs ? p.graphs[g] : p.single;
-    const int n = G.n;
-    for (int v = lane; v < n; v += 32)
-      sAdj[v] = p.adj[G.adj_off + v];
-    __syncwarp();
-    const TreeCtx ctx{sBinom, p.table + G.table_off, G.lb, G.nh, n};
-    const uint64_t query = p.query ? p.query : (n == 64 ? ~0ull : ((1ull << n) - 1));
-    const uint32_t td = query ? ctx.td_of(query) : 0u;
-    if (lane == 0 && p.td_out)
-      p.td_out[G.out_idx] = static_cast<int32_t>(td);
-
-    // Canonical tree of the query set: every component is rooted at
-    // ctx.root and its sub-components hang below that root
-    // (dynamic_cpu.hpp:59-81); kept in shared memory for the order below.
-    int32_t* sPar = sParAll[warp];
-    int32_t* sDep = sDepAll[warp];
-    int top = 0, height = 0;
-    for (uint64_t rest = query; rest;) {
-      const uint64_t c = warp_component(rest, __ffsll(static_cast<long long>(rest)) - 1, sAdj, n);
-      rest &= ~c;
-      if (lane == 0) {
-        stMask[top] = c;
-        stOwner[top] = -1;
-        stDepth[top] = 1;
-      }
-      ++top;
-    }
-    __syncwarp();
-    while (top > 0) {
-      --top;
-      const uint64_t C = stMask[top];
-      const int owner = stOwner[top], depth = stDepth[top];
-      __syncwarp();
-      const int r = ctx.root(C);
-      if (r < 0) {
-        if (lane == 0)
-          raise_error(p.error, kDevNoRoot, g);
-        return;
-      }
-      if (lane == 0) {
-        sPar[r] = owner;
-        sDep[r] = depth;
-      }
-      height = max(height, depth);
-      for (uint64_t rest = C & ~(1ull << r); rest;) {
-        const uint64_t c = warp_component(rest, __ffsll(static_cast<long long>(rest)) - 1, sAdj, n);
-        rest &= ~c;
-        if (lane == 0) {
-          stMask[top] = c;
-          stOwner[top] = r;
-          stDepth[top] = depth + 1;
-        }
-        ++top;
-      }
-      __syncwarp();
-    }
-    if (static_cast<uint32_t>(height) != td) {
-      if (lane == 0)
+    level_offsets(sBinom, G.nh, mem[warp].off);
+    const TreeCtx ctx{sBinom, mem[warp].off, p.table + G.table_off, G.lb, G.n};
+    if (!build_tree(p, G, ctx, mem[warp], p.query ? p.query : (1ull << G.n) - 1ull)) {
+      if ((threadIdx.x & 31) == 0)
         raise_error(p.error, kDevNoRoot, g);
       return;
-    }
-    if (p.parent_out) {
-      int32_t* parent = p.parent_out + G.adj_off;
-      for (int v = lane; v < n; v += 32)
-        if ((query >> v) & 1ull)
-          parent[v] = sPar[v];
-    }
-
-    if (p.order_out) {
-      // GetElimination (dynamic_gpu.hpp:58-63): repeatedly remove the stored
-      // root of the remaining set; for a disconnected set that is the root of
-      // its first deepest component, components taken in order of their
-      // lowest vertex (dynamic_gpu.cu:92-103). The components of the
-      // remaining set are subtrees of the canonical tree and a component's
-      // treedepth is its subtree's height, so the order is read off the tree:
-      // the active subtree of greatest height, ties to the lowest vertex,
-      // gives its root and is replaced by its children's subtrees.
-      uint32_t* sHgt = sHgtAll[warp];
-      uint32_t* sLow = sLowAll[warp];
-      unsigned long long* sKids = sKidsAll[warp];
-      for (int v = lane; v < n; v += 32) {
-        sHgt[v] = 0u;  // the tallest child so far
-        sLow[v] = 255u - static_cast<uint32_t>(v);
-        sKids[v] = 0ull;
-      }
-      __syncwarp();
-      for (int d = height; d >= 1; --d) {  // deepest first: children before parents
-        for (int v = lane; v < n; v += 32) {
-          if (((query >> v) & 1ull) && sDep[v] == d) {
-            const uint32_t h = sHgt[v] + 1u;  // own height = tallest child + 1
-            sHgt[v] = h;
-            const int pv = sPar[v];
-            if (pv >= 0) {
-              atomicMax(&sHgt[pv], h);
-              atomicMax(&sLow[pv], sLow[v]);
-              atomicOr(&sKids[pv], 1ull << v);
-            }
-          }
-        }
-        __syncwarp();
-      }
-      int32_t* order = p.order_out + G.adj_off;
-      uint64_t active = 0;
-      for (int v = lane; v < n; v += 32)
-        if (((query >> v) & 1ull) && sPar[v] < 0)
-          active |= 1ull << v;
-      active = warp_or64(active);
-      for (int step = 0; active; ++step) {
-        // key: height << 8 | 255 - lowest vertex (unique: the subtrees are disjoint)
-        const uint32_t k_lo = ((active >> lane) & 1ull) ? (sHgt[lane] << 8 | sLow[lane]) : 0u;
-        const uint32_t k_hi = (lane + 32 < n && ((active >> (lane + 32)) & 1ull))
-                                  ? (sHgt[lane + 32] << 8 | sLow[lane + 32]) : 0u;
-        const uint32_t m = __reduce_max_sync(0xffffffffu, max(k_lo, k_hi));
-        const uint64_t hit = ballot64(k_lo == m && k_lo != 0u, k_hi == m && k_hi != 0u);
-        const int a = __ffsll(static_cast<long long>(hit)) - 1;
-        if (lane == 0)
-          order[step] = a;
-        active = (active & ~(1ull << a)) | sKids[a];
-      }
     }
     __syncwarp();
   }
@@ -1076,16 +1124,6 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
 // ---------------------------------------------------------------------------
 // Host-side launch helpers.
 // ---------------------------------------------------------------------------
-
-void dp_fill_binom(DpBatchParams& p) {
-  for (int a = 0; a <= kDpMaxHigh; ++a) {
-    for (int b = 0; b <= kDpMaxHigh; ++b)
-      p.binom[a][b] = 0;
-    p.binom[a][0] = 1;
-    for (int b = 1; b <= a; ++b)
-      p.binom[a][b] = p.binom[a - 1][b - 1] + (b <= a - 1 ? p.binom[a - 1][b] : 0u);
-  }
-}
 
 template <int LB>
 static cudaError_t launch_tiles(const DpBatchParams& p, int ctas, cudaStream_t s) {
@@ -1175,13 +1213,16 @@ cudaError_t dp_launch_tree(const DpBatchParams& p, cudaStream_t s) {
 __global__ void __launch_bounds__(32 * kTreeWarps)
     dp_labels_kernel(const __grid_constant__ DpBatchParams p, const uint64_t* subsets, int count, int32_t* td_out,
                      uint64_t* roots_out) {
-  __shared__ Binom sBinom;  // lanes rank different subsets: shared memory, not the parameter bank
-  for (int i = threadIdx.x; i < (kDpMaxHigh + 1) * (kDpMaxHigh + 1); i += blockDim.x)
-    (&sBinom[0][0])[i] = (&p.binom[0][0])[i];
+  __shared__ Binom sBinom;
+  fill_binom(sBinom);
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const DpGraph G = p.single;
-  const TreeCtx ctx{sBinom, p.table + G.table_off, G.lb, G.nh, G.n};
+  __shared__ uint32_t sOff[32];
+  if (warp == 0)
+    level_offsets(sBinom, G.nh, sOff);
+  __syncthreads();
+  const TreeCtx ctx{sBinom, sOff, p.table + G.table_off, G.lb, G.n};
   for (int i = blockIdx.x * kTreeWarps + warp; i < count; i += gridDim.x * kTreeWarps) {
     const uint64_t S = subsets[i];
     if (S == 0) {
@@ -1191,12 +1232,12 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
       }
       continue;
     }
-    const uint32_t td = ctx.td_of(S), below = (td + 2u) % 3u;  // residue of td - 1
-    bool lo = false, hi = false;
-    if ((S >> lane) & 1ull)
-      lo = ctx.residue(S & ~(1ull << lane)) == below;
-    if (lane + 32 < G.n && ((S >> (lane + 32)) & 1ull))
-      hi = ctx.residue(S & ~(1ull << (lane + 32))) == below;
+    const Chain chain = load_chain(ctx, S);
+    const bool in_lo = (S >> lane) & 1ull, in_hi = (S >> (lane + 32)) & 1ull;
+    const uint32_t t_lo = in_lo ? ctx.residue(S & ~(1ull << lane)) : 3u;
+    const uint32_t t_hi = in_hi ? ctx.residue(S & ~(1ull << (lane + 32))) : 3u;
+    const uint32_t td = chain_td(chain, G.n), below = (td + 2u) % 3u;  // residue of td - 1
+    const bool lo = t_lo == below, hi = t_hi == below;
     const uint64_t roots = ballot64(lo, hi);
     if (lane == 0) {
       td_out[i] = static_cast<int32_t>(td);
@@ -1223,12 +1264,15 @@ cudaError_t dp_launch_labels(const DpBatchParams& p, const uint64_t* subsets, in
 __global__ void __launch_bounds__(32 * kTreeWarps)
     dp_expand_kernel(const __grid_constant__ DpBatchParams p, int lb, uint32_t tiles, uint8_t* out, uint64_t bytes) {
   __shared__ Binom sBinom;
-  for (int i = threadIdx.x; i < (kDpMaxHigh + 1) * (kDpMaxHigh + 1); i += blockDim.x)
-    (&sBinom[0][0])[i] = (&p.binom[0][0])[i];
+  fill_binom(sBinom);
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const DpGraph G = p.single;
-  const TreeCtx ctx{sBinom, p.table + G.table_off, G.lb, G.nh, G.n};
+  __shared__ uint32_t sOff[32];
+  if (warp == 0)
+    level_offsets(sBinom, G.nh, sOff);
+  __syncthreads();
+  const TreeCtx ctx{sBinom, sOff, p.table + G.table_off, G.lb, G.n};
   const int nh = G.n > lb ? G.n - lb : 0;
   const uint32_t words = lb > 5 ? 1u << (lb - 5) : 1u;
   for (uint32_t t = blockIdx.x * kTreeWarps + warp; t < tiles; t += gridDim.x * kTreeWarps) {
@@ -1242,7 +1286,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
         H |= 1u << a;
       }
     const uint64_t high = static_cast<uint64_t>(H) << lb;
-    const uint32_t base = ctx.td_of(high);
+    const uint32_t base = chain_td(load_chain(ctx, high), G.n);
     auto first = [&](uint32_t w) { return ctx.residue(high | (static_cast<uint64_t>(w) << 5)); };
     for (uint32_t w = lane; w < words; w += 32) {
       uint32_t td[32];

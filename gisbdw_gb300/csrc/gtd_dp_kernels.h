@@ -23,10 +23,8 @@ struct DpGraph {
   int32_t lb = 0;          // tile bits of this graph's table
 };
 
-// Passed by value as a __grid_constant__ kernel parameter: the binomial
-// table is read through the constant cache.
+// Passed by value as a __grid_constant__ kernel parameter.
 struct DpBatchParams {
-  uint32_t binom[kDpMaxHigh + 1][kDpMaxHigh + 1] = {};  // C(a, b)
   const DpGraph* graphs = nullptr;  // device descriptors; nullptr: only `single`
   DpGraph single;
   uint2* tile_map = nullptr;        // ticket -> (graph, its tile group) (batches)
@@ -52,7 +50,6 @@ struct DpBatchParams {
   int32_t* order_out = nullptr;
 };
 
-void dp_fill_binom(DpBatchParams& p);
 // CTAs per SM with tiles of lb bits and up to kid_rows high vertices, and of
 // the mixed-tile-size kernel with tiles of up to lb bits.
 int dp_tile_occupancy(int lb, int kid_rows);

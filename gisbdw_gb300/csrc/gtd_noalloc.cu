@@ -95,7 +95,6 @@ extern "C" gtd_status gtd_dp_solve_noalloc(const uint64_t* d_adj, int n, int32_t
   if (L.ntiles > kNoallocMaxTiles)
     return GTD_INVALID_ARG;
   DpBatchParams p;
-  dp_fill_binom(p);
   p.single.ntiles = L.ntiles;
   p.single.n = n;
   p.single.nh = L.nh;
