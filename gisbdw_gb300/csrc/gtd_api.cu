@@ -139,8 +139,8 @@ namespace {
 // and 803 with 12; n = 33: 4.68 ms against 5.14 and 5.23).
 int default_tile_bits(int n) { return n >= 26 ? 11 : 10; }
 
-// Up to this n the level kernel solves a graph, unless the caller gives tile
-// bits (level / 11-bit tile kernel: n = 12 20 / 24 us, 16 31 / 56, 20 45 / 117,
+// Up to this n the level kernel solves a graph (up to kDpSmallMaxN the small
+// kernel), unless the caller gives tile bits (level / 11-bit tile kernel: n = 12 20 / 24 us, 16 31 / 56, 20 45 / 117,
 // 25 112 / 234, 27 176 / 299, 28 264 / 344, 29 436 / 436, 30 806 / 690).
 constexpr int kLevelMaxN = 28;
 
@@ -151,9 +151,12 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, int n, const gtd_dp_o
                       int32_t* d_td, int32_t* d_parent, int32_t* d_order) {
   const int tile_bits = (opts && opts->tile_bits > 0) ? opts->tile_bits : default_tile_bits(n);
   const DpLayout L = make_dp_layout(n, tile_bits);
-  const bool by_level = !(opts && opts->tile_bits > 0) && n <= kLevelMaxN;
+  const bool stall = take_stall_fault();  // test injection: needs a kernel whose tiles wait
+  const bool given_bits = opts && opts->tile_bits > 0;
+  const bool small = !given_bits && !stall && n <= kDpSmallMaxN;
+  const bool by_level = !given_bits && !small && n <= kLevelMaxN;
   // the planes' tiles: n < lb is padded to one tile
-  const int lb = by_level ? kDpLevelTileBits : L.lb < kDpMinTileBits ? kDpMinTileBits : L.lb;
+  const int lb = small ? kDpSmallTileBits : by_level ? kDpLevelTileBits : L.lb < kDpMinTileBits ? kDpMinTileBits : L.lb;
   const int nh = n > lb ? n - lb : 0;
   const uint32_t ntiles = 1u << nh;
   const size_t table_bytes = size_t(1) << n;
@@ -197,7 +200,7 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, int n, const gtd_dp_o
 
   p.kid_rows = nh;
   int& dp_occ = h->dp_occ[by_level ? 0 : p.lb][nh];
-  if (dp_occ <= 0)
+  if (dp_occ <= 0 && !small)
     dp_occ = by_level ? dp_level_occupancy(nh) : dp_tile_occupancy(p.lb, nh);
   int occ = dp_occ;
   if (opts && opts->ctas_per_sm > 0 && opts->ctas_per_sm < occ)
@@ -205,20 +208,23 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, int n, const gtd_dp_o
   if (occ < 1)
     occ = 1;
   long long ctas = static_cast<long long>(h->num_sms) * occ;
-  if (ctas > p.total_groups)
-    ctas = p.total_groups;
+  if (ctas > p.total_groups || small)
+    ctas = small ? 1 : p.total_groups;
 
   GTD_CUDA(h, cudaMemsetAsync(h->d_io, 0, kIoWords * sizeof(int32_t), h->stream));
   if (take_poison_fault())  // test injection: every byte must be written before it is read
     GTD_CUDA(h, cudaMemsetAsync(h->d_table, 0xFF, h->table_cap, h->stream));
-  if (take_stall_fault())  // test injection: ticket 0 (the level-0 group) is never taken
+  if (stall)  // ticket 0 (the level-0 group) is never taken
     GTD_CUDA(h, cudaMemsetAsync(h->d_io + kIoTicket, 1, 1, h->stream));
-  GTD_CUDA(h, dp_launch_validate(p, h->stream));
+  if (!small)
+    GTD_CUDA(h, dp_launch_validate(p, h->stream));
   GTD_CUDA(h, cudaEventRecord(h->ev[0], h->stream));
-  GTD_CUDA(h, by_level ? dp_launch_levels(p, static_cast<int>(ctas), h->stream)
-                       : dp_launch_tiles(p, static_cast<int>(ctas), h->stream));
+  GTD_CUDA(h, small      ? dp_launch_small(p, n, h->stream)
+              : by_level ? dp_launch_levels(p, static_cast<int>(ctas), h->stream)
+                         : dp_launch_tiles(p, static_cast<int>(ctas), h->stream));
   GTD_CUDA(h, cudaEventRecord(h->ev[1], h->stream));
-  GTD_CUDA(h, dp_launch_tree(p, h->stream));
+  if (!small)  // the small kernel builds the tree itself
+    GTD_CUDA(h, dp_launch_tree(p, h->stream));
   GTD_CUDA(h, cudaEventRecord(h->ev[2], h->stream));
 
   h->last_params = p;

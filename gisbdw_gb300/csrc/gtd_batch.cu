@@ -1,6 +1,8 @@
 // Batched subset DP: many graphs of uneven size in one persistent launch.
 //
-// Planning (host): graphs are put in descending n, each gets a table region,
+// Planning (host): graphs are put in descending n; those of at most
+// kBatchSmallMaxN vertices are solved one CTA each, with no table; the others
+// go through the tile kernel. Of these each gets a table region,
 // a flag range and a descriptor. Tickets run level-major across graphs
 // (level 0 of every graph, then level 1, ...), so the children a tile waits
 // for were issued long before it; the ticket -> (graph, tile) map is filled
@@ -35,6 +37,7 @@ struct Plan {
   uint32_t total_tiles = 0;
   uint32_t total_groups = 0;    // tickets
   int kid_rows = 0;             // largest nh
+  int small = 0;                // graphs at the end of `graphs` that the small kernel takes (no tiles)
   uint64_t plane_bytes = 0;     // the pool itself; table_bytes counts one byte per padded subset
   uint64_t subsets = 0;
   uint64_t alg_bytes = 0;
@@ -42,6 +45,12 @@ struct Plan {
 };
 
 constexpr int kLevelSlots = kDpMaxHigh + 2;
+
+// Graphs of a batch that the small kernel takes, one CTA each, unless the
+// caller gives tile bits (2048 graphs of 15 vertices: 68 us against 265 in the
+// tile kernel, of 16: 111 against 306; from 17 on the widest level has seven
+// words per thread of the CTA and shared memory holds fewer CTAs).
+constexpr int kBatchSmallMaxN = 16;
 
 // Tile bits per vertex count. An explicit opts->tile_bits gives every graph
 // that size. Otherwise, when the autotuner has rates (subsets per us of the
@@ -140,7 +149,7 @@ void pick_tile_bits(gtd_handle h, const gtd_graph_desc* descs, int count, const 
   }
 }
 
-void make_plan(Plan& P, const gtd_graph_desc* descs, int count) {
+void make_plan(Plan& P, const gtd_graph_desc* descs, int count, bool small_kernel) {
   std::vector<int> order(count);
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return descs[a].n > descs[b].n; });
@@ -165,11 +174,15 @@ void make_plan(Plan& P, const gtd_graph_desc* descs, int count) {
     G.flag_base = group;
     G.adj_off = static_cast<uint32_t>(d.offset);
     G.out_idx = order[k];
-    off += uint64_t(G.ntiles) * dp_tile_bytes(lb);
     P.table_bytes += uint64_t(G.ntiles) << lb;
     tile += G.ntiles;
-    group += dp_groups(binom, G.nh, dp_group_tiles(lb));
-    P.kid_rows = std::max(P.kid_rows, G.nh);
+    if (small_kernel && d.n <= kBatchSmallMaxN) {
+      ++P.small;
+    } else {
+      off += uint64_t(G.ntiles) * dp_tile_bytes(lb);
+      group += dp_groups(binom, G.nh, dp_group_tiles(lb));
+      P.kid_rows = std::max(P.kid_rows, G.nh);
+    }
     const uint64_t sub = uint64_t(1) << d.n;
     P.subsets += sub;
     P.alg_bytes += sub + uint64_t(d.n) * (sub / 2);
@@ -181,7 +194,7 @@ void make_plan(Plan& P, const gtd_graph_desc* descs, int count) {
   P.level_base.assign(size_t(count) * kLevelSlots, 0);
   uint32_t ticket = 0;
   for (int j = 0; j <= kDpMaxHigh; ++j)
-    for (int k = 0; k < count; ++k) {
+    for (int k = 0; k < count - P.small; ++k) {
       const DpGraph& G = P.graphs[k];
       if (j <= G.nh) {
         P.level_base[size_t(k) * kLevelSlots + j] = ticket;
@@ -198,6 +211,7 @@ uint64_t fingerprint(const Plan& P, const void* adj, const void* td, const void*
   };
   mix(P.lb);
   mix(P.mixed);
+  mix(P.small);
   mix(P.graphs.size());
   for (const DpGraph& G : P.graphs) {
     mix(G.n);
@@ -232,7 +246,7 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
                          int32_t* d_td, int32_t* d_parent, const gtd_dp_batch_opts* opts, int force_cap = 0) {
   Plan P;
   pick_tile_bits(h, descs, count, opts, P, force_cap);
-  make_plan(P, descs, count);
+  make_plan(P, descs, count, !(opts && opts->tile_bits > 0) && force_cap == 0);
   const int lb = P.lb;
   const uint64_t timeout = (opts && opts->timeout_ns) ? opts->timeout_ns : 10ull * 1000 * 1000 * 1000;
   int occ = P.mixed ? dp_mixed_occupancy(lb, P.kid_rows) : dp_tile_occupancy(lb, P.kid_rows);
@@ -307,7 +321,7 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
   bp.graphs = h->d_bgraphs;
   bp.tile_map = h->d_tile_map;
   bp.level_base = h->d_level_base;
-  bp.num_graphs = count;
+  bp.num_graphs = count - P.small;
   bp.lb = lb;
   bp.mixed = P.mixed ? 1 : 0;
   bp.kid_rows = P.kid_rows;
@@ -320,7 +334,26 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
   bp.timeout_ns = timeout;
   bp.td_out = d_td;
   bp.parent_out = d_parent;
-  GTD_CUDA(h, dp_launch_fill_tile_map(bp, h->stream));
+  if (bp.num_graphs > 0)
+    GTD_CUDA(h, dp_launch_fill_tile_map(bp, h->stream));
+  const auto launch = [&]() -> cudaError_t {
+    cudaError_t e = cudaSuccess;
+    if (bp.num_graphs > 0) {
+      e = dp_launch_validate(bp, h->stream);
+      if (e == cudaSuccess)
+        e = dp_launch_tiles(bp, static_cast<int>(ctas), h->stream);
+      if (e == cudaSuccess)
+        e = dp_launch_tree(bp, h->stream);
+    }
+    if (e == cudaSuccess && P.small > 0) {
+      DpBatchParams sp = bp;
+      sp.first_graph = bp.num_graphs;
+      sp.num_graphs = P.small;
+      sp.table = nullptr;
+      e = dp_launch_small(sp, P.graphs[bp.num_graphs].n, h->stream);
+    }
+    return e;
+  };
   if (poison)
     GTD_CUDA(h, cudaMemsetAsync(h->d_table, 0xFF, P.plane_bytes, h->stream));
 
@@ -336,11 +369,7 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
     if (ce == cudaSuccess)
       ce = cudaMemsetAsync(h->d_io, 0, 4 * sizeof(int32_t), h->stream);
     if (ce == cudaSuccess)
-      ce = dp_launch_validate(bp, h->stream);
-    if (ce == cudaSuccess)
-      ce = dp_launch_tiles(bp, static_cast<int>(ctas), h->stream);
-    if (ce == cudaSuccess)
-      ce = dp_launch_tree(bp, h->stream);
+      ce = launch();
     cudaError_t ee = cudaStreamEndCapture(h->stream, &graph);
     if (ce == cudaSuccess)
       ce = ee;
@@ -360,9 +389,7 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
       return s;
     GTD_CUDA(h, cudaMemsetAsync(h->d_io, 0, 4 * sizeof(int32_t), h->stream));
     GTD_CUDA(h, cudaEventRecord(h->ev[0], h->stream));
-    GTD_CUDA(h, dp_launch_validate(bp, h->stream));
-    GTD_CUDA(h, dp_launch_tiles(bp, static_cast<int>(ctas), h->stream));
-    GTD_CUDA(h, dp_launch_tree(bp, h->stream));
+    GTD_CUDA(h, launch());
     GTD_CUDA(h, cudaEventRecord(h->ev[1], h->stream));
   }
   return GTD_OK;

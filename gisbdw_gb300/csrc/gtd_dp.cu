@@ -264,19 +264,12 @@ __device__ __forceinline__ uint32_t rank_colex(const Binom& binom, uint32_t H) {
   return r;
 }
 
-// Checks each graph's adjacency masks — no self loop, no bit >= n,
-// symmetric — one warp per graph, lane v checking vertex v (and v + 32).
-__global__ void dp_validate_kernel(const __grid_constant__ DpBatchParams p) {
-  const int lane = threadIdx.x & 31;
-  const int g = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (g >= p.num_graphs)
-    return;  // the whole warp
-  const DpGraph G = p.graphs ? p.graphs[g] : p.single;
-  const uint64_t* adj = p.adj + G.adj_off;
-  const int n = G.n;
+// Are a graph's adjacency masks well formed — no self loop, no bit >= n,
+// symmetric? Whole warp, lane v checking vertex v (and v + 32).
+__device__ __forceinline__ bool adjacency_ok(const uint64_t* adj, int n) {
   const uint64_t allowed = n >= 64 ? ~0ull : ((1ull << n) - 1);
   bool ok = true;
-  for (int v = lane; v < n && ok; v += 32) {
+  for (int v = threadIdx.x & 31; v < n && ok; v += 32) {
     const uint64_t a = adj[v];
     if (((a >> v) & 1ull) || (a & ~allowed))
       ok = false;
@@ -284,7 +277,16 @@ __global__ void dp_validate_kernel(const __grid_constant__ DpBatchParams p) {
       if (!((adj[__ffsll(static_cast<long long>(s)) - 1] >> v) & 1ull))
         ok = false;
   }
-  if (__any_sync(0xffffffffu, !ok) && lane == 0)
+  return __all_sync(0xffffffffu, ok);
+}
+
+// Checks every graph, one warp per graph.
+__global__ void dp_validate_kernel(const __grid_constant__ DpBatchParams p) {
+  const int g = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (g >= p.num_graphs)
+    return;  // the whole warp
+  const DpGraph G = p.graphs ? p.graphs[g] : p.single;
+  if (!adjacency_ok(p.adj + G.adj_off, G.n) && (threadIdx.x & 31) == 0)
     raise_error(p.error, kDevInvalidInput, g);
 }
 
@@ -1122,6 +1124,98 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
 }
 
 // ---------------------------------------------------------------------------
+// Small graphs: check, table and tree in one CTA.
+// ---------------------------------------------------------------------------
+
+// Subsets of a table in shared memory, words in natural order.
+struct SmallCtx {
+  const uint32_t* p0;
+  const uint32_t* p1;
+  int n;
+  __device__ uint32_t residue(uint64_t S) const {
+    const uint32_t w = static_cast<uint32_t>(S) >> 5, bit = static_cast<uint32_t>(S) & 31u;
+    return ((p0[w] >> bit) & 1u) ? 0u : 2u - ((p1[w] >> bit) & 1u);
+  }
+};
+
+// Dynamic shared memory for graphs of up to n vertices: three planes of
+// 2^(n-5) words and the words' order.
+__host__ __device__ constexpr uint32_t small_words(int n) { return n > 5 ? 1u << (n - 5) : 1u; }
+constexpr size_t small_smem(int n) { return size_t(small_words(n)) * (3 * 4 + 2); }
+
+// One CTA per graph of n <= kDpSmallMaxN vertices: a thread per word of 32
+// subsets, the words of a level between two CTA barriers, children at W ^ bit
+// in shared memory; then the first warp builds the tree from there while the
+// others copy the planes out (single-graph solves: tiles of 5 bits, for later
+// queries). One launch and no flag, count or gather from L2, each of which
+// costs a microsecond a level in the other kernels: bound by the latency of a
+// level's word chain, about 1 us (n = 12, all of check, table and tree: 18 us
+// against 4 + 21 + 14; n = 16: 25 against 4 + 30 + 16; n = 18: 49 against 58).
+__global__ void __launch_bounds__(512) dp_small_kernel(const __grid_constant__ DpBatchParams p, int max_n) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ Binom binom;
+  __shared__ TreeMem mem;
+  __shared__ int sBad;
+  const uint32_t tid = threadIdx.x, threads = blockDim.x;
+  const int g = p.first_graph + static_cast<int>(blockIdx.x);
+  const DpGraph G = p.graphs ? p.graphs[g] : p.single;
+  const uint64_t* const adj = p.adj + G.adj_off;
+  const int n = G.n, m = n > 5 ? n - 5 : 0;
+  const uint32_t words = 1u << m, stride = small_words(max_n);
+  uint32_t* const p0 = reinterpret_cast<uint32_t*>(smem);
+  uint32_t* const p1 = p0 + stride;
+  uint32_t* const pc = p1 + stride;
+  uint16_t* const order = reinterpret_cast<uint16_t*>(pc + stride);
+  fill_binom(binom);
+  if (tid < 32) {
+    __syncwarp();
+    level_offsets(binom, m, mem.off);
+    const bool bad = !adjacency_ok(adj, n);
+    if (tid == 0) {
+      sBad = bad ? 1 : 0;
+      if (bad)
+        raise_error(p.error, kDevInvalidInput, g);
+    }
+  }
+  __syncthreads();
+  if (sBad)
+    return;
+  for (uint32_t w = tid; w < words; w += threads)
+    order[mem.off[__popc(w)] + rank_colex(binom, w)] = static_cast<uint16_t>(w);
+  for (int j = 0; j <= m; ++j) {
+    __syncthreads();
+    const uint32_t begin = mem.off[j], count = binom[m][j];
+    for (uint32_t e = tid; e < count; e += threads) {
+      const uint32_t w = order[begin + e];
+      Acc a;
+      for (uint32_t bits = w; bits; bits &= bits - 1u) {
+        const uint32_t child = w ^ (bits & (0u - bits));
+        acc_add1(a, p0[child], p1[child], pc[child]);
+      }
+      const Planes r = j > 2 ? resolve_word(a, SmallSets{})
+                             : resolve_word(a, small_sets(static_cast<uint64_t>(w) << 5, j, adj, n));
+      p0[w] = r.p0;
+      p1[w] = r.p1;
+      pc[w] = r.c;
+    }
+  }
+  __syncthreads();
+  if (tid < 32) {
+    const SmallCtx ctx{p0, p1, n};
+    if (!build_tree(p, G, ctx, mem, (1ull << n) - 1ull) && tid == 0)
+      raise_error(p.error, kDevNoRoot, g);
+  } else if (p.table) {
+    uint32_t* const out = reinterpret_cast<uint32_t*>(p.table + G.table_off);
+    for (uint32_t t = tid - 32; t < words; t += threads - 32) {
+      const uint32_t w = order[t];
+      out[3 * t] = p0[w];
+      out[3 * t + 1] = p1[w];
+      out[3 * t + 2] = pc[w];
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Host-side launch helpers.
 // ---------------------------------------------------------------------------
 
@@ -1167,6 +1261,21 @@ cudaError_t dp_launch_fill_tile_map(const DpBatchParams& p, cudaStream_t s) {
 int dp_mixed_occupancy(int lb, int kid_rows) {
   return occupancy_of(dp_tile_kernel_mixed, smem_layout_for(kDpMinTileBits, lb, kid_rows),
                       smem_layout_for(kDpMinTileBits, kDpMaxTileBits, kDpMaxHigh));
+}
+
+cudaError_t dp_launch_small(const DpBatchParams& p, int max_n, cudaStream_t s) {
+  const size_t smem = small_smem(max_n);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(dp_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(small_smem(kDpSmallMaxN)));
+    if (e != cudaSuccess)
+      return e;
+  }
+  // threads: the words of the widest level, 64 to 512 (128 for many graphs,
+  // which fill the GPU side by side)
+  const int threads = max_n <= 13 ? 64 : max_n == 14 || p.num_graphs > 1 ? 128 : max_n == 15 ? 256 : 512;
+  dp_small_kernel<<<p.num_graphs, threads, smem, s>>>(p, max_n);
+  return cudaGetLastError();
 }
 
 int dp_level_occupancy(int kid_rows) {

@@ -30,6 +30,7 @@ struct DpBatchParams {
   uint2* tile_map = nullptr;        // ticket -> (graph, its tile group) (batches)
   const uint32_t* level_base = nullptr;  // [graph][level] first ticket (batches)
   int num_graphs = 1;
+  int first_graph = 0;              // number of graphs[0] (the small kernel starts there)
   int lb = 0;                       // tile bits of this launch (mixed batches: the largest)
   int kid_rows = 0;                 // largest nh of the launch's graphs
   int mixed = 0;                    // 1: graphs carry their own tile bits (DpGraph::lb)
@@ -61,6 +62,10 @@ cudaError_t dp_launch_tiles(const DpBatchParams& p, int ctas, cudaStream_t s);
 // counts chunks of kDpLevelChunk tiles of one level.
 int dp_level_occupancy(int kid_rows);
 cudaError_t dp_launch_levels(const DpBatchParams& p, int ctas, cudaStream_t s);
+// The small kernel: p.num_graphs graphs, from p.first_graph on, of at most
+// max_n <= kDpSmallMaxN vertices, checked, solved and reconstructed; p.table
+// (tiles of kDpSmallTileBits) may be null.
+cudaError_t dp_launch_small(const DpBatchParams& p, int max_n, cudaStream_t s);
 cudaError_t dp_launch_tree(const DpBatchParams& p, cudaStream_t s);
 cudaError_t dp_launch_labels(const DpBatchParams& p, const uint64_t* subsets, int count, int32_t* td_out,
                              uint64_t* roots_out, cudaStream_t s);

@@ -43,6 +43,10 @@ static_assert(dp_group_tiles(9) == kDpThreads && (dp_group_tiles(11) << (11 - 5)
 constexpr int kDpLevelTileBits = 7;
 constexpr int kDpLevelChunk = 128;
 
+// The small kernel's largest graph (its table in shared memory) and tiles.
+constexpr int kDpSmallMaxN = 18;
+constexpr int kDpSmallTileBits = 5;
+
 // Bytes of a tile of the solve's table.
 GTD_HD constexpr uint32_t dp_tile_bytes(int lb) { return 12u << (lb - 5); }
 
