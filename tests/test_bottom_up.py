@@ -88,3 +88,23 @@ def test_reference_chain_is_the_bnbgpu_incumbent(handle):
         td, par = reference_chain(handle, g)
         parts = [handle.bottom_up(g)[0], _lib.heuristic(g, 2)[0], _lib.heuristic(g, 1)[0]]
         assert td == min(parts), g.name
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [3, 11, 12, 13, 21])
+def test_bottom_up_gpu_at_the_table_sizes(handle, port, n):
+    """Up to 12 vertices are looked up, the others unranked."""
+    g = G.gnp_connected(n, 0.25, 60 + n)
+    td, par, order = handle.bottom_up(g)
+    otd, opar, oorder = port.bottom_up(g)
+    assert (td, order.tolist(), par.tolist()) == (otd, oorder, opar.tolist())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 12, 23, 24, 31, 32])
+def test_bottom_up_gpu_clique_heights(handle, n):
+    """A clique's forests are paths: heights up to n use every height plane,
+    and the last level's history starts at 2^n - 1; one subset per thread of a
+    chunk up to n = 23, four from n = 24 on."""
+    td, par, order = handle.bottom_up(G.complete(n))
+    assert td == n and order.tolist() == list(range(n)) and par.tolist() == [-1] + list(range(n - 1))
