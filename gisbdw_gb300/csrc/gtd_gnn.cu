@@ -21,6 +21,7 @@
 #include <cstring>
 #include <new>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "gtd_handle.h"
@@ -298,6 +299,612 @@ __global__ void to_bf16(int64_t n, const float* __restrict__ src, __nv_bfloat16*
 
 unsigned blocks_for(size_t n, unsigned t) { return static_cast<unsigned>((n + t - 1) / t); }
 
+// ---------------------------------------------------------------------------
+// Whole network per tile. A node's neighbours lie in its own graph, so a CTA
+// that holds a run of whole graphs (a tile, at most M nodes) computes every
+// layer, and for training the backward pass, from shared memory in one launch.
+// Training then takes the weight gradients of all layers in a second launch and
+// their sums in a third. Every sum runs in the order of the layer-by-layer
+// kernels above, so results are the same bit for bit (but for the loss, whose
+// order those leave open). Width 64; other widths, graphs larger than a tile
+// and neighbours outside their graph take the layer-by-layer kernels.
+// ---------------------------------------------------------------------------
+
+constexpr int kWide = 64;            // hidden width
+constexpr int kRow = kWide + 4;      // row stride in shared memory (16-byte rows, banks spread)
+constexpr int kTileThreads = 256;
+constexpr int kRowGroups = kTileThreads / 16;  // 16 threads take the 64 columns of a row
+constexpr int kGradThreads = 256;
+
+struct TileParams {
+  int fin, layers;
+  const float* x;
+  const int32_t* gstart;
+  const int32_t* nbr_start;
+  const int32_t* nbr;
+  const int32_t* tile_graph;   // [tiles + 1]: first graph of every tile
+  const __nv_bfloat16* w;      // all parameters
+  float* logits;
+  float* td_est;
+  int32_t* outside;            // set when a neighbour lies outside its tile
+  // training
+  const float* y;
+  const float* mask;
+  const float* td_label;
+  float inv_mask_sum, td_weight;
+  int num_nodes, num_graphs;
+  float *hs, *as, *dzs;        // [layers + 1], [layers], [layers + 1] x nodes x 64: kept for the weight gradients
+  float *pooled, *dlogit, *dtd;
+  float* tile_loss;            // [tiles]
+  int64_t nparams;
+  float* part;                 // [chunks of 64 rows][nparams]: weight gradients of every chunk
+};
+
+// BF16 weights (rows of 64, 16-byte aligned: every parameter block starts at a
+// multiple of 64 values) to FP32 rows of kRow, in two halves: the loads can be
+// on their way while the destination is still in use.
+template <int ROWS>
+struct WeightRegs {
+  static constexpr int kVec = ROWS * kWide / 8 / kTileThreads;
+  uint4 v[kVec];
+  __device__ __forceinline__ void load(const __nv_bfloat16* __restrict__ w) {
+#pragma unroll
+    for (int q = 0; q < kVec; ++q)
+      v[q] = __ldg(reinterpret_cast<const uint4*>(w) + threadIdx.x + q * kTileThreads);
+  }
+  __device__ __forceinline__ void store(float* out) const {
+#pragma unroll
+    for (int q = 0; q < kVec; ++q) {
+      const int t = threadIdx.x + q * kTileThreads;
+      float* const to = out + (t / 8) * kRow + 8 * (t % 8);
+      const uint32_t w[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
+      float f[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        f[2 * i] = __uint_as_float(w[i] << 16);
+        f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+      }
+      *reinterpret_cast<float4*>(to) = make_float4(f[0], f[1], f[2], f[3]);
+      *reinterpret_cast<float4*>(to + 4) = make_float4(f[4], f[5], f[6], f[7]);
+    }
+  }
+};
+
+// x / d, correctly rounded as the division is, from inv = 1 / d correctly
+// rounded: with the residue of q = x inv exact in a fused multiply-add,
+// q + residue * inv rounds to the quotient (Markstein's theorem; every
+// significand over every d up to 128 compared with the division). The residue
+// is exact above the denormal range; an infinite or NaN q is the quotient
+// itself. One division per node in place of one per channel, which took 60 %
+// of the aggregation.
+__device__ __forceinline__ float quotient(float x, float d, float inv) {
+  const float q = x * inv, residue = fmaf(-q, d, x);
+  return residue == residue ? fmaf(residue, inv, q) : q;
+}
+
+// acc[i][c] += X[row i][k] W[k][4 col + c] for k < K (a multiple of 4), in
+// ascending k: the same sums, bit for bit, as one thread per output. With few
+// rows per thread the next four k are loaded while these are multiplied.
+template <int R>
+struct Step {
+  float4 x[R], w[4];
+};
+
+template <int R>
+__device__ __forceinline__ void step_mul(const Step<R>& s, float (&acc)[R][4]) {
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const float xs[4] = {s.x[i].x, s.x[i].y, s.x[i].z, s.x[i].w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      acc[i][0] = fmaf(xs[q], s.w[q].x, acc[i][0]);
+      acc[i][1] = fmaf(xs[q], s.w[q].y, acc[i][1]);
+      acc[i][2] = fmaf(xs[q], s.w[q].z, acc[i][2]);
+      acc[i][3] = fmaf(xs[q], s.w[q].w, acc[i][3]);
+    }
+  }
+}
+
+template <int R>
+__device__ __forceinline__ void tile_product(const float* X, const float* W, int K, float (&acc)[R][4]) {
+  const int col = 4 * (threadIdx.x % 16), row = threadIdx.x / 16;
+  auto load = [&](int k, Step<R>& s) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      s.w[q] = *reinterpret_cast<const float4*>(W + (k + q) * kRow + col);
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      s.x[i] = *reinterpret_cast<const float4*>(X + (i * kRowGroups + row) * kRow + k);
+  };
+  if constexpr (R > 4) {  // enough independent products per load; registers for two CTAs per SM
+#pragma unroll 2
+    for (int k = 0; k < K; k += 4) {
+      Step<R> a;
+      load(k, a);
+      step_mul<R>(a, acc);
+    }
+    return;
+  }
+  Step<R> a, b;
+  load(0, a);
+#pragma unroll 1
+  for (int k = 0; k < K; k += 8) {
+    if (k + 4 < K)
+      load(k + 4, b);
+    step_mul<R>(a, acc);
+    if (k + 8 < K)
+      load(k + 8, a);
+    if (k + 4 < K)
+      step_mul<R>(b, acc);
+  }
+}
+
+// out = relu(b + X1 W1 (+ X2 W2)), rows < kRowGroups R; out may be X1.
+template <int R>
+__device__ __forceinline__ void tile_layer(const float* X1, const float* W1, int K1, const float* X2, const float* W2,
+                                           const __nv_bfloat16* __restrict__ bias, float* out) {
+  const int col = 4 * (threadIdx.x % 16), row = threadIdx.x / 16;
+  float acc[R][4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const float b = bf(bias[col + c]);
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      acc[i][c] = b;
+  }
+  tile_product<R>(X1, W1, K1, acc);
+  if (X2)
+    tile_product<R>(X2, W2, kWide, acc);
+  __syncthreads();  // every read of X1 before `out` is written
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+    *reinterpret_cast<float4*>(out + (i * kRowGroups + row) * kRow + col) =
+        make_float4(fmaxf(acc[i][0], 0.f), fmaxf(acc[i][1], 0.f), fmaxf(acc[i][2], 0.f), fmaxf(acc[i][3], 0.f));
+}
+
+// out[v][i] = sum_j Z[v][j] W[i][j], rows < kRowGroups R; with `start` divided by the
+// number of v's neighbours.
+template <int R>
+__device__ __forceinline__ void tile_product_t(const float* Z, const float* W, float* out,
+                                               const int32_t* start = nullptr) {
+  const int c = threadIdx.x % 16, row = threadIdx.x / 16;
+  float acc[R][4] = {};
+  auto load = [&](int j, Step<R>& s) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      s.w[q] = *reinterpret_cast<const float4*>(W + (c + 16 * q) * kRow + j);
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      s.x[i] = *reinterpret_cast<const float4*>(Z + (i * kRowGroups + row) * kRow + j);
+  };
+  auto mul = [&](const Step<R>& s) {
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        acc[i][q] = fmaf(s.x[i].w, s.w[q].w,
+                         fmaf(s.x[i].z, s.w[q].z, fmaf(s.x[i].y, s.w[q].y, fmaf(s.x[i].x, s.w[q].x, acc[i][q]))));
+  };
+  Step<R> s, t;
+  load(0, s);
+#pragma unroll 1
+  for (int j = 0; j < kWide; j += 8) {
+    load(j + 4, t);
+    mul(s);
+    if (j + 8 < kWide)
+      load(j + 8, s);
+    mul(t);
+  }
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int v = i * kRowGroups + row;
+    if (start) {
+      const float d = static_cast<float>(max(1, start[v + 1] - start[v]));  // without neighbours: not read
+      const float inv = 1.f / d;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        out[v * kRow + c + 16 * q] = quotient(acc[i][q], d, inv);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        out[v * kRow + c + 16 * q] = acc[i][q];
+    }
+  }
+}
+
+// Rows per thread that hold nodes: only those are computed.
+template <int M, typename F>
+__device__ __forceinline__ void for_rows(int nodes, F f) {
+  switch ((nodes + kRowGroups - 1) / kRowGroups) {
+    case 1: f(std::integral_constant<int, 1>{}); break;
+    case 2: f(std::integral_constant<int, 2>{}); break;
+    case 3: if constexpr (M >= 64) f(std::integral_constant<int, 3>{}); break;
+    case 4: if constexpr (M >= 64) f(std::integral_constant<int, 4>{}); break;
+    case 5: if constexpr (M >= 128) f(std::integral_constant<int, 5>{}); break;
+    case 6: if constexpr (M >= 128) f(std::integral_constant<int, 6>{}); break;
+    case 7: if constexpr (M >= 128) f(std::integral_constant<int, 7>{}); break;
+    default: if constexpr (M >= 128) f(std::integral_constant<int, 8>{}); break;
+  }
+}
+
+// Neighbour lists of a tile: first list entry of every node (relative to the
+// tile's first) and, where they fit, the neighbours as node numbers inside the
+// tile (else they are read from the batch's list each time).
+struct TileGraph {
+  const int32_t* start;   // [M + 1] shared; padding nodes have no neighbours
+  const uint8_t* local;   // shared, or null
+  const int32_t* nbr;     // the tile's part of the batch's list
+  int v0;
+  __device__ __forceinline__ int neighbour(int k) const { return local ? local[k] : __ldg(nbr + k) - v0; }
+};
+
+// Sum over v's neighbours, in list order, of h(u): 16 threads per node, 4
+// channels each; each of the 16 fetches one neighbour's number, so that the
+// rows follow one another without waiting for it. MEAN: out(v) = the sum over
+// their number, 0 without any; else out(v) += the sum. Whole CTA.
+template <bool MEAN>
+__device__ __forceinline__ void tile_aggregate(const TileGraph& t, int nodes, const float* h, float* out) {
+  const int sub = threadIdx.x % 16, col = 4 * sub, lane = threadIdx.x & 31;
+  for (int v0 = 0; v0 < nodes; v0 += kRowGroups) {
+    const int v = v0 + threadIdx.x / 16;
+    const int s = v < nodes ? t.start[v] : 0, deg = v < nodes ? t.start[v + 1] - s : 0;
+    const int most = max(deg, __shfl_xor_sync(0xffffffffu, deg, 16));  // of the warp's two nodes
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k0 = 0; k0 < most; k0 += 16) {
+      const int mine = k0 + sub < deg ? t.neighbour(s + k0 + sub) : 0;
+      const int trip = min(16, most - k0);
+#pragma unroll 4
+      for (int k = 0; k < trip; ++k) {
+        const int u = __shfl_sync(0xffffffffu, mine, (lane & 16) + k);
+        const float4 x = *reinterpret_cast<const float4*>(h + u * kRow + col);
+        if (k0 + k < deg) {
+          acc.x += x.x;
+          acc.y += x.y;
+          acc.z += x.z;
+          acc.w += x.w;
+        }
+      }
+    }
+    if (v < nodes) {
+      float4* const to = reinterpret_cast<float4*>(out + v * kRow + col);
+      if constexpr (MEAN) {
+        // without neighbours the sum is 0
+        const float d = static_cast<float>(max(1, deg)), inv = 1.f / d;
+        *to = make_float4(quotient(acc.x, d, inv), quotient(acc.y, d, inv), quotient(acc.z, d, inv),
+                          quotient(acc.w, d, inv));
+      } else {
+        const float4 o = *to;
+        *to = make_float4(o.x + acc.x, o.y + acc.y, o.z + acc.z, o.w + acc.w);
+      }
+    }
+  }
+}
+
+// Neighbours held in shared memory per tile: a complete graph of 32 vertices,
+// or sparse ones.
+template <int M>
+constexpr int kTileEdges = M == 32 ? 1024 : 4096;
+
+// Shared memory (floats) of a tile: rows of activations (forward two buffers,
+// training a third), two weight matrices, and for training the signs of every
+// layer's activations and dlogit, dtd, loss terms.
+template <int M>
+size_t tile_smem(bool train, int layers) {
+  return 4 * ((train ? 3 : 2) * size_t(M) * kRow + 2 * size_t(kWide) * kRow +
+              (train ? (2 * (size_t(layers) + 1) + 3) * M : 0) + M + 32) + kTileEdges<M>;
+}
+
+// One tile: forward, and for TRAIN the backward pass up to the weight
+// gradients. The products are bound by FP32 issue where two CTAs share an SM
+// (forward, M = 128: 1024 graphs of 20..80 nodes 100 us, where the layer-by-layer
+// kernels took 580), by the latency of shared loads at 8 warps per SM (training,
+// M = 32: 256 graphs of 5..24 nodes 48 us, 18 with gnn_weight_grads and
+// gnn_sum_chunks after it, against 530). 512 threads per CTA: 76 us in training.
+template <int M, bool TRAIN>
+__global__ void __launch_bounds__(kTileThreads, TRAIN ? 1 : 2) gnn_tile_kernel(const __grid_constant__ TileParams p) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int kBuf = M * kRow;
+  const int tid = threadIdx.x, H = kWide, L = p.layers, fin = p.fin;
+  const int g0 = p.tile_graph[blockIdx.x], g1 = p.tile_graph[blockIdx.x + 1];
+  const int v0 = p.gstart[g0], nodes = p.gstart[g1] - v0, graphs = g1 - g0;
+  float* const h = sm;            // the layer's activations; backward: dh
+  float* const agg = sm + kBuf;   // neighbour means (first: input features); backward: dz
+  float* const W1 = sm + (TRAIN ? 3 : 2) * kBuf;
+  float* const W2 = W1 + H * kRow;
+  int32_t* const start = reinterpret_cast<int32_t*>(W2 + H * kRow);  // [M + 32]
+  uint8_t* const local = reinterpret_cast<uint8_t*>(start + M + 32);
+  uint32_t* const sign = reinterpret_cast<uint32_t*>(local + kTileEdges<M>);  // training: [layer][node][2]
+  const __nv_bfloat16* const w = p.w;
+  const int64_t layer0 = int64_t(fin) * H + H, stride = 2 * int64_t(H) * H + H, head = layer0 + L * stride;
+  const size_t NH = size_t(p.num_nodes) * H;
+
+  // training keeps a layer for the weight gradients, and its signs here
+  auto keep = [&](const float* from, float* to) {
+    for (int t = tid; t < nodes * (H / 4); t += kTileThreads)
+      reinterpret_cast<float4*>(to + size_t(v0) * H)[t] =
+          *reinterpret_cast<const float4*>(from + (t / (H / 4)) * kRow + 4 * (t % (H / 4)));
+  };
+  auto keep_signs = [&](int l) {
+    for (int t = tid; t < nodes * H; t += kTileThreads) {  // whole warps: H is 64
+      const uint32_t bits = __ballot_sync(0xffffffffu, h[(t / H) * kRow + t % H] > 0.f);
+      if ((tid & 31) == 0)
+        sign[l * 2 * M + t / 32] = bits;
+    }
+  };
+
+  // input features, padded with zeros to a multiple of 4 and to whole row groups
+  const int fin4 = (fin + 3) & ~3, rows = (nodes + kRowGroups - 1) / kRowGroups * kRowGroups;
+  for (int t = tid; t < rows * fin4; t += kTileThreads) {
+    const int r = t / fin4, i = t % fin4;
+    agg[r * kRow + i] = r < nodes && i < fin ? p.x[size_t(v0 + r) * fin + i] : 0.f;
+  }
+  for (int t = tid; t < fin4 * H; t += kTileThreads)
+    W1[(t / H) * kRow + t % H] = t / H < fin ? bf(w[t]) : 0.f;
+  // neighbour lists; a neighbour outside the tile is reported and the batch
+  // taken up again layer by layer
+  const int e0 = p.nbr_start[v0], edges = p.nbr_start[v0 + nodes] - e0;
+  const TileGraph graph{start, edges <= kTileEdges<M> ? local : nullptr, p.nbr + e0, v0};
+  for (int v = tid; v < rows + 1; v += kTileThreads)
+    start[v] = v <= nodes ? p.nbr_start[v0 + v] - e0 : edges;
+  int bad = 0;
+  for (int k = tid; k < edges; k += kTileThreads) {
+    const int u = p.nbr[e0 + k] - v0;
+    bad |= static_cast<unsigned>(u) >= static_cast<unsigned>(nodes);
+    if (graph.local)
+      local[k] = static_cast<uint8_t>(u);
+  }
+  if (__syncthreads_or(bad)) {
+    if (tid == 0)
+      *p.outside = 1;
+    return;
+  }
+  WeightRegs<kWide> r1, r2;
+  for_rows<M>(nodes, [&](auto R) {
+    tile_layer<decltype(R)::value>(agg, W1, fin4, nullptr, nullptr, w + int64_t(fin) * H, h);
+  });
+  for (int l = 0; l < L; ++l) {
+    r1.load(w + layer0 + l * stride);
+    r2.load(w + layer0 + l * stride + H * H);
+    __syncthreads();
+    tile_aggregate<true>(graph, nodes, h, agg);
+    r1.store(W1);
+    r2.store(W2);
+    if constexpr (TRAIN) {
+      keep(h, p.hs + l * NH);
+      keep_signs(l);
+    }
+    __syncthreads();
+    if constexpr (TRAIN)
+      keep(agg, p.as + l * NH);
+    for_rows<M>(nodes, [&](auto R) {
+      tile_layer<decltype(R)::value>(h, W1, H, agg, W2, w + layer0 + l * stride + 2 * H * H, h);
+    });
+  }
+  __syncthreads();
+
+  // heads: a thread per node, then a warp per graph
+  const __nv_bfloat16 *w_out = w + head, *w_g = w + head + H + 1;
+  float* const dl = reinterpret_cast<float*>(sign + 2 * (L + 1) * M);  // training: dlogit per node
+  float* const dt = dl + M;         // dtd per graph
+  float* const loss = dt + M;       // loss terms per node
+  if constexpr (TRAIN) {
+    keep(h, p.hs + L * NH);
+    keep_signs(L);
+  }
+  if (tid < H) {
+    W1[tid] = bf(w_out[tid]);
+    W1[kRow + tid] = bf(w_g[tid]);
+  }
+  __syncthreads();
+  for (int v = tid; v < nodes; v += kTileThreads) {
+    float acc = bf(w_out[H]);
+    for (int j = 0; j < H; j += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(h + v * kRow + j);
+      acc = fmaf(x.x, W1[j], acc);
+      acc = fmaf(x.y, W1[j + 1], acc);
+      acc = fmaf(x.z, W1[j + 2], acc);
+      acc = fmaf(x.w, W1[j + 3], acc);
+    }
+    if constexpr (!TRAIN) {
+      p.logits[v0 + v] = acc;
+    } else {
+      const float m = p.mask[v0 + v], y = p.y[v0 + v], sig = 1.f / (1.f + expf(-acc));
+      const float d = m * (sig - y) * p.inv_mask_sum;
+      dl[v] = d;
+      p.dlogit[v0 + v] = d;
+      loss[v] = m * (fmaxf(acc, 0.f) - acc * y + log1pf(expf(-fabsf(acc)))) * p.inv_mask_sum;
+    }
+  }
+  for (int g = tid / 32; g < graphs; g += kTileThreads / 32) {
+    const int lane = tid & 31, s = p.gstart[g0 + g] - v0, e = p.gstart[g0 + g + 1] - v0;
+    float a = 0.f, b = 0.f;
+    for (int v = s; v < e; ++v) {
+      a += h[v * kRow + lane];
+      b += h[v * kRow + lane + 32];
+    }
+    a = a / static_cast<float>(e - s);  // no empty graphs here
+    b = b / static_cast<float>(e - s);
+    float sum = __fadd_rn(__fmul_rn(a, W1[kRow + lane]), __fmul_rn(b, W1[kRow + lane + 32]));
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+      sum += __shfl_down_sync(0xffffffffu, sum, off);
+    const float est = __shfl_sync(0xffffffffu, sum, 0) + bf(w_g[H]);
+    if constexpr (!TRAIN) {
+      if (lane == 0)
+        p.td_est[g0 + g] = est;
+    } else {
+      const float diff = est - p.td_label[g0 + g], d = 2.f * p.td_weight * diff / static_cast<float>(p.num_graphs);
+      if (lane == 0) {
+        dt[g] = d;
+        p.dtd[g0 + g] = d;
+        W2[g] = p.td_weight * diff * diff / static_cast<float>(p.num_graphs);  // g < M <= 128: two rows
+      }
+      p.pooled[size_t(g0 + g) * H + lane] = a;
+      p.pooled[size_t(g0 + g) * H + lane + 32] = b;
+    }
+  }
+  if constexpr (TRAIN) {
+    float* const dz = agg;
+    float* const da = sm + 2 * kBuf;
+    __syncthreads();
+    if (tid == 0) {
+      float a = 0.f;
+      for (int v = 0; v < nodes; ++v)
+        a += loss[v];
+      for (int g = 0; g < graphs; ++g)
+        a += W2[g];
+      p.tile_loss[blockIdx.x] = a;
+    }
+    // dh of the last layer (over its activations: only their signs are needed)
+    for (int g = tid / H; g < graphs; g += kTileThreads / H) {
+      const int j = tid % H, s = p.gstart[g0 + g] - v0, e = p.gstart[g0 + g + 1] - v0;
+      for (int v = s; v < e; ++v)
+        h[v * kRow + j] = dl[v] * W1[j] + dt[g] * W1[kRow + j] / static_cast<float>(e - s);
+    }
+    for (int l = L; l >= 0; --l) {
+      if (l > 0) {
+        r1.load(w + layer0 + (l - 1) * stride);
+        r2.load(w + layer0 + (l - 1) * stride + H * H);
+      }
+      __syncthreads();
+      // dz = dh where the activation is positive; zero padding rows
+      for (int t = tid; t < rows * H; t += kTileThreads) {
+        const int v = t / H, j = t % H;
+        const bool on = v < nodes && (sign[l * 2 * M + t / 32] >> (t & 31) & 1u);
+        dz[v * kRow + j] = on ? h[v * kRow + j] : 0.f;
+      }
+      if (l > 0) {
+        r1.store(W1);
+        r2.store(W2);
+      }
+      __syncthreads();
+      keep(dz, p.dzs + l * NH);
+      if (l == 0)
+        break;
+      // dh of the layer below: dz Ws^T + aggregate^T(dz Wn^T)
+      for_rows<M>(nodes, [&](auto R) {
+        tile_product_t<decltype(R)::value>(dz, W2, da, start);
+        tile_product_t<decltype(R)::value>(dz, W1, h);
+      });
+      __syncthreads();
+      tile_aggregate<false>(graph, nodes, da, h);
+    }
+  }
+}
+
+// Weight gradients of a chunk of 64 rows: dW[i][j] = sum_v X[v][i] dZ[v][j] and
+// the bias's column sums, in ascending v. blockIdx.y: 0 .. layers - 1 the two
+// matrices of a layer, `layers` the input projection, then the node head and
+// the graph head (rows: graphs).
+__global__ void __launch_bounds__(kGradThreads) gnn_weight_grads(const __grid_constant__ TileParams p) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int kChunk = 64;
+  const int tid = threadIdx.x, H = kWide, L = p.layers, fin = p.fin, what = static_cast<int>(blockIdx.y);
+  const int total = what == L + 2 ? p.num_graphs : p.num_nodes;
+  const int r0 = static_cast<int>(blockIdx.x) * kChunk, rows = min(kChunk, total - r0);
+  if (rows <= 0)
+    return;
+  const int64_t layer0 = int64_t(fin) * H + H, stride = 2 * int64_t(H) * H + H, head = layer0 + L * stride;
+  const size_t NH = size_t(p.num_nodes) * H;
+  float* const out = p.part + size_t(blockIdx.x) * p.nparams;
+  float *const X = sm, *const Y = sm + kChunk * kRow, *const Z = sm + 2 * kChunk * kRow;
+  auto load = [&](const float* from, float* to) {
+    for (int t = tid; t < rows * (H / 4); t += kGradThreads)
+      *reinterpret_cast<float4*>(to + (t / (H / 4)) * kRow + 4 * (t % (H / 4))) =
+          reinterpret_cast<const float4*>(from + size_t(r0) * H)[t];
+  };
+  if (what < L) {
+    load(p.hs + what * NH, X);
+    load(p.as + what * NH, Y);
+    load(p.dzs + (what + 1) * NH, Z);
+    __syncthreads();
+    const int j0 = 4 * (tid % 16), i0 = 4 * (tid / 16);
+    float a[4][4] = {}, b[4][4] = {};
+#pragma unroll 2
+    for (int v = 0; v < rows; ++v) {
+      const float4 z = *reinterpret_cast<const float4*>(Z + v * kRow + j0);
+      const float4 x = *reinterpret_cast<const float4*>(X + v * kRow + i0);
+      const float4 y = *reinterpret_cast<const float4*>(Y + v * kRow + i0);
+      const float zs[4] = {z.x, z.y, z.z, z.w}, xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          a[i][j] = fmaf(xs[i], zs[j], a[i][j]);
+          b[i][j] = fmaf(ys[i], zs[j], b[i][j]);
+        }
+    }
+    float* const g = out + layer0 + what * stride;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        g[(i0 + i) * H + j0 + j] = a[i][j];
+        g[H * H + (i0 + i) * H + j0 + j] = b[i][j];
+      }
+    if (tid < H) {
+      float sum = 0.f;
+      for (int v = 0; v < rows; ++v)
+        sum += Z[v * kRow + tid];
+      g[2 * H * H + tid] = sum;
+    }
+  } else if (what == L) {
+    load(p.dzs, Z);
+    for (int t = tid; t < rows * fin; t += kGradThreads)
+      X[(t / fin) * kRow + t % fin] = p.x[size_t(r0) * fin + t];
+    __syncthreads();
+    for (int t = tid; t < fin * H; t += kGradThreads) {
+      float a = 0.f;
+      for (int v = 0; v < rows; ++v)
+        a = fmaf(X[v * kRow + t / H], Z[v * kRow + t % H], a);
+      out[t] = a;
+    }
+    if (tid < H) {
+      float sum = 0.f;
+      for (int v = 0; v < rows; ++v)
+        sum += Z[v * kRow + tid];
+      out[int64_t(fin) * H + tid] = sum;
+    }
+  } else {
+    const bool graph = what == L + 2;
+    const float* const from = graph ? p.pooled : p.hs + L * NH;
+    const float* const d = (graph ? p.dtd : p.dlogit) + r0;
+    float* const g = out + head + (graph ? H + 1 : 0);
+    if (tid < H) {
+      float a = 0.f;
+      for (int v = 0; v < rows; ++v)
+        a = fmaf(from[size_t(r0 + v) * H + tid], d[v], a);
+      g[tid] = a;
+    } else if (tid == H) {
+      float a = 0.f;
+      for (int v = 0; v < rows; ++v)
+        a += d[v];
+      g[H] = a;
+    }
+  }
+}
+
+// The gradient: every parameter's chunks in ascending order; the loss: the
+// tiles' likewise.
+__global__ void __launch_bounds__(128) gnn_sum_chunks(const __grid_constant__ TileParams p, int tiles,
+                                                      float* __restrict__ grad, float* __restrict__ loss) {
+  const int64_t t = int64_t(blockIdx.x) * 128 + threadIdx.x;
+  if (t > p.nparams)
+    return;
+  const int64_t graph_head = p.nparams - kWide - 1;
+  const int count = t == p.nparams ? tiles : ((t >= graph_head ? p.num_graphs : p.num_nodes) + 63) / 64;
+  const float* from = t == p.nparams ? p.tile_loss : p.part + t;
+  const int64_t step = t == p.nparams ? 1 : p.nparams;
+  float acc = 0.f;
+#pragma unroll 8
+  for (int c = 0; c < count; ++c)
+    acc += from[c * step];
+  if (t == p.nparams)
+    *loss = acc;
+  else
+    grad[t] = 0.f + acc;
+}
+
 }  // namespace
 }  // namespace gtd
 
@@ -314,6 +921,9 @@ struct gtd_gnn_s {
   // batch and activation buffers (grown as needed)
   void* buf = nullptr;
   size_t buf_cap = 0;
+  void* stage = nullptr;  // pinned: small arrays of a batch in, results out
+  size_t stage_cap = 0;
+  bool smem_set = false;  // the tile kernels' shared-memory limits are raised
 };
 
 namespace {
@@ -483,6 +1093,190 @@ gtd_status backward(gtd_gnn g, const gtd_gnn_batch* b, const Views& V, float td_
   return GTD_OK;
 }
 
+// The most shared memory a CTA of these kernels may take (227 KB).
+constexpr size_t kTileSmemMost = 227 * 1024;
+
+template <int M, bool TRAIN>
+cudaError_t launch_tile_kernel(const gtd::TileParams& p, int tiles, cudaStream_t s) {
+  gtd::gnn_tile_kernel<M, TRAIN><<<tiles, gtd::kTileThreads, gtd::tile_smem<M>(TRAIN, p.layers), s>>>(p);
+  return cudaGetLastError();
+}
+
+// Nodes per tile for this batch, 0 where the tile kernels do not apply: the
+// largest graph decides, small tiles spread a small training batch over more
+// SMs.
+int tile_nodes(const gtd_gnn_s* g, const gtd_gnn_batch* b, bool train) {
+  if (g->hid != gtd::kWide)
+    return 0;
+  int most = 0;
+  for (int i = 0; i < b->num_graphs; ++i) {
+    const int n = b->graph_start[i + 1] - b->graph_start[i];
+    if (n < 1)
+      return 0;
+    most = std::max(most, n);
+  }
+  if (most <= 32 && b->num_nodes <= 32 * 3 * g->h->num_sms)
+    return 32;
+  return most <= 64 ? 64 : most <= 128 ? 128 : 0;
+}
+
+// Forward (train = false: logits and td estimates) or loss and gradients
+// (train = true: g->grad and *loss_out) by tiles. *done is false, and nothing
+// else has happened, where the batch needs the layer-by-layer kernels.
+gtd_status run_tiles(gtd_gnn g, const gtd_gnn_batch* b, bool train, float td_weight, float* logits_out, float* td_out,
+                     float* grad_out, float* loss_out, bool* done) {
+  *done = false;
+  const int M = tile_nodes(g, b, train);
+  if (M == 0)
+    return GTD_OK;
+  gtd_handle h = g->h;
+  cudaStream_t s = h->stream;
+  const size_t N = size_t(b->num_nodes), G = size_t(b->num_graphs), E = size_t(b->nbr_start[b->num_nodes]);
+  std::vector<int32_t> first;  // first graph of every tile
+  int nodes = M + 1;
+  for (size_t i = 0; i < G; ++i) {
+    const int n = b->graph_start[i + 1] - b->graph_start[i];
+    if (nodes + n > M) {
+      first.push_back(static_cast<int32_t>(i));
+      nodes = 0;
+    }
+    nodes += n;
+  }
+  const int tiles = static_cast<int>(first.size());
+  first.push_back(static_cast<int32_t>(G));
+
+  // one buffer: the batch's arrays, then results; the small ones (up to
+  // kStaged bytes each) lie in front and go up in one copy from pinned memory,
+  // the others straight from the caller's arrays (the host takes longer over a
+  // pass of its own: 78 us against 18 for 1.6 MB)
+  constexpr size_t kStaged = 64 * 1024;
+  struct Array {
+    const void* from;
+    size_t bytes, at;
+  };
+  enum { kX, kGraphStart, kNbrStart, kNbr, kTiles, kY, kMask, kTd, kArrays };
+  Array in[kArrays] = {{b->x, N * g->fin * 4, 0},
+                       {b->graph_start, (G + 1) * 4, 0},
+                       {b->nbr_start, (N + 1) * 4, 0},
+                       {b->nbr, E * 4, 0},
+                       {first.data(), first.size() * 4, 0},
+                       {b->root_label, train ? N * 4 : 0, 0},
+                       {b->node_mask, train ? N * 4 : 0, 0},
+                       {b->td_label, train ? G * 4 : 0, 0}};
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    const size_t o = off;
+    off += (bytes + 255) & ~size_t(255);
+    return o;
+  };
+  for (Array& a : in)
+    if (a.bytes <= kStaged)
+      a.at = take(a.bytes);
+  const size_t staged = off;
+  for (Array& a : in)
+    if (a.bytes > kStaged)
+      a.at = take(a.bytes);
+  const size_t chunks = (std::max(N, G) + 63) / 64, NH = N * size_t(gtd::kWide), L = size_t(g->layers);
+  // results, in one copy back: the flag, the loss or the td estimates, the logits
+  const size_t ores = take(256), otde = take(G * 4), olog = take(N * 4), res_bytes = train ? 8 : off - ores;
+  const size_t ohs = take(train ? (L + 1) * NH * 4 : 0), oas = take(train ? L * NH * 4 : 0),
+               odz = take(train ? (L + 1) * NH * 4 : 0), opool = take(train ? G * gtd::kWide * 4 : 0),
+               otl2 = take(train ? size_t(tiles) * 4 : 0), opart = take(train ? chunks * size_t(g->nparams) * 4 : 0);
+  GTD_CUDA(h, gtd::ensure_device(&g->buf, &g->buf_cap, off));
+  const size_t stage = std::max(staged, res_bytes);
+  if (g->stage_cap < stage) {
+    if (g->stage)
+      cudaFreeHost(g->stage);
+    g->stage = nullptr;
+    g->stage_cap = 0;
+    GTD_CUDA(h, cudaMallocHost(&g->stage, stage));
+    g->stage_cap = stage;
+  }
+  if (!g->smem_set) {
+    const int most = static_cast<int>(kTileSmemMost);
+    for (auto kernel : {gtd::gnn_tile_kernel<32, false>, gtd::gnn_tile_kernel<64, false>,
+                        gtd::gnn_tile_kernel<128, false>, gtd::gnn_tile_kernel<32, true>,
+                        gtd::gnn_tile_kernel<64, true>, gtd::gnn_tile_kernel<128, true>, gtd::gnn_weight_grads})
+      GTD_CUDA(h, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    g->smem_set = true;
+  }
+  char* const base = static_cast<char*>(g->buf);
+  char* const pinned = static_cast<char*>(g->stage);
+  for (const Array& a : in)
+    if (a.bytes > kStaged)
+      GTD_CUDA(h, cudaMemcpyAsync(base + a.at, a.from, a.bytes, cudaMemcpyHostToDevice, s));
+    else if (a.bytes)
+      std::memcpy(pinned + a.at, a.from, a.bytes);
+  GTD_CUDA(h, cudaMemcpyAsync(base, pinned, staged, cudaMemcpyHostToDevice, s));
+  GTD_CUDA(h, cudaMemsetAsync(base + ores, 0, 8, s));
+  double msum = 0;
+  for (size_t v = 0; train && v < N; ++v)
+    msum += b->node_mask[v];
+  auto f = [&](size_t o) { return reinterpret_cast<float*>(base + o); };
+  auto i32 = [&](size_t o) { return reinterpret_cast<int32_t*>(base + o); };
+  gtd::TileParams p = {};
+  p.fin = g->fin;
+  p.layers = g->layers;
+  p.x = f(in[kX].at);
+  p.gstart = i32(in[kGraphStart].at);
+  p.nbr_start = i32(in[kNbrStart].at);
+  p.nbr = i32(in[kNbr].at);
+  p.tile_graph = i32(in[kTiles].at);
+  p.w = g->w;
+  p.logits = f(olog);
+  p.td_est = f(otde);
+  p.outside = i32(ores);
+  p.y = f(in[kY].at);
+  p.mask = f(in[kMask].at);
+  p.td_label = f(in[kTd].at);
+  p.inv_mask_sum = msum > 0 ? float(1.0 / msum) : 0.f;
+  p.td_weight = td_weight;
+  p.num_nodes = b->num_nodes;
+  p.num_graphs = b->num_graphs;
+  p.hs = f(ohs);
+  p.as = f(oas);
+  p.dzs = f(odz);
+  p.pooled = f(opool);
+  p.dlogit = f(olog);
+  p.dtd = f(otde);
+  p.tile_loss = f(otl2);
+  p.nparams = g->nparams;
+  p.part = f(opart);
+  if (train) {
+    GTD_CUDA(h, (M == 32   ? launch_tile_kernel<32, true>(p, tiles, s)
+                 : M == 64 ? launch_tile_kernel<64, true>(p, tiles, s)
+                           : launch_tile_kernel<128, true>(p, tiles, s)));
+    const dim3 grid(static_cast<unsigned>(chunks), static_cast<unsigned>(g->layers + 3));
+    gtd::gnn_weight_grads<<<grid, gtd::kGradThreads, 3 * 64 * gtd::kRow * 4, s>>>(p);
+    gtd::gnn_sum_chunks<<<gtd::blocks_for(size_t(g->nparams) + 1, 128), 128, 0, s>>>(p, tiles, g->grad,
+                                                                                    f(ores) + 1);
+    GTD_CUDA(h, cudaGetLastError());
+  } else {
+    GTD_CUDA(h, (M == 32   ? launch_tile_kernel<32, false>(p, tiles, s)
+                 : M == 64 ? launch_tile_kernel<64, false>(p, tiles, s)
+                           : launch_tile_kernel<128, false>(p, tiles, s)));
+  }
+  GTD_CUDA(h, cudaMemcpyAsync(pinned, base + ores, res_bytes, cudaMemcpyDeviceToHost, s));
+  if (train && grad_out)
+    GTD_CUDA(h, cudaMemcpyAsync(grad_out, g->grad, size_t(g->nparams) * 4, cudaMemcpyDeviceToHost, s));
+  GTD_CUDA(h, cudaStreamSynchronize(s));
+  int32_t outside = 0;
+  std::memcpy(&outside, pinned, 4);
+  if (outside)
+    return GTD_OK;  // a neighbour lies outside its graph: layer by layer
+  *done = true;
+  if (train) {
+    if (loss_out)
+      std::memcpy(loss_out, pinned + 4, 4);
+  } else {
+    if (td_out)
+      std::memcpy(td_out, pinned + (otde - ores), G * 4);
+    if (logits_out)
+      std::memcpy(logits_out, pinned + (olog - ores), N * 4);
+  }
+  return GTD_OK;
+}
+
 uint64_t splitmix(uint64_t& s) {
   s += 0x9E3779B97F4A7C15ull;
   uint64_t z = s;
@@ -560,6 +1354,8 @@ gtd_status gtd_gnn_destroy(gtd_gnn g) {
   cudaFree(g->grad);
   cudaFree(g->w);
   cudaFree(g->buf);
+  if (g->stage)
+    cudaFreeHost(g->stage);
   delete g;
   return GTD_OK;
 }
@@ -606,6 +1402,9 @@ gtd_status gtd_gnn_forward(gtd_gnn g, const gtd_gnn_batch* b, float* logits_out,
   if (s != GTD_OK)
     return s;
   DeviceGuard dg(g->h->device);
+  bool done = false;
+  if ((s = run_tiles(g, b, false, 0.f, logits_out, td_out, nullptr, nullptr, &done)) != GTD_OK || done)
+    return s;
   Views V;
   if ((s = prepare(g, b, false, V)) != GTD_OK)
     return s;
@@ -625,6 +1424,9 @@ gtd_status gtd_gnn_gradients(gtd_gnn g, const gtd_gnn_batch* b, float td_weight,
   if (s != GTD_OK)
     return s;
   DeviceGuard dg(g->h->device);
+  bool done = false;
+  if ((s = run_tiles(g, b, true, td_weight, nullptr, nullptr, grad_out, loss_out, &done)) != GTD_OK || done)
+    return s;
   Views V;
   if ((s = prepare(g, b, true, V)) != GTD_OK)
     return s;
@@ -646,13 +1448,18 @@ gtd_status gtd_gnn_train_step(gtd_gnn g, const gtd_gnn_batch* b, float lr, float
   if (s != GTD_OK)
     return s;
   DeviceGuard dg(g->h->device);
+  bool done = false;
+  if ((s = run_tiles(g, b, true, td_weight, nullptr, nullptr, nullptr, loss_out, &done)) != GTD_OK)
+    return s;
   Views V;
-  if ((s = prepare(g, b, true, V)) != GTD_OK)
-    return s;
-  if ((s = forward(g, b, V)) != GTD_OK)
-    return s;
-  if ((s = backward(g, b, V, td_weight)) != GTD_OK)
-    return s;
+  if (!done) {
+    if ((s = prepare(g, b, true, V)) != GTD_OK)
+      return s;
+    if ((s = forward(g, b, V)) != GTD_OK)
+      return s;
+    if ((s = backward(g, b, V, td_weight)) != GTD_OK)
+      return s;
+  }
   ++g->step;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - std::pow(b1, float(g->step)), c2 = 1.f - std::pow(b2, float(g->step));
@@ -660,7 +1467,7 @@ gtd_status gtd_gnn_train_step(gtd_gnn g, const gtd_gnn_batch* b, float lr, float
   adam_step<<<blocks_for(size_t(g->nparams), 256), 256, 0, st>>>(g->nparams, g->master, g->m, g->v, g->grad, g->w,
                                                                   lr, b1, b2, 1e-8f, c1, c2);
   GTD_CUDA(g->h, cudaGetLastError());
-  if (loss_out)
+  if (loss_out && !done)
     GTD_CUDA(g->h, cudaMemcpyAsync(loss_out, V.loss, 4, cudaMemcpyDeviceToHost, st));
   GTD_CUDA(g->h, cudaStreamSynchronize(st));
   return GTD_OK;

@@ -173,3 +173,53 @@ def test_learned_order_keeps_treedepth_and_cuts_search(handle):
     # so compare the typical graph, not the total (dominated by a few hard ones)
     ratio = (learned["nodes"][both] + 1.0) / (plain["nodes"][both] + 1.0)
     assert np.median(ratio) < 1.0
+
+
+def _layerwise(b):
+    """The same nodes, neighbours and labels with an empty graph at the end:
+    batches with one take the layer-by-layer kernels."""
+    return gnn.Batch(b.x, np.append(b.graph_start, b.graph_start[-1]).astype(np.int32), b.nbr_start, b.nbr,
+                     b.root_label, b.node_mask, np.append(b.td_label, np.float32(1.0)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes", [(1,), (32,) * 3, (33, 31, 1), (64, 64), (65, 2, 60), (128, 5), (24,) * 40])
+def test_tile_kernels_equal_the_layerwise_kernels(handle, sizes):
+    """Tiles just filled, overfull and with padding rows: logits bit for bit,
+    estimates and gradients (whose mean over graphs counts the empty graph)
+    against float64."""
+    rng = np.random.default_rng(len(sizes))
+    gs = [G.gnp_connected(n, min(1.0, 3.0 / max(1, n - 1) + 0.1), 7 + i) if n > 1 else G.Graph(1, [])
+          for i, n in enumerate(sizes)]
+    b = gnn.make_batch(gs, roots=[(rng.random(g.n) < 0.4).astype(np.float32) for g in gs],
+                       tds=[3.0] * len(gs))
+    net = gnn.GNN(handle, seed=9)
+    logits, td = net.forward(b)
+    logits2, td2 = net.forward(_layerwise(b))
+    assert np.array_equal(logits, logits2) and np.array_equal(td, td2[:-1])
+    rlogits, rtd = gnn.reference_loss(net.params(), b, want_grad=False)
+    # float32 sums of at most 128 terms per layer, four layers
+    np.testing.assert_allclose(logits, rlogits, rtol=2e-4, atol=2e-5)
+    np.testing.assert_allclose(td, rtd, rtol=2e-4, atol=2e-5)
+    grad, loss = net.gradients(b)
+    rloss, rgrad = gnn.reference_loss(net.params(), b)
+    assert abs(loss - rloss) < 1e-4 * max(1.0, abs(rloss))
+    assert np.linalg.norm(grad - rgrad) < 1e-4 * np.linalg.norm(rgrad)
+
+
+@pytest.mark.gpu
+def test_neighbours_outside_their_graph_take_the_layerwise_kernels(handle):
+    """Two graphs joined by an edge of the neighbour lists: one network over
+    all nodes, as the reference computes it."""
+    _, b = _toy_batch(3)
+    n = int(b.graph_start[-1])
+    lists = [b.nbr[b.nbr_start[v]:b.nbr_start[v + 1]].tolist() for v in range(n)]
+    lists[0].append(n - 1)
+    lists[n - 1].append(0)
+    c = gnn.Batch(b.x, b.graph_start, np.concatenate([[0], np.cumsum([len(x) for x in lists])]).astype(np.int32),
+                  np.array(sum(lists, []), dtype=np.int32), b.root_label, b.node_mask, b.td_label)
+    net = gnn.GNN(handle, seed=4)
+    logits, td = net.forward(c)
+    rlogits, rtd = gnn.reference_loss(net.params(), c, want_grad=False)
+    np.testing.assert_allclose(logits, rlogits, rtol=2e-4, atol=2e-5)
+    np.testing.assert_allclose(td, rtd, rtol=2e-4, atol=2e-5)
