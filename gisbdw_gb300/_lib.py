@@ -309,18 +309,45 @@ class PerGraph(Sequence):
         return self._flat[o:o + self._n[i]]
 
 
+_PACK = None
+
+
+def _pack_edges():
+    global _PACK
+    if _PACK is None:
+        load()  # builds both libraries when needed
+        fn = ctypes.PyDLL(_build.PACK_LIB).gtd_pack_edges
+        fn.argtypes = [ctypes.py_object, _vp, _vp, _i, _vp]
+        _PACK = fn
+    return _PACK
+
+
+def adjacency_pool(graphs, words: int) -> np.ndarray:
+    """The masks of every graph one after another: adj64() (words = 1) or
+    adj128() (words = 2, lo and hi per vertex) of each, built in one native
+    pass over the edge lists."""
+    graphs = list(graphs)
+    ns = np.array([g.n for g in graphs], dtype=np.int64)
+    offs = np.zeros(len(graphs) + 1, dtype=np.int64)
+    np.cumsum(ns, out=offs[1:])
+    out = np.zeros(words * int(offs[-1]), dtype=np.uint64)
+    if len(graphs) and int(ns.max()) <= 64 * words and \
+            _pack_edges()([g.edges for g in graphs], _ptr(ns), _ptr(offs), words, _ptr(out)) == 0:
+        return out
+    parts = [g.adj64() if words == 1 else g.adj128() for g in graphs]
+    return np.concatenate(parts).astype(np.uint64) if parts else out
+
+
 def pack_batch(graphs):
     """Adjacency pool and descriptors for a list of graphs (offsets = running
     sum of n)."""
     descs = (GraphDesc * len(graphs))()
     off = 0
-    pool = np.zeros(sum(g.n for g in graphs), dtype=np.uint64)
     for i, g in enumerate(graphs):
         descs[i].n = g.n
         descs[i].offset = off
-        pool[off:off + g.n] = g.adj64()
         off += g.n
-    return descs, pool
+    return descs, adjacency_pool(graphs, 1)
 
 
 def table_index(n: int, tile_bits: int, subset_mask: int) -> int:
@@ -367,7 +394,7 @@ def _heuristic_batch(self, graphs, kind: int = 0, scores=None):
     ns = np.array([g.n for g in graphs], dtype=np.int32)
     offs = np.concatenate([[0], np.cumsum(ns)[:-1]]).astype(np.int32)
     descs = np.ascontiguousarray(np.stack([ns, offs], axis=1))
-    adj = np.ascontiguousarray(np.concatenate([g.adj128() for g in graphs]).astype(np.uint64))
+    adj = adjacency_pool(graphs, 2)
     total = int(ns.sum())
     sc = np.ascontiguousarray(np.concatenate(scores), dtype=np.float32) if scores is not None else None
     td = np.zeros(len(graphs), dtype=np.int32)
@@ -419,7 +446,7 @@ def pack_bnb(graphs, orders=None, seeds=None, seed_kind: int = 0):
     """Descriptors, 128-bit adjacency pool, order pool and seeds."""
     descs = (GraphDesc * len(graphs))()
     total = sum(g.n for g in graphs)
-    adj = np.zeros(2 * max(total, 1), dtype=np.uint64)
+    adj = adjacency_pool(graphs, 2) if total else np.zeros(2, dtype=np.uint64)
     order = np.zeros(max(total, 1), dtype=np.uint8)
     seed_td = np.zeros(len(graphs), dtype=np.int32)
     seed_par = np.zeros(max(total, 1), dtype=np.int32)
@@ -427,7 +454,6 @@ def pack_bnb(graphs, orders=None, seeds=None, seed_kind: int = 0):
     for i, g in enumerate(graphs):
         descs[i].n = g.n
         descs[i].offset = off
-        adj[2 * off:2 * (off + g.n)] = g.adj128()
         order[off:off + g.n] = orders[i] if orders is not None else np.arange(g.n)
         if seeds is not None:
             t, p = seeds[i]

@@ -3,7 +3,8 @@
 Every translation unit under csrc/ is compiled by nvcc in parallel with
 ``-gencode arch=compute_103a,code=sm_103a`` and linked into
 ``gisbdw_gb300/_build/libgtd.so`` (cudart linked statically, so the library
-only needs the driver at run time).
+only needs the driver at run time). gtd_pack.c, the batch packer over Python
+edge lists, becomes a library of its own next to it.
 """
 from __future__ import annotations
 
@@ -11,12 +12,14 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT_DIR, "libgtd.so")
+PACK_LIB = os.path.join(OUT_DIR, "libgtdpack.so")  # edge lists to masks (CPython)
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
@@ -44,16 +47,26 @@ def _compile(src: str, verbose: bool) -> str:
     return obj
 
 
+def _compile_pack() -> None:
+    tmp = PACK_LIB + ".tmp"
+    cmd = ["gcc", "-O2", "-fPIC", "-shared", "-I" + sysconfig.get_paths()["include"],
+           os.path.join(CSRC, "gtd_pack.c"), "-o", tmp]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"gcc failed on gtd_pack.c:\n{r.stderr}")
+    os.replace(tmp, PACK_LIB)
+
+
 def sources():
     return sorted(glob.glob(os.path.join(CSRC, "*.cu")))
 
 
 def up_to_date() -> bool:
-    if not os.path.exists(LIB):
+    if not os.path.exists(LIB) or not os.path.exists(PACK_LIB):
         return False
-    t = os.path.getmtime(LIB)
+    t = min(os.path.getmtime(LIB), os.path.getmtime(PACK_LIB))
     deps = sources() + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(CSRC, "*.cuh"))
-    deps += glob.glob(os.path.join(INCLUDE, "*.h")) + [__file__]
+    deps += glob.glob(os.path.join(CSRC, "*.c")) + glob.glob(os.path.join(INCLUDE, "*.h")) + [__file__]
     return all(os.path.getmtime(d) <= t for d in deps)
 
 
@@ -63,7 +76,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OUT_DIR, exist_ok=True)
     srcs = sources()
     with ThreadPoolExecutor(max_workers=max(1, min(len(srcs), os.cpu_count() or 4))) as ex:
+        pack = ex.submit(_compile_pack)
         objs = list(ex.map(lambda s: _compile(s, verbose), srcs))
+        pack.result()
     tmp = LIB + ".tmp"
     cmd = [nvcc()] + ARCH + ["-shared", "-o", tmp] + objs + ["-lpthread", "-ldl", "-lrt"]
     r = subprocess.run(cmd, capture_output=True, text=True)

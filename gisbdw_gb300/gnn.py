@@ -175,7 +175,7 @@ def make_batch(graphs: Sequence[Graph], roots: Optional[Sequence[np.ndarray]] = 
                tds: Optional[Sequence[int]] = None) -> Batch:
     ns = np.array([g.n for g in graphs], dtype=np.int64)
     offs = np.concatenate([[0], np.cumsum(ns)[:-1]]).astype(np.int64)
-    adj2 = np.concatenate([g.adj128() for g in graphs]).astype(np.uint64)
+    adj2 = _lib.adjacency_pool(graphs, 2)
     b = pack(adj2, ns, offs)
     if roots is not None:
         b.root_label = np.concatenate(roots).astype(np.float32)
@@ -506,7 +506,7 @@ def label_set(handle: _lib.Handle, graphs: Sequence[Graph], per_graph: int, seed
     L = _bind(handle.L)
     ns = np.array([g.n for g in graphs], dtype=np.int64)
     offs = np.concatenate([[0], np.cumsum(ns)[:-1]]).astype(np.int64)
-    adj2 = np.concatenate([g.adj128() for g in graphs]).astype(np.uint64)
+    adj2 = _lib.adjacency_pool(graphs, 2)
     descs = _descs(ns, offs)
     cap = len(graphs) * (per_graph + 1)
     sub_adj = np.zeros(2 * 24 * cap, dtype=np.uint64)

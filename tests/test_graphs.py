@@ -1,5 +1,6 @@
 """Generators and the reference's text format."""
 import numpy as np
+import pytest
 
 from gisbdw_gb300 import graphs as G
 
@@ -43,3 +44,24 @@ def test_masks():
     assert all(((int(adj[v]) >> v) & 1) == 0 for v in range(9))
     a2 = g.adj128()
     assert np.all(a2[0::2] == adj) and np.all(a2[1::2] == 0)
+
+
+def test_adjacency_pool_equals_the_per_graph_masks():
+    """The native packer against adj64 / adj128, and its way out: anything but
+    pairs of plain integers in range takes the per-graph path."""
+    from gisbdw_gb300 import _lib
+    gs = [G.Graph(1, []), G.path(2), G.complete(64), G.grid(4, 5), G.Graph(3, [])]
+    assert np.array_equal(_lib.adjacency_pool(gs, 1), np.concatenate([g.adj64() for g in gs]))
+    wide = gs + [G.cycle(65), G.complete(128), G.star(127)]
+    assert np.array_equal(_lib.adjacency_pool(wide, 2), np.concatenate([g.adj128() for g in wide]))
+    assert _lib.adjacency_pool([], 2).size == 0
+    odd = G.path(5)
+    odd.edges = [(np.int64(0), 1), [2, 3]]  # not tuples of int
+    assert np.array_equal(_lib.adjacency_pool([G.path(3), odd], 1),
+                          np.concatenate([G.path(3).adj64(), odd.adj64()]))
+    bad = G.path(4)
+    bad.edges = [(0, 7)]
+    with pytest.raises(IndexError):
+        _lib.adjacency_pool([bad], 1)
+    with pytest.raises(ValueError):
+        _lib.adjacency_pool([G.path(65)], 1)
