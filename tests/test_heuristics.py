@@ -51,3 +51,16 @@ def test_gpu_batch_heuristics_equal_host(handle, kind):
         htd, hpar = _lib.heuristic(g, kind, scores[i] if scores is not None else None)
         assert td[i] == htd, (g.name, kind)
         assert pars[i].tolist() == hpar.tolist(), (g.name, kind)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", [0, 1, 2])
+def test_gpu_rounds_at_the_word_and_warp_edges(handle, kind):
+    """A thread per vertex: vertex counts around 32, 64, 96 and 128, in one
+    launch with single vertices, a clique, a star and separate components."""
+    gs = [G.Graph(1, []), G.path(2), G.star(33), G.complete(32), G.cycle(64), G.tree_plus_edges(65, 9, 1),
+          G.random_geometric(96, 4.0, 2), G.tree_plus_edges(97, 40, 3), G.path(104), G.Graph(70, [(0, 69), (64, 1)])]
+    td, pars = handle.heuristic_batch(gs, kind)
+    for i, g in enumerate(gs):
+        htd, hpar = _lib.heuristic(g, kind)
+        assert td[i] == htd and pars[i].tolist() == hpar.tolist(), (i, g.name)
