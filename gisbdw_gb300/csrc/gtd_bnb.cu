@@ -51,7 +51,13 @@
 //    Split items: when a batch has fewer first-root items than the GPU has
 //    warps, an item is a pair (first root v, second root u) deciding C - v
 //    under root u at depth k - 1 (C - v connected; else the u = 0 item
-//    decides all of v), so a single graph uses n^2 warps.
+//    decides all of v), so a single graph uses n^2 warps. A larger batch
+//    changes over to split items at the end of the pass that leaves few
+//    (kSplitPerSm): one hard graph has 3 n first-root items for 3,648 warps,
+//    and the last ones decide how long the batch takes (48 graphs of 24..36
+//    vertices: 100 ms with first-root items to the end, 23 ms changed over).
+//    A done first-root item counts as its n pairs, an open one hands its
+//    budget to them.
 //    A success at level k improves the graph's best (atomicMin) and
 //    cancels every remaining item at levels >= k; when every candidate at
 //    level k has failed, the graph's proven lower bound becomes k + 1 and
@@ -122,9 +128,16 @@ constexpr int kIoExited = 200;           // d_io words: warps that left the curr
 constexpr int kIoPassDone = 202;         // d_io word: warps that finished the current pass
 constexpr int kIoPassGen = 203;          // d_io word: passes completed (released by the pass's last warp)
 constexpr int kIoPassStop = 204;         // d_io word: 1 when no further pass is needed
+constexpr int kIoSplitNow = 205;         // d_io word: 1 once the items are split
 constexpr uint64_t kFirstBudget = 1024;  // search nodes of an item's first run
 constexpr uint32_t kMaxDoublings = 30;   // an item's budget grows to at most 2^30 times the first
 constexpr uint32_t kItemDone = 0xFF;
+// A batch changes over to split items once fewer than this many first-root
+// items per SM are open (24 warps are resident): 32 leaves no warp of the next
+// passes idle. 8 / 16 / 24 / 32 / 64 per SM, ms: 48 graphs of 24..36 vertices
+// 67 / 23 / 23 / 23 / 23, 64 of 28..34 70 / 70 / 35 / 35 / 35, 256 of 28..34
+// - / 132 / - / 105 / 105, 300 of 16..36 - / 188 / - / 147 / 148.
+constexpr int kSplitPerSm = 32;
 constexpr int kRoundWindow = 3;          // levels run at a time per graph
 constexpr int kMaxRounds = 4096;
 
@@ -151,12 +164,15 @@ struct BnbParams {
   uint32_t memo_mask = 0;
   uint32_t* best = nullptr;        // per graph: k << 8 | root (kSeedRoot = seed tree)
   uint32_t* lbp = nullptr;         // per graph: proven lower bound
-  uint32_t* fails = nullptr;       // per graph x level: failed candidates
+  uint32_t* fails = nullptr;       // per graph x level: failed pairs (first root, second root)
   uint32_t* claim = nullptr;       // per graph x level: tree buffer taken
   uint8_t* item_state = nullptr;   // per graph x level x rank: kItemDone, or the item's budget doublings so far
+  uint8_t* split_state = nullptr;  // the same for split items (per second rank); null: items are never split
   uint64_t budget = 0;             // an item's first budget in search nodes (0 = unlimited)
   int window = 0;                  // levels run at a time below a graph's top level (0 = all)
-  int split = 0;                   // 1: an item is a pair (first root, second root)
+  int split = 0;                   // 1: an item is a pair (first root, second root) from the start
+  uint32_t split_below = 0;        // split once fewer first-root items than this are open
+  uint32_t* split_now = nullptr;   // set by the last warp of a pass
   uint32_t* unfinished = nullptr;  // items that used up their budget this round
   uint8_t* mini = nullptr;         // per warp: 2^kMiniMax-byte small-component DP table
   uint32_t* exited = nullptr;      // [0] warps that found no ticket left, [1] items started (this pass)
@@ -1073,11 +1089,18 @@ __device__ bool next_pass(const BnbParams& p, uint32_t pass) {
   }
   last = __shfl_sync(0xffffffffu, last, 0);
   if (last) {
-    uint32_t open = 0;
-    for (int g = lane; g < p.num_graphs; g += 32)
-      open += ld_relaxed_s32(p.status + g) != kBnbTimeout &&
-              ld_acquire_u32(p.lbp + g) < (ld_acquire_u32(p.best + g) >> 8);
+    uint32_t open = 0, items = 0;  // graphs, first-root items in their windows
+    for (int g = lane; g < p.num_graphs; g += 32) {
+      const uint32_t lb = ld_acquire_u32(p.lbp + g), best = ld_acquire_u32(p.best + g) >> 8;
+      if (ld_relaxed_s32(p.status + g) != kBnbTimeout && lb < best) {
+        ++open;
+        const uint32_t levels = best - lb;
+        items += static_cast<uint32_t>(p.graphs[g].n) *
+                 (p.window && levels > static_cast<uint32_t>(p.window) ? static_cast<uint32_t>(p.window) : levels);
+      }
+    }
     open = __reduce_add_sync(0xffffffffu, open);
+    items = __reduce_add_sync(0xffffffffu, items);
     if (lane == 0) {
       const bool stop = open == 0 || ld_relaxed_s32(p.error) != 0 || pass + 1 >= static_cast<uint32_t>(kMaxRounds);
       *reinterpret_cast<volatile uint32_t*>(p.ticket) = 0u;
@@ -1086,6 +1109,8 @@ __device__ bool next_pass(const BnbParams& p, uint32_t pass) {
       reinterpret_cast<volatile uint32_t*>(p.exited)[1] = 0u;
       *reinterpret_cast<volatile uint32_t*>(p.pass_done) = 0u;
       *reinterpret_cast<volatile uint32_t*>(p.pass_stop) = stop ? 1u : 0u;
+      if (p.split_state && items < p.split_below)
+        *reinterpret_cast<volatile uint32_t*>(p.split_now) = 1u;
       __threadfence();
       st_release_u32(p.pass_gen, pass + 1u);
     }
@@ -1113,10 +1138,14 @@ __global__ void __launch_bounds__(32 * kBnbWarps, 6) bnb_kernel(const __grid_con
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   WarpMem* w = reinterpret_cast<WarpMem*>(smem) + warp;
   int cur_g = -1;
-  const uint32_t S = p.split ? static_cast<uint32_t>(p.max_n) : 1u;  // second roots per first root
+  for (uint32_t pass = 0;; ++pass) {
+  uint32_t split_now = 0;
+  if (lane == 0)
+    split_now = p.split || (p.split_state && ld_acquire_u32(p.split_now) != 0u);
+  const bool split = __shfl_sync(0xffffffffu, split_now, 0) != 0u;
+  const uint32_t S = split ? static_cast<uint32_t>(p.max_n) : 1u;  // second roots per first root
   const uint32_t per_level = static_cast<uint32_t>(p.max_n) * S * static_cast<uint32_t>(p.num_graphs);
   const uint32_t total = per_level * static_cast<uint32_t>(p.levels);
-  for (uint32_t pass = 0;; ++pass) {
   for (;;) {
     uint32_t item = 0;
     if (lane == 0)
@@ -1134,12 +1163,21 @@ __global__ void __launch_bounds__(32 * kBnbWarps, 6) bnb_kernel(const __grid_con
     const int r = static_cast<int>(rr / S), r2 = static_cast<int>(rr % S);
     const BnbGraph G = p.graphs[g];
     const int k = G.ub0 - 1 - li;
-    if (r >= G.n || r2 >= (p.split ? G.n : 1) || k < G.lb0)
+    if (r >= G.n || r2 >= (split ? G.n : 1) || k < G.lb0)
       continue;
-    const size_t item_idx = ((size_t(g) * p.levels + li) * p.max_n + r) * S + r2;
-    const uint32_t istate = p.item_state[item_idx];
+    const size_t first_idx = (size_t(g) * p.levels + li) * p.max_n + r;
+    uint32_t istate = p.item_state[first_idx];
     if (istate == kItemDone)
       continue;  // finished in an earlier round
+    uint8_t* state = p.item_state + first_idx;
+    if (split) {  // a pair starts with its first root's budget
+      state = p.split_state + first_idx * S + r2;
+      const uint32_t own = *state;
+      if (own == kItemDone)
+        continue;
+      if (own != 0)
+        istate = own;
+    }
     int useful = 0;
     if (lane == 0) {
       const unsigned long long now = global_ns();
@@ -1160,7 +1198,7 @@ __global__ void __launch_bounds__(32 * kBnbWarps, 6) bnb_kernel(const __grid_con
       // best only falls, the proven bound only rises and a timeout is final:
       // a useless item stays useless
       if (lane == 0)
-        p.item_state[item_idx] = kItemDone;
+        *state = kItemDone;
       continue;
     }
     if (g != cur_g) {
@@ -1191,7 +1229,7 @@ __global__ void __launch_bounds__(32 * kBnbWarps, 6) bnb_kernel(const __grid_con
     bool ok = false;
     int u = -1;  // fixed second root (split items)
     const bool skip = G.n >= 3 && s.dominated(v, fl, fh);  // another root is at least as good
-    if (!skip && !p.split) {
+    if (!skip && !split) {
       ok = s.decide(fl, fh, k, v, nullptr);
     } else if (!skip) {
       // Split item (v, order[r2]): when C - v is connected, decide C - v under
@@ -1240,9 +1278,9 @@ __global__ void __launch_bounds__(32 * kBnbWarps, 6) bnb_kernel(const __grid_con
       atomicAdd(p.nodes + g, s.nodes);
       if (s.yielded && !s.timed_out && !s.cancelled) {
         atomicAdd(p.unfinished, 1u);  // run again next pass with twice the budget
-        p.item_state[item_idx] = static_cast<uint8_t>(min(istate + 1, kMaxDoublings));
+        *state = static_cast<uint8_t>(min(istate + 1, kMaxDoublings));
       } else {
-        p.item_state[item_idx] = kItemDone;
+        *state = kItemDone;
       }
       if (s.timed_out) {
         atomicExch(p.status + g, kBnbTimeout);
@@ -1250,9 +1288,10 @@ __global__ void __launch_bounds__(32 * kBnbWarps, 6) bnb_kernel(const __grid_con
         if (ok) {
           if (publish)
             atomicMin(p.best + g, (static_cast<uint32_t>(k) << 8) | static_cast<uint32_t>(v));
-        } else if (atomicAdd(p.fails + size_t(g) * p.levels + li, 1u) + 1 ==
-                   static_cast<uint32_t>(p.split ? G.n * G.n : G.n)) {
-          atomicMax(p.lbp + g, static_cast<uint32_t>(k + 1));  // every root failed: td > k
+        } else {
+          const uint32_t pairs = split ? 1u : static_cast<uint32_t>(G.n);
+          if (atomicAdd(p.fails + size_t(g) * p.levels + li, pairs) + pairs == static_cast<uint32_t>(G.n * G.n))
+            atomicMax(p.lbp + g, static_cast<uint32_t>(k + 1));  // every root failed: td > k
         }
         check_proved(p, g);
       }
@@ -1519,8 +1558,12 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
     first_items += size_t(descs[i].n) * std::min(levels, kRoundWindow);
   const int split = (first_items < size_t(h->num_sms) * 16 &&
                      size_t(count) * levels * max_n * max_n < (size_t(1) << 31)) ? 1 : 0;
+  // Larger batches change over to split items when as few first-root items are
+  // left (a byte per pair of roots: at most 256 MB).
+  const size_t firsts = size_t(count) * levels * max_n, pairs = firsts * size_t(max_n);
+  const bool may_split = split || pairs <= (size_t(1) << 28);
   const size_t S = split ? size_t(max_n) : 1;
-  if ((s = grow(h, &B.i8, &B.i8_cap, size_t(count) * levels * max_n * (1 + S))) != GTD_OK) return s;
+  if ((s = grow(h, &B.i8, &B.i8_cap, 2 * firsts + (may_split ? pairs : 0))) != GTD_OK) return s;
   if ((s = grow(h, &B.u64, &B.u64_cap, 3 * size_t(count) + 1)) != GTD_OK) return s;
   int32_t* d_seed_parent = B.i32;
   int32_t* d_parent = B.i32 + pool_len;
@@ -1545,8 +1588,7 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   GTD_CUDA(h, cudaMemcpyAsync(d_best, best.data(), count * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream));
   GTD_CUDA(h, cudaMemcpyAsync(d_lbp, lbp.data(), count * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream));
   GTD_CUDA(h, cudaMemsetAsync(d_fails, 0, 2 * size_t(count) * levels * sizeof(uint32_t), h->stream));
-  GTD_CUDA(h, cudaMemsetAsync(B.i8 + size_t(count) * levels * max_n, 0, size_t(count) * levels * max_n * S,
-                              h->stream));
+  GTD_CUDA(h, cudaMemsetAsync(B.i8 + firsts, 0, firsts + (may_split ? pairs : 0), h->stream));
   GTD_CUDA(h, cudaMemsetAsync(B.memo, 0, slots * count * sizeof(uint4), h->stream));
   GTD_CUDA(h, cudaMemsetAsync(d_status, 0, count * sizeof(int32_t), h->stream));
   GTD_CUDA(h, cudaMemsetAsync(B.u64, 0, 3 * size_t(count) * sizeof(uint64_t), h->stream));
@@ -1567,8 +1609,11 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   p.fails = d_fails;
   p.claim = d_claim;
   p.lvl_parent = B.i8;
-  p.item_state = reinterpret_cast<uint8_t*>(B.i8 + size_t(count) * levels * max_n);
+  p.item_state = reinterpret_cast<uint8_t*>(B.i8 + firsts);
+  p.split_state = may_split ? p.item_state + firsts : nullptr;
   p.split = split;
+  p.split_below = static_cast<uint32_t>(h->num_sms) * kSplitPerSm;
+  p.split_now = reinterpret_cast<uint32_t*>(h->d_io + kIoSplitNow);
   p.unfinished = reinterpret_cast<uint32_t*>(h->d_io + kIoUnfinished);
   p.exited = reinterpret_cast<uint32_t*>(h->d_io + kIoExited);
   p.window = (opts && opts->window > 0) ? opts->window : kRoundWindow;
@@ -1609,7 +1654,7 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   p.pass_gen = reinterpret_cast<uint32_t*>(h->d_io + kIoPassGen);
   p.pass_stop = reinterpret_cast<uint32_t*>(h->d_io + kIoPassStop);
   p.pass_wait_ns = p.deadline_ns + 30ull * 1000 * 1000 * 1000;
-  GTD_CUDA(h, cudaMemsetAsync(h->d_io + kIoExited, 0, 5 * sizeof(int32_t), h->stream));
+  GTD_CUDA(h, cudaMemsetAsync(h->d_io + kIoExited, 0, 6 * sizeof(int32_t), h->stream));
   GTD_CUDA(h, cudaEventRecord(h->ev[0], h->stream));
   {
     void* args[] = {&p};

@@ -204,3 +204,15 @@ def test_smallest_graphs_every_solver(handle):
     assert htd.tolist() == want  # greedy is optimal on these
     for g, t, par in zip(gs, htd, hpar):
         assert check_tree(g, int(t), par)
+
+
+@pytest.mark.parametrize("easy,hard,n", [(60, 1, 24), (60, 3, 25), (20, 60, 18), (300, 8, 22)])
+@pytest.mark.parametrize("first_budget", [0, 64])
+def test_bnb_batch_that_ends_in_split_items(handle, easy, hard, n, first_budget):
+    # more first-root items than warps at the start; the easy graphs go first,
+    # the hard ones are finished as (first root, second root) items
+    gs = [G.tree_plus_edges(16 + s % 3, 2 + s % 3, s) for s in range(easy)]
+    gs += [G.sparse_connected(n - s % 2, 90 + s) for s in range(hard)]
+    res = _check(handle, gs, **({"first_budget": first_budget} if first_budget else {}))
+    dtd, _, _ = handle.dp_solve_batch(gs)
+    assert res["td"].tolist() == dtd.tolist()
