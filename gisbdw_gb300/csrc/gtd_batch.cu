@@ -64,13 +64,20 @@ constexpr int kBatchSmallMaxN = 16;
 //    the autotuner's measured mixed-kernel efficiency at c with its own
 //    occupancy share taken out (what is left: the dispatch's extra work);
 // and the least predicted time wins. No rates: 10 bits. force_cap > 0 (the
-// autotuner's own measurement) plans a mixed launch at that cap.
+// autotuner's own measurement) plans a mixed launch at that cap. A size that
+// leaves more than kDpMaxHigh high vertices is raised to the least that does
+// not, as in a single solve (n = 35 needs 9 bits, n = 36 needs 10).
 void pick_tile_bits(gtd_handle h, const gtd_graph_desc* descs, int count, const gtd_dp_batch_opts* opts, Plan& P,
                     int force_cap = 0) {
   std::vector<int> count_by_n(GTD_DP_MAX_N + 1, 0);
-  for (int i = 0; i < count; ++i)
+  int max_n = 0;
+  for (int i = 0; i < count; ++i) {
     ++count_by_n[descs[i].n];
+    max_n = std::max(max_n, descs[i].n);
+  }
+  const int lb_min = std::max(kTuneLbMin, max_n - kDpMaxHigh);
   auto uniform = [&](int lb) {
+    lb = std::max(lb, lb_min);
     P.lb = lb;
     P.mixed = false;
     for (int n = 0; n <= GTD_DP_MAX_N; ++n)
@@ -113,7 +120,7 @@ void pick_tile_bits(gtd_handle h, const gtd_graph_desc* descs, int count, const 
   int occ_one[kTuneLbMax + 1] = {};
   for (int lb = kTuneLbMin; lb <= kTuneLbMax; ++lb)
     occ_one[lb] = std::max(1, dp_tile_occupancy(lb, high_at(lb)));
-  for (int c = kTuneLbMin; c <= kTuneLbMax; ++c) {
+  for (int c = lb_min; c <= kTuneLbMax; ++c) {
     const int occ_mixed = dp_mixed_occupancy(c, high_at(kTuneLbMin));
     const float eff = h->tune_mixed_eff[c];
     if (eff <= 0 || occ_mixed < 1)
@@ -127,7 +134,7 @@ void pick_tile_bits(gtd_handle h, const gtd_graph_desc* descs, int count, const 
       if (!count_by_n[n])
         continue;
       double best_t = -1;
-      for (int lb = kTuneLbMin; lb <= c; ++lb) {
+      for (int lb = std::max(kTuneLbMin, n - kDpMaxHigh); lb <= c; ++lb) {
         const double t = t_of(n, lb) * std::max(1.0, double(occ_one[lb]) / occ_mixed);
         if (best_t < 0 || t < best_t) {
           best_t = t;

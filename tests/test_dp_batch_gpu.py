@@ -7,6 +7,7 @@ import pytest
 
 from gisbdw_gb300 import InvalidArgument, _lib
 from gisbdw_gb300 import graphs as G
+from gisbdw_gb300.validate import check_tree
 
 pytestmark = pytest.mark.gpu
 
@@ -126,3 +127,13 @@ def test_planner_never_mixes_without_a_measured_gain(port):
     for g, t in zip(gs, td):
         assert t == port.dp_solve(g)[0]
     h.close()
+
+
+def test_batch_tile_bits_too_small_for_the_largest_graph(handle):
+    # 8-bit tiles would leave 27 high vertices at n = 35: raised to 9 bits
+    gs = [G.cycle(35), G.path(20)]
+    td, parents, stats = handle.dp_solve_batch(gs, tile_bits=8)
+    assert stats["tile_bits_by_n"][35] == 9 and stats["tile_bits"] == 9
+    assert td.tolist() == [7, 5]
+    for g, t, par in zip(gs, td, parents):
+        assert check_tree(g, t, par)
