@@ -145,10 +145,12 @@ int default_tile_bits(int n) { return n >= 26 ? 11 : 10; }
 constexpr int kLevelMaxN = 28;
 
 // Allocates (or grows) the table and flag buffers and enqueues the
-// validation, DP and tree kernels for one graph. Outputs go to
-// td/parent/order (device pointers, possibly the handle's IO block).
-gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, int n, const gtd_dp_opts* opts,
-                      int32_t* d_td, int32_t* d_parent, int32_t* d_order) {
+// validation, DP and tree kernels for one graph. The adjacency is at d_adj,
+// or h_adj's masks go to the first kernel by value (which puts them down at
+// d_adj). Outputs go to td/parent/order (device pointers, or pinned host
+// memory), the error words to `report` as well when it is given.
+gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, const uint64_t* h_adj, int n, const gtd_dp_opts* opts,
+                      int32_t* d_td, int32_t* d_parent, int32_t* d_order, int32_t* report) {
   const int tile_bits = (opts && opts->tile_bits > 0) ? opts->tile_bits : default_tile_bits(n);
   const DpLayout L = make_dp_layout(n, tile_bits);
   const bool stall = take_stall_fault();  // test injection: needs a kernel whose tiles wait
@@ -197,6 +199,14 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, int n, const gtd_dp_o
   p.td_out = d_td;
   p.parent_out = d_parent;
   p.order_out = d_order;
+  p.report = report;
+  DpInput in;
+  in.clear = h->d_io;
+  in.clear_words = kIoWords;
+  if (h_adj) {
+    in.by_value = 1;
+    std::memcpy(in.adj, h_adj, sizeof(uint64_t) * n);
+  }
 
   p.kid_rows = nh;
   int& dp_occ = h->dp_occ[by_level ? 0 : p.lb][nh];
@@ -211,23 +221,25 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, int n, const gtd_dp_o
   if (ctas > p.total_groups || small)
     ctas = small ? 1 : p.total_groups;
 
-  GTD_CUDA(h, cudaMemsetAsync(h->d_io, 0, kIoWords * sizeof(int32_t), h->stream));
   if (take_poison_fault())  // test injection: every byte must be written before it is read
     GTD_CUDA(h, cudaMemsetAsync(h->d_table, 0xFF, h->table_cap, h->stream));
+  if (!small)
+    GTD_CUDA(h, dp_launch_validate(p, h->stream, in));
   if (stall)  // ticket 0 (the level-0 group) is never taken
     GTD_CUDA(h, cudaMemsetAsync(h->d_io + kIoTicket, 1, 1, h->stream));
-  if (!small)
-    GTD_CUDA(h, dp_launch_validate(p, h->stream));
   GTD_CUDA(h, cudaEventRecord(h->ev[0], h->stream));
-  GTD_CUDA(h, small      ? dp_launch_small(p, n, h->stream)
+  GTD_CUDA(h, small      ? dp_launch_small(p, n, h->stream, in)
               : by_level ? dp_launch_levels(p, static_cast<int>(ctas), h->stream)
                          : dp_launch_tiles(p, static_cast<int>(ctas), h->stream));
   GTD_CUDA(h, cudaEventRecord(h->ev[1], h->stream));
-  if (!small)  // the small kernel builds the tree itself
+  if (!small) {  // the small kernel builds the tree itself
     GTD_CUDA(h, dp_launch_tree(p, h->stream));
-  GTD_CUDA(h, cudaEventRecord(h->ev[2], h->stream));
+    GTD_CUDA(h, cudaEventRecord(h->ev[2], h->stream));
+  }
 
   h->last_params = p;
+  h->last_params.report = nullptr;
+  h->tree_timed = !small;
   h->have_table = true;
   h->pending_stats = true;
   gtd_dp_stats& st = h->last_stats;
@@ -259,7 +271,7 @@ void collect_stats(gtd_handle h) {
   float a = 0, b = 0;
   if (cudaEventElapsedTime(&a, h->ev[0], h->ev[1]) == cudaSuccess)
     h->last_stats.dp_ms = a;
-  if (cudaEventElapsedTime(&b, h->ev[1], h->ev[2]) == cudaSuccess)
+  if (h->tree_timed && cudaEventElapsedTime(&b, h->ev[1], h->ev[2]) == cudaSuccess)
     h->last_stats.tree_ms = b;
   h->pending_stats = false;
 }
@@ -351,8 +363,7 @@ gtd_status gtd_destroy(gtd_handle h) {
     cudaFree(h->d_tile_map);
     cudaFree(h->d_level_base);
     cudaFree(h->d_badj);
-    cudaFree(h->d_btd);
-    cudaFree(h->d_bparent);
+    cudaFree(h->d_bout);
     cudaFree(h->d_scratch);
     cudaFree(h->d_bu);
     if (h->h_pinned)
@@ -394,15 +405,11 @@ gtd_status gtd_dp_solve(gtd_handle h, const uint64_t* adj, int n, int32_t* td_ou
       *stats = gtd_dp_stats{};
     return GTD_OK;
   }
-  uint64_t* h_adj = static_cast<uint64_t*>(h->h_pinned);
-  std::memcpy(h_adj, adj, sizeof(uint64_t) * n);
-  GTD_CUDA(h, cudaMemcpyAsync(h->d_adj, h_adj, sizeof(uint64_t) * n, cudaMemcpyHostToDevice, h->stream));
-  s = dp_enqueue(h, h->d_adj, n, opts, h->d_io + kIoTd, h->d_io + kIoParent, h->d_io + kIoOrder);
+  // the last kernel writes its results to the pinned block
+  int32_t* h_io = reinterpret_cast<int32_t*>(static_cast<char*>(h->h_pinned) + kPinnedIo);
+  s = dp_enqueue(h, h->d_adj, adj, n, opts, h_io + kIoTd, h_io + kIoParent, h_io + kIoOrder, h_io + kIoError);
   if (s != GTD_OK)
     return s;
-  int32_t* h_io = reinterpret_cast<int32_t*>(static_cast<char*>(h->h_pinned) + kPinnedIo);
-  GTD_CUDA(h, cudaMemcpyAsync(h_io, h->d_io, (kIoOrder + 64) * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                              h->stream));
   GTD_CUDA(h, cudaStreamSynchronize(h->stream));
   collect_stats(h);
   s = map_device_error(h, h_io[kIoError], h_io[kIoError + 1]);
@@ -430,7 +437,7 @@ gtd_status gtd_dp_solve_device(gtd_handle h, const uint64_t* d_adj, int n, int32
   if (n < 2 || n > GTD_DP_MAX_N)
     return fail(h, GTD_INVALID_ARG, "device solve needs n in [2, " + std::to_string(GTD_DP_MAX_N) + "]");
   DeviceGuard g(h->device);
-  return dp_enqueue(h, d_adj, n, opts, d_td, d_parent, d_order);
+  return dp_enqueue(h, d_adj, nullptr, n, opts, d_td, d_parent, d_order, nullptr);
 }
 
 gtd_status gtd_sync(gtd_handle h, gtd_dp_stats* stats) {

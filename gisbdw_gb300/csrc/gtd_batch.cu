@@ -256,7 +256,9 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
   make_plan(P, descs, count, !(opts && opts->tile_bits > 0) && force_cap == 0);
   const int lb = P.lb;
   const uint64_t timeout = (opts && opts->timeout_ns) ? opts->timeout_ns : 10ull * 1000 * 1000 * 1000;
-  int occ = P.mixed ? dp_mixed_occupancy(lb, P.kid_rows) : dp_tile_occupancy(lb, P.kid_rows);
+  int occ = 1;
+  if (P.total_groups > 0)
+    occ = P.mixed ? dp_mixed_occupancy(lb, P.kid_rows) : dp_tile_occupancy(lb, P.kid_rows);
   if (opts && opts->ctas_per_sm > 0 && opts->ctas_per_sm < occ)
     occ = opts->ctas_per_sm;
   if (occ < 1)
@@ -372,7 +374,9 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
     bp.epoch = kGraphEpoch;
     cudaGraph_t graph = nullptr;
     GTD_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t ce = cudaMemsetAsync(h->d_flags, 0, size_t(P.total_groups) * sizeof(uint32_t), h->stream);
+    cudaError_t ce = cudaSuccess;
+    if (P.total_groups > 0)
+      ce = cudaMemsetAsync(h->d_flags, 0, size_t(P.total_groups) * sizeof(uint32_t), h->stream);
     if (ce == cudaSuccess)
       ce = cudaMemsetAsync(h->d_io, 0, 4 * sizeof(int32_t), h->stream);
     if (ce == cudaSuccess)
@@ -515,20 +519,17 @@ gtd_status solve_batch_host(gtd_handle h, const gtd_graph_desc* descs, int count
   if (s != GTD_OK)
     return s;
   GTD_CUDA(h, ensure_field(&h->d_badj, &h->badj_cap, size_t(pool_len)));
-  GTD_CUDA(h, ensure_field(&h->d_btd, &h->btd_cap, size_t(count)));
-  GTD_CUDA(h, ensure_field(&h->d_bparent, &h->bparent_cap, size_t(pool_len)));
+  GTD_CUDA(h, ensure_field(&h->d_bout, &h->bout_cap, size_t(count) + size_t(pool_len)));
 
   char* stage = static_cast<char*>(h->h_bstage);
   std::memcpy(stage, adj_pool, adj_bytes);
   GTD_CUDA(h, cudaMemcpyAsync(h->d_badj, stage, adj_bytes, cudaMemcpyHostToDevice, h->stream));
-  s = batch_enqueue(h, descs, count, h->d_badj, h->d_btd, h->d_bparent, opts, force_cap);
+  s = batch_enqueue(h, descs, count, h->d_badj, h->d_bout, h->d_bout + count, opts, force_cap);
   if (s != GTD_OK)
     return s;
   int32_t* h_td = reinterpret_cast<int32_t*>(stage + adj_bytes);
   int32_t* h_par = h_td + count;
-  GTD_CUDA(h, cudaMemcpyAsync(h_td, h->d_btd, count * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-  GTD_CUDA(h, cudaMemcpyAsync(h_par, h->d_bparent, size_t(pool_len) * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                              h->stream));
+  GTD_CUDA(h, cudaMemcpyAsync(h_td, h->d_bout, out_bytes, cudaMemcpyDeviceToHost, h->stream));
   s = batch_finish(h, nullptr);
   if (s != GTD_OK)
     return s;

@@ -236,7 +236,7 @@ __device__ __forceinline__ uint32_t spread5(uint32_t a) {
 // SmallSets of the word whose position 0 is the set S0 of k <= 2 vertices
 // >= 5 (vertices >= n are padding, isolated).
 __device__ __noinline__ SmallSets small_sets(uint64_t S0, int k, const uint64_t* adj, int n) {
-  auto at = [&](int v) -> uint64_t { return v < n ? __ldg(adj + v) : 0ull; };
+  auto at = [&](int v) -> uint64_t { return v < n ? adj[v] : 0ull; };
   constexpr uint32_t kSingles = 0x00010116u, kPairs = 0x01161668u;  // |x| = 1, 2
   SmallSets s;
   if (k == 2) {
@@ -280,8 +280,23 @@ __device__ __forceinline__ bool adjacency_ok(const uint64_t* adj, int n) {
   return __all_sync(0xffffffffu, ok);
 }
 
+// What the first kernel of a single solve does with its input (one CTA; a
+// barrier before the adjacency or the control words are used). Together with
+// results written to pinned memory by the last kernel, a copy in, a memset, a
+// copy out and an event fewer per call (n = 12: 50 -> 37 us, n = 20: 104 -> 95).
+__device__ __forceinline__ void take_input(const DpBatchParams& p, const DpInput& in) {
+  for (int i = threadIdx.x; i < in.clear_words; i += blockDim.x)
+    in.clear[i] = 0;
+  if (in.by_value && threadIdx.x < p.single.n)
+    const_cast<uint64_t*>(p.adj)[threadIdx.x] = in.adj[threadIdx.x];
+}
+
 // Checks every graph, one warp per graph.
-__global__ void dp_validate_kernel(const __grid_constant__ DpBatchParams p) {
+__global__ void dp_validate_kernel(const __grid_constant__ DpBatchParams p, const __grid_constant__ DpInput in) {
+  if (!p.graphs) {
+    take_input(p, in);
+    __syncthreads();
+  }
   const int g = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (g >= p.num_graphs)
     return;  // the whole warp
@@ -951,10 +966,11 @@ struct TreeMem {
 // the depth of the tree times one load's latency and the component searches
 // (n = 30: 61 us when each component took a round of its own).
 template <class Ctx>
-__device__ bool build_tree(const DpBatchParams& p, const DpGraph& G, const Ctx& ctx, TreeMem& m, uint64_t query) {
+__device__ bool build_tree(const DpBatchParams& p, const DpGraph& G, const uint64_t* adj, const Ctx& ctx, TreeMem& m,
+                           uint64_t query) {
   const int lane = threadIdx.x & 31, n = G.n;
-  const uint64_t adj_lo = lane < n ? __ldg(p.adj + G.adj_off + lane) : 0ull;
-  const uint64_t adj_hi = lane + 32 < n ? __ldg(p.adj + G.adj_off + lane + 32) : 0ull;
+  const uint64_t adj_lo = lane < n ? adj[lane] : 0ull;
+  const uint64_t adj_hi = lane + 32 < n ? adj[lane + 32] : 0ull;
   const Chain chain = load_chain(ctx, query);
   int height = 0, count = 0;      // count: components of the next depth
   uint64_t in_next = 0;           // their union
@@ -1101,6 +1117,14 @@ __device__ bool build_tree(const DpBatchParams& p, const DpGraph& G, const Ctx& 
   return true;
 }
 
+// The error words of a single solve for the host (its graph is warp 0's).
+__device__ __forceinline__ void report_error(const DpBatchParams& p) {
+  if (p.report && blockIdx.x == 0 && threadIdx.x == 0) {
+    p.report[0] = ld_relaxed_s32(p.error);
+    p.report[1] = ld_relaxed_s32(p.error + 1);
+  }
+}
+
 __global__ void __launch_bounds__(32 * kTreeWarps)
     dp_tree_kernel(const __grid_constant__ DpBatchParams p) {
   __shared__ Binom sBinom;
@@ -1108,19 +1132,19 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
   fill_binom(sBinom);
   __syncthreads();
   const int warp = threadIdx.x >> 5;
-  if (ld_relaxed_s32(p.error) != 0)
-    return;
-  for (int g = blockIdx.x * kTreeWarps + warp; g < p.num_graphs; g += gridDim.x * kTreeWarps) {
+  const bool failed = ld_relaxed_s32(p.error) != 0;
+  for (int g = blockIdx.x * kTreeWarps + warp; g < p.num_graphs && !failed; g += gridDim.x * kTreeWarps) {
     const DpGraph G = p.graphs ? p.graphs[g] : p.single;
     level_offsets(sBinom, G.nh, mem[warp].off);
     const TreeCtx ctx{sBinom, mem[warp].off, p.table + G.table_off, G.lb, G.n};
-    if (!build_tree(p, G, ctx, mem[warp], p.query ? p.query : (1ull << G.n) - 1ull)) {
+    if (!build_tree(p, G, p.adj + G.adj_off, ctx, mem[warp], p.query ? p.query : (1ull << G.n) - 1ull)) {
       if ((threadIdx.x & 31) == 0)
         raise_error(p.error, kDevNoRoot, g);
-      return;
+      break;
     }
     __syncwarp();
   }
+  report_error(p);
 }
 
 // ---------------------------------------------------------------------------
@@ -1151,7 +1175,8 @@ constexpr size_t small_smem(int n) { return size_t(small_words(n)) * (3 * 4 + 2)
 // costs a microsecond a level in the other kernels: bound by the latency of a
 // level's word chain, about 1 us (n = 12, all of check, table and tree: 18 us
 // against 4 + 21 + 14; n = 16: 25 against 4 + 30 + 16; n = 18: 49 against 58).
-__global__ void __launch_bounds__(512) dp_small_kernel(const __grid_constant__ DpBatchParams p, int max_n) {
+__global__ void __launch_bounds__(512)
+    dp_small_kernel(const __grid_constant__ DpBatchParams p, int max_n, const __grid_constant__ DpInput in) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ Binom binom;
   __shared__ TreeMem mem;
@@ -1159,16 +1184,20 @@ __global__ void __launch_bounds__(512) dp_small_kernel(const __grid_constant__ D
   const uint32_t tid = threadIdx.x, threads = blockDim.x;
   const int g = p.first_graph + static_cast<int>(blockIdx.x);
   const DpGraph G = p.graphs ? p.graphs[g] : p.single;
-  const uint64_t* const adj = p.adj + G.adj_off;
+  __shared__ uint64_t adj[kDpSmallMaxN];
   const int n = G.n, m = n > 5 ? n - 5 : 0;
   const uint32_t words = 1u << m, stride = small_words(max_n);
   uint32_t* const p0 = reinterpret_cast<uint32_t*>(smem);
   uint32_t* const p1 = p0 + stride;
   uint32_t* const pc = p1 + stride;
   uint16_t* const order = reinterpret_cast<uint16_t*>(pc + stride);
+  if (!p.graphs)
+    take_input(p, in);
+  if (tid < n)
+    adj[tid] = in.by_value ? in.adj[tid] : p.adj[G.adj_off + tid];
   fill_binom(binom);
+  __syncthreads();
   if (tid < 32) {
-    __syncwarp();
     level_offsets(binom, m, mem.off);
     const bool bad = !adjacency_ok(adj, n);
     if (tid == 0) {
@@ -1178,8 +1207,10 @@ __global__ void __launch_bounds__(512) dp_small_kernel(const __grid_constant__ D
     }
   }
   __syncthreads();
-  if (sBad)
+  if (sBad) {
+    report_error(p);
     return;
+  }
   for (uint32_t w = tid; w < words; w += threads)
     order[mem.off[__popc(w)] + rank_colex(binom, w)] = static_cast<uint16_t>(w);
   for (int j = 0; j <= m; ++j) {
@@ -1202,8 +1233,9 @@ __global__ void __launch_bounds__(512) dp_small_kernel(const __grid_constant__ D
   __syncthreads();
   if (tid < 32) {
     const SmallCtx ctx{p0, p1, n};
-    if (!build_tree(p, G, ctx, mem, (1ull << n) - 1ull) && tid == 0)
+    if (!build_tree(p, G, adj, ctx, mem, (1ull << n) - 1ull) && tid == 0)
       raise_error(p.error, kDevNoRoot, g);
+    report_error(p);
   } else if (p.table) {
     uint32_t* const out = reinterpret_cast<uint32_t*>(p.table + G.table_off);
     for (uint32_t t = tid - 32; t < words; t += threads - 32) {
@@ -1247,8 +1279,8 @@ int dp_tile_occupancy(int lb, int kid_rows) {
   }
 }
 
-cudaError_t dp_launch_validate(const DpBatchParams& p, cudaStream_t s) {
-  dp_validate_kernel<<<(p.num_graphs + 3) / 4, 128, 0, s>>>(p);  // one warp per graph
+cudaError_t dp_launch_validate(const DpBatchParams& p, cudaStream_t s, const DpInput& in) {
+  dp_validate_kernel<<<(p.num_graphs + 3) / 4, 128, 0, s>>>(p, in);  // one warp per graph
   return cudaGetLastError();
 }
 
@@ -1263,7 +1295,7 @@ int dp_mixed_occupancy(int lb, int kid_rows) {
                       smem_layout_for(kDpMinTileBits, kDpMaxTileBits, kDpMaxHigh));
 }
 
-cudaError_t dp_launch_small(const DpBatchParams& p, int max_n, cudaStream_t s) {
+cudaError_t dp_launch_small(const DpBatchParams& p, int max_n, cudaStream_t s, const DpInput& in) {
   const size_t smem = small_smem(max_n);
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(dp_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1274,7 +1306,7 @@ cudaError_t dp_launch_small(const DpBatchParams& p, int max_n, cudaStream_t s) {
   // threads: the words of the widest level, 64 to 512 (128 for many graphs,
   // which fill the GPU side by side)
   const int threads = max_n <= 13 ? 64 : max_n == 14 || p.num_graphs > 1 ? 128 : max_n == 15 ? 256 : 512;
-  dp_small_kernel<<<p.num_graphs, threads, smem, s>>>(p, max_n);
+  dp_small_kernel<<<p.num_graphs, threads, smem, s>>>(p, max_n, in);
   return cudaGetLastError();
 }
 

@@ -49,13 +49,24 @@ struct DpBatchParams {
   int32_t* td_out = nullptr;
   int32_t* parent_out = nullptr;
   int32_t* order_out = nullptr;
+  int32_t* report = nullptr;        // error code and info once the tree is built (host memory; may be null)
+};
+
+// What a single solve hands its first kernel instead of copying and clearing
+// beforehand: the adjacency by value (put down at p.adj for the kernels after
+// it) and the control words to zero.
+struct DpInput {
+  uint64_t adj[kDpMaxN] = {};
+  int32_t by_value = 0;      // 1: adj holds the graph's masks
+  int32_t clear_words = 0;
+  int32_t* clear = nullptr;
 };
 
 // CTAs per SM with tiles of lb bits and up to kid_rows high vertices, and of
 // the mixed-tile-size kernel with tiles of up to lb bits.
 int dp_tile_occupancy(int lb, int kid_rows);
 int dp_mixed_occupancy(int lb, int kid_rows);
-cudaError_t dp_launch_validate(const DpBatchParams& p, cudaStream_t s);
+cudaError_t dp_launch_validate(const DpBatchParams& p, cudaStream_t s, const DpInput& in = DpInput{});
 cudaError_t dp_launch_fill_tile_map(const DpBatchParams& p, cudaStream_t s);
 cudaError_t dp_launch_tiles(const DpBatchParams& p, int ctas, cudaStream_t s);
 // The level kernel (single graph, tiles of kDpLevelTileBits): total_groups
@@ -65,7 +76,7 @@ cudaError_t dp_launch_levels(const DpBatchParams& p, int ctas, cudaStream_t s);
 // The small kernel: p.num_graphs graphs, from p.first_graph on, of at most
 // max_n <= kDpSmallMaxN vertices, checked, solved and reconstructed; p.table
 // (tiles of kDpSmallTileBits) may be null.
-cudaError_t dp_launch_small(const DpBatchParams& p, int max_n, cudaStream_t s);
+cudaError_t dp_launch_small(const DpBatchParams& p, int max_n, cudaStream_t s, const DpInput& in = DpInput{});
 cudaError_t dp_launch_tree(const DpBatchParams& p, cudaStream_t s);
 cudaError_t dp_launch_labels(const DpBatchParams& p, const uint64_t* subsets, int count, int32_t* td_out,
                              uint64_t* roots_out, cudaStream_t s);

@@ -68,10 +68,8 @@ struct gtd_handle_s {
   size_t level_base_cap = 0;
   uint64_t* d_badj = nullptr;
   size_t badj_cap = 0;
-  int32_t* d_btd = nullptr;
-  size_t btd_cap = 0;
-  int32_t* d_bparent = nullptr;
-  size_t bparent_cap = 0;
+  int32_t* d_bout = nullptr;  // td of every graph, then the parents
+  size_t bout_cap = 0;
   void* h_bstage = nullptr;  // pinned: adjacency pool in, td + parent out
   size_t bstage_cap = 0;
   cudaGraphExec_t bgraph = nullptr;
@@ -98,6 +96,7 @@ struct gtd_handle_s {
   // Last DP solve (for gtd_dp_query / gtd_sync).
   bool have_table = false;
   bool pending_stats = false;
+  bool tree_timed = false;    // the tree kernel ran on its own, before ev[2]
   int last_tile_bits = 0;  // of the byte table's layout (the planes' tiles may differ)
   uint32_t last_tiles = 0;
   gtd::DpBatchParams last_params;

@@ -251,3 +251,19 @@ def test_dp_device_path_reports_timeout_at_sync(handle):
     handle.dp_solve_device(d_adj.data_ptr(), g.n, d_out.data_ptr(), d_out[2:].data_ptr())
     handle.sync()
     assert int(d_out[0].item()) == handle.dp_solve(g.adj64(), g.n)[0]
+
+
+@pytest.mark.parametrize("n", [2, 12, 18, 19, 28, 29])
+def test_adjacency_handed_over_by_value_serves_later_queries(handle, n):
+    # the first kernel puts the masks down for the tree kernel of a query; a
+    # rejected graph and a smaller one before it leave nothing behind
+    bad = np.zeros(n, dtype=np.uint64)
+    bad[0] = 2
+    with pytest.raises(InvalidArgument):
+        handle.dp_solve(bad, n)
+    handle.dp_solve(G.complete(5).adj64(), 5)
+    td, parent, order, _ = handle.dp_solve(G.path(n).adj64(), n)
+    assert td == int(np.ceil(np.log2(n + 1))) and sorted(order.tolist()) == list(range(n))
+    half = n // 2
+    td, order = handle.dp_query((1 << half) - 1)
+    assert td == int(np.ceil(np.log2(half + 1))) and sorted(order) == list(range(half))
