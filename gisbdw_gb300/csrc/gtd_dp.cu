@@ -961,12 +961,100 @@ struct TreeMem {
 // The canonical tree of `query` and what p asks of it (whole warp): every
 // component is rooted at the first vertex v with td(C - v) = td(C) - 1 and its
 // sub-components hang below that root (dynamic_cpu.hpp:59-81). All components
-// of a depth are taken together: their vertices are disjoint, so one round of
-// loads, lane v reading C(v) - v, finds every root of the depth. The time is
-// the depth of the tree times one load's latency and the component searches
-// (n = 30: 61 us when each component took a round of its own).
+// of a depth are taken together. They are the components of the graph on the
+// vertices not yet placed (an edge between two of them would have kept them in
+// one), so lane v holds the set C(v) of its vertex in a register: one round of
+// loads reads C(v) - v, three ballots of the residues give every component its
+// root, and a root's C is its subtree. The latency of one warp bounds
+// it: with lists of components in shared memory, taken one after another, and
+// the order from shared-memory atomics it took 15 us at n = 16 (9 depths, 11
+// components; the small kernel as a whole 29 us, now 22; n = 12 19, now 15).
 template <class Ctx>
-__device__ bool build_tree(const DpBatchParams& p, const DpGraph& G, const uint64_t* adj, const Ctx& ctx, TreeMem& m,
+__device__ __forceinline__ bool build_tree(const DpBatchParams& p, const DpGraph& G, const uint64_t* adj_masks,
+                                           const Ctx& ctx, uint32_t query) {
+  const int lane = threadIdx.x & 31, n = G.n;
+  const uint32_t adj = lane < n ? static_cast<uint32_t>(adj_masks[lane]) : 0u;
+  const Chain chain = load_chain(ctx, query);
+  uint32_t comp = 0u, sub = 0u;  // the vertex's component; its subtree once placed
+  int parent = -1, owner = -1;   // owner: root of the component around it
+  int dep = 0, deepest = 0, height = 0;
+  for (uint32_t rest = query; rest;) {
+    ++height;
+    const bool in = (rest >> lane) & 1u, alone = in && (adj & rest) == 0u;
+    if (alone)
+      comp = 1u << lane;
+    uint32_t todo = rest & ~__ballot_sync(0xffffffffu, alone);
+    while (todo) {
+      uint32_t reach = todo & (0u - todo), front = reach;
+      while (front) {
+        front = __reduce_or_sync(0xffffffffu, ((front >> lane) & 1u) ? adj : 0u) & todo & ~reach;
+        reach |= front;
+      }
+      if ((reach >> lane) & 1u)
+        comp = reach;
+      todo &= ~reach;
+    }
+    const bool look = in && !alone;
+    const uint32_t t = look ? ctx.residue(comp & ~(1u << lane)) : 3u;
+    const uint32_t h0 = __ballot_sync(0xffffffffu, t == 0u) & comp, h1 = __ballot_sync(0xffffffffu, t == 1u) & comp,
+                   h2 = __ballot_sync(0xffffffffu, t == 2u) & comp;
+    // td(C - v) over v in C is a and possibly a + 1: residue a is the one
+    // present whose predecessor is absent (three: a corrupt table)
+    const uint32_t hits = h0 && h2 ? h2 : h0 ? h0 : h1 ? h1 : h2;
+    if (__any_sync(0xffffffffu, look && ((h0 && h1 && h2) || hits == 0u)))
+      return false;
+    const int root = look ? __ffs(hits) - 1 : lane;
+    const bool placed = in && root == lane;
+    if (placed) {
+      parent = owner;
+      dep = height;
+      sub = comp;
+    }
+    owner = root;
+    const uint32_t now = __ballot_sync(0xffffffffu, placed);
+    if (now & sub)
+      deepest = height;
+    rest &= ~now;
+  }
+  const uint32_t td = chain_td(chain, n);
+  if (lane == 0 && p.td_out)
+    p.td_out[G.out_idx] = static_cast<int32_t>(td);
+  if (static_cast<uint32_t>(height) != td)
+    return false;
+  const bool in = (query >> lane) & 1u;
+  if (p.parent_out && in)
+    p.parent_out[G.adj_off + lane] = parent;
+  if (p.order_out) {
+    // GetElimination (dynamic_gpu.hpp:58-63): repeatedly remove the stored
+    // root of the remaining set; for a disconnected set that is the root of
+    // its first deepest component, components taken in order of their
+    // lowest vertex (dynamic_gpu.cu:92-103). The components of the
+    // remaining set are subtrees of the canonical tree and a component's
+    // treedepth is its subtree's height, so the order is read off the tree:
+    // the active subtree of greatest height, ties to the lowest vertex,
+    // gives its root and is replaced by its children's subtrees.
+    const uint32_t key = static_cast<uint32_t>(deepest - dep + 1) << 10 |
+                         static_cast<uint32_t>(32 - __ffs(sub)) << 5 | static_cast<uint32_t>(lane);
+    bool active = in && parent < 0;
+    const int count = __popc(query);
+    int own = 0;
+    for (int step = 0; step < count; ++step) {
+      const int v = static_cast<int>(__reduce_max_sync(0xffffffffu, active ? key : 0u) & 31u);
+      if (lane == step)
+        own = v;
+      active = (active && lane != v) || (in && parent == v);
+    }
+    if (lane < count)
+      p.order_out[G.adj_off + lane] = own;
+  }
+  return true;
+}
+
+// The same for more than 32 vertices, two to a lane, the components of a depth
+// in lists in shared memory. A table of this size takes milliseconds, its tree
+// a few dozen microseconds.
+template <class Ctx>
+__device__ __noinline__ bool build_wide_tree(const DpBatchParams& p, const DpGraph& G, const uint64_t* adj, const Ctx& ctx, TreeMem& m,
                            uint64_t query) {
   const int lane = threadIdx.x & 31, n = G.n;
   const uint64_t adj_lo = lane < n ? adj[lane] : 0ull;
@@ -976,7 +1064,6 @@ __device__ bool build_tree(const DpBatchParams& p, const DpGraph& G, const uint6
   uint64_t in_next = 0;           // their union
   // The components of `rest`, below `owner` at depth d: single vertices are
   // done, the others join list `to`.
-  const bool wide = n > 32;
   auto split = [&](uint64_t rest, int owner, int d, int to) {
     if (rest)
       height = max(height, d);
@@ -994,16 +1081,6 @@ __device__ bool build_tree(const DpBatchParams& p, const DpGraph& G, const uint6
     rest &= ~ballot64(one_lo, one_hi);
     while (rest) {
       uint64_t reach = rest & (0ull - rest), frontier = reach;
-      if (!wide) {
-        uint32_t r32 = static_cast<uint32_t>(reach), f32 = r32;
-        while (f32) {
-          const uint32_t nb = ((f32 >> lane) & 1u) ? static_cast<uint32_t>(adj_lo) : 0u;
-          f32 = __reduce_or_sync(0xffffffffu, nb) & static_cast<uint32_t>(rest) & ~r32;
-          r32 |= f32;
-        }
-        reach = r32;
-        frontier = 0ull;
-      }
       while (frontier) {
         const uint64_t nb = (((frontier >> lane) & 1ull) ? adj_lo : 0ull) |
                             (((frontier >> (lane + 32)) & 1ull) ? adj_hi : 0ull);
@@ -1065,14 +1142,6 @@ __device__ bool build_tree(const DpBatchParams& p, const DpGraph& G, const uint6
   }
 
   if (p.order_out) {
-    // GetElimination (dynamic_gpu.hpp:58-63): repeatedly remove the stored
-    // root of the remaining set; for a disconnected set that is the root of
-    // its first deepest component, components taken in order of their
-    // lowest vertex (dynamic_gpu.cu:92-103). The components of the
-    // remaining set are subtrees of the canonical tree and a component's
-    // treedepth is its subtree's height, so the order is read off the tree:
-    // the active subtree of greatest height, ties to the lowest vertex,
-    // gives its root and is replaced by its children's subtrees.
     for (int v = lane; v < n; v += 32) {
       m.hgt[v] = 0u;  // the tallest child so far
       m.low[v] = 255u - static_cast<uint32_t>(v);
@@ -1137,7 +1206,10 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
     const DpGraph G = p.graphs ? p.graphs[g] : p.single;
     level_offsets(sBinom, G.nh, mem[warp].off);
     const TreeCtx ctx{sBinom, mem[warp].off, p.table + G.table_off, G.lb, G.n};
-    if (!build_tree(p, G, p.adj + G.adj_off, ctx, mem[warp], p.query ? p.query : (1ull << G.n) - 1ull)) {
+    const uint64_t query = p.query ? p.query : (1ull << G.n) - 1ull;
+    const uint64_t* const adj = p.adj + G.adj_off;
+    if (!(G.n <= 32 ? build_tree(p, G, adj, ctx, static_cast<uint32_t>(query))
+                    : build_wide_tree(p, G, adj, ctx, mem[warp], query))) {
       if ((threadIdx.x & 31) == 0)
         raise_error(p.error, kDevNoRoot, g);
       break;
@@ -1179,7 +1251,7 @@ __global__ void __launch_bounds__(512)
     dp_small_kernel(const __grid_constant__ DpBatchParams p, int max_n, const __grid_constant__ DpInput in) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ Binom binom;
-  __shared__ TreeMem mem;
+  __shared__ uint32_t off[32];  // first place of a level
   __shared__ int sBad;
   const uint32_t tid = threadIdx.x, threads = blockDim.x;
   const int g = p.first_graph + static_cast<int>(blockIdx.x);
@@ -1198,7 +1270,7 @@ __global__ void __launch_bounds__(512)
   fill_binom(binom);
   __syncthreads();
   if (tid < 32) {
-    level_offsets(binom, m, mem.off);
+    level_offsets(binom, m, off);
     const bool bad = !adjacency_ok(adj, n);
     if (tid == 0) {
       sBad = bad ? 1 : 0;
@@ -1212,10 +1284,10 @@ __global__ void __launch_bounds__(512)
     return;
   }
   for (uint32_t w = tid; w < words; w += threads)
-    order[mem.off[__popc(w)] + rank_colex(binom, w)] = static_cast<uint16_t>(w);
+    order[off[__popc(w)] + rank_colex(binom, w)] = static_cast<uint16_t>(w);
   for (int j = 0; j <= m; ++j) {
     __syncthreads();
-    const uint32_t begin = mem.off[j], count = binom[m][j];
+    const uint32_t begin = off[j], count = binom[m][j];
     for (uint32_t e = tid; e < count; e += threads) {
       const uint32_t w = order[begin + e];
       Acc a;
@@ -1233,7 +1305,7 @@ __global__ void __launch_bounds__(512)
   __syncthreads();
   if (tid < 32) {
     const SmallCtx ctx{p0, p1, n};
-    if (!build_tree(p, G, adj, ctx, mem, (1ull << n) - 1ull) && tid == 0)
+    if (!build_tree(p, G, adj, ctx, (1u << n) - 1u) && tid == 0)
       raise_error(p.error, kDevNoRoot, g);
     report_error(p);
   } else if (p.table) {

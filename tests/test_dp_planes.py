@@ -20,6 +20,7 @@ import numpy as np
 import pytest
 
 from gisbdw_gb300 import graphs as G
+from gisbdw_gb300.validate import check_tree
 
 M32 = 0xFFFFFFFF
 SINGLES = 0x10116            # positions with one of the five bits
@@ -223,3 +224,22 @@ def test_kernel_at_tile_edges_matches_oracle(handle, port, tile_bits, n):
         assert np.array_equal(tab >> 1, T), g.name
         for s in (1, (1 << n) - 1, 3, 5 % (1 << n), (1 << n) - 2):
             assert tab[s] & 1 == connected(g, s), (g.name, s)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 3, 12, 18, 19, 31, 32])
+def test_tree_of_deep_wide_and_forest_shaped_graphs(handle, port, n):
+    # one warp, a vertex per lane: all lanes in use, one component per depth
+    # (complete), many (path, star), none but single vertices, and a forest
+    gs = [G.path(n), G.star(n), G.Graph(n, [])]
+    gs += [G.complete(n)] if n <= 19 else []
+    gs += [G.Graph(n, [(v, v + 2) for v in range(n - 2)]), G.relabel(G.path(n), list(reversed(range(n))))]
+    for g in gs:
+        otd, oparent = (port.dp_solve(g) if n <= 19 else (None, None))
+        td, parent, order, _ = handle.dp_solve(g.adj64(), n)
+        if otd is not None:
+            assert td == otd and parent.tolist() == oparent.tolist(), (n, g.edges[:3])
+        assert check_tree(g, td, parent, allow_forest=True) and sorted(order.tolist()) == list(range(n))
+        # the order removes a root only after every vertex above it
+        place = {v: i for i, v in enumerate(order.tolist())}
+        assert all(parent[v] < 0 or place[parent[v]] < place[v] for v in range(n))
