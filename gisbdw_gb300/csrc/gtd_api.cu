@@ -139,9 +139,11 @@ namespace {
 // and 803 with 12; n = 33: 4.68 ms against 5.14 and 5.23).
 int default_tile_bits(int n) { return n >= 26 ? 11 : 10; }
 
-// Up to this n the level kernel solves a graph (up to kDpSmallMaxN the small
-// kernel), unless the caller gives tile bits (level / 11-bit tile kernel: n = 12 20 / 24 us, 16 31 / 56, 20 45 / 117,
-// 25 112 / 234, 27 176 / 299, 28 264 / 344, 29 436 / 436, 30 806 / 690).
+// Up to this n the level kernel solves a graph (up to kDpSmallBestN the small,
+// up to kDpClusterMaxN the cluster kernel; the small kernel up to kDpSmallMaxN
+// where that does not fit), unless the caller gives tile bits (level / 11-bit
+// tile kernel: n = 20 45 / 117 us, 25 112 / 234, 27 176 / 299, 28 264 / 344,
+// 29 436 / 436, 30 806 / 690).
 constexpr int kLevelMaxN = 28;
 
 // Allocates (or grows) the table and flag buffers and enqueues the
@@ -155,7 +157,10 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, const uint64_t* h_adj
   const DpLayout L = make_dp_layout(n, tile_bits);
   const bool stall = take_stall_fault();  // test injection: needs a kernel whose tiles wait
   const bool given_bits = opts && opts->tile_bits > 0;
-  const bool small = !given_bits && !stall && n <= kDpSmallMaxN;
+  if (h->dp_cluster < 0 && n > kDpSmallBestN && n <= kDpClusterMaxN)
+    h->dp_cluster = dp_cluster_fits() ? 1 : 0;
+  const bool cluster = !given_bits && !stall && n > kDpSmallBestN && n <= kDpClusterMaxN && h->dp_cluster == 1;
+  const bool small = !given_bits && !stall && (n <= kDpSmallMaxN || cluster);
   const bool by_level = !given_bits && !small && n <= kLevelMaxN;
   // the planes' tiles: n < lb is padded to one tile
   const int lb = small ? kDpSmallTileBits : by_level ? kDpLevelTileBits : L.lb < kDpMinTileBits ? kDpMinTileBits : L.lb;
@@ -219,7 +224,7 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, const uint64_t* h_adj
     occ = 1;
   long long ctas = static_cast<long long>(h->num_sms) * occ;
   if (ctas > p.total_groups || small)
-    ctas = small ? 1 : p.total_groups;
+    ctas = cluster ? kDpClusterCtas : small ? 1 : p.total_groups;
 
   if (take_poison_fault())  // test injection: every byte must be written before it is read
     GTD_CUDA(h, cudaMemsetAsync(h->d_table, 0xFF, h->table_cap, h->stream));
@@ -228,7 +233,8 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, const uint64_t* h_adj
   if (stall)  // ticket 0 (the level-0 group) is never taken
     GTD_CUDA(h, cudaMemsetAsync(h->d_io + kIoTicket, 1, 1, h->stream));
   GTD_CUDA(h, cudaEventRecord(h->ev[0], h->stream));
-  GTD_CUDA(h, small      ? dp_launch_small(p, n, h->stream, in)
+  GTD_CUDA(h, cluster    ? dp_launch_cluster(p, h->stream, in)
+              : small    ? dp_launch_small(p, n, h->stream, in)
               : by_level ? dp_launch_levels(p, static_cast<int>(ctas), h->stream)
                          : dp_launch_tiles(p, static_cast<int>(ctas), h->stream));
   GTD_CUDA(h, cudaEventRecord(h->ev[1], h->stream));

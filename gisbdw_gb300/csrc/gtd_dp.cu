@@ -1234,6 +1234,31 @@ struct SmallCtx {
   }
 };
 
+// Place of every word among all words by size and colex rank: f(word, place)
+// for the words base << mh + ..., by the given warps, the m < 5 case in one of
+// them. 32 words of one h = word / 32 at a time: the rank is that of the five
+// low bits plus, by their number, one of six sums over the bits of h (a lane
+// each); a loop over the bits of every word took 7 of the 62 us at n = 20.
+template <class F>
+__device__ __forceinline__ void for_places(const Binom& binom, const uint32_t* off, uint32_t base, int m, int warp,
+                                           int warps, F&& f) {
+  const int lane = threadIdx.x & 31, q = __popc(lane), mh = m > 5 ? m - 5 : 0;
+  const uint32_t low = rank_colex(binom, static_cast<uint32_t>(lane));
+  for (uint32_t h = warp; h < (1u << mh); h += warps) {
+    const uint32_t H = base << mh | h;
+    const bool in_H = (H >> lane) & 1u;
+    const int k = __popc(H & ((2u << lane) - 1u));
+    uint32_t high = 0;
+#pragma unroll
+    for (int i = 0; i <= 5; ++i) {
+      const uint32_t sum = __reduce_add_sync(0xffffffffu, in_H ? binom[5 + lane][k + i] : 0u);
+      high = i == q ? sum : high;
+    }
+    if (lane < (1 << m))
+      f(h << 5 | lane, off[__popc(H) + q] + low + high);
+  }
+}
+
 // Dynamic shared memory for graphs of up to n vertices: three planes of
 // 2^(n-5) words and the words' order.
 __host__ __device__ constexpr uint32_t small_words(int n) { return n > 5 ? 1u << (n - 5) : 1u; }
@@ -1245,8 +1270,9 @@ constexpr size_t small_smem(int n) { return size_t(small_words(n)) * (3 * 4 + 2)
 // others copy the planes out (single-graph solves: tiles of 5 bits, for later
 // queries). One launch and no flag, count or gather from L2, each of which
 // costs a microsecond a level in the other kernels: bound by the latency of a
-// level's word chain, about 1 us (n = 12, all of check, table and tree: 18 us
-// against 4 + 21 + 14; n = 16: 25 against 4 + 30 + 16; n = 18: 49 against 58).
+// level's word chain, about 0.8 us, and half as much again for the tree (n = 12,
+// all of check, table and tree: 15 us against 4 + 21 + 9 in the level kernel's
+// three; n = 16: 22 against 4 + 30 + 11).
 __global__ void __launch_bounds__(512)
     dp_small_kernel(const __grid_constant__ DpBatchParams p, int max_n, const __grid_constant__ DpInput in) {
   extern __shared__ __align__(16) uint8_t smem[];
@@ -1283,8 +1309,8 @@ __global__ void __launch_bounds__(512)
     report_error(p);
     return;
   }
-  for (uint32_t w = tid; w < words; w += threads)
-    order[off[__popc(w)] + rank_colex(binom, w)] = static_cast<uint16_t>(w);
+  for_places(binom, off, 0u, m, tid >> 5, threads >> 5,
+             [&](uint32_t w, uint32_t at) { order[at] = static_cast<uint16_t>(w); });
   for (int j = 0; j <= m; ++j) {
     __syncthreads();
     const uint32_t begin = off[j], count = binom[m][j];
@@ -1320,8 +1346,197 @@ __global__ void __launch_bounds__(512)
 }
 
 // ---------------------------------------------------------------------------
+// Middle-sized graphs: the table in the shared memory of one cluster.
+// ---------------------------------------------------------------------------
+
+constexpr int kClusterBits = 4, kClusterThreads = 512;
+static_assert(1 << kClusterBits == kDpClusterCtas);
+
+// Three planes and the words' order, of a CTA's share.
+constexpr size_t cluster_smem(int n) { return size_t(14) << (n - 5 - kClusterBits); }
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+
+// Shared-memory address `a` of this CTA as that of CTA `rank`.
+__device__ __forceinline__ uint32_t map_rank(uint32_t a, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+
+__device__ __forceinline__ uint32_t ld_cluster(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+
+// All threads of the cluster; stores to shared memory before it are seen after it.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// Words of a table over the cluster's CTAs, by the top bits of the word.
+struct ClusterCtx {
+  uint32_t p0, p1;  // shared-memory addresses of the planes
+  int m, n;         // bits of a word within a CTA
+  __device__ uint32_t residue(uint64_t S) const {
+    const uint32_t w = static_cast<uint32_t>(S) >> 5, bit = static_cast<uint32_t>(S) & 31u;
+    const uint32_t rank = w >> m, at = 4u * (w & ((1u << m) - 1u));
+    const uint32_t a = ld_cluster(map_rank(p0 + at, rank)), b = ld_cluster(map_rank(p1 + at, rank));
+    return ((a >> bit) & 1u) ? 0u : 2u - ((b >> bit) & 1u);
+  }
+};
+
+// The small kernel over a cluster, a CTA per value of the word's top bits (a
+// single graph of kDpSmallBestN < n <= kDpClusterMaxN vertices): every CTA has
+// the same words of 2^(n-9) to go through, a level later for every top bit it
+// has; children without one of those are read from the neighbour CTAs' shared
+// memory, and a cluster barrier parts the levels. Bound by the word chain and
+// the barrier of its levels (0.8 us), the widest ones by what 16 SMs issue.
+// Kernel time, us, against the small / the level and tree kernels: n = 16 25 /
+// 22, 17 26 / 28, 18 29 / 39, 19 35 / 59, 20 45 / 61, 21 61 / 67, 22 - / 80.
+// 8 CTAs: n = 18 30, 20 50, 21 74.
+__global__ void __launch_bounds__(kClusterThreads)
+    dp_cluster_kernel(const __grid_constant__ DpBatchParams p, const __grid_constant__ DpInput in) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ Binom binom;
+  __shared__ uint32_t off[32];        // first place of a level within the CTA
+  __shared__ uint32_t table_off[32];
+  __shared__ uint64_t adj[kDpClusterMaxN];
+  const uint32_t tid = threadIdx.x, threads = blockDim.x, cta = cluster_rank();
+  const DpGraph G = p.single;
+  const int n = G.n, M = n - 5, m = M - kClusterBits, top = __popc(cta);
+  const uint32_t words = 1u << m;
+  uint32_t* const p0 = reinterpret_cast<uint32_t*>(smem);
+  uint32_t* const p1 = p0 + words;
+  uint32_t* const pc = p1 + words;
+  uint16_t* const order = reinterpret_cast<uint16_t*>(pc + words);
+  if (cta == 0)
+    take_input(p, in);
+  if (tid < n)
+    adj[tid] = in.by_value ? in.adj[tid] : p.adj[tid];
+  fill_binom(binom);
+  __syncthreads();
+  bool bad = false;
+  if (tid < 32) {
+    level_offsets(binom, m, off);
+    level_offsets(binom, M, table_off);
+    bad = cta == 0 && !adjacency_ok(adj, n);
+  }
+  __syncthreads();
+  for_places(binom, off, 0u, m, tid >> 5, threads >> 5,
+             [&](uint32_t w, uint32_t at) { order[at] = static_cast<uint16_t>(w); });
+  const uint32_t a0 = static_cast<uint32_t>(__cvta_generic_to_shared(p0)), plane = 4u * words;
+  uint32_t other[kClusterBits];
+  bool has[kClusterBits];
+#pragma unroll
+  for (int i = 0; i < kClusterBits; ++i) {
+    has[i] = (cta >> i) & 1u;
+    other[i] = map_rank(a0, has[i] ? cta ^ (1u << i) : cta);
+  }
+  for (int j = 0; j <= M; ++j) {
+    cluster_sync();
+    const int own = j - top;
+    if (own < 0 || own > m)
+      continue;
+    const uint32_t begin = off[own], count = binom[m][own];
+    for (uint32_t e = tid; e < count; e += threads) {
+      const uint32_t w = order[begin + e];
+      Acc a;
+      uint32_t r0[kClusterBits], r1[kClusterBits], rc[kClusterBits];
+#pragma unroll
+      for (int i = 0; i < kClusterBits; ++i) {
+        r0[i] = r1[i] = rc[i] = 0u;
+        if (has[i]) {
+          r0[i] = ld_cluster(other[i] + 4u * w);
+          r1[i] = ld_cluster(other[i] + 4u * w + plane);
+          rc[i] = ld_cluster(other[i] + 4u * w + 2u * plane);
+        }
+      }
+      for (uint32_t bits = w; bits; bits &= bits - 1u) {
+        const uint32_t child = w ^ (bits & (0u - bits));
+        acc_add1(a, p0[child], p1[child], pc[child]);
+      }
+#pragma unroll
+      for (int i = 0; i < kClusterBits; ++i)
+        if (has[i])
+          acc_add1(a, r0[i], r1[i], rc[i]);
+      const uint64_t S0 = (static_cast<uint64_t>(cta) << m | w) << 5;
+      const Planes r = j > 2 ? resolve_word(a, SmallSets{}) : resolve_word(a, small_sets(S0, j, adj, n));
+      p0[w] = r.p0;
+      p1[w] = r.p1;
+      pc[w] = r.c;
+    }
+  }
+  cluster_sync();
+  if (cta == 0 && tid < 32) {
+    if (bad) {
+      if (tid == 0)
+        raise_error(p.error, kDevInvalidInput, 0);
+    } else {
+      const ClusterCtx ctx{a0, a0 + plane, m, n};
+      if (!build_tree(p, G, adj, ctx, (1u << n) - 1u) && tid == 0)
+        raise_error(p.error, kDevNoRoot, 0);
+    }
+    report_error(p);
+  } else {
+    uint32_t* const out = reinterpret_cast<uint32_t*>(p.table + G.table_off);
+    const int first = cta == 0 ? 1 : 0;
+    for_places(binom, table_off, cta, m, (tid >> 5) - first, (threads >> 5) - first, [&](uint32_t w, size_t t) {
+      out[3 * t] = p0[w];
+      out[3 * t + 1] = p1[w];
+      out[3 * t + 2] = pc[w];
+    });
+  }
+  cluster_sync();  // CTA 0's tree reads every CTA's planes
+}
+
+// ---------------------------------------------------------------------------
 // Host-side launch helpers.
 // ---------------------------------------------------------------------------
+
+// A launch of the cluster kernel. 16 CTAs are above the portable cluster size:
+// dp_cluster_fits says whether the device has room for them.
+struct ClusterLaunch {
+  cudaLaunchAttribute attr = {};
+  cudaLaunchConfig_t cfg = {};
+  cudaError_t status;
+  ClusterLaunch(int n, cudaStream_t s) {
+    status = cudaFuncSetAttribute(dp_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(cluster_smem(kDpClusterMaxN)));
+    if (status == cudaSuccess)
+      status = cudaFuncSetAttribute(dp_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = kDpClusterCtas;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(kDpClusterCtas);
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.dynamicSmemBytes = cluster_smem(n);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+  }
+};
+
+bool dp_cluster_fits() {
+  ClusterLaunch l(kDpClusterMaxN, nullptr);
+  int clusters = 0;
+  if (l.status == cudaSuccess)
+    l.status = cudaOccupancyMaxActiveClusters(&clusters, dp_cluster_kernel, &l.cfg);
+  if (l.status != cudaSuccess)
+    cudaGetLastError();  // not an error of the call that asked
+  return l.status == cudaSuccess && clusters > 0;
+}
+
+cudaError_t dp_launch_cluster(const DpBatchParams& p, cudaStream_t s, const DpInput& in) {
+  ClusterLaunch l(p.single.n, s);
+  return l.status != cudaSuccess ? l.status : cudaLaunchKernelEx(&l.cfg, dp_cluster_kernel, p, in);
+}
 
 template <int LB>
 static cudaError_t launch_tiles(const DpBatchParams& p, int ctas, cudaStream_t s) {

@@ -77,6 +77,10 @@ cudaError_t dp_launch_levels(const DpBatchParams& p, int ctas, cudaStream_t s);
 // max_n <= kDpSmallMaxN vertices, checked, solved and reconstructed; p.table
 // (tiles of kDpSmallTileBits) may be null.
 cudaError_t dp_launch_small(const DpBatchParams& p, int max_n, cudaStream_t s, const DpInput& in = DpInput{});
+// The cluster kernel: as the small kernel, for one graph of kDpSmallBestN <
+// n <= kDpClusterMaxN vertices, on a device that has room for the cluster.
+bool dp_cluster_fits();
+cudaError_t dp_launch_cluster(const DpBatchParams& p, cudaStream_t s, const DpInput& in);
 cudaError_t dp_launch_tree(const DpBatchParams& p, cudaStream_t s);
 cudaError_t dp_launch_labels(const DpBatchParams& p, const uint64_t* subsets, int count, int32_t* td_out,
                              uint64_t* roots_out, cudaStream_t s);

@@ -46,6 +46,11 @@ constexpr int kDpLevelChunk = 128;
 // The small kernel's largest graph (its table in shared memory) and tiles.
 constexpr int kDpSmallMaxN = 18;
 constexpr int kDpSmallTileBits = 5;
+// Above kDpSmallBestN and up to kDpClusterMaxN the cluster kernel of
+// kDpClusterCtas CTAs is faster than the small and the level kernel.
+constexpr int kDpSmallBestN = 16;
+constexpr int kDpClusterMaxN = 21;
+constexpr int kDpClusterCtas = 16;
 
 // Bytes of a tile of the solve's table.
 GTD_HD constexpr uint32_t dp_tile_bytes(int lb) { return 12u << (lb - 5); }

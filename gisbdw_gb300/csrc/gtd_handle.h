@@ -87,6 +87,8 @@ struct gtd_handle_s {
   // a property of the kernel and the device, looked up once per handle.
   int dp_occ[gtd::kDpMaxTileBits + 1][gtd::kDpMaxHigh + 1] = {};
 
+  int dp_cluster = -1;        // 1: the device takes the cluster kernel (-1: not asked yet)
+
   gtd_bnb_state* bnb = nullptr;
   void* d_scratch = nullptr;  // general device scratch (labels, GNN batches)
   size_t scratch_cap = 0;

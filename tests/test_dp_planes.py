@@ -243,3 +243,18 @@ def test_tree_of_deep_wide_and_forest_shaped_graphs(handle, port, n):
         # the order removes a root only after every vertex above it
         place = {v: i for i, v in enumerate(order.tolist())}
         assert all(parent[v] < 0 or place[parent[v]] < place[v] for v in range(n))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [16, 17, 18, 20, 21, 22])
+def test_cluster_kernel_equals_the_tile_kernel(handle, n):
+    # 17..21: words over 16 CTAs by their top bits; one vertex less and more on
+    # either side. Whole tables, trees, orders and queries.
+    for g in (G.gnp_connected(n, 0.25, n), G.grid(2, n // 2), G.Graph(n, [(v, v + 3) for v in range(n - 3)])):
+        adj = np.zeros(n, dtype=np.uint64)
+        adj[:g.n] = g.adj64()
+        a = handle.dp_solve(adj, n, tile_bits=10)
+        table, query = handle.dp_read_table()[0], handle.dp_query((1 << n) - 6)
+        b = handle.dp_solve(adj, n)
+        assert a[0] == b[0] and a[1].tolist() == b[1].tolist() and a[2].tolist() == b[2].tolist()
+        assert np.array_equal(table, handle.dp_read_table()[0]) and query == handle.dp_query((1 << n) - 6)
