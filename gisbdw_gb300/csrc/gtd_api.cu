@@ -368,6 +368,7 @@ gtd_status gtd_destroy(gtd_handle h) {
     cudaFree(h->d_bgraphs);
     cudaFree(h->d_tile_map);
     cudaFree(h->d_level_base);
+    cudaFree(h->d_levels);
     cudaFree(h->d_badj);
     cudaFree(h->d_bout);
     cudaFree(h->d_scratch);

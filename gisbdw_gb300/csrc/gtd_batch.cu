@@ -37,6 +37,8 @@ struct Plan {
   uint32_t total_tiles = 0;
   uint32_t total_groups = 0;    // tickets
   int kid_rows = 0;             // largest nh
+  bool rated = false;           // the tile sizes come from the autotuner's rates
+  bool by_level = false;        // the other graphs go to the level kernel
   int small = 0;                // graphs at the end of `graphs` that the small kernel takes (no tiles)
   uint64_t plane_bytes = 0;     // the pool itself; table_bytes counts one byte per padded subset
   uint64_t subsets = 0;
@@ -51,6 +53,16 @@ constexpr int kLevelSlots = kDpMaxHigh + 2;
 // tile kernel, of 16: 111 against 306; from 17 on the widest level has seven
 // words per thread of the CTA and shared memory holds fewer CTAs).
 constexpr int kBatchSmallMaxN = 16;
+
+// The other graphs go to the level kernel while their subsets together are too
+// few to fill the GPU with the tile kernel's groups, unless the caller gives
+// tile bits or has them measured (level / tile kernel, us, whole batch:
+// 2 graphs of 20 vertices 65 / 139, 6 of 17..24 112 / 218, 48 of 17..21 91 /
+// 178, 300 of 17..21 190 / 230, 48 of 22..24, 450 M subsets, 328 / 340; above:
+// 1000 of 17..21, 813 M, 510 / 499, 200 of 17..24 534 / 493, 4096 of 10..24
+// 5316 / 4380: its gathers are 48 bytes).
+constexpr int kBatchLevelMaxN = 28;
+constexpr uint64_t kBatchLevelSubsets = uint64_t(1) << 29;
 
 // Tile bits per vertex count. An explicit opts->tile_bits gives every graph
 // that size. Otherwise, when the autotuner has rates (subsets per us of the
@@ -98,6 +110,7 @@ void pick_tile_bits(gtd_handle h, const gtd_graph_desc* descs, int count, const 
         uniform(10);
         return;
       }
+  P.rated = true;
   auto t_of = [&](int n, int lb) { return double(uint64_t(1) << std::max(n, lb)) / h->tune[n][lb]; };
   double best_cost = -1;
   for (int lb = kTuneLbMin; lb <= kTuneLbMax; ++lb) {
@@ -172,7 +185,8 @@ void make_plan(Plan& P, const gtd_graph_desc* descs, int count, bool small_kerne
   for (int k = 0; k < count; ++k) {
     const gtd_graph_desc& d = descs[order[k]];
     DpGraph& G = P.graphs[k];
-    const int lb = P.lb_by_n[d.n];
+    const bool in_small = small_kernel && d.n <= kBatchSmallMaxN;
+    const int planned = P.lb_by_n[d.n], lb = P.by_level && !in_small ? kDpLevelTileBits : planned;
     G.n = d.n;
     G.lb = lb;
     G.nh = d.n > lb ? d.n - lb : 0;
@@ -181,13 +195,13 @@ void make_plan(Plan& P, const gtd_graph_desc* descs, int count, bool small_kerne
     G.flag_base = group;
     G.adj_off = static_cast<uint32_t>(d.offset);
     G.out_idx = order[k];
-    P.table_bytes += uint64_t(G.ntiles) << lb;
-    tile += G.ntiles;
-    if (small_kernel && d.n <= kBatchSmallMaxN) {
+    P.table_bytes += uint64_t(1) << std::max(d.n, planned);
+    tile += 1u << std::max(0, d.n - planned);
+    if (in_small) {
       ++P.small;
     } else {
       off += uint64_t(G.ntiles) * dp_tile_bytes(lb);
-      group += dp_groups(binom, G.nh, dp_group_tiles(lb));
+      group += dp_groups(binom, G.nh, dp_chunk_tiles(lb));
       P.kid_rows = std::max(P.kid_rows, G.nh);
     }
     const uint64_t sub = uint64_t(1) << d.n;
@@ -205,7 +219,7 @@ void make_plan(Plan& P, const gtd_graph_desc* descs, int count, bool small_kerne
       const DpGraph& G = P.graphs[k];
       if (j <= G.nh) {
         P.level_base[size_t(k) * kLevelSlots + j] = ticket;
-        ticket += (binom[G.nh][j] + dp_group_tiles(G.lb) - 1) / dp_group_tiles(G.lb);
+        ticket += (binom[G.nh][j] + dp_chunk_tiles(G.lb) - 1) / dp_chunk_tiles(G.lb);
       }
     }
 }
@@ -219,6 +233,7 @@ uint64_t fingerprint(const Plan& P, const void* adj, const void* td, const void*
   mix(P.lb);
   mix(P.mixed);
   mix(P.small);
+  mix(P.by_level);
   mix(P.graphs.size());
   for (const DpGraph& G : P.graphs) {
     mix(G.n);
@@ -253,12 +268,23 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
                          int32_t* d_td, int32_t* d_parent, const gtd_dp_batch_opts* opts, int force_cap = 0) {
   Plan P;
   pick_tile_bits(h, descs, count, opts, P, force_cap);
-  make_plan(P, descs, count, !(opts && opts->tile_bits > 0) && force_cap == 0);
+  const bool own_choice = !(opts && opts->tile_bits > 0) && force_cap == 0;
+  uint64_t work = 0;
+  int max_n = 0;
+  for (int i = 0; i < count; ++i) {
+    max_n = std::max(max_n, descs[i].n);
+    if (descs[i].n > kBatchSmallMaxN)
+      work += uint64_t(1) << descs[i].n;
+  }
+  P.by_level = own_choice && !P.rated && max_n <= kBatchLevelMaxN && work <= kBatchLevelSubsets;
+  make_plan(P, descs, count, own_choice);
   const int lb = P.lb;
   const uint64_t timeout = (opts && opts->timeout_ns) ? opts->timeout_ns : 10ull * 1000 * 1000 * 1000;
   int occ = 1;
   if (P.total_groups > 0)
-    occ = P.mixed ? dp_mixed_occupancy(lb, P.kid_rows) : dp_tile_occupancy(lb, P.kid_rows);
+    occ = P.by_level ? dp_level_occupancy(P.kid_rows)
+          : P.mixed  ? dp_mixed_occupancy(lb, P.kid_rows)
+                     : dp_tile_occupancy(lb, P.kid_rows);
   if (opts && opts->ctas_per_sm > 0 && opts->ctas_per_sm < occ)
     occ = opts->ctas_per_sm;
   if (occ < 1)
@@ -284,7 +310,8 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
   // no other call has reallocated them (a larger single solve grows the table).
   const DpBatchParams& cap = h->bparams;
   const bool same_buffers = cap.table == h->d_table && cap.flags == h->d_flags && cap.tile_map == h->d_tile_map &&
-                            cap.level_base == h->d_level_base && cap.graphs == h->d_bgraphs;
+                            cap.level_base == h->d_level_base && cap.graphs == h->d_bgraphs &&
+                            cap.level_done == (P.by_level ? h->d_levels : nullptr);
   const bool poison = take_poison_fault();  // test injection (gtd_inject_fault)
   if (use_graph && h->bgraph_valid && h->bgraph_key == key && same_buffers) {
     st.graph_replayed = 1;
@@ -308,6 +335,9 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
     return s;
   GTD_CUDA(h, ensure_field(&h->d_tile_map, &h->tile_map_cap, P.total_groups));
   GTD_CUDA(h, ensure_field(&h->d_level_base, &h->level_base_cap, P.level_base.size()));
+  const size_t level_words = P.by_level ? 32 * size_t(count) : 0;
+  if (P.by_level)
+    GTD_CUDA(h, ensure_field(&h->d_levels, &h->levels_cap, level_words));
   GTD_CUDA(h, ensure_field(&h->d_bgraphs, &h->bgraphs_cap, size_t(count)));
   // Descriptors and level bases go up through pinned staging (synchronised
   // below, so the staging is released right after).
@@ -337,6 +367,7 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
   bp.total_groups = P.total_groups;
   bp.table = h->d_table;
   bp.flags = h->d_flags;
+  bp.level_done = P.by_level ? h->d_levels : nullptr;
   bp.ticket = reinterpret_cast<uint32_t*>(h->d_io + kIoTicket);
   bp.error = h->d_io + kIoError;
   bp.adj = d_adj;
@@ -350,7 +381,8 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
     if (bp.num_graphs > 0) {
       e = dp_launch_validate(bp, h->stream);
       if (e == cudaSuccess)
-        e = dp_launch_tiles(bp, static_cast<int>(ctas), h->stream);
+        e = P.by_level ? dp_launch_levels(bp, static_cast<int>(ctas), h->stream)
+                       : dp_launch_tiles(bp, static_cast<int>(ctas), h->stream);
       if (e == cudaSuccess)
         e = dp_launch_tree(bp, h->stream);
     }
@@ -375,7 +407,9 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
     cudaGraph_t graph = nullptr;
     GTD_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t ce = cudaSuccess;
-    if (P.total_groups > 0)
+    if (P.by_level)
+      ce = cudaMemsetAsync(h->d_levels, 0, level_words * sizeof(uint32_t), h->stream);
+    else if (P.total_groups > 0)
       ce = cudaMemsetAsync(h->d_flags, 0, size_t(P.total_groups) * sizeof(uint32_t), h->stream);
     if (ce == cudaSuccess)
       ce = cudaMemsetAsync(h->d_io, 0, 4 * sizeof(int32_t), h->stream);
@@ -398,6 +432,8 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
     s = next_epoch(h, &bp.epoch);
     if (s != GTD_OK)
       return s;
+    if (P.by_level)
+      GTD_CUDA(h, cudaMemsetAsync(h->d_levels, 0, level_words * sizeof(uint32_t), h->stream));
     GTD_CUDA(h, cudaMemsetAsync(h->d_io, 0, 4 * sizeof(int32_t), h->stream));
     GTD_CUDA(h, cudaEventRecord(h->ev[0], h->stream));
     GTD_CUDA(h, launch());

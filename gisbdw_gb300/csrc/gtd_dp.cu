@@ -314,7 +314,7 @@ __global__ void dp_fill_tile_map_kernel(const __grid_constant__ DpBatchParams p)
   __syncthreads();
   for (int g = blockIdx.x; g < p.num_graphs; g += gridDim.x) {
     const DpGraph G = p.graphs[g];
-    const uint32_t per = dp_group_tiles(G.lb);
+    const uint32_t per = dp_chunk_tiles(G.lb);
     uint32_t local = 0;
     for (int j = 0; j <= G.nh; ++j) {
       const uint32_t count = (binom[G.nh][j] + per - 1u) / per;
@@ -728,6 +728,10 @@ constexpr int kLevelThreads = kDpLevelChunk;
 // 2.5 to 3 us here (n = 20: 45 us), most of it the count, the gathers and the
 // chain through three words. A tile of 48 bytes is also the widest load that
 // the gathers can use, so tables beyond the L2 (n >= 29) go to the tile kernel.
+//
+// BATCH: chunks of many graphs, level-major as in the tile kernel, counters
+// per graph.
+template <bool BATCH>
 __global__ void __launch_bounds__(kLevelThreads, 4) dp_level_kernel(const __grid_constant__ DpBatchParams p) {
   constexpr int LB = kDpLevelTileBits;
   constexpr uint32_t kTileBytes = dp_tile_bytes(LB);
@@ -741,16 +745,23 @@ __global__ void __launch_bounds__(kLevelThreads, 4) dp_level_kernel(const __grid
   uint32_t ticket = 0;
   if (tid == 0)
     ticket = atomicAdd(p.ticket, 1u);
-  const DpGraph G = p.single;
-  uint8_t* const table = p.table + G.table_off;
-  const int nh = G.nh;
   for (;;) {
     if (tid == 0)
       sTicket = ticket;
     __syncthreads();
-    const uint32_t chunk = sTicket;
+    uint32_t chunk = sTicket;
     if (chunk >= p.total_groups)
       return;
+    uint32_t g = 0;
+    if (BATCH) {
+      const uint2 at = __ldg(p.tile_map + chunk);
+      g = at.x;
+      chunk = at.y;
+    }
+    const DpGraph G = BATCH ? p.graphs[g] : p.single;
+    uint8_t* const table = p.table + G.table_off;
+    uint32_t* const level_done = p.level_done + 32u * g;
+    const int nh = G.nh;
     if (tid == 0)
       ticket = atomicAdd(p.ticket, 1u);
     // Level j of the chunk: lane i holds the tiles and chunks of levels 0..i.
@@ -793,7 +804,7 @@ __global__ void __launch_bounds__(kLevelThreads, 4) dp_level_kernel(const __grid
     }
     if (j > 0) {
       if (tid == 0)
-        sStop = wait_count(p.level_done + (j - 1), chunks_prev, p.timeout_ns, p.error) ? 0 : 1;
+        sStop = wait_count(level_done + (j - 1), chunks_prev, p.timeout_ns, p.error) ? 0 : 1;
       __syncthreads();
       if (sStop)
         return;
@@ -861,7 +872,7 @@ __global__ void __launch_bounds__(kLevelThreads, 4) dp_level_kernel(const __grid
     // chunk's stores to the thread that acquires the final value.
     __syncthreads();
     if (tid == 0)
-      red_release_add_u32(p.level_done + j, 1u);
+      red_release_add_u32(level_done + j, 1u);
   }
 }
 
@@ -1600,12 +1611,16 @@ cudaError_t dp_launch_small(const DpBatchParams& p, int max_n, cudaStream_t s, c
 int dp_level_occupancy(int kid_rows) {
   const int smem = static_cast<int>(sizeof(uint32_t)) * kLevelThreads * kid_rows;
   int blocks = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, dp_level_kernel, kLevelThreads, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, dp_level_kernel<true>, kLevelThreads, smem);
   return blocks;
 }
 
 cudaError_t dp_launch_levels(const DpBatchParams& p, int ctas, cudaStream_t s) {
-  dp_level_kernel<<<ctas, kLevelThreads, sizeof(uint32_t) * kLevelThreads * p.kid_rows, s>>>(p);
+  const size_t smem = sizeof(uint32_t) * kLevelThreads * p.kid_rows;
+  if (p.graphs)
+    dp_level_kernel<true><<<ctas, kLevelThreads, smem, s>>>(p);
+  else
+    dp_level_kernel<false><<<ctas, kLevelThreads, smem, s>>>(p);
   return cudaGetLastError();
 }
 

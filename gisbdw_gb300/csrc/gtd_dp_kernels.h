@@ -38,7 +38,7 @@ struct DpBatchParams {
   uint8_t* table = nullptr;         // table pool: tiles of three bit planes
   uint32_t* flags = nullptr;        // one ready stamp per tile group
   uint32_t* ticket = nullptr;       // work counter, zeroed before each launch
-  uint32_t* level_done = nullptr;   // chunks done per level (level kernel), zeroed before each launch
+  uint32_t* level_done = nullptr;   // chunks done per level (level kernel), 32 words per graph, zeroed before each launch
   int32_t* error = nullptr;         // [0] code, [1] info
   const uint64_t* adj = nullptr;    // adjacency pool (device)
   uint32_t epoch = 0;               // flags equal to epoch are ready
@@ -69,8 +69,8 @@ int dp_mixed_occupancy(int lb, int kid_rows);
 cudaError_t dp_launch_validate(const DpBatchParams& p, cudaStream_t s, const DpInput& in = DpInput{});
 cudaError_t dp_launch_fill_tile_map(const DpBatchParams& p, cudaStream_t s);
 cudaError_t dp_launch_tiles(const DpBatchParams& p, int ctas, cudaStream_t s);
-// The level kernel (single graph, tiles of kDpLevelTileBits): total_groups
-// counts chunks of kDpLevelChunk tiles of one level.
+// The level kernel (tiles of kDpLevelTileBits, n >= that): total_groups counts
+// chunks of kDpLevelChunk tiles of one level.
 int dp_level_occupancy(int kid_rows);
 cudaError_t dp_launch_levels(const DpBatchParams& p, int ctas, cudaStream_t s);
 // The small kernel: p.num_graphs graphs, from p.first_graph on, of at most

@@ -43,6 +43,11 @@ static_assert(dp_group_tiles(9) == kDpThreads && (dp_group_tiles(11) << (11 - 5)
 constexpr int kDpLevelTileBits = 7;
 constexpr int kDpLevelChunk = 128;
 
+// Tiles per ticket.
+GTD_HD constexpr uint32_t dp_chunk_tiles(int lb) {
+  return lb == kDpLevelTileBits ? uint32_t(kDpLevelChunk) : dp_group_tiles(lb);
+}
+
 // The small kernel's largest graph (its table in shared memory) and tiles.
 constexpr int kDpSmallMaxN = 18;
 constexpr int kDpSmallTileBits = 5;

@@ -66,6 +66,8 @@ struct gtd_handle_s {
   size_t tile_map_cap = 0;
   uint32_t* d_level_base = nullptr;
   size_t level_base_cap = 0;
+  uint32_t* d_levels = nullptr;  // chunks done per graph and level (level kernel)
+  size_t levels_cap = 0;
   uint64_t* d_badj = nullptr;
   size_t badj_cap = 0;
   int32_t* d_bout = nullptr;  // td of every graph, then the parents

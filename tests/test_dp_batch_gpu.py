@@ -137,3 +137,17 @@ def test_batch_tile_bits_too_small_for_the_largest_graph(handle):
     assert td.tolist() == [7, 5]
     for g, t, par in zip(gs, td, parents):
         assert check_tree(g, t, par)
+
+
+@pytest.mark.parametrize("sizes", [[17], [17, 24, 3, 16, 20, 1, 18], [28, 17], [19] * 40])
+@pytest.mark.parametrize("use_cuda_graph", [True, False])
+def test_batches_with_few_subsets_by_level(handle, sizes, use_cuda_graph):
+    # the level kernel's chunks of many graphs against the tile kernel's groups;
+    # a second call with other contents (counters cleared), then a tile-kernel batch
+    for seed in (1, 2):
+        gs = [G.gnp_connected(n, 0.25, 10 * seed + n) if n > 1 else G.Graph(1, []) for n in sizes]
+        td, parents, stats = handle.dp_solve_batch(gs, use_cuda_graph=use_cuda_graph)
+        etd, eparents, _ = handle.dp_solve_batch(gs, tile_bits=10, use_cuda_graph=use_cuda_graph)
+        assert stats["tile_bits"] == 10 and td.tolist() == etd.tolist()
+        for a, b in zip(parents, eparents):
+            assert a.tolist() == b.tolist()
