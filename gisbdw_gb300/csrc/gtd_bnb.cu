@@ -162,6 +162,7 @@ struct BnbParams {
   const uint8_t* order = nullptr;  // order[adj_off + r] = vertex of rank r
   uint4* memo = nullptr;
   uint32_t memo_mask = 0;
+  uint64_t memo_tag = 0;           // number of this solve (1 .. 2^40 - 1)
   uint32_t* best = nullptr;        // per graph: k << 8 | root (kSeedRoot = seed tree)
   uint32_t* lbp = nullptr;         // per graph: proven lower bound
   uint32_t* fails = nullptr;       // per graph x level: failed pairs (first root, second root)
@@ -259,8 +260,15 @@ __device__ __forceinline__ void cas128(uint4* addr, uint64_t clo, uint64_t chi, 
 
 // Memo slot: lo = mask bits 0..63; hi = mask bits 64..103 (bits 0..39) |
 // lb << 40 | ub << 47 | root << 54. An all-zero slot is empty (the empty set
-// is never stored).
+// is never stored). Graphs of at most 64 vertices have the solve's number (its
+// tag) where bits 64..103 would be: a slot of an earlier solve is empty, and
+// the memo, 256 MB a graph, is not cleared for every call (2.1 ms for 48
+// graphs). Wider graphs (tag 0) use a cleared memo.
 constexpr uint64_t kKeyHiMask = (1ull << 40) - 1;
+
+__device__ __forceinline__ bool memo_empty(uint64_t clo, uint64_t chi, uint64_t tag) {
+  return (clo == 0 && chi == 0) || (tag != 0 && (chi & kKeyHiMask) != tag);
+}
 
 __device__ __forceinline__ uint64_t memo_hash(uint64_t lo, uint64_t hi) {
   uint64_t x = lo * 0x9E3779B97F4A7C15ull ^ (hi + 0x632BE59BD9B4E019ull) * 0xC2B2AE3D27D4EB4Full;
@@ -280,13 +288,14 @@ __device__ __forceinline__ MemoHit unpack(uint64_t chi) {
 
 // Lookup (lane 0). Reads are atomic: a CAS that can only write back the
 // value it found.
-__device__ MemoHit memo_get(uint4* table, uint32_t mask, uint64_t lo, uint64_t hi) {
+__device__ MemoHit memo_get(uint4* table, uint32_t mask, uint64_t tag, uint64_t lo, uint64_t hi) {
   const uint64_t h = memo_hash(lo, hi);
+  hi |= tag;
   for (int p = 0; p < kMemoProbes; ++p) {
     uint4* slot = table + ((h + p) & mask);
     uint64_t clo, chi;
     cas128(slot, 0, 0, 0, 0, clo, chi);
-    if (clo == 0 && chi == 0)
+    if (memo_empty(clo, chi, tag))
       break;
     if (clo == lo && (chi & kKeyHiMask) == hi)
       return unpack(chi);
@@ -295,8 +304,10 @@ __device__ MemoHit memo_get(uint4* table, uint32_t mask, uint64_t lo, uint64_t h
 }
 
 // Merges bounds into the memo (lane 0): lb = max, ub = min (with its root).
-__device__ void memo_put(uint4* table, uint32_t mask, uint64_t lo, uint64_t hi, int lb, int ub, int root) {
+__device__ void memo_put(uint4* table, uint32_t mask, uint64_t tag, uint64_t lo, uint64_t hi, int lb, int ub,
+                         int root) {
   const uint64_t h = memo_hash(lo, hi);
+  hi |= tag;
   auto merged = [&](uint64_t chi, bool empty) {
     MemoHit c = empty ? MemoHit{0, kUnknownUb, 0} : unpack(chi);
     const int nlb = max(c.lb, lb);
@@ -314,9 +325,9 @@ __device__ void memo_put(uint4* table, uint32_t mask, uint64_t lo, uint64_t hi, 
     uint64_t clo = 0, chi = 0;
     cas128(slot, 0, 0, 0, 0, clo, chi);
     for (int tries = 0; tries < 64; ++tries) {
-      const bool empty = clo == 0 && chi == 0;
+      const bool empty = memo_empty(clo, chi, tag);
       if (!empty && !(clo == lo && (chi & kKeyHiMask) == hi)) {
-        const int sz = __popcll(clo) + __popcll(chi & kKeyHiMask);
+        const int sz = __popcll(clo) + (tag ? 0 : __popcll(chi & kKeyHiMask));
         if (sz < victim_size) {
           victim_size = sz;
           victim = p;
@@ -367,6 +378,7 @@ struct Search {
   int lane, n;
   uint4* memo;
   uint32_t memo_mask;
+  uint64_t tag;  // of the memo's slots
   StopCheck stop;
   unsigned long long nodes;
   bool timed_out, cancelled;
@@ -572,7 +584,7 @@ struct Search {
       if (v < n && has(Clo, Chi, v)) {
         uint64_t lo = Clo, hi = Chi;
         bit_clear(lo, hi, v);
-        const MemoHit m = memo_get(memo, memo_mask, lo, hi);
+        const MemoHit m = memo_get(memo, memo_mask, tag, lo, hi);
         best = max(best, m.lb);
         if (m.ub < kUnknownUb)
           ubr = min(ubr, (static_cast<uint32_t>(m.ub) << 8) | static_cast<uint32_t>(v));
@@ -818,7 +830,7 @@ struct Search {
           } else {
             MemoHit hit{0, kUnknownUb, 0};
             if (lane == 0)
-              hit = memo_get(memo, memo_mask, f.lo, f.hi);
+              hit = memo_get(memo, memo_mask, tag, f.lo, f.hi);
             hit.lb = __shfl_sync(0xffffffffu, hit.lb, 0);
             hit.ub = __shfl_sync(0xffffffffu, hit.ub, 0);
             hit.root = __shfl_sync(0xffffffffu, hit.root, 0);
@@ -831,7 +843,7 @@ struct Search {
               int r = 0;
               const int td = mini_dp(f.lo, f.hi, csize, &r);
               if (lane == 0)
-                memo_put(memo, memo_mask, f.lo, f.hi, td, td, r);
+                memo_put(memo, memo_mask, tag, f.lo, f.hi, td, td, r);
               decision = td <= fk ? 1 : 0;
               vroot = r;
             } else {
@@ -840,7 +852,7 @@ struct Search {
               if (lb <= fk && hit.lb == 0 && csize >= kMmdMin) {
                 lb = max(lb, mmd_lb(f.lo, f.hi));
                 if (lane == 0)
-                  memo_put(memo, memo_mask, f.lo, f.hi, lb, kUnknownUb, 0);
+                  memo_put(memo, memo_mask, tag, f.lo, f.hi, lb, kUnknownUb, 0);
               }
               // a path of 2^fk vertices, or a cycle of 2^(fk-1) + 1, would
               // refute td <= fk (a tree, with fewer edges than vertices, has
@@ -850,7 +862,7 @@ struct Search {
                 if (pl > fk) {
                   lb = pl;
                   if (lane == 0)
-                    memo_put(memo, memo_mask, f.lo, f.hi, lb, kUnknownUb, 0);
+                    memo_put(memo, memo_mask, tag, f.lo, f.hi, lb, kUnknownUb, 0);
                 }
               }
               // td is monotone under vertex deletion: a memo entry proving
@@ -862,7 +874,7 @@ struct Search {
                 if (sl > fk) {
                   lb = sl;
                   if (lane == 0)
-                    memo_put(memo, memo_mask, f.lo, f.hi, lb, kUnknownUb, 0);
+                    memo_put(memo, memo_mask, tag, f.lo, f.hi, lb, kUnknownUb, 0);
                 }
               }
               if (lb > fk) {
@@ -871,7 +883,7 @@ struct Search {
                 decision = 1;
                 vroot = static_cast<int>(ubr & 0xFF);
                 if (lane == 0)
-                  memo_put(memo, memo_mask, f.lo, f.hi, 0, fk, vroot);
+                  memo_put(memo, memo_mask, tag, f.lo, f.hi, 0, fk, vroot);
               }
             }
           }
@@ -968,9 +980,9 @@ struct Search {
       const int fv = f.v;
       if (!f.single && lane == 0) {
         if (ok)
-          memo_put(memo, memo_mask, f.lo, f.hi, 0, fk, fv);
+          memo_put(memo, memo_mask, tag, f.lo, f.hi, 0, fk, fv);
         else
-          memo_put(memo, memo_mask, f.lo, f.hi, fk + 1, kUnknownUb, 0);
+          memo_put(memo, memo_mask, tag, f.lo, f.hi, fk + 1, kUnknownUb, 0);
       }
       ret = ok;
       ret_root = ok ? fv : -1;
@@ -1208,7 +1220,7 @@ __global__ void __launch_bounds__(32 * kBnbWarps, 6) bnb_kernel(const __grid_con
     const int v = w->order[r];
     uint64_t fl, fh;
     full_set(G.n, fl, fh);
-    Search s{w, lane, G.n, p.memo + G.memo_off, p.memo_mask, StopCheck{}, 0ull, false, false};
+    Search s{w, lane, G.n, p.memo + G.memo_off, p.memo_mask, G.n <= 64 ? p.memo_tag : 0ull, StopCheck{}, 0ull, false, false};
     s.mini = p.mini ? p.mini + (size_t(blockIdx.x) * kBnbWarps + warp) * (1u << kMiniMax) : nullptr;
     s.stop.best = p.best + g;
     s.stop.lbp = p.lbp + g;
@@ -1438,6 +1450,8 @@ struct gtd_bnb_state {
   size_t order_cap = 0;
   uint4* memo = nullptr;
   size_t memo_cap = 0;
+  uint64_t memo_tag = 0;   // solves so far
+  bool memo_plain = false; // the memo may hold slots that no solve has tagged
   int32_t* i32 = nullptr;  // seed parents, parents, td, status
   size_t i32_cap = 0;
   uint32_t* u32 = nullptr; // best, lbp, fails
@@ -1498,8 +1512,10 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   if (memo_log2 == 0) {
     // HBM is the memo: up to a quarter of the free memory (at most 32 GiB),
     // 2^16 .. 2^24 slots of 16 bytes per graph
+    // (a memo kept from an earlier call that reaches 2^24 already answers it)
     size_t free_b = 0, total_b = 0;
-    GTD_CUDA(h, cudaMemGetInfo(&free_b, &total_b));
+    if (B.memo_cap < size_t(count) << 24)
+      GTD_CUDA(h, cudaMemGetInfo(&free_b, &total_b));
     const size_t budget = std::min(free_b / 4 + B.memo_cap * sizeof(uint4), size_t(32) << 30);
     const size_t per_graph = budget / sizeof(uint4) / size_t(count);
     memo_log2 = 16;
@@ -1548,6 +1564,8 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   if ((s = grow(h, &B.graphs, &B.graphs_cap, count)) != GTD_OK) return s;
   if ((s = grow(h, &B.adj, &B.adj_cap, 2 * size_t(pool_len))) != GTD_OK) return s;
   if ((s = grow(h, &B.order, &B.order_cap, size_t(pool_len) + 16)) != GTD_OK) return s;
+  if (B.memo_cap < slots * count)
+    B.memo_plain = true;  // fresh memory
   if ((s = grow(h, &B.memo, &B.memo_cap, slots * count)) != GTD_OK) return s;
   if ((s = grow(h, &B.i32, &B.i32_cap, 2 * size_t(pool_len) + 2 * size_t(count))) != GTD_OK) return s;
   if ((s = grow(h, &B.u32, &B.u32_cap, size_t(count) * (2 + 2 * size_t(levels)))) != GTD_OK) return s;
@@ -1589,7 +1607,12 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   GTD_CUDA(h, cudaMemcpyAsync(d_lbp, lbp.data(), count * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream));
   GTD_CUDA(h, cudaMemsetAsync(d_fails, 0, 2 * size_t(count) * levels * sizeof(uint32_t), h->stream));
   GTD_CUDA(h, cudaMemsetAsync(B.i8 + firsts, 0, firsts + (may_split ? pairs : 0), h->stream));
-  GTD_CUDA(h, cudaMemsetAsync(B.memo, 0, slots * count * sizeof(uint4), h->stream));
+  if (B.memo_plain)
+    GTD_CUDA(h, cudaMemsetAsync(B.memo, 0, B.memo_cap * sizeof(uint4), h->stream));
+  else if (max_n > 64)
+    GTD_CUDA(h, cudaMemsetAsync(B.memo, 0, slots * count * sizeof(uint4), h->stream));
+  B.memo_plain = max_n > 64;
+  B.memo_tag = B.memo_tag % kKeyHiMask + 1;
   GTD_CUDA(h, cudaMemsetAsync(d_status, 0, count * sizeof(int32_t), h->stream));
   GTD_CUDA(h, cudaMemsetAsync(B.u64, 0, 3 * size_t(count) * sizeof(uint64_t), h->stream));
   GTD_CUDA(h, cudaMemsetAsync(d_t0, 0xFF, sizeof(uint64_t), h->stream));
@@ -1604,6 +1627,7 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   p.order = B.order;
   p.memo = B.memo;
   p.memo_mask = static_cast<uint32_t>(slots - 1);
+  p.memo_tag = B.memo_tag;
   p.best = d_best;
   p.lbp = d_lbp;
   p.fails = d_fails;

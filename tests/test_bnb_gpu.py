@@ -216,3 +216,21 @@ def test_bnb_batch_that_ends_in_split_items(handle, easy, hard, n, first_budget)
     res = _check(handle, gs, **({"first_budget": first_budget} if first_budget else {}))
     dtd, _, _ = handle.dp_solve_batch(gs)
     assert res["td"].tolist() == dtd.tolist()
+
+
+@pytest.mark.parametrize("memo_log2", [0, 6])
+def test_bnb_memo_of_earlier_solves_is_empty(memo_log2):
+    # other graphs on the same vertex sets, one solve after another on one
+    # handle, wide graphs (whose slots have no solve number) in between, a
+    # memo so small that slots are overwritten, and a larger one after it
+    from gisbdw_gb300 import Handle
+    h = Handle(0)
+    for rep in range(3):
+        for s in range(4):
+            gs = [G.sparse_connected(22, 10 * s + i) for i in range(6)] + [G.complete(9), G.path(20 + s)]
+            res = _check(h, gs, memo_log2=memo_log2 + rep if memo_log2 else 0)
+            dtd, _, _ = h.dp_solve_batch(gs)
+            assert res["td"].tolist() == dtd.tolist()
+        wide = _check(h, [G.cycle(70 + rep), G.path(100), G.grid(4, 5)], memo_log2=memo_log2)
+        assert wide["td"].tolist()[:2] == [8, 7]
+    h.close()
