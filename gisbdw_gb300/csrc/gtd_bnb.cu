@@ -1442,24 +1442,12 @@ gtd_status grow(gtd_handle h, T** p, size_t* cap, size_t count) {
 
 // Branch-and-bound buffers of a handle.
 struct gtd_bnb_state {
-  BnbGraph* graphs = nullptr;
-  size_t graphs_cap = 0;
-  uint64_t* adj = nullptr;
-  size_t adj_cap = 0;
-  uint8_t* order = nullptr;
-  size_t order_cap = 0;
   uint4* memo = nullptr;
   size_t memo_cap = 0;
   uint64_t memo_tag = 0;   // solves so far
   bool memo_plain = false; // the memo may hold slots that no solve has tagged
-  int32_t* i32 = nullptr;  // seed parents, parents, td, status
-  size_t i32_cap = 0;
-  uint32_t* u32 = nullptr; // best, lbp, fails
-  size_t u32_cap = 0;
-  uint64_t* u64 = nullptr; // t_begin, t_end, nodes, t0
-  size_t u64_cap = 0;
-  int8_t* i8 = nullptr;    // per-level trees
-  size_t i8_cap = 0;
+  uint8_t* arena = nullptr;  // inputs, results, items (see gtd_bnb_solve_batch)
+  size_t arena_cap = 0;
   uint8_t* mini = nullptr; // per-warp small-component DP tables
   size_t mini_cap = 0;
   std::vector<int32_t> last_lb;  // proven lower bound per graph of the last solve
@@ -1469,14 +1457,8 @@ void gtd_bnb_release(gtd_handle h) {
   if (!h->bnb)
     return;
   gtd_bnb_state* b = h->bnb;
-  cudaFree(b->graphs);
-  cudaFree(b->adj);
-  cudaFree(b->order);
+  cudaFree(b->arena);
   cudaFree(b->memo);
-  cudaFree(b->i32);
-  cudaFree(b->u32);
-  cudaFree(b->u64);
-  cudaFree(b->i8);
   cudaFree(b->mini);
   delete b;
   h->bnb = nullptr;
@@ -1561,14 +1543,9 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   }
 
   gtd_status s;
-  if ((s = grow(h, &B.graphs, &B.graphs_cap, count)) != GTD_OK) return s;
-  if ((s = grow(h, &B.adj, &B.adj_cap, 2 * size_t(pool_len))) != GTD_OK) return s;
-  if ((s = grow(h, &B.order, &B.order_cap, size_t(pool_len) + 16)) != GTD_OK) return s;
   if (B.memo_cap < slots * count)
     B.memo_plain = true;  // fresh memory
   if ((s = grow(h, &B.memo, &B.memo_cap, slots * count)) != GTD_OK) return s;
-  if ((s = grow(h, &B.i32, &B.i32_cap, 2 * size_t(pool_len) + 2 * size_t(count))) != GTD_OK) return s;
-  if ((s = grow(h, &B.u32, &B.u32_cap, size_t(count) * (2 + 2 * size_t(levels)))) != GTD_OK) return s;
   // Split items (first root x second root) when the batch is too small to
   // give every warp a first-root item: a single graph then uses n^2 warps.
   size_t first_items = 0;
@@ -1581,59 +1558,68 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   const size_t firsts = size_t(count) * levels * max_n, pairs = firsts * size_t(max_n);
   const bool may_split = split || pairs <= (size_t(1) << 28);
   const size_t S = split ? size_t(max_n) : 1;
-  if ((s = grow(h, &B.i8, &B.i8_cap, 2 * firsts + (may_split ? pairs : 0))) != GTD_OK) return s;
-  if ((s = grow(h, &B.u64, &B.u64_cap, 3 * size_t(count) + 1)) != GTD_OK) return s;
-  int32_t* d_seed_parent = B.i32;
-  int32_t* d_parent = B.i32 + pool_len;
-  int32_t* d_td = B.i32 + 2 * pool_len;
-  int32_t* d_status = d_td + count;
-  uint32_t* d_best = B.u32;
-  uint32_t* d_lbp = B.u32 + count;
-  uint32_t* d_fails = B.u32 + 2 * count;
-  uint32_t* d_claim = d_fails + size_t(count) * levels;
-  uint64_t* d_tbeg = B.u64;
-  uint64_t* d_tend = B.u64 + count;
-  uint64_t* d_nodes = B.u64 + 2 * count;
-  uint64_t* d_t0 = B.u64 + 3 * count;
+  // One block on the device: inputs, then the bounds (also results), then
+  // words that start at zero, the results among them first, then the
+  // per-level trees. One copy in, one clearing, one copy out.
+  size_t at = 0;
+  auto take = [&](size_t bytes) {
+    const size_t off = at;
+    at += (bytes + 15) / 16 * 16;
+    return off;
+  };
+  const size_t n_pool = size_t(pool_len), n_graphs = size_t(count);
+  const size_t o_graphs = take(n_graphs * sizeof(BnbGraph)), o_adj = take(2 * n_pool * sizeof(uint64_t));
+  const size_t o_order = take(n_pool + 16), o_seed = take(n_pool * sizeof(int32_t));
+  const size_t o_t0 = take(sizeof(uint64_t)), o_best = take(n_graphs * sizeof(uint32_t));
+  const size_t o_lbp = take(n_graphs * sizeof(uint32_t));
+  const size_t in_end = at;
+  const size_t o_tend = take(n_graphs * sizeof(uint64_t)), o_nodes = take(n_graphs * sizeof(uint64_t));
+  const size_t o_status = take(n_graphs * sizeof(int32_t)), o_td = take(n_graphs * sizeof(int32_t));
+  const size_t o_parent = take(n_pool * sizeof(int32_t));
+  const size_t out_end = at;
+  const size_t o_tbeg = take(n_graphs * sizeof(uint64_t)), o_fails = take(2 * n_graphs * levels * sizeof(uint32_t));
+  const size_t o_items = take(firsts + (may_split ? pairs : 0));
+  const size_t zero_end = at;
+  const size_t o_trees = take(firsts);
+  if ((s = grow(h, &B.arena, &B.arena_cap, at)) != GTD_OK) return s;
+  std::vector<uint8_t> stage(out_end, 0);
+  std::memcpy(stage.data() + o_graphs, graphs.data(), n_graphs * sizeof(BnbGraph));
+  std::memcpy(stage.data() + o_adj, adj2_pool, 2 * n_pool * sizeof(uint64_t));
+  std::memcpy(stage.data() + o_order, order.data(), n_pool);
+  std::memcpy(stage.data() + o_seed, seed_parent, n_pool * sizeof(int32_t));
+  std::memset(stage.data() + o_t0, 0xFF, sizeof(uint64_t));
+  std::memcpy(stage.data() + o_best, best.data(), n_graphs * sizeof(uint32_t));
+  std::memcpy(stage.data() + o_lbp, lbp.data(), n_graphs * sizeof(uint32_t));
+  auto dev = [&](size_t off, auto* like) { return reinterpret_cast<decltype(like)>(B.arena + off); };
+  uint32_t* const d_fails = dev(o_fails, static_cast<uint32_t*>(nullptr));
 
   // plain (pageable) copies: this entry point is host-synchronous anyway
-  GTD_CUDA(h, cudaMemcpyAsync(B.graphs, graphs.data(), count * sizeof(BnbGraph), cudaMemcpyHostToDevice, h->stream));
-  GTD_CUDA(h, cudaMemcpyAsync(B.adj, adj2_pool, 2 * size_t(pool_len) * sizeof(uint64_t), cudaMemcpyHostToDevice,
-                              h->stream));
-  GTD_CUDA(h, cudaMemcpyAsync(B.order, order.data(), size_t(pool_len), cudaMemcpyHostToDevice, h->stream));
-  GTD_CUDA(h, cudaMemcpyAsync(d_seed_parent, seed_parent, size_t(pool_len) * sizeof(int32_t), cudaMemcpyHostToDevice,
-                              h->stream));
-  GTD_CUDA(h, cudaMemcpyAsync(d_best, best.data(), count * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream));
-  GTD_CUDA(h, cudaMemcpyAsync(d_lbp, lbp.data(), count * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream));
-  GTD_CUDA(h, cudaMemsetAsync(d_fails, 0, 2 * size_t(count) * levels * sizeof(uint32_t), h->stream));
-  GTD_CUDA(h, cudaMemsetAsync(B.i8 + firsts, 0, firsts + (may_split ? pairs : 0), h->stream));
+  GTD_CUDA(h, cudaMemcpyAsync(B.arena, stage.data(), in_end, cudaMemcpyHostToDevice, h->stream));
+  GTD_CUDA(h, cudaMemsetAsync(B.arena + in_end, 0, zero_end - in_end, h->stream));
   if (B.memo_plain)
     GTD_CUDA(h, cudaMemsetAsync(B.memo, 0, B.memo_cap * sizeof(uint4), h->stream));
   else if (max_n > 64)
     GTD_CUDA(h, cudaMemsetAsync(B.memo, 0, slots * count * sizeof(uint4), h->stream));
   B.memo_plain = max_n > 64;
   B.memo_tag = B.memo_tag % kKeyHiMask + 1;
-  GTD_CUDA(h, cudaMemsetAsync(d_status, 0, count * sizeof(int32_t), h->stream));
-  GTD_CUDA(h, cudaMemsetAsync(B.u64, 0, 3 * size_t(count) * sizeof(uint64_t), h->stream));
-  GTD_CUDA(h, cudaMemsetAsync(d_t0, 0xFF, sizeof(uint64_t), h->stream));
-  GTD_CUDA(h, cudaMemsetAsync(h->d_io, 0, 4 * sizeof(int32_t), h->stream));
+  GTD_CUDA(h, cudaMemsetAsync(h->d_io, 0, kIoWords * sizeof(int32_t), h->stream));
 
   BnbParams p;
-  p.graphs = B.graphs;
+  p.graphs = dev(o_graphs, static_cast<BnbGraph*>(nullptr));
   p.num_graphs = count;
   p.max_n = max_n;
   p.levels = levels;
-  p.adj = B.adj;
-  p.order = B.order;
+  p.adj = dev(o_adj, static_cast<uint64_t*>(nullptr));
+  p.order = B.arena + o_order;
   p.memo = B.memo;
   p.memo_mask = static_cast<uint32_t>(slots - 1);
   p.memo_tag = B.memo_tag;
-  p.best = d_best;
-  p.lbp = d_lbp;
+  p.best = dev(o_best, static_cast<uint32_t*>(nullptr));
+  p.lbp = dev(o_lbp, static_cast<uint32_t*>(nullptr));
   p.fails = d_fails;
-  p.claim = d_claim;
-  p.lvl_parent = B.i8;
-  p.item_state = reinterpret_cast<uint8_t*>(B.i8 + firsts);
+  p.claim = d_fails + n_graphs * levels;
+  p.lvl_parent = dev(o_trees, static_cast<int8_t*>(nullptr));
+  p.item_state = B.arena + o_items;
   p.split_state = may_split ? p.item_state + firsts : nullptr;
   p.split = split;
   p.split_below = static_cast<uint32_t>(h->num_sms) * kSplitPerSm;
@@ -1641,17 +1627,17 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   p.unfinished = reinterpret_cast<uint32_t*>(h->d_io + kIoUnfinished);
   p.exited = reinterpret_cast<uint32_t*>(h->d_io + kIoExited);
   p.window = (opts && opts->window > 0) ? opts->window : kRoundWindow;
-  p.status = d_status;
-  p.t_begin = d_tbeg;
-  p.t_end = reinterpret_cast<unsigned long long*>(d_tend);
-  p.t0 = reinterpret_cast<unsigned long long*>(d_t0);
-  p.nodes = reinterpret_cast<unsigned long long*>(d_nodes);
+  p.status = dev(o_status, static_cast<int32_t*>(nullptr));
+  p.t_begin = dev(o_tbeg, static_cast<uint64_t*>(nullptr));
+  p.t_end = dev(o_tend, static_cast<unsigned long long*>(nullptr));
+  p.t0 = dev(o_t0, static_cast<unsigned long long*>(nullptr));
+  p.nodes = dev(o_nodes, static_cast<unsigned long long*>(nullptr));
   p.ticket = reinterpret_cast<uint32_t*>(h->d_io + kIoTicket);
   p.error = h->d_io + kIoError;
   p.deadline_ns = (opts && opts->deadline_ns) ? opts->deadline_ns : 120ull * 1000 * 1000 * 1000;
-  p.seed_parent = d_seed_parent;
-  p.td_out = d_td;
-  p.parent_out = d_parent;
+  p.seed_parent = dev(o_seed, static_cast<int32_t*>(nullptr));
+  p.td_out = dev(o_td, static_cast<int32_t*>(nullptr));
+  p.parent_out = dev(o_parent, static_cast<int32_t*>(nullptr));
 
   const size_t smem = sizeof(WarpMem) * kBnbWarps;
   GTD_CUDA(h, cudaFuncSetAttribute(bnb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
@@ -1678,7 +1664,6 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   p.pass_gen = reinterpret_cast<uint32_t*>(h->d_io + kIoPassGen);
   p.pass_stop = reinterpret_cast<uint32_t*>(h->d_io + kIoPassStop);
   p.pass_wait_ns = p.deadline_ns + 30ull * 1000 * 1000 * 1000;
-  GTD_CUDA(h, cudaMemsetAsync(h->d_io + kIoExited, 0, 6 * sizeof(int32_t), h->stream));
   GTD_CUDA(h, cudaEventRecord(h->ev[0], h->stream));
   {
     void* args[] = {&p};
@@ -1690,34 +1675,27 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   GTD_CUDA(h, cudaGetLastError());
   GTD_CUDA(h, cudaEventRecord(h->ev[1], h->stream));
 
-  std::vector<int32_t> st(count);
-  std::vector<uint32_t> bst(count), lb(count);
-  std::vector<uint64_t> te(count), nd(count);
-  uint64_t t_first = 0;
-  int32_t io[4] = {0, 0, 0, 0};
-  std::vector<int32_t> par(static_cast<size_t>(pool_len));
-  GTD_CUDA(h, cudaMemcpyAsync(td_out, d_td, count * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-  GTD_CUDA(h, cudaMemcpyAsync(st.data(), d_status, count * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-  GTD_CUDA(h, cudaMemcpyAsync(bst.data(), d_best, count * sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
-  GTD_CUDA(h, cudaMemcpyAsync(lb.data(), d_lbp, count * sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
-  GTD_CUDA(h, cudaMemcpyAsync(te.data(), d_tend, count * sizeof(uint64_t), cudaMemcpyDeviceToHost, h->stream));
-  GTD_CUDA(h, cudaMemcpyAsync(nd.data(), d_nodes, count * sizeof(uint64_t), cudaMemcpyDeviceToHost, h->stream));
-  GTD_CUDA(h, cudaMemcpyAsync(&t_first, d_t0, sizeof(uint64_t), cudaMemcpyDeviceToHost, h->stream));
-  GTD_CUDA(h, cudaMemcpyAsync(io, h->d_io, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-  uint32_t passes = 0;
-  GTD_CUDA(h, cudaMemcpyAsync(&passes, h->d_io + kIoPassGen, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
-  GTD_CUDA(h, cudaMemcpyAsync(par.data(), d_parent, size_t(pool_len) * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                              h->stream));
+  GTD_CUDA(h, cudaMemcpyAsync(stage.data() + o_t0, B.arena + o_t0, out_end - o_t0, cudaMemcpyDeviceToHost, h->stream));
+  int32_t io[kIoWords];
+  GTD_CUDA(h, cudaMemcpyAsync(io, h->d_io, sizeof(io), cudaMemcpyDeviceToHost, h->stream));
   GTD_CUDA(h, cudaStreamSynchronize(h->stream));
-  gtd_status es = map_device_error(h, io[1], io[2]);
+  gtd_status es = map_device_error(h, io[kIoError], io[kIoError + 1]);
   if (es != GTD_OK)
     return es;
+  auto host = [&](size_t off, auto* like) { return reinterpret_cast<decltype(like)>(stage.data() + off); };
+  const uint64_t t_first = *host(o_t0, static_cast<uint64_t*>(nullptr));
+  const uint64_t* const te = host(o_tend, static_cast<uint64_t*>(nullptr));
+  const uint64_t* const nd = host(o_nodes, static_cast<uint64_t*>(nullptr));
+  const uint32_t* const bst = host(o_best, static_cast<uint32_t*>(nullptr));
+  const uint32_t* const lb = host(o_lbp, static_cast<uint32_t*>(nullptr));
+  const int32_t* const par = host(o_parent, static_cast<int32_t*>(nullptr));
+  std::memcpy(td_out, stage.data() + o_td, n_graphs * sizeof(int32_t));
   uint64_t total_nodes = 0;
   B.last_lb.assign(count, 0);
   for (int i = 0; i < count; ++i) {
     const gtd_graph_desc& d = descs[i];
     B.last_lb[i] = static_cast<int32_t>(std::min(lb[i], bst[i] >> 8));
-    std::memcpy(parent_out + d.offset, par.data() + d.offset, d.n * sizeof(int32_t));
+    std::memcpy(parent_out + d.offset, par + d.offset, d.n * sizeof(int32_t));
     const bool proved = lb[i] >= (bst[i] >> 8);
     status_out[i] = proved ? GTD_OK : GTD_TIMEOUT;
     if (proof_ms_out)
@@ -1731,7 +1709,7 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
     cudaEventElapsedTime(&ms, h->ev[0], h->ev[1]);
     stats->ms = ms;
     stats->nodes = total_nodes;
-    stats->passes = static_cast<int32_t>(passes);
+    stats->passes = io[kIoPassGen];
     stats->total_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t_call).count();
   }
   return GTD_OK;
