@@ -380,6 +380,11 @@ gtd_status gtd_destroy(gtd_handle h) {
     for (auto& e : h->ev)
       if (e)
         cudaEventDestroy(e);
+    for (auto& e : h->side_ev)
+      if (e)
+        cudaEventDestroy(e);
+    if (h->side_stream)
+      cudaStreamDestroy(h->side_stream);
     if (h->own_stream && h->stream)
       cudaStreamDestroy(h->stream);
     if (h->abort_stream)

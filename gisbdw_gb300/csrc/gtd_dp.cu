@@ -1601,9 +1601,11 @@ cudaError_t dp_launch_small(const DpBatchParams& p, int max_n, cudaStream_t s, c
     if (e != cudaSuccess)
       return e;
   }
-  // threads: the words of the widest level, 64 to 512 (128 for many graphs,
-  // which fill the GPU side by side)
-  const int threads = max_n <= 13 ? 64 : max_n == 14 || p.num_graphs > 1 ? 128 : max_n == 15 ? 256 : 512;
+  // threads: the words of the widest level, 64 to 512 (128 for thousands of
+  // graphs, which fill the GPU side by side; with 512, 48 graphs of up to 16
+  // vertices take 24 us instead of 29, 300 of 16 31 instead of 34, 1000 the same)
+  const bool many = p.num_graphs > 1024;
+  const int threads = max_n <= 13 ? 64 : max_n == 14 || many ? 128 : max_n == 15 ? 256 : 512;
   dp_small_kernel<<<p.num_graphs, threads, smem, s>>>(p, max_n, in);
   return cudaGetLastError();
 }

@@ -75,6 +75,8 @@ struct gtd_handle_s {
   void* h_bstage = nullptr;  // pinned: adjacency pool in, td + parent out
   size_t bstage_cap = 0;
   cudaGraphExec_t bgraph = nullptr;
+  cudaStream_t side_stream = nullptr;  // a batch's small graphs next to its others, in the captured graph
+  cudaEvent_t side_ev[2] = {nullptr, nullptr};
   uint64_t bgraph_key = 0;
   bool bgraph_valid = false;
   gtd::DpBatchParams bparams;
