@@ -169,90 +169,171 @@ __global__ void __launch_bounds__(32 * kHWarps) heuristic_kernel(const HeurGraph
 // Kinds 0, 1, 2: a thread per vertex, every component at once.
 // ---------------------------------------------------------------------------
 
-struct Set {
-  uint64_t lo, hi;
+// A vertex set of W words.
+template <int W>
+struct Bits {
+  uint32_t w[W];
 };
 
-// Component of S holding u, by one thread. WIDE: vertices from 64 on.
-template <bool WIDE>
-__device__ __forceinline__ Set component_of(const ulonglong2* adj, const Set& S, int u) {
-  Set reach{0, 0};
-  if (!WIDE || u < 64)
-    reach.lo = 1ull << u;
-  else
-    reach.hi = 1ull << (u - 64);
-  Set front = reach;
-  for (;;) {
-    Set next{0, 0};
-    while (front.lo) {  // two vertices at a time: their loads overlap
-      const ulonglong2 a = adj[__ffsll(static_cast<long long>(front.lo)) - 1];
-      front.lo &= front.lo - 1;
-      const ulonglong2 b = front.lo ? adj[__ffsll(static_cast<long long>(front.lo)) - 1] : a;
-      front.lo &= front.lo - 1;
-      next.lo |= a.x | b.x;
-      if constexpr (WIDE)
-        next.hi |= a.y | b.y;
+template <int W>
+__device__ __forceinline__ bool any(const Bits<W>& s) {
+  uint32_t x = 0;
+#pragma unroll
+  for (int i = 0; i < W; ++i)
+    x |= s.w[i];
+  return x != 0;
+}
+template <int W>
+__device__ __forceinline__ bool has(const Bits<W>& s, int v) {
+  uint32_t x = 0;
+#pragma unroll
+  for (int i = 0; i < W; ++i)
+    x = (v >> 5) == i ? s.w[i] : x;
+  return (x >> (v & 31)) & 1u;
+}
+template <int W>
+__device__ __forceinline__ void set_bit(Bits<W>& s, int v, bool on) {
+#pragma unroll
+  for (int i = 0; i < W; ++i) {
+    const uint32_t bit = (v >> 5) == i ? 1u << (v & 31) : 0u;
+    s.w[i] = on ? s.w[i] | bit : s.w[i] & ~bit;
+  }
+}
+template <int W>
+__device__ __forceinline__ int first(const Bits<W>& s) {
+  int r = -1;
+#pragma unroll
+  for (int i = W - 1; i >= 0; --i)
+    r = s.w[i] ? 32 * i + __ffs(s.w[i]) - 1 : r;
+  return r;
+}
+template <int W>
+__device__ __forceinline__ int size(const Bits<W>& s) {
+  int r = 0;
+#pragma unroll
+  for (int i = 0; i < W; ++i)
+    r += __popc(s.w[i]);
+  return r;
+}
+
+// Adjacency rows of W words; row kHMaxN is empty.
+template <int W>
+__device__ __forceinline__ Bits<W> row(const uint32_t* adj, int v) {
+  Bits<W> r;
+  if constexpr (W == 4) {
+    const uint4 x = reinterpret_cast<const uint4*>(adj)[v];
+    r.w[0] = x.x;
+    r.w[1] = x.y;
+    r.w[2] = x.z;
+    r.w[3] = x.w;
+  } else if constexpr (W == 2) {
+    const uint2 x = reinterpret_cast<const uint2*>(adj)[v];
+    r.w[0] = x.x;
+    r.w[1] = x.y;
+  } else {
+    r.w[0] = adj[v];
+  }
+  return r;
+}
+
+// The components of S by one thread, f(component) for each in the order of
+// their lowest vertices. One loop over all of them, up to four vertices a step
+// in no particular order, the lowest of every word (and the highest, of one or
+// two words): their loads overlap, and lanes with different sets take about as
+// many steps, where the levels of a breadth-first search, or components, nested
+// in it would wait for the widest of the warp's.
+template <int W, class F>
+__device__ __forceinline__ void for_components(const uint32_t* adj, Bits<W> S, F&& f) {
+  Bits<W> reach = {}, todo = {};
+  while (any(S)) {
+    if (!any(todo)) {
+      set_bit(todo, first(S), true);
+      reach = todo;
     }
-    if constexpr (WIDE) {
-      while (front.hi) {
-        const ulonglong2 a = adj[63 + __ffsll(static_cast<long long>(front.hi))];
-        front.hi &= front.hi - 1;
-        const ulonglong2 b = front.hi ? adj[63 + __ffsll(static_cast<long long>(front.hi))] : a;
-        front.hi &= front.hi - 1;
-        next.lo |= a.x | b.x;
-        next.hi |= a.y | b.y;
+    Bits<W> next = {};
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+      const uint32_t t = todo.w[i];
+      const Bits<W> a = row<W>(adj, t ? 32 * i + __ffs(t) - 1 : kHMaxN);
+      uint32_t left = t & (t - 1u);
+#pragma unroll
+      for (int k = 0; k < W; ++k)
+        next.w[k] |= a.w[k];
+      if constexpr (W <= 2) {
+        const int top = 31 - __clz(left);
+        const Bits<W> b = row<W>(adj, left ? 32 * i + top : kHMaxN);
+        left &= ~(left ? 1u << top : 0u);
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+          next.w[k] |= b.w[k];
+      }
+      todo.w[i] = left;
+    }
+    uint32_t missing = 0;
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      const uint32_t fresh = next.w[k] & S.w[k] & ~reach.w[k];
+      reach.w[k] |= fresh;
+      todo.w[k] |= fresh;
+      missing |= reach.w[k] ^ S.w[k];
+    }
+    if (missing == 0 || !any(todo)) {
+      f(reach);
+#pragma unroll
+      for (int k = 0; k < W; ++k) {
+        S.w[k] &= ~reach.w[k];
+        todo.w[k] = 0u;
       }
     }
-    front.lo = next.lo & S.lo & ~reach.lo;
-    reach.lo |= front.lo;
-    if constexpr (WIDE) {
-      front.hi = next.hi & S.hi & ~reach.hi;
-      reach.hi |= front.hi;
-    }
-    if ((front.lo | (WIDE ? front.hi : 0ull)) == 0 || (reach.lo == S.lo && (!WIDE || reach.hi == S.hi)))
-      return reach;
   }
 }
 
-// Variance score of removing v from C (variance_heuristic.hpp:40-56 as
-// restated on the host, same order of operations).
-template <bool WIDE>
-__device__ double variance_coef(const ulonglong2* adj, const Set& C, int v) {
-  const float A = 1.0f, D = 0.2f, E = 0.8f;
-  uint8_t sizes[kHMaxN];
-  int nc = 0;
-  Set rest = C;
-  hclear(rest.lo, rest.hi, v);
-  while (rest.lo | rest.hi) {
-    const Set c = component_of<WIDE>(adj, rest, hfirst(rest.lo, rest.hi));
-    rest.lo &= ~c.lo;
-    rest.hi &= ~c.hi;
-    sizes[nc++] = static_cast<uint8_t>(hpopc(c.lo, c.hi));
-  }
-  // explicit round-to-nearest operations: no contraction into FMAs, so the
-  // result is bit-identical to the host's
-  double gamma = 0.0;
-  if (nc > 1) {  // one component: the mean is its size, gamma 0
-    double acc = 0.0;
+// The order of the variance scores of the vertices that leave nc > 1 parts of
+// a component, `total` vertices together (variance_heuristic.hpp:40-56 as
+// restated on the host: gamma is the sum of the squared distances from the mean
+// size, the score D / sqrt(gamma + A) + E nc). Every score of the component has
+// the same nc, so a smaller gamma wins. For nc a power of two the host's gamma
+// is exact: gamma = (nc sum s^2 - total^2) / nc, whose steps of 1 / nc (gamma
+// below 2^14) move the score by more than 1e-9, and the integer orders as the
+// doubles do. Otherwise the host's double operations in their order, each
+// rounded to nearest (no contraction into FMAs).
+__device__ __forceinline__ unsigned long long variance_key(const uint8_t* sizes, int nc, int total) {
+  if ((nc & (nc - 1)) == 0) {
+    int squares = 0;
     for (int i = 0; i < nc; ++i)
-      acc = __dadd_rn(acc, static_cast<double>(sizes[i]));
-    const double avg = __ddiv_rn(acc, static_cast<double>(nc));
-    for (int i = 0; i < nc; ++i) {
-      const double d = __dsub_rn(static_cast<double>(sizes[i]), avg);
-      gamma = __dadd_rn(gamma, __dmul_rn(d, d));
-    }
+      squares += static_cast<int>(sizes[i]) * sizes[i];
+    return (1ull << 32) - static_cast<unsigned long long>(nc * squares - total * total);
+  }
+  const float A = 1.0f, D = 0.2f, E = 0.8f;
+  double acc = 0.0, gamma = 0.0;
+  for (int i = 0; i < nc; ++i)
+    acc = __dadd_rn(acc, static_cast<double>(sizes[i]));
+  const double avg = __ddiv_rn(acc, static_cast<double>(nc));
+  for (int i = 0; i < nc; ++i) {
+    const double d = __dsub_rn(static_cast<double>(sizes[i]), avg);
+    gamma = __dadd_rn(gamma, __dmul_rn(d, d));
   }
   const float enc = __fmul_rn(E, static_cast<float>(nc));
-  return __dadd_rn(__ddiv_rn(static_cast<double>(D), __dsqrt_rn(__dadd_rn(gamma, static_cast<double>(A)))),
-                   static_cast<double>(enc));
+  // positive doubles: their bits are in order
+  return static_cast<unsigned long long>(__double_as_longlong(
+      __dadd_rn(__ddiv_rn(static_cast<double>(D), __dsqrt_rn(__dadd_rn(gamma, static_cast<double>(A)))),
+                static_cast<double>(enc))));
 }
 
 // One greedy elimination by a group of `threads` threads (its own barrier).
+// Components are named by their lowest vertices.
 struct RoundMem {
-  unsigned long long coef[kHMaxN];  // per component (its lowest vertex): the best score's bits
-  uint32_t pick[kHMaxN];            // ... the best (degree, smallest id) among those
+  alignas(16) uint32_t sets[4 * kHMaxN];   // the components
+  alignas(16) uint32_t parts[4 * kHMaxN];  // per component eliminated from: the names of what is left of it
+  unsigned long long best[kHMaxN];  // per component: the best score among those that leave the most parts
+  unsigned long long own[kHMaxN];   // per vertex: its score
+  uint32_t most[kHMaxN];            // per component: the most parts that a removal leaves
+  uint32_t pick[kHMaxN];            // ... the best (degree, smallest id) among the best
   int32_t parent[kHMaxN];
-  int32_t left, height;
+  uint8_t leaves[kHMaxN];           // per vertex: parts that its removal leaves
+  uint8_t name[kHMaxN];             // the vertex's component
+  uint8_t inner[kHMaxN];            // the vertices to search from
+  int32_t left, height, inners;
 };
 
 __device__ __forceinline__ void group_sync(int id, int threads) {
@@ -260,81 +341,193 @@ __device__ __forceinline__ void group_sync(int id, int threads) {
 }
 
 // Rounds: every vertex scores itself within its component, each component
-// eliminates its best, the others search their new component. The number of
-// rounds is the tree's height, not its size. Bound by the latency of the
-// components' searches in shared memory.
-template <bool WIDE>
-__device__ void greedy_rounds(const ulonglong2* adj, int n, bool variance, RoundMem& m, int barrier, int threads) {
+// eliminates its best. The number of rounds is the tree's height, not its
+// size. The variance score needs a search of C - v per vertex, but not for a
+// vertex with one neighbour left, and the searches are taken by the first
+// threads, so that whole warps have none. A score lies in (E nc, E nc + D] and
+// D < E: only the vertices that leave the most parts can win. What is left of a
+// component is published by the thread that searched its vertex (which still
+// has it up to kKeep parts; kind 1 searches only here), the others look
+// themselves up in it. Bound by the latency of a search, |C| / 4 steps of some
+// 100 cycles, once a round.
+template <int W>
+__device__ void greedy_rounds(const uint32_t* adj, int n, bool variance, RoundMem& m, int barrier, int threads) {
+  constexpr int kKeep = 4;
   const int v = threadIdx.x % threads;
   const bool own = v < n;
   bool alive = own;
-  int owner = -1, depth = 0;
-  Set C{n >= 64 ? ~0ull : (1ull << n) - 1, n > 64 ? (n == 128 ? ~0ull : (1ull << (n - 64)) - 1) : 0ull};
-  if (own)
-    C = component_of<WIDE>(adj, C, v);
+  int owner = -1, depth = 0, name = 0;
+  auto store = [&](uint32_t* to, int at, const Bits<W>& s) {
+#pragma unroll
+    for (int i = 0; i < W; ++i)
+      to[at * W + i] = s.w[i];
+  };
+  auto look_up = [&](int from) {
+    Bits<W> names = row<W>(m.parts, from);
+    while (any(names)) {
+      name = first(names);
+      if (has(row<W>(m.sets, name), v))
+        break;
+      set_bit(names, name, false);
+    }
+    m.name[v] = static_cast<uint8_t>(name);
+  };
+  auto publish = [&](const Bits<W>& S, int from) {
+    Bits<W> names = {};
+    for_components<W>(adj, S, [&](const Bits<W>& c) {
+      store(m.sets, first(c), c);
+      set_bit(names, first(c), true);
+    });
+    store(m.parts, from, names);
+  };
   if (v == 0) {
     m.left = n;
     m.height = 0;
+    Bits<W> all;
+#pragma unroll
+    for (int i = 0; i < W; ++i)
+      all.w[i] = n >= 32 * (i + 1) ? ~0u : n > 32 * i ? (1u << (n - 32 * i)) - 1u : 0u;
+    publish(all, 0);
   }
+  group_sync(barrier, threads);
+  if (own)
+    look_up(0);
   for (;;) {
     if (own) {
-      m.coef[v] = 0ull;
+      m.most[v] = 0u;
+      m.best[v] = 0ull;
       m.pick[v] = 0u;
     }
+    if (v == 0)
+      m.inners = 0;
     group_sync(barrier, threads);
     if (m.left == 0)
       return;
-    const int id = alive ? hfirst(C.lo, C.hi) : 0;
-    uint32_t key = 0;
-    unsigned long long coef = 0;
+    uint32_t key = 0, deg = 0;
+    Bits<W> C = {};
     if (alive) {
-      const uint32_t deg = static_cast<uint32_t>(hpopc(adj[v].x & C.lo, adj[v].y & C.hi));
+      C = row<W>(m.sets, name);
+      const Bits<W> mine = row<W>(adj, v);
+#pragma unroll
+      for (int i = 0; i < W; ++i)
+        deg += __popc(mine.w[i] & C.w[i]);
       key = (deg + 1) << 8 | static_cast<uint32_t>(kHMaxN - 1 - v);  // > 0
-      if (variance) {  // positive doubles: their bits are in order
-        coef = static_cast<unsigned long long>(__double_as_longlong(variance_coef<WIDE>(adj, C, v)));
-        atomicMax(&m.coef[id], coef);
+      if (variance) {
+        if (deg >= 2) {
+          m.inner[atomicAdd(&m.inners, 1)] = static_cast<uint8_t>(v);
+        } else {
+          m.leaves[v] = static_cast<uint8_t>(deg);  // of a single vertex nothing is left
+          atomicMax(&m.most[name], deg);
+        }
       }
     }
-    if (variance)
+    Bits<W> kept[kKeep];
+    int u = -1, at = 0, nc = 0;
+    if (variance) {
       group_sync(barrier, threads);
-    if (alive && (!variance || m.coef[id] == coef))
-      atomicMax(&m.pick[id], key);
+      uint8_t sizes[kHMaxN];
+      int total = 0;
+      if (v < m.inners) {
+        u = m.inner[v];
+        at = m.name[u];
+        Bits<W> rest = row<W>(m.sets, at);
+        set_bit(rest, u, false);
+        total = size(rest);
+        for_components<W>(adj, rest, [&](const Bits<W>& c) {
+#pragma unroll
+          for (int i = 0; i < kKeep; ++i)
+            if (nc == i)
+              kept[i] = c;
+          sizes[nc++] = static_cast<uint8_t>(size(c));
+        });
+        m.leaves[u] = static_cast<uint8_t>(nc);
+        atomicMax(&m.most[at], static_cast<uint32_t>(nc));
+      }
+      group_sync(barrier, threads);
+      if (u >= 0 && nc > 1 && m.most[at] == static_cast<uint32_t>(nc)) {
+        m.own[u] = variance_key(sizes, nc, total);
+        atomicMax(&m.best[at], m.own[u]);
+      }
+      group_sync(barrier, threads);
+    }
+    bool candidate = alive;
+    if (alive && variance) {
+      const uint32_t most = m.most[name];  // of one part or none the scores are equal
+      candidate = m.leaves[v] == most && (most <= 1 || m.best[name] == m.own[v]);
+    }
+    if (candidate)
+      atomicMax(&m.pick[name], key);
     group_sync(barrier, threads);
+    const int from = name;
+    bool moved = false;
+    if (u >= 0 && kHMaxN - 1 - static_cast<int>(m.pick[at] & 0xFFu) == u) {  // what this thread searched is eliminated
+      if (nc <= kKeep) {
+        Bits<W> names = {};
+#pragma unroll
+        for (int i = 0; i < kKeep; ++i)
+          if (i < nc) {
+            store(m.sets, first(kept[i]), kept[i]);
+            set_bit(names, first(kept[i]), true);
+          }
+        store(m.parts, at, names);
+      } else {
+        Bits<W> rest = row<W>(m.sets, at);
+        set_bit(rest, u, false);
+        publish(rest, at);
+      }
+    }
     if (alive) {
-      const int chosen = kHMaxN - 1 - static_cast<int>(m.pick[id] & 0xFFu);
+      const int chosen = kHMaxN - 1 - static_cast<int>(m.pick[name] & 0xFFu);
       if (chosen == v) {
         m.parent[v] = owner;
         atomicMax(&m.height, depth + 1);
         atomicSub(&m.left, 1);
         alive = false;
+        set_bit(C, v, false);
+        if (!variance) {
+          publish(C, name);
+        } else if (deg == 1) {  // one part
+          Bits<W> names = {};
+          set_bit(names, first(C), true);
+          store(m.sets, first(C), C);
+          store(m.parts, name, names);
+        }
       } else {
         owner = chosen;
         ++depth;
-        hclear(C.lo, C.hi, chosen);
-        C = component_of<WIDE>(adj, C, v);
+        moved = true;
       }
     }
     group_sync(barrier, threads);
+    if (moved)
+      look_up(from);
   }
 }
 
 // One CTA per graph; kind 0 runs kinds 1 and 2 side by side, `threads` threads
 // each. 1024 graphs of 20..80 vertices, kind 0: 1.48 ms with one warp per graph
-// and one vertex per step.
+// and one vertex per step, 627 us when every vertex searched its new component
+// and scored itself in double, 324 us now (48 graphs of 24..36: 45 us).
 __global__ void heuristic_rounds_kernel(const HeurGraph* graphs, const uint64_t* adj2, int kind, int threads,
                                         int32_t* td_out, int32_t* parent_out) {
-  __shared__ ulonglong2 adj[kHMaxN];
+  __shared__ __align__(16) uint32_t adj[4 * (kHMaxN + 1)];
   __shared__ RoundMem mem[2];
   const HeurGraph G = graphs[blockIdx.x];
-  for (int u = threadIdx.x; u < G.n; u += blockDim.x)
-    adj[u] = make_ulonglong2(adj2[2 * (size_t(G.off) + u)], adj2[2 * (size_t(G.off) + u) + 1]);
+  const int words = G.n <= 32 ? 1 : G.n <= 64 ? 2 : 4;
+  const uint32_t* const rows = reinterpret_cast<const uint32_t*>(adj2 + 2 * size_t(G.off));
+  for (int t = threadIdx.x; t < G.n * words; t += blockDim.x)
+    adj[t] = rows[4 * (t / words) + t % words];
+  if (threadIdx.x < words)
+    adj[kHMaxN * words + threadIdx.x] = 0u;
   __syncthreads();
   const int half = threadIdx.x / threads;
   const bool variance = kind == 2 || half == 1;
-  if (G.n > 64)
-    greedy_rounds<true>(adj, G.n, variance, mem[half], 1 + half, threads);
+  if (words == 1)
+    greedy_rounds<1>(adj, G.n, variance, mem[half], 1 + half, threads);
+  else if (words == 2)
+    greedy_rounds<2>(adj, G.n, variance, mem[half], 1 + half, threads);
   else
-    greedy_rounds<false>(adj, G.n, variance, mem[half], 1 + half, threads);
+    greedy_rounds<4>(adj, G.n, variance, mem[half], 1 + half, threads);
   __syncthreads();
   // the variance tree only when strictly lower, as on the host
   const int from = kind == 0 && mem[1].height < mem[0].height ? 1 : 0;

@@ -64,3 +64,24 @@ def test_gpu_rounds_at_the_word_and_warp_edges(handle, kind):
     for i, g in enumerate(gs):
         htd, hpar = _lib.heuristic(g, kind)
         assert td[i] == htd and pars[i].tolist() == hpar.tolist(), (i, g.name)
+
+
+def _ary_tree(n, k):
+    return G.Graph(n, [(v, (v - 1) // k) for v in range(1, n)])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", [0, 2])
+@pytest.mark.parametrize("n", [31, 32, 64, 104])
+def test_gpu_variance_scores_that_tie_and_leave_many_parts(handle, kind, n):
+    """Parts in numbers that are powers of two (integer order) and not (double
+    order), more of them than a thread keeps, equal ones under other labels."""
+    rng = np.random.default_rng(n)
+    gs = [_ary_tree(n, k) for k in (2, 3, 4, 5, 7, 8)]
+    gs += [G.Graph(n, [(v, v // 3 * 3) for v in range(n) if v % 3] + [(v, v + 3) for v in range(0, n - 3, 3)])]
+    gs += [G.relabel(g, rng.permutation(n).tolist()) for g in list(gs) for _ in range(3)]
+    gs += [G.tree_plus_edges(n, k, k) for k in (0, 1, 3)]
+    td, pars = handle.heuristic_batch(gs, kind)
+    for i, g in enumerate(gs):
+        htd, hpar = _lib.heuristic(g, kind)
+        assert td[i] == htd and pars[i].tolist() == hpar.tolist(), i
