@@ -214,7 +214,7 @@ class ClockSampler:
 
 
 def ncu_profile_figure(key):
-    """A figure of the DP tile kernel's ncu capture on an n = 28 launch
+    """A figure of the DP tile kernel's ncu capture on an n = 30 launch
     (profiles/dp_tile_kernel.md, line '<key>: <value>')."""
     path = os.path.join(ROOT, "profiles", "dp_tile_kernel.md")
     try:
@@ -226,7 +226,7 @@ def ncu_profile_figure(key):
 
 
 def ncu_bytes_per_subset():
-    """DRAM bytes per subset of the DP tile kernel (ncu, n = 28 launch)."""
+    """DRAM bytes per subset of the DP tile kernel (ncu, n = 30 launch)."""
     return ncu_profile_figure("dram_bytes_per_subset")
 
 
@@ -714,7 +714,7 @@ def run_gpu(args, graphs):
     by_n_out = {str(n): {"dp_ms": statistics.median(x["dp_ms"] for x in v),
                          "alg_GBps": statistics.median(x["alg_bytes"] / (x["dp_ms"] / 1e3) / 1e9 for x in v)}
                 for n, v in sorted(by_n.items())}
-    # ncu's DRAM bytes per subset (n = 28 capture) scaled to each launch's 2^n
+    # ncu's DRAM bytes per subset (n = 30 capture) scaled to each launch's 2^n
     bps = ncu_bytes_per_subset()
     traffic = (bps * statistics.mean(2.0 ** g.n for g in graphs)) if bps else None
 
@@ -732,14 +732,15 @@ def run_gpu(args, graphs):
                      "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic,
                      "traffic_note": "profiled constant, not measured in this run: ncu DRAM read+write bytes "
-                                     "per subset of one n=28 launch (profiles/dp_tile_kernel.md), scaled by "
+                                     "per subset of one n=30 launch (profiles/dp_tile_kernel.md), scaled by "
                                      "2^n and averaged over the workload's launches",
                      "frac_note": "achieved counts 1 + n/2 algorithmic bytes per subset (one written, one "
-                                  "gathered per child); the tile layout serves the in-tile children from "
-                                  "shared memory and most cross-tile children from L2, so DRAM moves about "
-                                  "1.1 B per subset (traffic) and frac can exceed 1; the kernel is bound "
-                                  "by instruction issue and the cross-tile L2 latency",
-                     "issue_active_frac_profiled_n28": ncu_profile_figure("issue_active_frac"),
+                                  "gathered per child); the table holds three bits per subset and most "
+                                  "children come from shared memory or L2, so DRAM moves about 0.6 B per "
+                                  "subset (traffic) and frac exceeds 1; the kernel is bound by logic "
+                                  "instructions and the latency of a tile group's phases (n = 28 runs in "
+                                  "dp_level_kernel)",
+                     "issue_active_frac_profiled_n30": ncu_profile_figure("issue_active_frac"),
                      "alg_bytes_per_launch_mean": alg / launches,
                      "launch_ms_mean": kms / launches, "by_n": by_n_out},
         "e2e": {"value": e2e_value, "unit": "solves/s", "h2d_bytes_per_step": h2d,

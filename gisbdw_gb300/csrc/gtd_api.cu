@@ -135,8 +135,8 @@ gtd_status next_epoch(gtd_handle h, uint32_t* epoch) {
 namespace {
 
 // Tile bits of the table's layout unless the caller gives them; the tile
-// kernel's best from n = 26 on (n = 30: 718 us with 11 bits against 743 with 10
-// and 803 with 12; n = 33: 4.68 ms against 5.14 and 5.23).
+// kernel's best from n = 26 on (n = 30: 674 us with 11 bits against 712 with 10,
+// n = 32 2.37 ms against 2.64, n = 33 4.71 against 5.35).
 int default_tile_bits(int n) { return n >= 26 ? 11 : 10; }
 
 // Up to this n the level kernel solves a graph (up to kDpSmallBestN the small,

@@ -396,11 +396,11 @@ __device__ __forceinline__ Workspace make_workspace(const DpBatchParams& p, cons
 // the tiles in shared memory and stores them; the caller publishes the group
 // after a CTA barrier. False (for every thread) if a wait gave up.
 //
-// Bound by latency: 34 % of issue slots at n = 30 (16 warps per SM, as many as
+// Bound by latency: 37 % of issue slots at n = 30 (16 warps per SM, as many as
 // shared memory and registers take), a group's time going to unranking and
 // flags (15 %), the gathers (27 %), the classes of the in-tile phase (33 %)
 // and waits at the narrow levels (16 %). 8.5 warp instructions per word of 32
-// subsets; n = 30 takes 0.69 ms, n = 33 4.7 ms (at one byte per subset and one
+// subsets; n = 30 takes 0.67 ms, n = 33 4.7 ms (at one byte per subset and one
 // warp per tile, 1.52 warp instructions per subset: 1.92 and 14.9 ms). Tried
 // and not kept: a warp per group (0.91 ms), 64 threads per CTA (0.79), the next
 // group unranked by an idle warp beside the in-tile phase (0.72 and 5.2).
@@ -877,7 +877,7 @@ __global__ void __launch_bounds__(kLevelThreads, 4) dp_level_kernel(const __grid
 }
 
 // ---------------------------------------------------------------------------
-// Reconstruction: one warp per graph; lanes cover vertices lane, lane + 32.
+// Reconstruction: one warp per graph.
 // ---------------------------------------------------------------------------
 
 constexpr int kTreeWarps = 4;
