@@ -138,6 +138,13 @@ constexpr uint32_t kItemDone = 0xFF;
 // 67 / 23 / 23 / 23 / 23, 64 of 28..34 70 / 70 / 35 / 35 / 35, 256 of 28..34
 // - / 132 / - / 105 / 105, 300 of 16..36 - / 188 / - / 147 / 148.
 constexpr int kSplitPerSm = 32;
+// A batch that starts with fewer than that already will change over after its
+// first pass, which a few first-root items with whole budgets would draw out
+// while most warps wait: they get 2^-3 of it (budgets of 1024 / 128 / 64 nodes,
+// ms: 64 graphs of 16..24 vertices 6.1-13.4 / 3.5-5.1 / 3.2-4.4, 30 of 28..34
+// 34-42 / 19-27 / 18-26; the median graph is proven as early with 128, later
+// with 64; larger batches the same or slower).
+constexpr int kUnsplitShift = 3;
 constexpr int kRoundWindow = 3;          // levels run at a time per graph
 constexpr int kMaxRounds = 4096;
 
@@ -172,6 +179,7 @@ struct BnbParams {
   uint64_t budget = 0;             // an item's first budget in search nodes (0 = unlimited)
   int window = 0;                  // levels run at a time below a graph's top level (0 = all)
   int split = 0;                   // 1: an item is a pair (first root, second root) from the start
+  int unsplit_shift = 0;           // first-root items get budgets 2^-this as large
   uint32_t split_below = 0;        // split once fewer first-root items than this are open
   uint32_t* split_now = nullptr;   // set by the last warp of a pass
   uint32_t* unfinished = nullptr;  // items that used up their budget this round
@@ -1225,7 +1233,7 @@ __global__ void __launch_bounds__(32 * kBnbWarps, 6) bnb_kernel(const __grid_con
     s.stop.best = p.best + g;
     s.stop.lbp = p.lbp + g;
     s.stop.item_k = k;
-    s.stop.budget = p.budget ? (p.budget << istate) : 0;
+    s.stop.budget = p.budget ? max((p.budget << istate) >> (split ? 0 : p.unsplit_shift), uint64_t(1)) : 0;
     s.stop.exited = p.exited;
     s.stop.drain_at = p.drain_at;
     s.stop.full_at = p.full_at;
@@ -1660,6 +1668,9 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   // deadline (next_pass). Cooperative: every CTA is resident, so the warps
   // waiting at the end of a pass never wait on a CTA that cannot run.
   p.budget = (opts && opts->first_budget) ? opts->first_budget : kFirstBudget;
+  // few enough items to change over after the first pass: keep that one short
+  if (!split && may_split && !(opts && opts->first_budget) && first_items < p.split_below)
+    p.unsplit_shift = kUnsplitShift;
   p.pass_done = reinterpret_cast<uint32_t*>(h->d_io + kIoPassDone);
   p.pass_gen = reinterpret_cast<uint32_t*>(h->d_io + kIoPassGen);
   p.pass_stop = reinterpret_cast<uint32_t*>(h->d_io + kIoPassStop);
