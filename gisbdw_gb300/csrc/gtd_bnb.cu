@@ -76,6 +76,7 @@
 #include <string>
 #include <vector>
 
+#include "gtd_bnb_memo.h"
 #include "gtd_handle.h"
 
 namespace gtd {
@@ -1453,7 +1454,7 @@ struct gtd_bnb_state {
   uint4* memo = nullptr;
   size_t memo_cap = 0;
   uint64_t memo_tag = 0;   // solves so far
-  bool memo_plain = false; // the memo may hold slots that no solve has tagged
+  gtd::MemoSlots memo_plain;  // slots that may hold an entry without a solve's number
   uint8_t* arena = nullptr;  // inputs, results, items (see gtd_bnb_solve_batch)
   size_t arena_cap = 0;
   uint8_t* mini = nullptr; // per-warp small-component DP tables
@@ -1551,9 +1552,11 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   }
 
   gtd_status s;
-  if (B.memo_cap < slots * count)
-    B.memo_plain = true;  // fresh memory
-  if ((s = grow(h, &B.memo, &B.memo_cap, slots * count)) != GTD_OK) return s;
+  const size_t memo_used = slots * count;
+  if (B.memo_cap < memo_used) {
+    if ((s = grow(h, &B.memo, &B.memo_cap, memo_used)) != GTD_OK) return s;
+    B.memo_plain.fresh(B.memo_cap);
+  }
   // Split items (first root x second root) when the batch is too small to
   // give every warp a first-root item: a single graph then uses n^2 warps.
   size_t first_items = 0;
@@ -1604,11 +1607,10 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   // plain (pageable) copies: this entry point is host-synchronous anyway
   GTD_CUDA(h, cudaMemcpyAsync(B.arena, stage.data(), in_end, cudaMemcpyHostToDevice, h->stream));
   GTD_CUDA(h, cudaMemsetAsync(B.arena + in_end, 0, zero_end - in_end, h->stream));
-  if (B.memo_plain)
-    GTD_CUDA(h, cudaMemsetAsync(B.memo, 0, B.memo_cap * sizeof(uint4), h->stream));
-  else if (max_n > 64)
-    GTD_CUDA(h, cudaMemsetAsync(B.memo, 0, slots * count * sizeof(uint4), h->stream));
-  B.memo_plain = max_n > 64;
+  size_t clear_first = 0;
+  const size_t clear = B.memo_plain.clear_before(memo_used, max_n > 64, &clear_first);
+  if (clear > 0)
+    GTD_CUDA(h, cudaMemsetAsync(B.memo + clear_first, 0, clear * sizeof(uint4), h->stream));
   B.memo_tag = B.memo_tag % kKeyHiMask + 1;
   GTD_CUDA(h, cudaMemsetAsync(h->d_io, 0, kIoWords * sizeof(int32_t), h->stream));
 
