@@ -505,9 +505,12 @@ __device__ void greedy_rounds(const uint32_t* adj, int n, bool variance, RoundMe
 }
 
 // One CTA per graph; kind 0 runs kinds 1 and 2 side by side, `threads` threads
-// each. 1024 graphs of 20..80 vertices, kind 0: 1.48 ms with one warp per graph
-// and one vertex per step, 627 us when every vertex searched its new component
-// and scored itself in double, 324 us now (48 graphs of 24..36: 45 us).
+// each. Components that do not depend on where a search starts need symmetric
+// masks: a graph without them gets the height -1 and is left to the host (the
+// check adds nothing that shows). 1024 graphs of 20..80 vertices, kind 0:
+// 1.48 ms with one warp per graph and one vertex per step, 627 us when every
+// vertex searched its new component and scored itself in double, 324 us now
+// (48 graphs of 24..36: 45 us).
 __global__ void heuristic_rounds_kernel(const HeurGraph* graphs, const uint64_t* adj2, int kind, int threads,
                                         int32_t* td_out, int32_t* parent_out) {
   __shared__ __align__(16) uint32_t adj[4 * (kHMaxN + 1)];
@@ -520,6 +523,20 @@ __global__ void heuristic_rounds_kernel(const HeurGraph* graphs, const uint64_t*
   if (threadIdx.x < words)
     adj[kHMaxN * words + threadIdx.x] = 0u;
   __syncthreads();
+  bool one_way = false;
+  if (threadIdx.x < G.n) {
+    const int v = threadIdx.x;
+    for (int i = 0; i < words; ++i)
+      for (uint32_t left = adj[v * words + i]; left; left &= left - 1u) {
+        const int u = 32 * i + __ffs(static_cast<int>(left)) - 1;
+        one_way |= !((adj[u * words + (v >> 5)] >> (v & 31)) & 1u);
+      }
+  }
+  if (__syncthreads_or(one_way)) {
+    if (threadIdx.x == 0)
+      td_out[blockIdx.x] = -1;
+    return;
+  }
   const int half = threadIdx.x / threads;
   const bool variance = kind == 2 || half == 1;
   if (words == 1)
@@ -603,5 +620,12 @@ extern "C" gtd_status gtd_heuristic_batch(gtd_handle h, const gtd_graph_desc* de
   GTD_CUDA(h, cudaMemcpyAsync(td_out, d_td, size_t(count) * 4, cudaMemcpyDeviceToHost, s));
   GTD_CUDA(h, cudaMemcpyAsync(parent_out, d_par, n_pool * 4, cudaMemcpyDeviceToHost, s));
   GTD_CUDA(h, cudaStreamSynchronize(s));
+  for (int i = 0; i < count; ++i)
+    if (td_out[i] < 0) {  // masks that are not symmetric
+      const size_t off = size_t(descs[i].offset);
+      const gtd_status st = gtd_heuristic(adj2_pool + 2 * off, descs[i].n, kind, nullptr, td_out + i, parent_out + off);
+      if (st != GTD_OK)
+        return fail(h, st, "graph " + std::to_string(i));
+    }
   return GTD_OK;
 }

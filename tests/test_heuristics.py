@@ -85,3 +85,42 @@ def test_gpu_variance_scores_that_tie_and_leave_many_parts(handle, kind, n):
     for i, g in enumerate(gs):
         htd, hpar = _lib.heuristic(g, kind)
         assert td[i] == htd and pars[i].tolist() == hpar.tolist(), i
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", [0, 1, 2, 3])
+@pytest.mark.parametrize("n", [7, 32, 33, 70, 128])
+def test_gpu_heuristics_on_masks_that_are_not_symmetric_equal_host(handle, kind, n):
+    """Edges kept in one of the two masks, next to ordinary graphs: the batch
+    takes them as the host function does, with the same trees."""
+    import ctypes
+    rng = np.random.default_rng(100 * kind + n)
+    masks = []
+    for k in range(12):
+        a = rng.random((n, n)) < (2.0 + k % 3) / n
+        np.fill_diagonal(a, False)
+        if k % 4 == 0:
+            a |= a.T
+        elif k % 4 == 1:  # a single edge of an ordinary graph lacks its other direction
+            a |= a.T
+            u, v = np.argwhere(a)[rng.integers(int(a.sum()))] if a.any() else (0, 1)
+            a[u, v], a[v, u] = True, False
+        masks.append([sum(1 << int(u) for u in np.flatnonzero(row)) for row in a])
+    pool = np.array([w for m in masks for x in m for w in (x & (1 << 64) - 1, x >> 64)], dtype=np.uint64)
+    scores = rng.random(n * len(masks)).astype(np.float32)
+    descs = (_lib.GraphDesc * len(masks))()
+    for i in range(len(masks)):
+        descs[i].n, descs[i].offset = n, i * n
+    td = np.zeros(len(masks), dtype=np.int32)
+    par = np.zeros(n * len(masks), dtype=np.int32)
+    handle.heuristic_batch([G.path(3)], 1)  # binds the entry point
+    L, p = handle.L, _lib._ptr
+    sc = p(scores) if kind == 3 else None
+    assert L.gtd_heuristic_batch(handle._h, ctypes.cast(descs, ctypes.c_void_p), len(masks), p(pool), n * len(masks),
+                                 kind, sc, p(td), p(par)) == 0
+    _lib.heuristic(G.path(3))
+    for i in range(len(masks)):
+        t, q = ctypes.c_int32(), np.zeros(n, dtype=np.int32)
+        own, s = pool[2 * n * i:2 * n * (i + 1)].copy(), scores[n * i:n * (i + 1)].copy()
+        assert L.gtd_heuristic(p(own), n, kind, p(s), ctypes.byref(t), p(q)) == 0
+        assert td[i] == t.value and par[n * i:n * (i + 1)].tolist() == q.tolist(), i
