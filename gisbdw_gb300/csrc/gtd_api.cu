@@ -449,6 +449,7 @@ gtd_status gtd_dp_solve_device(gtd_handle h, const uint64_t* d_adj, int n, int32
   if (n < 2 || n > GTD_DP_MAX_N)
     return fail(h, GTD_INVALID_ARG, "device solve needs n in [2, " + std::to_string(GTD_DP_MAX_N) + "]");
   DeviceGuard g(h->device);
+  h->uncollected = true;
   return dp_enqueue(h, d_adj, nullptr, n, opts, d_td, d_parent, d_order, nullptr);
 }
 
@@ -459,6 +460,7 @@ gtd_status gtd_sync(gtd_handle h, gtd_dp_stats* stats) {
   int32_t* h_io = reinterpret_cast<int32_t*>(static_cast<char*>(h->h_pinned) + kPinnedIo);
   GTD_CUDA(h, cudaMemcpyAsync(h_io, h->d_io, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
   GTD_CUDA(h, cudaStreamSynchronize(h->stream));
+  h->uncollected = false;
   collect_stats(h);
   if (stats)
     *stats = h->last_stats;

@@ -468,6 +468,7 @@ gtd_status batch_finish(gtd_handle h, gtd_dp_batch_stats* stats) {
   int32_t* h_io = reinterpret_cast<int32_t*>(static_cast<char*>(h->h_pinned) + 1024);
   GTD_CUDA(h, cudaMemcpyAsync(h_io, h->d_io, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
   GTD_CUDA(h, cudaStreamSynchronize(h->stream));
+  h->uncollected = false;
   float ms = 0;
   if (cudaEventElapsedTime(&ms, h->ev[0], h->ev[1]) == cudaSuccess)
     h->bstats.dp_ms = ms;
@@ -533,6 +534,7 @@ gtd_status gtd_dp_solve_batch_device(gtd_handle h, const gtd_graph_desc* descs, 
   if (!d_adj_pool || !d_td || !d_parent)
     return fail(h, GTD_INVALID_ARG, "null pointer argument");
   DeviceGuard g(h->device);
+  h->uncollected = true;
   return batch_enqueue(h, descs, count, d_adj_pool, d_td, d_parent, opts);
 }
 

@@ -410,6 +410,11 @@ extern "C" gtd_status gtd_bottom_up(gtd_handle h, const uint64_t* adj, int n, in
   GTD_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, bu_kernel, kBuThreads, smem));
   const unsigned ctas = static_cast<unsigned>(
       std::min<uint64_t>(uint64_t(h->num_sms) * static_cast<unsigned>(std::max(1, occ)), p.chunks));
+  // a solve enqueued before may not have been asked for its errors yet: its
+  // words outlive this call, which has its own in their place meanwhile
+  int32_t* const kept = reinterpret_cast<int32_t*>(static_cast<char*>(h->h_pinned) + kPinnedError);
+  if (h->uncollected)
+    GTD_CUDA(h, cudaMemcpyAsync(kept, h->d_io + kIoError, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
   GTD_CUDA(h, cudaMemsetAsync(h->d_io, 0, kIoWords * sizeof(int32_t), h->stream));
   GTD_CUDA(h, cudaEventRecord(h->ev[0], h->stream));
   bu_kernel<<<ctas, kBuThreads, smem, h->stream>>>(p);
@@ -421,6 +426,8 @@ extern "C" gtd_status gtd_bottom_up(gtd_handle h, const uint64_t* adj, int n, in
   int32_t io[4] = {0, 0, 0, 0};
   GTD_CUDA(h, cudaMemcpyAsync(order.data(), p.order, n * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
   GTD_CUDA(h, cudaMemcpyAsync(io, h->d_io, sizeof(io), cudaMemcpyDeviceToHost, h->stream));
+  if (h->uncollected)  // the words kept have arrived by the time these are put back
+    GTD_CUDA(h, cudaMemcpyAsync(h->d_io + kIoError, kept, 2 * sizeof(int32_t), cudaMemcpyHostToDevice, h->stream));
   GTD_CUDA(h, cudaStreamSynchronize(h->stream));
   s = map_device_error(h, io[kIoError], io[kIoError + 1]);
   if (s != GTD_OK)

@@ -24,6 +24,7 @@ constexpr int kIoLevels = 208;  // chunks done per level (level kernel), 32 word
 constexpr int kIoWords = 256;
 // Byte offsets inside the handle's 4096-byte pinned staging block.
 constexpr size_t kPinnedIo = 1024;     // IO block copies (kIoOrder + 64 words)
+constexpr size_t kPinnedError = 2048;  // error words of an uncollected call, kept over another (bottom-up)
 constexpr size_t kPinnedAbort = 4092;  // gtd_abort's source word
 
 // Flag stamp reserved for CUDA-graph replays (the graph zeroes the flags
@@ -102,6 +103,7 @@ struct gtd_handle_s {
   // Last DP solve (for gtd_dp_query / gtd_sync).
   bool have_table = false;
   bool pending_stats = false;
+  bool uncollected = false;   // an enqueued solve (single or batch) whose error words nothing has read yet
   bool tree_timed = false;    // the tree kernel ran on its own, before ev[2]
   int last_tile_bits = 0;  // of the byte table's layout (the planes' tiles may differ)
   uint32_t last_tiles = 0;

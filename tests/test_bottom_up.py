@@ -108,3 +108,35 @@ def test_bottom_up_gpu_clique_heights(handle, n):
     chunk up to n = 23, four from n = 24 on."""
     td, par, order = handle.bottom_up(G.complete(n))
     assert td == n and order.tolist() == list(range(n)) and par.tolist() == [-1] + list(range(n - 1))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [12, 20, 24])
+@pytest.mark.parametrize("batch", [False, True])
+def test_bottom_up_keeps_the_errors_of_an_enqueued_solve(handle, port, n, batch):
+    """An enqueued solve of masks that the device rejects, a bottom-up call,
+    then the call that collects the solve's errors: it still reports them."""
+    import torch
+    good = G.gnp_connected(n, 0.3, 3)
+    masks = good.adj64().copy()
+    bad = masks.copy()
+    u = int(good.edges[0][1])
+    bad[u] &= ~(np.uint64(1) << np.uint64(good.edges[0][0]))  # the edge kept in one mask only
+    out = torch.zeros(1 + 2 * n, dtype=torch.int32, device="cuda")
+    otd, opar, oorder = port.bottom_up(G.cycle(9))
+    descs, _ = _lib.pack_batch([good])
+    for m, fails in ((bad, True), (masks, False)):
+        d = torch.from_numpy(m.view(np.int64)).cuda()
+        torch.cuda.synchronize()
+        if batch:
+            handle.dp_solve_batch_device(descs, 1, d.data_ptr(), n, out.data_ptr(), out[1:].data_ptr())
+        else:
+            handle.dp_solve_device(d.data_ptr(), n, out.data_ptr(), out[1:].data_ptr(), out[1 + n:].data_ptr())
+        td, par, order = handle.bottom_up(G.cycle(9))
+        assert (td, order.tolist(), par.tolist()) == (otd, oorder, opar.tolist())
+        collect = handle.dp_batch_sync if batch else handle.sync
+        if fails:
+            with pytest.raises(_lib.InvalidArgument):
+                collect()
+        else:
+            collect()
