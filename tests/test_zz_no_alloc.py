@@ -93,3 +93,74 @@ def test_noalloc_allocates_nothing_and_reports_bad_input():
     assert st == 1  # GTD_INVALID_ARG from the device-side check
     assert _noalloc(L, d_adj.data_ptr(), g.n, d_td.data_ptr(), d_par.data_ptr(), 0, stream.cuda_stream) == 0
     assert int(d_td.item()) == td_ref
+
+
+def _entry():
+    import torch
+
+    from gisbdw_gb300 import _lib
+    L = _lib.load()
+    L.gtd_dp_solve_noalloc.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p,
+                                       ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
+    return L, torch.cuda.Stream()
+
+
+@pytest.mark.parametrize("n", [2, 5, 6, 8, 15, 16, 17, 18, 19, 21, 22, 23])
+def test_noalloc_at_the_edges_of_its_kernels_matches_oracle(port, n):
+    """Small, cluster, level and tile kernel, one after another on the shared
+    scratch, with a rejected graph before each: treedepth, tree and order."""
+    import torch
+
+    from gisbdw_gb300 import graphs as G
+    L, stream = _entry()
+    for g in (G.gnp(n, 0.3, n), G.path(n), G.Graph(n, [(v, v + 2) for v in range(n - 2)])):
+        bad = g.adj64().copy()
+        bad[0] ^= np.uint64(2)  # in one mask only
+        out = torch.full((1 + 2 * n,), -7, dtype=torch.int32, device="cuda")
+        for masks, want in ((bad, 1), (g.adj64(), 0)):
+            d = torch.from_numpy(masks.view(np.int64)).cuda()
+            torch.cuda.synchronize()
+            assert _noalloc(L, d.data_ptr(), n, out.data_ptr(), out[1:].data_ptr(), out[1 + n:].data_ptr(),
+                            stream.cuda_stream) == want
+        T = port.dp_table(g, nthreads=8)
+        otd, opar = port.tree_from_table(g, T)
+        got = out.cpu().numpy().tolist()
+        assert got[0] == otd and got[1:1 + n] == list(opar), g.name
+        assert got[1 + n:] == port.get_elimination(g, T, (1 << n) - 1), g.name
+
+
+@pytest.mark.parametrize("n", [16, 18, 20, 22])
+def test_noalloc_is_as_fast_as_the_allocating_entry_point(n):
+    """Both take the same kernels: the call without an allocation, which leaves
+    its results on the device, within 1.5 times the other's median (the tile
+    kernel took 1.9 to 2.5 times as long)."""
+    import statistics
+    import time
+
+    import torch
+
+    from gisbdw_gb300 import Handle
+    from gisbdw_gb300 import graphs as G
+    L, stream = _entry()
+    g = G.gnp_connected(n, 0.3, 5)
+    adj = g.adj64()
+    d = torch.from_numpy(adj.view(np.int64)).cuda()
+    out = torch.zeros(1 + 2 * n, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    h = Handle(0)
+
+    def median(call):
+        for _ in range(5):
+            call()
+        t = []
+        for _ in range(40):
+            a = time.perf_counter()
+            call()
+            t.append(time.perf_counter() - a)
+        return statistics.median(t)
+
+    with h:
+        alloc = median(lambda: h.dp_solve(adj, n))
+        none = median(lambda: _noalloc(L, d.data_ptr(), n, out.data_ptr(), out[1:].data_ptr(), out[1 + n:].data_ptr(),
+                                       stream.cuda_stream))
+    assert none < 1.5 * alloc, (none * 1e6, alloc * 1e6)
