@@ -141,9 +141,11 @@ int default_tile_bits(int n) { return n >= 26 ? 11 : 10; }
 
 // Up to this n the level kernel solves a graph (up to kDpSmallBestN the small,
 // up to kDpClusterMaxN the cluster kernel; the small kernel up to kDpSmallMaxN
-// where that does not fit), unless the caller gives tile bits (level / 11-bit
-// tile kernel: n = 20 45 / 117 us, 25 112 / 234, 27 176 / 299, 28 264 / 344,
-// 29 436 / 436, 30 806 / 690).
+// where that does not fit; level / 11-bit tile kernel: n = 20 45 / 117 us,
+// 25 112 / 234, 27 176 / 299, 28 264 / 344, 29 436 / 436, 30 806 / 690).
+// Tile bits that the caller gives shape the byte table and the tile kernel
+// beyond (with them the tile kernel took 135 us at n = 18 and 10 bits, where
+// tiles of bytes had taken 122 and the cluster kernel takes 47).
 constexpr int kLevelMaxN = 28;
 
 // Allocates (or grows) the table and flag buffers and enqueues the
@@ -155,13 +157,15 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, const uint64_t* h_adj
                       int32_t* d_td, int32_t* d_parent, int32_t* d_order, int32_t* report) {
   const int tile_bits = (opts && opts->tile_bits > 0) ? opts->tile_bits : default_tile_bits(n);
   const DpLayout L = make_dp_layout(n, tile_bits);
-  const bool stall = take_stall_fault();  // test injection: needs a kernel whose tiles wait
-  const bool given_bits = opts && opts->tile_bits > 0;
+  // test injections: a stall needs a kernel whose tiles wait; a poisoned solve
+  // with tile bits runs the tile kernel, which is then under test
+  const bool stall = take_stall_fault(), poison = take_poison_fault();
+  const bool by_tile = poison && opts && opts->tile_bits > 0;
   if (h->dp_cluster < 0 && n > kDpSmallBestN && n <= kDpClusterMaxN)
     h->dp_cluster = dp_cluster_fits() ? 1 : 0;
-  const bool cluster = !given_bits && !stall && n > kDpSmallBestN && n <= kDpClusterMaxN && h->dp_cluster == 1;
-  const bool small = !given_bits && !stall && (n <= kDpSmallMaxN || cluster);
-  const bool by_level = !given_bits && !small && n <= kLevelMaxN;
+  const bool cluster = !by_tile && !stall && n > kDpSmallBestN && n <= kDpClusterMaxN && h->dp_cluster == 1;
+  const bool small = !by_tile && !stall && (n <= kDpSmallMaxN || cluster);
+  const bool by_level = !by_tile && !small && n <= kLevelMaxN;
   // the planes' tiles: n < lb is padded to one tile
   const int lb = small ? kDpSmallTileBits : by_level ? kDpLevelTileBits : L.lb < kDpMinTileBits ? kDpMinTileBits : L.lb;
   const int nh = n > lb ? n - lb : 0;
@@ -226,7 +230,7 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, const uint64_t* h_adj
   if (ctas > p.total_groups || small)
     ctas = cluster ? kDpClusterCtas : small ? 1 : p.total_groups;
 
-  if (take_poison_fault())  // test injection: every byte must be written before it is read
+  if (poison)  // every byte must be written before it is read
     GTD_CUDA(h, cudaMemsetAsync(h->d_table, 0xFF, h->table_cap, h->stream));
   if (!small)
     GTD_CUDA(h, dp_launch_validate(p, h->stream, in));

@@ -48,15 +48,17 @@ struct Plan {
 
 constexpr int kLevelSlots = kDpMaxHigh + 2;
 
-// Graphs of a batch that the small kernel takes, one CTA each, unless the
-// caller gives tile bits (2048 graphs of 15 vertices: 68 us against 265 in the
-// tile kernel, of 16: 111 against 306; from 17 on the widest level has seven
-// words per thread of the CTA and shared memory holds fewer CTAs).
+// Graphs of a batch that the small kernel takes, one CTA each (2048 graphs of
+// 15 vertices: 68 us against 265 in the tile kernel, of 16: 111 against 306;
+// from 17 on the widest level has seven words per thread of the CTA and shared
+// memory holds fewer CTAs). Tile bits that the caller gives are for the graphs
+// of the tile kernel: 2000 of 8..16 with 10 bits took 575 us in it, 538 when
+// its tiles were bytes.
 constexpr int kBatchSmallMaxN = 16;
 
 // The other graphs go to the level kernel while their subsets together are too
-// few to fill the GPU with the tile kernel's groups, unless the caller gives
-// tile bits or has them measured (level / tile kernel, us, whole batch:
+// few to fill the GPU with the tile kernel's groups, unless the caller has
+// their rates measured (level / tile kernel, us, whole batch:
 // 2 graphs of 20 vertices 65 / 139, 6 of 17..24 112 / 218, 48 of 17..21 91 /
 // 178, 300 of 17..21 190 / 230, 48 of 22..24, 450 M subsets, 328 / 340; above:
 // 1000 of 17..21, 813 M, 510 / 499, 200 of 17..24 534 / 493, 4096 of 10..24
@@ -265,10 +267,14 @@ gtd_status check_descs(gtd_handle h, const gtd_graph_desc* descs, int count, int
 // Plans the batch, (re)builds device state when the shape changed and
 // enqueues the launch (graph replay or direct). Device pointers in/out.
 gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, const uint64_t* d_adj,
-                         int32_t* d_td, int32_t* d_parent, const gtd_dp_batch_opts* opts, int force_cap = 0) {
+                         int32_t* d_td, int32_t* d_parent, const gtd_dp_batch_opts* opts, bool tuning = false,
+                         int force_cap = 0) {
   Plan P;
   pick_tile_bits(h, descs, count, opts, P, force_cap);
-  const bool own_choice = !(opts && opts->tile_bits > 0) && force_cap == 0;
+  // The tile kernel for every graph: the autotuner, which measures it, and a
+  // poisoned batch with tile bits (test injection), which is a test of it.
+  const bool poison = take_poison_fault();
+  const bool own_choice = !tuning && !(poison && opts && opts->tile_bits > 0);
   uint64_t work = 0;
   int max_n = 0;
   for (int i = 0; i < count; ++i) {
@@ -312,7 +318,6 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
   const bool same_buffers = cap.table == h->d_table && cap.flags == h->d_flags && cap.tile_map == h->d_tile_map &&
                             cap.level_base == h->d_level_base && cap.graphs == h->d_bgraphs &&
                             cap.level_done == (P.by_level ? h->d_levels : nullptr);
-  const bool poison = take_poison_fault();  // test injection (gtd_inject_fault)
   if (use_graph && h->bgraph_valid && h->bgraph_key == key && same_buffers) {
     st.graph_replayed = 1;
     if (poison)
@@ -515,7 +520,7 @@ namespace gtd {
 namespace {
 gtd_status solve_batch_host(gtd_handle h, const gtd_graph_desc* descs, int count, const uint64_t* adj_pool,
                             int64_t pool_len, int32_t* td_out, int32_t* parent_out, const gtd_dp_batch_opts* opts,
-                            gtd_dp_batch_stats* stats, int force_cap);
+                            gtd_dp_batch_stats* stats, bool tuning = false, int force_cap = 0);
 }  // namespace
 }  // namespace gtd
 
@@ -548,7 +553,7 @@ gtd_status gtd_dp_batch_sync(gtd_handle h, gtd_dp_batch_stats* stats) {
 gtd_status gtd_dp_solve_batch(gtd_handle h, const gtd_graph_desc* descs, int count, const uint64_t* adj_pool,
                               int64_t pool_len, int32_t* td_out, int32_t* parent_out,
                               const gtd_dp_batch_opts* opts, gtd_dp_batch_stats* stats) {
-  return solve_batch_host(h, descs, count, adj_pool, pool_len, td_out, parent_out, opts, stats, 0);
+  return solve_batch_host(h, descs, count, adj_pool, pool_len, td_out, parent_out, opts, stats);
 }
 
 }  // extern "C"
@@ -558,7 +563,7 @@ namespace {
 
 gtd_status solve_batch_host(gtd_handle h, const gtd_graph_desc* descs, int count, const uint64_t* adj_pool,
                             int64_t pool_len, int32_t* td_out, int32_t* parent_out, const gtd_dp_batch_opts* opts,
-                            gtd_dp_batch_stats* stats, int force_cap) {
+                            gtd_dp_batch_stats* stats, bool tuning, int force_cap) {
   if (!h)
     return GTD_INVALID_ARG;
   gtd_status s = check_descs(h, descs, count, pool_len);
@@ -584,7 +589,7 @@ gtd_status solve_batch_host(gtd_handle h, const gtd_graph_desc* descs, int count
   char* stage = static_cast<char*>(h->h_bstage);
   std::memcpy(stage, adj_pool, adj_bytes);
   GTD_CUDA(h, cudaMemcpyAsync(h->d_badj, stage, adj_bytes, cudaMemcpyHostToDevice, h->stream));
-  s = batch_enqueue(h, descs, count, h->d_badj, h->d_bout, h->d_bout + count, opts, force_cap);
+  s = batch_enqueue(h, descs, count, h->d_badj, h->d_bout, h->d_bout + count, opts, tuning, force_cap);
   if (s != GTD_OK)
     return s;
   int32_t* h_td = reinterpret_cast<int32_t*>(stage + adj_bytes);
@@ -650,7 +655,7 @@ gtd_status gtd_dp_autotune(gtd_handle h, int n_min, int n_max, float* rates_out,
         float best = 0;
         for (int rep = 0; rep < 3; ++rep) {
           gtd_status s = solve_batch_host(h, descs.data(), count, adj.data(), pool, td.data(), par.data(),
-                                          pass ? nullptr : &o, &st, pass ? lb : 0);
+                                          pass ? nullptr : &o, &st, true, pass ? lb : 0);
           if (s != GTD_OK)
             return s;
           if (rep > 0 && (best == 0 || st.dp_ms < best))

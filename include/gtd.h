@@ -80,7 +80,9 @@ gtd_status gtd_inject_fault(int kind, int count);
 
 /* Options and statistics of one subset-DP solve. */
 typedef struct {
-  int tile_bits;        /* low vertices per tile (0 = autotuned default) */
+  int tile_bits;        /* low vertices per tile of the byte table, and of the
+                           tile kernel where n is large enough for it (0 = 10,
+                           11 from n = 26 on) */
   int ctas_per_sm;      /* persistent CTAs per SM (0 = default) */
   uint64_t timeout_ns;  /* bound on every in-kernel wait (0 = 10 s) */
 } gtd_dp_opts;
@@ -153,8 +155,9 @@ typedef struct {
 } gtd_graph_desc;
 
 typedef struct {
-  int tile_bits;        /* 8..12 for every graph; 0 = planned per vertex
-                           count from gtd_dp_autotune's results (else 10) */
+  int tile_bits;        /* 8..12 for every graph of the tile kernel (larger
+                           graphs and batches); 0 = planned per vertex count
+                           from gtd_dp_autotune's results (else 10) */
   int ctas_per_sm;      /* 0 = occupancy limit */
   uint64_t timeout_ns;  /* bound on every in-kernel wait (0 = 10 s) */
   int use_cuda_graph;   /* capture the launch once, replay while the batch

@@ -1,0 +1,124 @@
+"""Which kernel a subset-DP call takes, by the number of CTAs that its
+statistics report, and each of them against the oracle. A poisoned solve
+(gtd_inject_fault) whose caller names tile bits runs the tile kernel whatever
+the sizes, so the tile kernel's edges are tested that way."""
+import numpy as np
+import pytest
+
+from gisbdw_gb300 import Handle, _lib
+from gisbdw_gb300 import graphs as G
+
+pytestmark = pytest.mark.gpu
+
+
+class poisoned:
+    def __init__(self, count=1):
+        self.count = count
+
+    def __enter__(self):
+        _lib.inject_fault(_lib.FAULT_POISON, self.count)
+
+    def __exit__(self, *exc):
+        _lib.inject_fault(_lib.FAULT_NONE, 0)
+
+
+def natural_order(raw, n, lb):
+    """The byte table by subset mask."""
+    S = np.arange(1 << n, dtype=np.int64)
+    tile = np.array([_lib.table_index(n, lb, h << lb) >> lb for h in range(1 << (n - lb))], dtype=np.int64)
+    return raw[(tile[S >> lb] << lb) | (S & ((1 << lb) - 1))]
+
+
+def same(got, want):
+    (td, parents), gs = got, want
+    for g, t, par in zip(gs, td, parents):
+        otd, opar = ORACLE(g)
+        assert t == otd and par.tolist() == list(opar), g.name
+
+
+ORACLE = None
+
+
+@pytest.fixture(autouse=True)
+def _oracle(port):
+    global ORACLE
+    known = {}
+
+    def solve(g):
+        key = (g.n, tuple(g.edges))
+        if key not in known:
+            known[key] = port.dp_solve(g)
+        return known[key]
+    ORACLE = solve
+
+
+@pytest.mark.parametrize("n", [9, 16, 18, 20, 22, 24])
+@pytest.mark.parametrize("tile_bits", [8, 9, 10, 12])
+def test_given_tile_bits_take_the_kernels_of_the_default(handle, port, n, tile_bits):
+    g = G.gnp_connected(n, 0.3, n)
+    ctas = handle.dp_solve(g.adj64(), n)[3]["ctas"]
+    td, parent, _, stats = handle.dp_solve(g.adj64(), n, tile_bits=tile_bits)
+    assert stats["ctas"] == ctas and stats["tile_bits"] == min(n, tile_bits)
+    raw, tn, lb = handle.dp_read_table()
+    assert (tn, lb) == (n, min(n, tile_bits))
+    if n <= 20:
+        T = port.dp_table(g)
+        assert np.array_equal(natural_order(raw, n, lb) >> 1, T)
+        otd, opar = port.tree_from_table(g, T)
+        assert (td, parent.tolist()) == (otd, opar.tolist())
+
+
+@pytest.mark.parametrize("tile_bits", [8, 9, 10, 11, 12])
+@pytest.mark.parametrize("n", [2, 4, 7, 8, 9, 12, 13, 16, 18])
+def test_tile_kernel_at_tile_edges_matches_oracle(handle, port, tile_bits, n):
+    """Padded tiles (n < 8), one tile, one to a few tiles per level, levels of
+    just under and over a group: every byte, the tree, the order."""
+    for g in (G.gnp(n, 0.35, 40 + n), G.path(n), G.complete(n)):
+        with poisoned():
+            td, parent, order, _ = handle.dp_solve(g.adj64(), n, tile_bits=tile_bits)
+        T = port.dp_table(g)
+        otd, opar = port.tree_from_table(g, T)
+        assert (td, parent.tolist()) == (otd, opar.tolist()), g.name
+        assert sorted(order.tolist()) == list(range(n))
+        raw, tn, lb = handle.dp_read_table()
+        assert tn == n and lb == min(n, tile_bits)
+        assert np.array_equal(natural_order(raw, n, lb) >> 1, T), g.name
+
+
+@pytest.mark.parametrize("n", [17, 20, 21, 22, 24])
+def test_cluster_and_level_kernels_equal_the_tile_kernel(handle, n):
+    """Whole tables, trees, orders and queries."""
+    for g in (G.gnp_connected(n, 0.25, n), G.grid(2, n // 2), G.Graph(n, [(v, v + 3) for v in range(n - 3)])):
+        adj = np.zeros(n, dtype=np.uint64)
+        adj[:g.n] = g.adj64()
+        with poisoned():
+            a = handle.dp_solve(adj, n, tile_bits=10)
+        table, query = handle.dp_read_table()[0], handle.dp_query((1 << n) - 6)
+        b = handle.dp_solve(adj, n)
+        assert a[3]["ctas"] != b[3]["ctas"]
+        assert a[0] == b[0] and a[1].tolist() == b[1].tolist() and a[2].tolist() == b[2].tolist()
+        assert np.array_equal(table, handle.dp_read_table()[0]) and query == handle.dp_query((1 << n) - 6)
+
+
+@pytest.mark.parametrize("tile_bits", [8, 10, 12])
+@pytest.mark.parametrize("sizes", [[20, 20], [17, 24, 3, 16, 20, 1, 18], [9, 12, 16] * 20])
+def test_batches_with_given_tile_bits_take_the_kernels_of_the_default(handle, tile_bits, sizes):
+    gs = [G.gnp_connected(n, 0.3, 10 + n) if n > 1 else G.Graph(1, []) for n in sizes]
+    ctas = handle.dp_solve_batch(gs)[2]["ctas"]
+    td, parents, stats = handle.dp_solve_batch(gs, tile_bits=tile_bits)
+    assert stats["ctas"] == ctas and stats["tile_bits"] == tile_bits
+    same((td, parents), gs)
+
+
+@pytest.mark.parametrize("tile_bits", [8, 9, 10, 11, 12])
+def test_tile_kernel_batches_match_oracle(handle, tile_bits):
+    """Graphs of every size, smaller than a tile as well, in the tile kernel:
+    a first call, a replay with other contents and a call without a graph."""
+    sizes = [1, 2, 5, 8, 9, 10, 11, 13, 16, 17, 18, 20, 21] * 2
+    default = handle.dp_solve_batch([G.gnp(n, 0.3, n) for n in sizes])[2]["ctas"]
+    for call, (seed, use_graph) in enumerate(((1, True), (2, True), (3, False))):
+        gs = [G.gnp(n, 0.3, 100 * seed + i % 13) for i, n in enumerate(sizes)]
+        with poisoned():
+            td, parents, stats = handle.dp_solve_batch(gs, tile_bits=tile_bits, use_cuda_graph=use_graph)
+        assert stats["graph_replayed"] == int(call == 1) and stats["ctas"] != default
+        same((td, parents), gs)
