@@ -2,8 +2,8 @@
 //
 // Planning (host): graphs are put in descending n; those of at most
 // kBatchSmallMaxN vertices are solved one CTA each, with no table; the others
-// go through the tile kernel. Of these each gets a table region,
-// a flag range and a descriptor. Tickets run level-major across graphs
+// go through the level kernel, or where they are many the tile kernel. Of
+// these each gets a table region, a flag range and a descriptor. Tickets run level-major across graphs
 // (level 0 of every graph, then level 1, ...), so the children a tile waits
 // for were issued long before it; the ticket -> (graph, tile) map is filled
 // on the device. The launch sequence (zero the flags and
@@ -11,15 +11,17 @@
 // replayed while the batch keeps its shape and buffers.
 //
 // The autotuner times the DP kernel per (n, tile bits) on seeded random
-// graphs; the planner then gives each vertex count its own tile size
-// (pick_tile_bits) and, when the sizes differ, launches the mixed-size
-// kernel, whose tiles dispatch on their graph's size.
+// graphs; where the tile kernel runs, the planner then gives each vertex count
+// its own tile size (pick_tile_bits) and, when the sizes differ, launches the
+// mixed-size kernel, whose tiles dispatch on their graph's size.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <chrono>
 #include <cstring>
 #include <numeric>
+#include <optional>
 #include <string>
 #include <vector>
 
@@ -29,15 +31,13 @@ namespace gtd {
 namespace {
 
 struct Plan {
-  int lb = 10;                  // the launch's (largest) tile bits
+  int lb = 10;                  // the tile kernel's (largest) tile bits
   bool mixed = false;           // graphs carry their own tile bits
-  int lb_by_n[GTD_DP_MAX_N + 1] = {};
   std::vector<DpGraph> graphs;  // processing order
   uint64_t table_bytes = 0;
   uint32_t total_tiles = 0;
   uint32_t total_groups = 0;    // tickets
   int kid_rows = 0;             // largest nh
-  bool rated = false;           // the tile sizes come from the autotuner's rates
   bool by_level = false;        // the other graphs go to the level kernel
   int small = 0;                // graphs at the end of `graphs` that the small kernel takes (no tiles)
   uint64_t plane_bytes = 0;     // the pool itself; table_bytes counts one byte per padded subset
@@ -57,8 +57,8 @@ constexpr int kLevelSlots = kDpMaxHigh + 2;
 constexpr int kBatchSmallMaxN = 16;
 
 // The other graphs go to the level kernel while their subsets together are too
-// few to fill the GPU with the tile kernel's groups, unless the caller has
-// their rates measured (level / tile kernel, us, whole batch:
+// few to fill the GPU with the tile kernel's groups, whose rates (of batches
+// that fill it) say nothing about them (level / tile kernel, us, whole batch:
 // 2 graphs of 20 vertices 65 / 139, 6 of 17..24 112 / 218, 48 of 17..21 91 /
 // 178, 300 of 17..21 190 / 230, 48 of 22..24, 450 M subsets, 328 / 340; above:
 // 1000 of 17..21, 813 M, 510 / 499, 200 of 17..24 534 / 493, 4096 of 10..24
@@ -81,37 +81,70 @@ constexpr uint64_t kBatchLevelSubsets = uint64_t(1) << 29;
 // autotuner's own measurement) plans a mixed launch at that cap. A size that
 // leaves more than kDpMaxHigh high vertices is raised to the least that does
 // not, as in a single solve (n = 35 needs 9 bits, n = 36 needs 10).
-void pick_tile_bits(gtd_handle h, const gtd_graph_desc* descs, int count, const gtd_dp_batch_opts* opts, Plan& P,
-                    int force_cap = 0) {
-  std::vector<int> count_by_n(GTD_DP_MAX_N + 1, 0);
-  int max_n = 0;
-  for (int i = 0; i < count; ++i) {
-    ++count_by_n[descs[i].n];
-    max_n = std::max(max_n, descs[i].n);
+struct TileSizes {
+  int lb = 10;         // the launch's (largest) tile bits
+  bool mixed = false;  // graphs carry their own tile bits
+  bool rated = false;  // chosen by the autotuner's rates
+  int by_n[GTD_DP_MAX_N + 1] = {};
+};
+
+// CTAs per SM by tile bits, of the one-size and the mixed kernel, for a batch
+// whose largest graph has max_n vertices.
+struct Occupancy {
+  int one[kTuneLbMax + 1] = {}, mixed[kTuneLbMax + 1] = {};
+  Occupancy(gtd_handle h, int max_n) {
+    auto high_at = [&](int lb) { return std::min(std::max(0, max_n - lb), kDpMaxHigh); };
+    for (int lb = kTuneLbMin; lb <= kTuneLbMax; ++lb) {
+      int& o = h->dp_occ[lb][high_at(lb)];
+      if (o <= 0)
+        o = dp_tile_occupancy(lb, high_at(lb));
+      int& m = h->dp_occ_mixed[lb][high_at(kTuneLbMin)];
+      if (m <= 0)
+        m = dp_mixed_occupancy(lb, high_at(kTuneLbMin));
+      one[lb] = std::max(1, o);
+      mixed[lb] = m;
+    }
   }
+};
+
+using CountByN = std::array<int, GTD_DP_MAX_N + 1>;
+
+// The autotuner has rates for every n of the batch.
+bool all_rated(gtd_handle h, const CountByN& count_by_n) {
+  for (int n = 0; n <= GTD_DP_MAX_N; ++n)
+    for (int lb = kTuneLbMin; lb <= kTuneLbMax && count_by_n[n]; ++lb)
+      if (h->tune[n][lb] <= 0)
+        return false;
+  return true;
+}
+
+TileSizes pick_tile_bits(gtd_handle h, const CountByN& count_by_n, const gtd_dp_batch_opts* opts, int force_cap,
+                         const Occupancy* occ) {
+  TileSizes P;
+  int max_n = GTD_DP_MAX_N;
+  while (max_n > 0 && !count_by_n[max_n])
+    --max_n;
   const int lb_min = std::max(kTuneLbMin, max_n - kDpMaxHigh);
   auto uniform = [&](int lb) {
     lb = std::max(lb, lb_min);
     P.lb = lb;
     P.mixed = false;
     for (int n = 0; n <= GTD_DP_MAX_N; ++n)
-      P.lb_by_n[n] = count_by_n[n] ? lb : 0;
+      P.by_n[n] = count_by_n[n] ? lb : 0;
   };
   if (force_cap > 0) {
     uniform(force_cap);
     P.mixed = true;
-    return;
+    return P;
   }
   if (opts && opts->tile_bits > 0) {
     uniform(std::min(std::max(opts->tile_bits, kTuneLbMin), kTuneLbMax));
-    return;
+    return P;
   }
-  for (int n = 0; n <= GTD_DP_MAX_N; ++n)
-    for (int lb = kTuneLbMin; lb <= kTuneLbMax && count_by_n[n]; ++lb)
-      if (h->tune[n][lb] <= 0) {
-        uniform(10);
-        return;
-      }
+  if (!occ || !all_rated(h, count_by_n)) {
+    uniform(10);
+    return P;
+  }
   P.rated = true;
   auto t_of = [&](int n, int lb) { return double(uint64_t(1) << std::max(n, lb)) / h->tune[n][lb]; };
   double best_cost = -1;
@@ -125,22 +158,12 @@ void pick_tile_bits(gtd_handle h, const gtd_graph_desc* descs, int count, const 
       uniform(lb);
     }
   }
-  // high vertices of the batch's largest graph at lb bits
-  auto high_at = [&](int lb) {
-    int n = GTD_DP_MAX_N;
-    while (n > 0 && !count_by_n[n])
-      --n;
-    return std::min(std::max(0, n - lb), kDpMaxHigh);
-  };
-  int occ_one[kTuneLbMax + 1] = {};
-  for (int lb = kTuneLbMin; lb <= kTuneLbMax; ++lb)
-    occ_one[lb] = std::max(1, dp_tile_occupancy(lb, high_at(lb)));
   for (int c = lb_min; c <= kTuneLbMax; ++c) {
-    const int occ_mixed = dp_mixed_occupancy(c, high_at(kTuneLbMin));
+    const int occ_mixed = occ->mixed[c];
     const float eff = h->tune_mixed_eff[c];
     if (eff <= 0 || occ_mixed < 1)
       continue;  // unmeasured: never mix at this cap
-    const double slow_c = std::max(1.0, double(occ_one[c]) / occ_mixed);
+    const double slow_c = std::max(1.0, double(occ->one[c]) / occ_mixed);
     const double residual = std::min(1.0, eff * slow_c);  // efficiency beyond the occupancy effect
     int choice[GTD_DP_MAX_N + 1] = {};
     double cost = 0;
@@ -150,7 +173,7 @@ void pick_tile_bits(gtd_handle h, const gtd_graph_desc* descs, int count, const 
         continue;
       double best_t = -1;
       for (int lb = std::max(kTuneLbMin, n - kDpMaxHigh); lb <= c; ++lb) {
-        const double t = t_of(n, lb) * std::max(1.0, double(occ_one[lb]) / occ_mixed);
+        const double t = t_of(n, lb) * std::max(1.0, double(occ->one[lb]) / occ_mixed);
         if (best_t < 0 || t < best_t) {
           best_t = t;
           choice[n] = lb;
@@ -166,12 +189,16 @@ void pick_tile_bits(gtd_handle h, const gtd_graph_desc* descs, int count, const 
       P.lb = c;
       P.mixed = true;
       for (int n = 0; n <= GTD_DP_MAX_N; ++n)
-        P.lb_by_n[n] = choice[n];
+        P.by_n[n] = choice[n];
     }
   }
+  return P;
 }
 
-void make_plan(Plan& P, const gtd_graph_desc* descs, int count, bool small_kernel) {
+// `planned`: tile bits by vertex count that the statistics report (as if the
+// tile kernel took every graph), `run`: those of the graphs that it takes.
+void make_plan(Plan& P, const gtd_graph_desc* descs, int count, bool small_kernel, const TileSizes& planned,
+               const TileSizes& run) {
   std::vector<int> order(count);
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return descs[a].n > descs[b].n; });
@@ -188,7 +215,8 @@ void make_plan(Plan& P, const gtd_graph_desc* descs, int count, bool small_kerne
     const gtd_graph_desc& d = descs[order[k]];
     DpGraph& G = P.graphs[k];
     const bool in_small = small_kernel && d.n <= kBatchSmallMaxN;
-    const int planned = P.lb_by_n[d.n], lb = P.by_level && !in_small ? kDpLevelTileBits : planned;
+    const int lb = in_small ? planned.by_n[d.n] : P.by_level ? kDpLevelTileBits : run.by_n[d.n];
+    const int bits = planned.by_n[d.n];
     G.n = d.n;
     G.lb = lb;
     G.nh = d.n > lb ? d.n - lb : 0;
@@ -197,8 +225,8 @@ void make_plan(Plan& P, const gtd_graph_desc* descs, int count, bool small_kerne
     G.flag_base = group;
     G.adj_off = static_cast<uint32_t>(d.offset);
     G.out_idx = order[k];
-    P.table_bytes += uint64_t(1) << std::max(d.n, planned);
-    tile += 1u << std::max(0, d.n - planned);
+    P.table_bytes += uint64_t(1) << std::max(d.n, bits);
+    tile += 1u << std::max(0, d.n - bits);
     if (in_small) {
       ++P.small;
     } else {
@@ -269,21 +297,39 @@ gtd_status check_descs(gtd_handle h, const gtd_graph_desc* descs, int count, int
 gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, const uint64_t* d_adj,
                          int32_t* d_td, int32_t* d_parent, const gtd_dp_batch_opts* opts, bool tuning = false,
                          int force_cap = 0) {
-  Plan P;
-  pick_tile_bits(h, descs, count, opts, P, force_cap);
+  CountByN all = {};
+  for (int i = 0; i < count; ++i)
+    ++all[descs[i].n];
+  int max_n = GTD_DP_MAX_N;
+  while (!all[max_n])
+    --max_n;
+  std::optional<Occupancy> occupancy;  // asked for where rates weigh tile sizes
+  if (!tuning && !(opts && opts->tile_bits > 0) && all_rated(h, all))
+    occupancy.emplace(h, max_n);
+  const TileSizes planned = pick_tile_bits(h, all, opts, force_cap, occupancy ? &*occupancy : nullptr);
   // The tile kernel for every graph: the autotuner, which measures it, and a
-  // poisoned batch with tile bits (test injection), which is a test of it.
+  // poisoned batch with tile bits or rates (test injection), a test of it.
   const bool poison = take_poison_fault();
-  const bool own_choice = !tuning && !(poison && opts && opts->tile_bits > 0);
+  const bool own_choice = !tuning && !(poison && ((opts && opts->tile_bits > 0) || planned.rated));
+  CountByN others = all;  // those that the small kernel does not take
   uint64_t work = 0;
-  int max_n = 0;
-  for (int i = 0; i < count; ++i) {
-    max_n = std::max(max_n, descs[i].n);
-    if (descs[i].n > kBatchSmallMaxN)
-      work += uint64_t(1) << descs[i].n;
+  for (int n = 0; n <= GTD_DP_MAX_N; ++n) {
+    if (own_choice && n <= kBatchSmallMaxN)
+      others[n] = 0;
+    work += others[n] * (uint64_t(1) << n);
   }
-  P.by_level = own_choice && !P.rated && max_n <= kBatchLevelMaxN && work <= kBatchLevelSubsets;
-  make_plan(P, descs, count, own_choice);
+  Plan P;
+  P.by_level = own_choice && max_n <= kBatchLevelMaxN && work <= kBatchLevelSubsets;
+  TileSizes run = planned;
+  if (own_choice && !P.by_level && max_n > kBatchSmallMaxN && others != all && !(opts && opts->tile_bits > 0)) {
+    // rates of the graphs that the tile kernel takes alone decide its sizes
+    if (!occupancy && all_rated(h, others))
+      occupancy.emplace(h, max_n);
+    run = pick_tile_bits(h, others, opts, force_cap, occupancy ? &*occupancy : nullptr);
+  }
+  P.lb = run.lb;
+  P.mixed = run.mixed;
+  make_plan(P, descs, count, own_choice, planned, run);
   const int lb = P.lb;
   const uint64_t timeout = (opts && opts->timeout_ns) ? opts->timeout_ns : 10ull * 1000 * 1000 * 1000;
   int occ = 1;
@@ -306,11 +352,11 @@ gtd_status batch_enqueue(gtd_handle h, const gtd_graph_desc* descs, int count, c
   st.subsets = P.subsets;
   st.alg_bytes = P.alg_bytes;
   st.table_bytes = P.table_bytes;
-  st.tile_bits = lb;
+  st.tile_bits = planned.lb;
   st.tiles = static_cast<int>(P.total_tiles);
   st.ctas = static_cast<int>(ctas);
   for (int n = 0; n <= GTD_DP_MAX_N; ++n)
-    st.tile_bits_by_n[n] = P.lb_by_n[n];
+    st.tile_bits_by_n[n] = planned.by_n[n];
 
   // The captured graph holds the handle's buffer addresses: replay only while
   // no other call has reallocated them (a larger single solve grows the table).

@@ -91,6 +91,7 @@ struct gtd_handle_s {
   // vertices, row 0 the level kernel's (0 = not asked yet):
   // a property of the kernel and the device, looked up once per handle.
   int dp_occ[gtd::kDpMaxTileBits + 1][gtd::kDpMaxHigh + 1] = {};
+  int dp_occ_mixed[gtd::kDpMaxTileBits + 1][gtd::kDpMaxHigh + 1] = {};  // of the mixed-size kernel
 
   int dp_cluster = -1;        // 1: the device takes the cluster kernel (-1: not asked yet)
 

@@ -122,3 +122,58 @@ def test_tile_kernel_batches_match_oracle(handle, tile_bits):
             td, parents, stats = handle.dp_solve_batch(gs, tile_bits=tile_bits, use_cuda_graph=use_graph)
         assert stats["graph_replayed"] == int(call == 1) and stats["ctas"] != default
         same((td, parents), gs)
+
+
+def _rated(choice, n_min=2, n_max=28, eff=1.0):
+    """A handle with rates that favour choice(n) tile bits."""
+    h = Handle(0)
+    r = np.ones((n_max - n_min + 1, 5), dtype=np.float32)
+    for n in range(n_min, n_max + 1):
+        r[n - n_min, choice(n) - 8] = 1e4
+    h.dp_set_rates(n_min, r, mixed_eff=np.full(5, eff))
+    return h
+
+
+@pytest.mark.parametrize("sizes", [[20, 20], [17, 24, 3, 16, 20, 18], [17, 18, 19, 20, 21] * 8, [9, 12, 16] * 20])
+def test_rated_handles_take_the_kernels_of_the_others(handle, sizes):
+    """Batches of few subsets: with rates as without them."""
+    gs = [G.gnp_connected(n, 0.3, 30 + n) for n in sizes]
+    ctas = handle.dp_solve_batch(gs)[2]["ctas"]
+    with _rated(lambda n: 9 + n % 3) as h:
+        td, parents, stats = h.dp_solve_batch(gs)
+        assert stats["ctas"] == ctas
+        assert stats["tile_bits_by_n"] == {n: 9 + n % 3 for n in set(sizes)} or len(set(sizes)) == 1
+        same((td, parents), gs)
+
+
+@pytest.mark.parametrize("choice", [lambda n: 8 if n <= 16 else 12, lambda n: 9 + n % 3, lambda n: 11 if n >= 20 else 10])
+def test_mixed_tile_kernel_matches_oracle(handle, choice):
+    """The mixed-size tile kernel on graphs of every size: a first call and a
+    replay with other contents."""
+    sizes = [2, 5, 8, 9, 10, 11, 13, 16, 17, 18, 20, 21] * 2
+    default = handle.dp_solve_batch([G.gnp(n, 0.3, n) for n in sizes])[2]["ctas"]
+    with _rated(choice) as h:
+        for call in range(2):
+            gs = [G.gnp(n, 0.3, 100 * call + i % 12) for i, n in enumerate(sizes)]
+            with poisoned():
+                td, parents, stats = h.dp_solve_batch(gs)
+            assert stats["tile_bits_by_n"] == {n: choice(n) for n in sizes}
+            assert stats["graph_replayed"] == call and stats["ctas"] != default
+            same((td, parents), gs)
+
+
+def test_rates_of_small_graphs_are_not_asked_for(handle):
+    """More subsets than the level kernel takes: the rates of the graphs in the
+    tile kernel choose its tile size, with or without rates of the others."""
+    gs = [G.gnp_connected(24, 0.2, i % 3) for i in range(40)] + [G.gnp_connected(10, 0.3, 1)]
+
+    def solve(h, **kw):  # treedepths, least device time of eight
+        runs = [h.dp_solve_batch(gs, **kw) for _ in range(8)]
+        return runs[0][0].tolist(), min(r[2]["dp_ms"] for r in runs)
+    td8, t8 = solve(handle, tile_bits=8)
+    td10, t10 = solve(handle)
+    with _rated(lambda n: 8, n_min=17) as h:
+        td, t = solve(h)
+    assert td == td8 == td10
+    # 8-bit tiles take a quarter more time here: which of the two sizes ran
+    assert t8 > 1.1 * t10 and t > (t8 + t10) / 2, (t8, t10, t)
