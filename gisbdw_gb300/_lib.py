@@ -313,26 +313,34 @@ _PACK = None
 
 
 def _pack_edges():
+    """The native packer, or None where its library cannot be built or loaded."""
     global _PACK
     if _PACK is None:
+        _PACK = False
         load()  # builds both libraries when needed
-        fn = ctypes.PyDLL(_build.PACK_LIB).gtd_pack_edges
-        fn.argtypes = [ctypes.py_object, _vp, _vp, _i, _vp]
-        _PACK = fn
-    return _PACK
+        path = _build.pack_library()
+        if path is not None:
+            try:
+                fn = ctypes.PyDLL(path).gtd_pack_edges
+            except OSError:
+                return None
+            fn.argtypes = [ctypes.py_object, _vp, _vp, _i, _vp]
+            _PACK = fn
+    return _PACK or None
 
 
 def adjacency_pool(graphs, words: int) -> np.ndarray:
     """The masks of every graph one after another: adj64() (words = 1) or
     adj128() (words = 2, lo and hi per vertex) of each, built in one native
-    pass over the edge lists."""
+    pass over the edge lists where that is to be had."""
     graphs = list(graphs)
     ns = np.array([g.n for g in graphs], dtype=np.int64)
     offs = np.zeros(len(graphs) + 1, dtype=np.int64)
     np.cumsum(ns, out=offs[1:])
     out = np.zeros(words * int(offs[-1]), dtype=np.uint64)
-    if len(graphs) and int(ns.max()) <= 64 * words and \
-            _pack_edges()([g.edges for g in graphs], _ptr(ns), _ptr(offs), words, _ptr(out)) == 0:
+    pack = _pack_edges()
+    if pack is not None and len(graphs) and int(ns.max()) <= 64 * words and \
+            pack([g.edges for g in graphs], _ptr(ns), _ptr(offs), words, _ptr(out)) == 0:
         return out
     parts = [g.adj64() if words == 1 else g.adj128() for g in graphs]
     return np.concatenate(parts).astype(np.uint64) if parts else out

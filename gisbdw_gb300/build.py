@@ -4,7 +4,8 @@ Every translation unit under csrc/ is compiled by nvcc in parallel with
 ``-gencode arch=compute_103a,code=sm_103a`` and linked into
 ``gisbdw_gb300/_build/libgtd.so`` (cudart linked statically, so the library
 only needs the driver at run time). gtd_pack.c, the batch packer over Python
-edge lists, becomes a library of its own next to it.
+edge lists, becomes a library of its own next to it, for the interpreter that
+builds it; without a C compiler or the Python headers the package does without.
 """
 from __future__ import annotations
 
@@ -14,12 +15,15 @@ import subprocess
 import sys
 import sysconfig
 from concurrent.futures import ThreadPoolExecutor
+from typing import Optional
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT_DIR, "libgtd.so")
-PACK_LIB = os.path.join(OUT_DIR, "libgtdpack.so")  # edge lists to masks (CPython)
+# edge lists to masks: reads CPython's objects, so one file per interpreter
+PACK_LIB = os.path.join(OUT_DIR, "libgtdpack" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+PACK_SRC = os.path.join(CSRC, "gtd_pack.c")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
@@ -47,27 +51,39 @@ def _compile(src: str, verbose: bool) -> str:
     return obj
 
 
-def _compile_pack() -> None:
+def _compile_pack() -> bool:
     tmp = PACK_LIB + ".tmp"
-    cmd = ["gcc", "-O2", "-fPIC", "-shared", "-I" + sysconfig.get_paths()["include"],
-           os.path.join(CSRC, "gtd_pack.c"), "-o", tmp]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError(f"gcc failed on gtd_pack.c:\n{r.stderr}")
-    os.replace(tmp, PACK_LIB)
+    cmd = ["gcc", "-O2", "-fPIC", "-shared", "-I" + sysconfig.get_paths()["include"], PACK_SRC, "-o", tmp]
+    try:
+        done = subprocess.run(cmd, capture_output=True, text=True).returncode == 0
+    except OSError:
+        done = False
+    if done:
+        os.replace(tmp, PACK_LIB)
+    elif os.path.exists(PACK_LIB):
+        os.remove(PACK_LIB)  # of an older source
+    return done
+
+
+def pack_library() -> Optional[str]:
+    """The batch packer's library, compiled when it is missing or stale; None
+    where it cannot be."""
+    if not _newer(PACK_LIB, [PACK_SRC, __file__]) and not _compile_pack():
+        return None
+    return PACK_LIB
 
 
 def sources():
     return sorted(glob.glob(os.path.join(CSRC, "*.cu")))
 
 
+def _newer(lib: str, deps) -> bool:
+    return os.path.exists(lib) and all(os.path.getmtime(d) <= os.path.getmtime(lib) for d in deps)
+
+
 def up_to_date() -> bool:
-    if not os.path.exists(LIB) or not os.path.exists(PACK_LIB):
-        return False
-    t = min(os.path.getmtime(LIB), os.path.getmtime(PACK_LIB))
     deps = sources() + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(CSRC, "*.cuh"))
-    deps += glob.glob(os.path.join(CSRC, "*.c")) + glob.glob(os.path.join(INCLUDE, "*.h")) + [__file__]
-    return all(os.path.getmtime(d) <= t for d in deps)
+    return _newer(LIB, deps + glob.glob(os.path.join(INCLUDE, "*.h")) + [__file__])
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -78,7 +94,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
     with ThreadPoolExecutor(max_workers=max(1, min(len(srcs), os.cpu_count() or 4))) as ex:
         pack = ex.submit(_compile_pack)
         objs = list(ex.map(lambda s: _compile(s, verbose), srcs))
-        pack.result()
+        if not pack.result():
+            sys.stderr.write("gtd_pack.c not compiled (gcc or Python headers missing): batches are packed in Python\n")
     tmp = LIB + ".tmp"
     cmd = [nvcc()] + ARCH + ["-shared", "-o", tmp] + objs + ["-lpthread", "-ldl", "-lrt"]
     r = subprocess.run(cmd, capture_output=True, text=True)
