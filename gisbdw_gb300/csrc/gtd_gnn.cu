@@ -337,8 +337,15 @@ struct TileParams {
   float *pooled, *dlogit, *dtd;
   float* tile_loss;            // [tiles]
   int64_t nparams;
-  float* part;                 // [chunks of 64 rows][nparams]: weight gradients of every chunk
+  float* part;                 // [kGradRun][nparams]: weight gradients of the chunks of 64 rows of a run
+  int first_chunk;             // of the run
 };
+
+// Chunks whose weight gradients are held at a time (51 MB with three layers).
+// More of them, from 32,769 nodes on, take further launches: all at once, with
+// eight layers, a training step took 1.4 times the memory of the layer-by-layer
+// kernels, which hold one matrix's.
+constexpr int kGradRun = 512;
 
 // BF16 weights (rows of 64, 16-byte aligned: every parameter block starts at a
 // multiple of 64 values) to FP32 rows of kRow, in two halves: the loads can be
@@ -801,7 +808,7 @@ __global__ void __launch_bounds__(kGradThreads) gnn_weight_grads(const __grid_co
   constexpr int kChunk = 64;
   const int tid = threadIdx.x, H = kWide, L = p.layers, fin = p.fin, what = static_cast<int>(blockIdx.y);
   const int total = what == L + 2 ? p.num_graphs : p.num_nodes;
-  const int r0 = static_cast<int>(blockIdx.x) * kChunk, rows = min(kChunk, total - r0);
+  const int r0 = (p.first_chunk + static_cast<int>(blockIdx.x)) * kChunk, rows = min(kChunk, total - r0);
   if (rows <= 0)
     return;
   const int64_t layer0 = int64_t(fin) * H + H, stride = 2 * int64_t(H) * H + H, head = layer0 + L * stride;
@@ -884,18 +891,22 @@ __global__ void __launch_bounds__(kGradThreads) gnn_weight_grads(const __grid_co
   }
 }
 
-// The gradient: every parameter's chunks in ascending order; the loss: the
-// tiles' likewise.
+// The gradient: every parameter's chunks in ascending order, on top of those of
+// earlier runs; the loss (with the first run): the tiles' likewise.
 __global__ void __launch_bounds__(128) gnn_sum_chunks(const __grid_constant__ TileParams p, int tiles,
                                                       float* __restrict__ grad, float* __restrict__ loss) {
   const int64_t t = int64_t(blockIdx.x) * 128 + threadIdx.x;
   if (t > p.nparams)
     return;
   const int64_t graph_head = p.nparams - kWide - 1;
-  const int count = t == p.nparams ? tiles : ((t >= graph_head ? p.num_graphs : p.num_nodes) + 63) / 64;
+  const bool again = p.first_chunk > 0;
+  if (again && t == p.nparams)
+    return;
+  const int chunks = ((t >= graph_head ? p.num_graphs : p.num_nodes) + 63) / 64 - p.first_chunk;
+  const int count = t == p.nparams ? tiles : min(chunks, kGradRun);
   const float* from = t == p.nparams ? p.tile_loss : p.part + t;
   const int64_t step = t == p.nparams ? 1 : p.nparams;
-  float acc = 0.f;
+  float acc = again ? grad[t] : 0.f;
 #pragma unroll 8
   for (int c = 0; c < count; ++c)
     acc += from[c * step];
@@ -1181,7 +1192,7 @@ gtd_status run_tiles(gtd_gnn g, const gtd_gnn_batch* b, bool train, float td_wei
   const size_t ores = take(256), otde = take(G * 4), olog = take(N * 4), res_bytes = train ? 8 : off - ores;
   const size_t ohs = take(train ? (L + 1) * NH * 4 : 0), oas = take(train ? L * NH * 4 : 0),
                odz = take(train ? (L + 1) * NH * 4 : 0), opool = take(train ? G * gtd::kWide * 4 : 0),
-               otl2 = take(train ? size_t(tiles) * 4 : 0), opart = take(train ? chunks * size_t(g->nparams) * 4 : 0);
+               otl2 = take(train ? size_t(tiles) * 4 : 0), opart = take(train ? std::min(chunks, size_t(gtd::kGradRun)) * size_t(g->nparams) * 4 : 0);
   GTD_CUDA(h, gtd::ensure_device(&g->buf, &g->buf_cap, off));
   const size_t stage = std::max(staged, res_bytes);
   if (g->stage_cap < stage) {
@@ -1246,10 +1257,14 @@ gtd_status run_tiles(gtd_gnn g, const gtd_gnn_batch* b, bool train, float td_wei
     GTD_CUDA(h, (M == 32   ? launch_tile_kernel<32, true>(p, tiles, s)
                  : M == 64 ? launch_tile_kernel<64, true>(p, tiles, s)
                            : launch_tile_kernel<128, true>(p, tiles, s)));
-    const dim3 grid(static_cast<unsigned>(chunks), static_cast<unsigned>(g->layers + 3));
-    gtd::gnn_weight_grads<<<grid, gtd::kGradThreads, 3 * 64 * gtd::kRow * 4, s>>>(p);
-    gtd::gnn_sum_chunks<<<gtd::blocks_for(size_t(g->nparams) + 1, 128), 128, 0, s>>>(p, tiles, g->grad,
-                                                                                    f(ores) + 1);
+    for (size_t first = 0; first < chunks; first += gtd::kGradRun) {
+      p.first_chunk = static_cast<int>(first);
+      const dim3 grid(static_cast<unsigned>(std::min(chunks - first, size_t(gtd::kGradRun))),
+                      static_cast<unsigned>(g->layers + 3));
+      gtd::gnn_weight_grads<<<grid, gtd::kGradThreads, 3 * 64 * gtd::kRow * 4, s>>>(p);
+      gtd::gnn_sum_chunks<<<gtd::blocks_for(size_t(g->nparams) + 1, 128), 128, 0, s>>>(p, tiles, g->grad,
+                                                                                      f(ores) + 1);
+    }
     GTD_CUDA(h, cudaGetLastError());
   } else {
     GTD_CUDA(h, (M == 32   ? launch_tile_kernel<32, false>(p, tiles, s)

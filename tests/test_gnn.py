@@ -223,3 +223,51 @@ def test_neighbours_outside_their_graph_take_the_layerwise_kernels(handle):
     rlogits, rtd = gnn.reference_loss(net.params(), c, want_grad=False)
     np.testing.assert_allclose(logits, rlogits, rtol=2e-4, atol=2e-5)
     np.testing.assert_allclose(td, rtd, rtol=2e-4, atol=2e-5)
+
+
+def _joined_singles(count, n, seed, across):
+    """A training batch of `count` graphs of n vertices between two single
+    vertices of the same features and labels. These are each other's neighbours
+    (`across`: the batch takes the layer-by-layer kernels) or each its own (the
+    tile kernels), which makes the same network: every sum has the same terms."""
+    rng = np.random.default_rng(seed)
+    kinds = [G.tree_plus_edges(n, n // 4, seed + i) for i in range(16)]
+    one = G.Graph(1, [])
+    gs = [one] + [kinds[i % 16] for i in range(count)] + [one]
+    roots = [(rng.random(g.n) < 0.4).astype(np.float32) for g in gs]
+    roots[-1] = roots[0]
+    b = gnn.make_batch(gs, roots=roots, tds=[2.0 + i % 5 for i in range(count + 1)] + [2.0])
+    last = int(b.graph_start[-1]) - 1
+    ends = (last, 0) if across else (0, last)
+    nbr = np.concatenate([[ends[0]], b.nbr[:b.nbr_start[-1]], [ends[1]]]).astype(np.int32)
+    start = b.nbr_start + 1
+    start[0], start[-1] = 0, len(nbr)
+    return gnn.Batch(b.x, b.graph_start, start.astype(np.int32), nbr, b.root_label, b.node_mask, b.td_label)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count", [1600, 1700, 3400])  # 500, 532 and 1063 chunks of 64 nodes
+def test_weight_gradients_of_many_chunks_equal_the_layerwise_kernels(handle, count):
+    """Runs of 512 chunks, one to three of them: the sums go on where the run
+    before ended, so the bits are those of the layer-by-layer kernels."""
+    net = gnn.GNN(handle, seed=2)
+    tiles, layers = (net.gradients(_joined_singles(count, 20, 5, across))[0] for across in (False, True))
+    assert np.array_equal(tiles, layers)
+
+
+@pytest.mark.gpu
+def test_a_large_training_batch_takes_no_more_memory_than_layer_by_layer():
+    import torch
+
+    from gisbdw_gb300 import Handle
+    layers, hid = 8, 64
+    b = _joined_singles(9000, 24, 1, False)  # 216,002 nodes
+    nodes = len(b.x)
+    with Handle(0) as h:
+        net = gnn.GNN(h, seed=1, layers=layers)
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        net.gradients(b)
+        used = before - torch.cuda.mem_get_info()[0]
+    # features; Z and h of every layer and the input, the means; dh, dz, da and one more
+    assert used < 4 * nodes * (gnn.IN_FEATURES + hid * (2 * (layers + 1) + layers + 4)), used
