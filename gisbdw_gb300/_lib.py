@@ -279,10 +279,11 @@ class Handle:
 
     def dp_read_table(self) -> Tuple[np.ndarray, int, int]:
         """Raw table bytes (tiled layout), n and tile bits of the last solve."""
-        _, nbytes, n, lb = self.dp_table_info()
-        out = np.empty(nbytes, dtype=np.uint8)
-        self._check(self.L.gtd_dp_read_table(self._h, _ptr(out), nbytes))
-        return out, n, lb
+        nbytes, n, lb = _u64(), _i(), _i()
+        self._check(self.L.gtd_dp_table(self._h, None, ctypes.byref(nbytes), ctypes.byref(n), ctypes.byref(lb)))
+        out = np.empty(nbytes.value, dtype=np.uint8)
+        self._check(self.L.gtd_dp_read_table(self._h, _ptr(out), nbytes.value))
+        return out, n.value, lb.value
 
 
 class PerGraph(Sequence):

@@ -3,6 +3,7 @@
 // gtd_status and keeps a message for gtd_last_error.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <cstdio>
@@ -104,6 +105,8 @@ cudaError_t ensure_device(void** ptr, size_t* cap, size_t bytes) {
   cudaError_t e = cudaMalloc(ptr, want);
   if (e == cudaSuccess)
     *cap = want;
+  else
+    cudaGetLastError();  // reported by this call, not by the next launch
   return e;
 }
 
@@ -264,13 +267,16 @@ gtd_status dp_enqueue(gtd_handle h, const uint64_t* d_adj, const uint64_t* h_adj
   return GTD_OK;
 }
 
+// What gtd_dp_read_table expands at a time where 2^n bytes are not to be had.
+constexpr uint64_t kTablePiece = uint64_t(1) << 26;
+
 // The last solve's byte table in h->d_bytes (enqueued on the stream).
 gtd_status make_byte_table(gtd_handle h) {
   if (h->bytes_valid)
     return GTD_OK;
   const size_t bytes = size_t(1) << h->last_params.single.n;
   GTD_CUDA(h, ensure_field(&h->d_bytes, &h->bytes_cap, bytes));
-  GTD_CUDA(h, dp_launch_expand(h->last_params, h->last_tile_bits, h->last_tiles, h->d_bytes, bytes, h->stream));
+  GTD_CUDA(h, dp_launch_expand(h->last_params, h->last_tile_bits, 0, h->last_tiles, h->d_bytes, bytes, h->stream));
   h->bytes_valid = true;
   return GTD_OK;
 }
@@ -541,9 +547,21 @@ gtd_status gtd_dp_read_table(gtd_handle h, uint8_t* out, uint64_t bytes) {
     return fail(h, GTD_INVALID_ARG, "output buffer smaller than the table");
   DeviceGuard g(h->device);
   const gtd_status s = make_byte_table(h);
-  if (s != GTD_OK)
+  if (s == GTD_OK) {
+    GTD_CUDA(h, cudaMemcpyAsync(out, h->d_bytes, need, cudaMemcpyDeviceToHost, h->stream));
+  } else if (s == GTD_OOM) {  // no room for all of it: piece by piece
+    GTD_CUDA(h, ensure_field(&h->d_bytes, &h->bytes_cap, size_t(std::min<uint64_t>(need, kTablePiece))));
+    const int lb = h->last_tile_bits;
+    const uint32_t step = static_cast<uint32_t>(kTablePiece >> lb);
+    for (uint32_t t = 0; t < h->last_tiles; t += step) {
+      const uint32_t end = std::min(h->last_tiles, t + step);
+      const uint64_t bytes = std::min(need, uint64_t(end) << lb) - (uint64_t(t) << lb);
+      GTD_CUDA(h, dp_launch_expand(h->last_params, lb, t, end, h->d_bytes, bytes, h->stream));
+      GTD_CUDA(h, cudaMemcpyAsync(out + (uint64_t(t) << lb), h->d_bytes, bytes, cudaMemcpyDeviceToHost, h->stream));
+    }
+  } else {
     return s;
-  GTD_CUDA(h, cudaMemcpyAsync(out, h->d_bytes, need, cudaMemcpyDeviceToHost, h->stream));
+  }
   GTD_CUDA(h, cudaStreamSynchronize(h->stream));
   return GTD_OK;
 }

@@ -1702,12 +1702,13 @@ cudaError_t dp_launch_labels(const DpBatchParams& p, const uint64_t* subsets, in
   return cudaGetLastError();
 }
 
-// The byte table of gtd_dp_table (td << 1 | connected per subset, tiles of
-// 2^lb bytes in tile order; the planes may have tiles of another size), one
-// warp per tile: td(H) from the warp's chain, each word's first subset along
+// Tiles [first, end) of the byte table of gtd_dp_table (td << 1 | connected per
+// subset, tiles of 2^lb bytes in tile order; the planes may have tiles of
+// another size), one warp per tile: td(H) from the warp's chain, each word's first subset along
 // the chain of its bits, the word's subsets from one another.
 __global__ void __launch_bounds__(32 * kTreeWarps)
-    dp_expand_kernel(const __grid_constant__ DpBatchParams p, int lb, uint32_t tiles, uint8_t* out, uint64_t bytes) {
+    dp_expand_kernel(const __grid_constant__ DpBatchParams p, int lb, uint32_t first_tile, uint32_t end, uint8_t* out,
+                     uint64_t bytes) {
   __shared__ Binom sBinom;
   fill_binom(sBinom);
   __syncthreads();
@@ -1720,7 +1721,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
   const TreeCtx ctx{sBinom, sOff, p.table + G.table_off, G.lb, G.n};
   const int nh = G.n > lb ? G.n - lb : 0;
   const uint32_t words = lb > 5 ? 1u << (lb - 5) : 1u;
-  for (uint32_t t = blockIdx.x * kTreeWarps + warp; t < tiles; t += gridDim.x * kTreeWarps) {
+  for (uint32_t t = first_tile + blockIdx.x * kTreeWarps + warp; t < end; t += gridDim.x * kTreeWarps) {
     uint32_t r = t, H = 0;
     int j = 0;
     while (r >= sBinom[nh][j])
@@ -1750,7 +1751,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
         const int y = x & (x - 1);
         td[x] = td[y] + ((((p0 >> x) ^ (p0 >> y)) | ((p1 >> x) ^ (p1 >> y))) & 1u);
       }
-      const uint64_t at = (static_cast<uint64_t>(t) << lb) + w * 32u;
+      const uint64_t at = (static_cast<uint64_t>(t - first_tile) << lb) + w * 32u;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         uint32_t v = 0;
@@ -1764,10 +1765,10 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
   }
 }
 
-cudaError_t dp_launch_expand(const DpBatchParams& p, int lb, uint32_t tiles, uint8_t* out, uint64_t bytes,
-                             cudaStream_t s) {
-  const uint32_t ctas = (tiles + kTreeWarps - 1) / kTreeWarps;
-  dp_expand_kernel<<<ctas < 16384u ? ctas : 16384u, 32 * kTreeWarps, 0, s>>>(p, lb, tiles, out, bytes);
+cudaError_t dp_launch_expand(const DpBatchParams& p, int lb, uint32_t first, uint32_t end, uint8_t* out,
+                             uint64_t bytes, cudaStream_t s) {
+  const uint32_t ctas = (end - first + kTreeWarps - 1) / kTreeWarps;
+  dp_expand_kernel<<<ctas < 16384u ? ctas : 16384u, 32 * kTreeWarps, 0, s>>>(p, lb, first, end, out, bytes);
   return cudaGetLastError();
 }
 

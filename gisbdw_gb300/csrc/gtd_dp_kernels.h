@@ -84,9 +84,9 @@ cudaError_t dp_launch_cluster(const DpBatchParams& p, cudaStream_t s, const DpIn
 cudaError_t dp_launch_tree(const DpBatchParams& p, cudaStream_t s);
 cudaError_t dp_launch_labels(const DpBatchParams& p, const uint64_t* subsets, int count, int32_t* td_out,
                              uint64_t* roots_out, cudaStream_t s);
-// The byte table (td << 1 | connected, 2^n bytes) of a solved single graph,
-// in `tiles` tiles of 2^lb bytes.
-cudaError_t dp_launch_expand(const DpBatchParams& p, int lb, uint32_t tiles, uint8_t* out, uint64_t bytes,
-                             cudaStream_t s);
+// Tiles [first, end) (2^lb bytes each, `bytes` in all) of the byte table (td << 1
+// | connected, 2^n bytes) of a solved single graph.
+cudaError_t dp_launch_expand(const DpBatchParams& p, int lb, uint32_t first, uint32_t end, uint8_t* out,
+                             uint64_t bytes, cudaStream_t s);
 
 }  // namespace gtd

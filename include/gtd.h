@@ -135,7 +135,8 @@ gtd_status gtd_dp_query(gtd_handle h, uint64_t subset_mask, int32_t* td_out,
  * induced subgraph is connected). The solve keeps three bits per subset; the
  * bytes are written from them by the first of gtd_dp_table and
  * gtd_dp_read_table after a solve, into a buffer of 2^n bytes that the handle
- * keeps until a larger solve (GTD_OOM if it cannot be had). */
+ * keeps until a larger solve. If it cannot be had, gtd_dp_table gives GTD_OOM
+ * and gtd_dp_read_table reads the table in pieces of 64 MiB. */
 gtd_status gtd_dp_table(gtd_handle h, const uint8_t** d_table, uint64_t* bytes,
                         int* n, int* tile_bits);
 uint64_t gtd_dp_table_index(int n, int tile_bits, uint64_t subset_mask);

@@ -177,3 +177,23 @@ def test_rates_of_small_graphs_are_not_asked_for(handle):
     assert td == td8 == td10
     # 8-bit tiles take a quarter more time here: which of the two sizes ran
     assert t8 > 1.1 * t10 and t > (t8 + t10) / 2, (t8, t10, t)
+
+
+@pytest.mark.parametrize("n,tile_bits", [(2, 0), (8, 0), (20, 10), (26, 0), (27, 8), (28, 12)])
+def test_table_is_read_in_pieces_where_there_is_no_room_for_it(n, tile_bits):
+    """The allocation of the byte table fails: gtd_dp_read_table still gives
+    every byte (27 and 28 vertices: two and four pieces), gtd_dp_table GTD_OOM."""
+    g = G.gnp(n, 0.2, n)
+    with Handle(0) as h:
+        h.dp_solve(g.adj64(), n, tile_bits=tile_bits)
+        _lib.inject_fault(_lib.FAULT_ALLOC, 1)
+        try:
+            with pytest.raises(_lib.GtdError) as e:
+                h.dp_table_info()
+            assert e.value.status == 3
+            _lib.inject_fault(_lib.FAULT_ALLOC, 1)
+            pieces = h.dp_read_table()
+        finally:
+            _lib.inject_fault(_lib.FAULT_NONE, 0)
+        whole = h.dp_read_table()
+        assert pieces[1:] == whole[1:] and np.array_equal(pieces[0], whole[0])
