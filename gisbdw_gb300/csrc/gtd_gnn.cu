@@ -244,8 +244,8 @@ __global__ void heads_forward(int N, int G, int H, const float* __restrict__ h, 
     td_est[g] = part[0] + bf(b_g[0]);
 }
 
-// Loss and the head gradients w.r.t. the logits and td estimates: writes
-// dlogit (per node), dtd (per graph) and dh_L = dlogit w_out + dtd w_g / |g|.
+// Loss and the head gradients w.r.t. the logits and td estimates (a thread per
+// node and per graph): writes dlogit (per node), dtd (per graph) and dh_L = dlogit w_out + dtd w_g / |g|.
 __global__ void heads_backward(int N, int G, int H, const int32_t* __restrict__ gstart,
                                const int32_t* __restrict__ graph_of, const float* __restrict__ logits,
                                const float* __restrict__ td_est, const float* __restrict__ y,
@@ -254,6 +254,11 @@ __global__ void heads_backward(int N, int G, int H, const int32_t* __restrict__ 
                                const __nv_bfloat16* __restrict__ w_g, float* __restrict__ dlogit,
                                float* __restrict__ dtd, float* __restrict__ dh, float* __restrict__ loss) {
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v < G) {  // graph v, which may have no node
+    const float diff = td_est[v] - td_label[v];
+    dtd[v] = 2.f * td_weight * diff / float(G);
+    atomicAdd(loss, td_weight * diff * diff / float(G));
+  }
   if (v >= N)
     return;
   const float z = logits[v];
@@ -265,10 +270,6 @@ __global__ void heads_backward(int N, int G, int H, const int32_t* __restrict__ 
   const int g = graph_of[v];
   const float diff = td_est[g] - td_label[g];
   const float dt = 2.f * td_weight * diff / float(G);
-  if (v == gstart[g]) {
-    dtd[g] = dt;
-    atomicAdd(loss, td_weight * diff * diff / float(G));
-  }
   const float ng = float(gstart[g + 1] - gstart[g]);
   for (int j = 0; j < H; ++j)
     dh[size_t(v) * H + j] = dl * bf(w_out[j]) + dt * bf(w_g[j]) / ng;
@@ -1077,7 +1078,7 @@ gtd_status backward(gtd_gnn g, const gtd_gnn_batch* b, const Views& V, float td_
   GTD_CUDA(h, cudaMemsetAsync(g->grad, 0, g->nparams * 4, s));
   GTD_CUDA(h, cudaMemsetAsync(V.loss, 0, 4, s));
   float* gr = g->grad;
-  gtd::heads_backward<<<gtd::blocks_for(size_t(N), 128), 128, 0, s>>>(
+  gtd::heads_backward<<<gtd::blocks_for(size_t(std::max(N, G)), 128), 128, 0, s>>>(
       N, G, H, V.gstart, V.graph_of, V.logits, V.td_est, V.y, V.mask, V.td_label, inv, td_weight, g->w + P.head,
       g->w + P.head + H + 1, V.dlogit, V.dtd, V.dh, V.loss);
   // w_out, b_out from h_L and dlogit; w_g, b_g from the pooled means and dtd

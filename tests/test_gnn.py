@@ -269,5 +269,26 @@ def test_a_large_training_batch_takes_no_more_memory_than_layer_by_layer():
         before = torch.cuda.mem_get_info()[0]
         net.gradients(b)
         used = before - torch.cuda.mem_get_info()[0]
+        net.close()
     # features; Z and h of every layer and the input, the means; dh, dz, da and one more
     assert used < 4 * nodes * (gnn.IN_FEATURES + hid * (2 * (layers + 1) + layers + 4)), used
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("where", [0, 2, 5])
+@pytest.mark.parametrize("empties", [1, 70])
+def test_graphs_without_nodes_count_in_loss_and_gradients(handle, where, empties):
+    """Their estimate is the graph head's bias: its gradient and the loss have
+    their terms, at the start, between others and at the end (more of them than
+    nodes as well), whatever the buffers held before."""
+    _, b = _toy_batch(5)
+    net = gnn.GNN(handle, seed=6)
+    noise = gnn.Batch(b.x * 50, b.graph_start, b.nbr_start, b.nbr, b.root_label, b.node_mask, b.td_label + 500)
+    net.gradients(_layerwise(noise))  # other values in the buffers
+    c = gnn.Batch(b.x, np.insert(b.graph_start, where, [b.graph_start[where]] * empties).astype(np.int32), b.nbr_start,
+                  b.nbr, b.root_label, b.node_mask, np.insert(b.td_label, where, [7.0] * empties).astype(np.float32))
+    grad, loss = net.gradients(c)
+    with np.errstate(divide="ignore"):
+        rloss, rgrad = gnn.reference_loss(net.params(), c)
+    assert abs(loss - rloss) < 1e-4 * max(1.0, abs(rloss))
+    np.testing.assert_allclose(grad, rgrad, rtol=2e-3, atol=2e-5)
