@@ -1133,8 +1133,9 @@ int tile_nodes(const gtd_gnn_s* g, const gtd_gnn_batch* b, bool train) {
 }
 
 // Forward (train = false: logits and td estimates) or loss and gradients
-// (train = true: g->grad and *loss_out) by tiles. *done is false, and nothing
-// else has happened, where the batch needs the layer-by-layer kernels.
+// (train = true: g->grad, grad_out and *loss_out) by tiles. *done is false, and
+// no output written (g->grad is), where the batch needs the layer-by-layer
+// kernels.
 gtd_status run_tiles(gtd_gnn g, const gtd_gnn_batch* b, bool train, float td_weight, float* logits_out, float* td_out,
                      float* grad_out, float* loss_out, bool* done) {
   *done = false;
@@ -1195,7 +1196,8 @@ gtd_status run_tiles(gtd_gnn g, const gtd_gnn_batch* b, bool train, float td_wei
                odz = take(train ? (L + 1) * NH * 4 : 0), opool = take(train ? G * gtd::kWide * 4 : 0),
                otl2 = take(train ? size_t(tiles) * 4 : 0), opart = take(train ? std::min(chunks, size_t(gtd::kGradRun)) * size_t(g->nparams) * 4 : 0);
   GTD_CUDA(h, gtd::ensure_device(&g->buf, &g->buf_cap, off));
-  const size_t stage = std::max(staged, res_bytes);
+  const size_t grad_bytes = train && grad_out ? size_t(g->nparams) * 4 : 0;
+  const size_t stage = std::max(staged, res_bytes + grad_bytes);
   if (g->stage_cap < stage) {
     if (g->stage)
       cudaFreeHost(g->stage);
@@ -1273,8 +1275,8 @@ gtd_status run_tiles(gtd_gnn g, const gtd_gnn_batch* b, bool train, float td_wei
                            : launch_tile_kernel<128, false>(p, tiles, s)));
   }
   GTD_CUDA(h, cudaMemcpyAsync(pinned, base + ores, res_bytes, cudaMemcpyDeviceToHost, s));
-  if (train && grad_out)
-    GTD_CUDA(h, cudaMemcpyAsync(grad_out, g->grad, size_t(g->nparams) * 4, cudaMemcpyDeviceToHost, s));
+  if (grad_bytes)
+    GTD_CUDA(h, cudaMemcpyAsync(pinned + res_bytes, g->grad, grad_bytes, cudaMemcpyDeviceToHost, s));
   GTD_CUDA(h, cudaStreamSynchronize(s));
   int32_t outside = 0;
   std::memcpy(&outside, pinned, 4);
@@ -1284,6 +1286,8 @@ gtd_status run_tiles(gtd_gnn g, const gtd_gnn_batch* b, bool train, float td_wei
   if (train) {
     if (loss_out)
       std::memcpy(loss_out, pinned + 4, 4);
+    if (grad_bytes)
+      std::memcpy(grad_out, pinned + res_bytes, grad_bytes);
   } else {
     if (td_out)
       std::memcpy(td_out, pinned + (otde - ores), G * 4);

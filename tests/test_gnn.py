@@ -292,3 +292,26 @@ def test_graphs_without_nodes_count_in_loss_and_gradients(handle, where, empties
         rloss, rgrad = gnn.reference_loss(net.params(), c)
     assert abs(loss - rloss) < 1e-4 * max(1.0, abs(rloss))
     np.testing.assert_allclose(grad, rgrad, rtol=2e-3, atol=2e-5)
+
+
+@pytest.mark.gpu
+def test_gradients_that_cannot_be_had_leave_the_output_untouched():
+    """A batch with a neighbour outside its graph, taken up again layer by
+    layer, without room for that: GTD_OOM, and neither array written."""
+    import ctypes
+
+    from gisbdw_gb300 import Handle, _lib
+    b = _joined_singles(40, 20, 3, True)
+    with Handle(0) as h:
+        net = gnn.GNN(h, seed=1, layers=1)  # with one layer the second buffer is the larger one
+        grad, loss = np.full(net.nparams, 7.0, dtype=np.float32), np.full(1, 7.0, dtype=np.float32)
+        cb, p = b.c(), _lib._ptr
+        _lib.inject_fault(_lib.FAULT_ALLOC, 2)  # the tile kernels' buffer, then the other's
+        try:
+            st = h.L.gtd_gnn_gradients(net._g, ctypes.byref(cb), 0.05, p(grad), p(loss))
+        finally:
+            _lib.inject_fault(_lib.FAULT_NONE, 0)
+        assert st == 3 and np.all(grad == 7.0) and loss[0] == 7.0
+        assert h.L.gtd_gnn_gradients(net._g, ctypes.byref(cb), 0.05, p(grad), p(loss)) == 0
+        assert np.array_equal(grad, net.gradients(b)[0])
+        net.close()
