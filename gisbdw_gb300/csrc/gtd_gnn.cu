@@ -922,6 +922,7 @@ __global__ void __launch_bounds__(128) gnn_sum_chunks(const __grid_constant__ Ti
 
 struct gtd_gnn_s {
   gtd_handle h = nullptr;
+  int device = 0;  // the handle's, which may be gone when the network is destroyed
   int fin = 0, hid = 0, layers = 0;
   int64_t nparams = 0;
   float* master = nullptr;
@@ -1321,6 +1322,7 @@ gtd_status gtd_gnn_create(gtd_handle h, int in_features, int hidden, int layers,
   if (!g)
     return GTD_OOM;
   g->h = h;
+  g->device = h->device;
   g->fin = in_features;
   g->hid = hidden;
   g->layers = layers;
@@ -1367,7 +1369,7 @@ gtd_status gtd_gnn_create(gtd_handle h, int in_features, int hidden, int layers,
 gtd_status gtd_gnn_destroy(gtd_gnn g) {
   if (!g)
     return GTD_INVALID_ARG;
-  DeviceGuard dg(g->h->device);
+  DeviceGuard dg(g->device);
   cudaFree(g->master);
   cudaFree(g->m);
   cudaFree(g->v);

@@ -315,3 +315,24 @@ def test_gradients_that_cannot_be_had_leave_the_output_untouched():
         assert h.L.gtd_gnn_gradients(net._g, ctypes.byref(cb), 0.05, p(grad), p(loss)) == 0
         assert np.array_equal(grad, net.gradients(b)[0])
         net.close()
+
+
+@pytest.mark.gpu
+def test_a_network_may_outlive_its_handle():
+    """Closed in either order, also by the garbage collector: nothing is left
+    for a later call to trip over."""
+    from gisbdw_gb300 import Handle
+    _, b = _toy_batch(2)
+    for _ in range(3):
+        h = Handle(0)
+        net = gnn.GNN(h, seed=1)
+        want = net.forward(b)[0]
+        h.close()
+        others = [Handle(0) for _ in range(4)]  # take the freed memory
+        net.close()
+        with Handle(0) as h2:
+            again = gnn.GNN(h2, seed=1)
+            assert np.array_equal(again.forward(b)[0], want)
+            again.close()
+        for o in others:
+            o.close()
