@@ -336,3 +336,37 @@ def test_a_network_may_outlive_its_handle():
             again.close()
         for o in others:
             o.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("hidden", [8, 32, 63, 64])
+def test_layerwise_gradients_match_reference(handle, hidden):
+    """The layer-by-layer kernels, which other widths than 64 and neighbours
+    outside their graph take."""
+    c = _joined_singles(3, 14, 8, True)
+    net = gnn.GNN(handle, seed=7, hidden=hidden)
+    shape = (gnn.IN_FEATURES, hidden, gnn.LAYERS)
+    logits, td = net.forward(c)
+    rl, rtd = gnn.reference_loss(net.params(), c, shape, want_grad=False)
+    np.testing.assert_allclose(logits, rl, rtol=2e-4, atol=2e-5)
+    np.testing.assert_allclose(td, rtd, rtol=2e-4, atol=2e-5)
+    grad, loss = net.gradients(c)
+    rloss, rgrad = gnn.reference_loss(net.params(), c, shape)
+    assert abs(loss - rloss) < 1e-4 * max(1.0, abs(rloss))
+    # FP32 accumulation in a different order than the FP64 reference
+    np.testing.assert_allclose(grad, rgrad, rtol=2e-3, atol=2e-5)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count,n", [(1, 2), (5, 32), (3, 64), (4, 128), (70, 20)])
+def test_tile_gradients_and_steps_equal_the_layerwise_ones(handle, count, n):
+    """The same network by either kernels, bit for bit: gradients, and the
+    parameters after three steps. The loss is summed in another order."""
+    tiles, layers = (_joined_singles(count, n, 11, across) for across in (False, True))
+    nets = [gnn.GNN(handle, seed=12) for _ in range(2)]
+    (g0, l0), (g1, l1) = nets[0].gradients(tiles), nets[1].gradients(layers)
+    assert np.array_equal(g0, g1) and abs(l0 - l1) < 1e-5 * max(1.0, abs(l0))
+    for _ in range(3):
+        a, b = nets[0].train_step(tiles), nets[1].train_step(layers)
+        assert abs(a - b) < 1e-5 * max(1.0, abs(a))
+    assert np.array_equal(nets[0].params(), nets[1].params())
