@@ -69,11 +69,13 @@ gtd_status gtd_abort(gtd_handle h);
  *     depends on it waits until its bound (gtd_dp_opts.timeout_ns) runs out:
  *     GTD_TIMEOUT, and the handle stays usable;
  *   GTD_FAULT_POISON, c: the next c subset-DP solves (single graphs and
- *     batches) first fill their table with 0xFF bytes (treedepth 127, a
- *     value no solve writes). Every table byte is written before any tile
- *     reads it, so results are unchanged; a tile read before its
- *     producer's stores were visible would see the poison and corrupt the
- *     result (the stress test of the tiles' release/acquire publication);
+ *     batches) first fill their table with 0xFF bytes (both residue planes
+ *     and the connected plane set, which no solve writes). Every word of the
+ *     table is written before it is read, so results are unchanged; one read
+ *     before its producer's stores were visible would give 32 subsets of a
+ *     connected graph a wrong child and change some of them (a stress test
+ *     of the kernels' release/acquire publication). Such a solve whose caller gives tile bits
+ *     (a batch: or has loaded rates) runs the tile kernel at any size;
  *   GTD_FAULT_NONE: clears all. */
 enum { GTD_FAULT_NONE = 0, GTD_FAULT_ALLOC = 1, GTD_FAULT_STALL = 2, GTD_FAULT_POISON = 3 };
 gtd_status gtd_inject_fault(int kind, int count);
