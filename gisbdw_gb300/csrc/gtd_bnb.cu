@@ -1567,7 +1567,7 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   // Larger batches change over to split items when as few first-root items are
   // left (a byte per pair of roots: at most 256 MB).
   const size_t firsts = size_t(count) * levels * max_n, pairs = firsts * size_t(max_n);
-  const bool may_split = split || pairs <= (size_t(1) << 28);
+  bool may_split = split || pairs <= (size_t(1) << 28);
   const size_t S = split ? size_t(max_n) : 1;
   // One block on the device: inputs, then the bounds (also results), then
   // words that start at zero, the results among them first, then the
@@ -1589,10 +1589,21 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   const size_t o_parent = take(n_pool * sizeof(int32_t));
   const size_t out_end = at;
   const size_t o_tbeg = take(n_graphs * sizeof(uint64_t)), o_fails = take(2 * n_graphs * levels * sizeof(uint32_t));
-  const size_t o_items = take(firsts + (may_split ? pairs : 0));
-  const size_t zero_end = at;
-  const size_t o_trees = take(firsts);
-  if ((s = grow(h, &B.arena, &B.arena_cap, at)) != GTD_OK) return s;
+  const size_t items_at = at;
+  size_t o_items = 0, zero_end = 0, o_trees = 0;
+  auto grow_arena = [&]() {
+    at = items_at;
+    o_items = take(firsts + (may_split ? pairs : 0));
+    zero_end = at;
+    o_trees = take(firsts);
+    return grow(h, &B.arena, &B.arena_cap, at);
+  };
+  s = grow_arena();
+  if (s == GTD_OOM && may_split && !split) {  // no room for the pairs: first-root items to the end
+    may_split = false;
+    s = grow_arena();
+  }
+  if (s != GTD_OK) return s;
   std::vector<uint8_t> stage(out_end, 0);
   std::memcpy(stage.data() + o_graphs, graphs.data(), n_graphs * sizeof(BnbGraph));
   std::memcpy(stage.data() + o_adj, adj2_pool, 2 * n_pool * sizeof(uint64_t));

@@ -234,3 +234,26 @@ def test_bnb_memo_of_earlier_solves_is_empty(memo_log2):
         wide = _check(h, [G.cycle(70 + rep), G.path(100), G.grid(4, 5)], memo_log2=memo_log2)
         assert wide["td"].tolist()[:2] == [8, 7]
     h.close()
+
+
+def _easy_and_hard(easy, hard, n):
+    gs = [G.tree_plus_edges(16 + s % 3, 2 + s % 3, s) for s in range(easy)]
+    return gs + [G.sparse_connected(n - s % 2, 90 + s) for s in range(hard)]
+
+
+def test_bnb_without_room_for_split_items_goes_on_without_them():
+    """The memo fits, the block with a state per pair of roots does not: the
+    batch is solved with first-root items to the end."""
+    from gisbdw_gb300 import Handle
+    gs = _easy_and_hard(150, 4, 22)
+    with Handle(0) as h:
+        packed = _lib.pack_bnb(gs)
+        _lib.inject_fault(_lib.FAULT_ALLOC, 2)  # the memo, then the block
+        try:
+            res = h.bnb_solve_batch(gs, packed=packed, deadline_ns=CAP_NS)
+        finally:
+            _lib.inject_fault(_lib.FAULT_NONE, 0)
+        assert np.all(res["status"] == 0)
+        assert res["td"].tolist() == h.dp_solve_batch(gs)[0].tolist()
+        for g, t, par in zip(gs, res["td"], res["parents"]):
+            assert check_tree(g, int(t), par), g.name
