@@ -257,3 +257,19 @@ def test_bnb_without_room_for_split_items_goes_on_without_them():
         assert res["td"].tolist() == h.dp_solve_batch(gs)[0].tolist()
         for g, t, par in zip(gs, res["td"], res["parents"]):
             assert check_tree(g, int(t), par), g.name
+
+
+@pytest.mark.parametrize("wide", [False, True])
+def test_bnb_change_over_with_hints_and_with_wide_graphs(handle, wide):
+    """Batches that change over to split items, with level hints above, at and
+    below the treedepth, and with graphs of more than 64 vertices among them
+    (two mask words, memo slots without a number)."""
+    gs = _easy_and_hard(120, 6, 22)
+    want = handle.dp_solve_batch(gs)[0].tolist()
+    if wide:
+        gs += [G.path(70), G.cycle(90), G.star(104), G.tree_plus_edges(70, 0, 3)]
+        want += [7, 8, 2]
+    rng = np.random.default_rng(3)
+    for hints in (None, np.zeros(len(gs), np.int32), rng.integers(1, 9, len(gs)).astype(np.int32)):
+        res = _check(handle, gs, **({} if hints is None else {"hints": hints}))
+        assert res["td"].tolist()[:len(want)] == want
