@@ -380,10 +380,11 @@ struct WeightRegs {
 
 // x / d, correctly rounded as the division is, from inv = 1 / d correctly
 // rounded: with the residue of q = x inv exact in a fused multiply-add,
-// q + residue * inv rounds to the quotient (Markstein's theorem; every
-// significand over every d up to 128 compared with the division). The residue
-// is exact above the denormal range; an infinite or NaN q is the quotient
-// itself. One division per node in place of one per channel, which took 60 %
+// q + residue * inv rounds to the quotient (Markstein's theorem; compared in
+// integers for every significand over every odd d below 300, and for random
+// ones over every d up to 4096: a node may have more neighbours than a tile has
+// nodes, where its list repeats them). The residue is exact above the denormal
+// range; an infinite or NaN q is the quotient itself. One division per node in place of one per channel, which took 60 %
 // of the aggregation.
 __device__ __forceinline__ float quotient(float x, float d, float inv) {
   const float q = x * inv, residue = fmaf(-q, d, x);

@@ -370,3 +370,26 @@ def test_tile_gradients_and_steps_equal_the_layerwise_ones(handle, count, n):
         a, b = nets[0].train_step(tiles), nets[1].train_step(layers)
         assert abs(a - b) < 1e-5 * max(1.0, abs(a))
     assert np.array_equal(nets[0].params(), nets[1].params())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("repeat", [1, 43, 300])
+def test_neighbour_lists_that_repeat_entries(handle, repeat):
+    """Degrees far above the number of nodes (43 and 300 times every entry, in
+    lists that no longer fit the tile's shared memory): means and gradients as
+    layer by layer, bit for bit, and against float64."""
+    pair = []
+    for across in (False, True):
+        b = _joined_singles(3, 14, 8, across)
+        deg = np.diff(b.nbr_start)
+        nbr = np.concatenate([np.tile(b.nbr[s:s + d], repeat) for s, d in zip(b.nbr_start, deg)]).astype(np.int32)
+        start = np.concatenate([[0], np.cumsum(deg * repeat)]).astype(np.int32)
+        pair.append(gnn.Batch(b.x, b.graph_start, start, nbr, b.root_label, b.node_mask, b.td_label))
+    net = gnn.GNN(handle, seed=13)
+    (logits, td), (logits2, td2) = net.forward(pair[0]), net.forward(_layerwise(pair[0]))
+    assert np.array_equal(logits, logits2) and np.array_equal(td, td2[:-1])
+    rl, rtd = gnn.reference_loss(net.params(), pair[0], want_grad=False)
+    np.testing.assert_allclose(logits, rl, rtol=2e-3, atol=2e-4)  # sums of up to 2000 terms
+    np.testing.assert_allclose(td, rtd, rtol=2e-3, atol=2e-4)
+    tiles, layers = (net.gradients(b)[0] for b in pair)
+    assert np.array_equal(tiles, layers)
