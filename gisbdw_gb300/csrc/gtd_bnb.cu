@@ -134,8 +134,9 @@ constexpr uint64_t kFirstBudget = 1024;  // search nodes of an item's first run
 constexpr uint32_t kMaxDoublings = 30;   // an item's budget grows to at most 2^30 times the first
 constexpr uint32_t kItemDone = 0xFF;
 // A batch changes over to split items once fewer than this many first-root
-// items per SM are open (24 warps are resident): 32 leaves no warp of the next
-// passes idle. 8 / 16 / 24 / 32 / 64 per SM, ms: 48 graphs of 24..36 vertices
+// items per SM are open (24 warps are resident; a batch of few levels launches
+// as few as 16 per SM, one for each first-root item, which made no difference:
+// 40 graphs of 20 vertices 2.5 ms with either, 100 of 16 0.77). 8 / 16 / 24 / 32 / 64 per SM, ms: 48 graphs of 24..36 vertices
 // 67 / 23 / 23 / 23 / 23, 64 of 28..34 70 / 70 / 35 / 35 / 35, 256 of 28..34
 // - / 132 / - / 105 / 105, 300 of 16..36 - / 188 / - / 147 / 148.
 constexpr int kSplitPerSm = 32;

@@ -9,7 +9,7 @@
 
 namespace gtd {
 
-// One graph of a DP launch (48 bytes). A graph with n < lb is padded with
+// One graph of a DP launch (40 bytes). A graph with n < lb is padded with
 // isolated vertices up to lb (one tile); padding changes no treedepth of a
 // real subset and the reconstruction never touches padded vertices.
 struct DpGraph {
@@ -22,6 +22,7 @@ struct DpGraph {
   int32_t out_idx = 0;     // position of the graph in the caller's arrays (td_out)
   int32_t lb = 0;          // tile bits of this graph's table
 };
+static_assert(sizeof(DpGraph) == 40);
 
 // Passed by value as a __grid_constant__ kernel parameter.
 struct DpBatchParams {

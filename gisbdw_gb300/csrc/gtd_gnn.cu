@@ -1117,9 +1117,8 @@ cudaError_t launch_tile_kernel(const gtd::TileParams& p, int tiles, cudaStream_t
 }
 
 // Nodes per tile for this batch, 0 where the tile kernels do not apply: the
-// largest graph decides, small tiles spread a small training batch over more
-// SMs.
-int tile_nodes(const gtd_gnn_s* g, const gtd_gnn_batch* b, bool train) {
+// largest graph decides, small tiles spread a small batch over more SMs.
+int tile_nodes(const gtd_gnn_s* g, const gtd_gnn_batch* b) {
   if (g->hid != gtd::kWide)
     return 0;
   int most = 0;
@@ -1141,7 +1140,7 @@ int tile_nodes(const gtd_gnn_s* g, const gtd_gnn_batch* b, bool train) {
 gtd_status run_tiles(gtd_gnn g, const gtd_gnn_batch* b, bool train, float td_weight, float* logits_out, float* td_out,
                      float* grad_out, float* loss_out, bool* done) {
   *done = false;
-  const int M = tile_nodes(g, b, train);
+  const int M = tile_nodes(g, b);
   if (M == 0)
     return GTD_OK;
   gtd_handle h = g->h;

@@ -53,7 +53,6 @@ __device__ __forceinline__ void hclear(uint64_t& lo, uint64_t& hi, int v) {
 __device__ __forceinline__ int hfirst(uint64_t lo, uint64_t hi) {
   return lo ? __ffsll(static_cast<long long>(lo)) - 1 : 63 + __ffsll(static_cast<long long>(hi));
 }
-__device__ __forceinline__ int hpopc(uint64_t lo, uint64_t hi) { return __popcll(lo) + __popcll(hi); }
 
 // Component of S holding v, by one lane (serial BFS).
 __device__ void lane_component(const HeurWarp* w, uint64_t Slo, uint64_t Shi, int v, uint64_t& rlo, uint64_t& rhi) {
@@ -78,19 +77,17 @@ __device__ void lane_component(const HeurWarp* w, uint64_t Slo, uint64_t Shi, in
 }
 
 struct Pick {
-  double coef;
-  int deg, v;
+  double score;
+  int v;
 };
-// The host's scan order: higher coef, then higher degree, then smaller id.
+// The host's scan order: higher score, then smaller id.
 __device__ __forceinline__ bool better(const Pick& a, const Pick& b) {
   if (a.v < 0)
     return false;
   if (b.v < 0)
     return true;
-  if (a.coef != b.coef)
-    return a.coef > b.coef;
-  if (a.deg != b.deg)
-    return a.deg > b.deg;
+  if (a.score != b.score)
+    return a.score > b.score;
   return a.v < b.v;
 }
 
@@ -109,19 +106,18 @@ __device__ int greedy(HeurWarp* w, int n, const float* scores, int32_t* parent) 
     // component of the smallest remaining vertex (every lane computes it)
     uint64_t Clo, Chi;
     lane_component(w, rem_lo, rem_hi, hfirst(rem_lo, rem_hi), Clo, Chi);
-    Pick best{0.0, -1, -1};
+    Pick best{0.0, -1};
     for (int k = 0; k < kHMaxN / 32; ++k) {
       const int u = lane + 32 * k;
       if (u >= n || !hhas(Clo, Chi, u))
         continue;
-      const Pick c{static_cast<double>(scores[u]), 0, u};
+      const Pick c{static_cast<double>(scores[u]), u};
       if (better(c, best))
         best = c;
     }
     for (int off = 16; off > 0; off >>= 1) {
       Pick o;
-      o.coef = __shfl_xor_sync(0xffffffffu, best.coef, off);
-      o.deg = __shfl_xor_sync(0xffffffffu, best.deg, off);
+      o.score = __shfl_xor_sync(0xffffffffu, best.score, off);
       o.v = __shfl_xor_sync(0xffffffffu, best.v, off);
       if (better(o, best))
         best = o;

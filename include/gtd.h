@@ -50,8 +50,9 @@ const char* gtd_status_string(gtd_status s);
 const char* gtd_last_error(gtd_handle h);
 
 /* Stops the call in flight on handle h: the persistent kernels see the
- * request at their next poll (every DP tile ticket and dependency wait,
- * every 64 branch-and-bound search nodes) and that call returns GTD_ABORTED
+ * request at their next poll (every ticket of the DP's tile kernel and every
+ * dependency wait, every 64 branch-and-bound search nodes; DP launches of up to
+ * 28 vertices may run to their end first) and that call returns GTD_ABORTED
  * with its outputs undefined; the handle stays usable. This is the one call
  * that may be made from another host thread while a call on the same handle
  * runs. A request made while no call runs is dropped when the next call
@@ -63,7 +64,8 @@ gtd_status gtd_abort(gtd_handle h);
  * reference), process-wide:
  *   GTD_FAULT_ALLOC, c: the c-th device buffer allocation made by this
  *     library from now on fails as if the GPU were out of memory; the call
- *     returns GTD_OOM and the handle stays usable;
+ *     returns GTD_OOM, or goes on with less where it can, and the handle
+ *     stays usable;
  *   GTD_FAULT_STALL, c: the next c single-graph DP solves (gtd_dp_solve,
  *     gtd_dp_solve_device) never take their first tile, so every tile that
  *     depends on it waits until its bound (gtd_dp_opts.timeout_ns) runs out:
@@ -85,19 +87,22 @@ typedef struct {
   int tile_bits;        /* low vertices per tile of the byte table, and of the
                            tile kernel where n is large enough for it (0 = 10,
                            11 from n = 26 on) */
-  int ctas_per_sm;      /* persistent CTAs per SM (0 = default) */
+  int ctas_per_sm;      /* persistent CTAs per SM (0 = default; without effect up
+                           to n = 21, where one CTA or one cluster runs) */
   uint64_t timeout_ns;  /* bound on every in-kernel wait (0 = 10 s) */
 } gtd_dp_opts;
 
 typedef struct {
-  float dp_ms;          /* DP kernel time, CUDA events on the handle's stream */
-  float tree_ms;        /* tree reconstruction kernel */
+  float dp_ms;          /* DP kernel time, CUDA events on the handle's stream; up
+                           to n = 21 one kernel checks the graph, fills the
+                           table and builds the tree: all of it */
+  float tree_ms;        /* tree reconstruction kernel (0 up to n = 21) */
   float total_ms;       /* whole call including copies */
   uint64_t table_bytes; /* 2^n, the byte table of gtd_dp_table */
   uint64_t alg_bytes;   /* 2^n + n 2^(n-1): one write + |S| one-byte gathers per subset */
-  int tile_bits;
+  int tile_bits;        /* of the byte table */
   int tiles;
-  int ctas;
+  int ctas;             /* of the DP kernel that ran */
 } gtd_dp_stats;
 
 /* DynamicGPU (Treedepth/src/dynamic_gpu/dynamic_gpu.cu:171-201 Run, with
@@ -174,12 +179,14 @@ typedef struct {
   uint64_t alg_bytes;   /* sum of 2^n + n 2^(n-1) */
   uint64_t table_bytes; /* subsets in the table pool, graphs with n < tile bits
                            padded (the pool takes three bits for each) */
-  int tile_bits;        /* the launch's largest tile size */
+  int tile_bits;        /* the largest tile size planned for the tile kernel, and
+                           its tiles, as if it took every graph (graphs of up to
+                           16 vertices and batches of few subsets do without) */
   int tiles;
-  int ctas;
+  int ctas;             /* of the tile or the level kernel, as it ran */
   int graph_replayed;   /* 1 if an existing CUDA graph was replayed */
-  int tile_bits_by_n[GTD_DP_MAX_N + 1]; /* tile size of the graphs with n
-                                           vertices (0: none in the batch) */
+  int tile_bits_by_n[GTD_DP_MAX_N + 1]; /* tile size planned for the graphs with
+                                           n vertices (0: none in the batch) */
 } gtd_dp_batch_stats;
 
 /* DynamicGPU over many graphs of uneven size in ONE persistent launch
@@ -213,8 +220,9 @@ gtd_status gtd_dp_batch_sync(gtd_handle h, gtd_dp_batch_stats* stats);
  * one that runs graphs of different tile sizes in one launch; it holds fewer
  * CTAs per SM) at each largest tile size 8..12: mixed_eff_out (may be NULL)
  * receives its 5 throughputs relative to the one-size kernel. Batches solved
- * with tile_bits = 0 then give each vertex count its own tile size when the
- * predicted time, mixed-kernel efficiency included, beats one size for all. */
+ * with tile_bits = 0 then give each vertex count its own tile size in the tile
+ * kernel when the predicted time, mixed-kernel efficiency included, beats one
+ * size for all; which graphs the tile kernel takes does not depend on rates. */
 gtd_status gtd_dp_autotune(gtd_handle h, int n_min, int n_max,
                            float* rates_out, float* mixed_eff_out);
 
@@ -309,8 +317,8 @@ gtd_status gtd_bottom_up(gtd_handle h, const uint64_t* adj, int n,
                          int32_t* td_out, int32_t* parent_out,
                          int32_t* order_out);
 
-/* The same heuristics for many graphs in one GPU launch (one warp per
- * graph, n <= 128), trees identical to gtd_heuristic's: descs and the
+/* The same heuristics for many graphs in one GPU launch (n <= 128; a thread
+ * per vertex, kind 3 a warp per graph), trees identical to gtd_heuristic's: descs and the
  * (lo, hi) adjacency pool as for gtd_bnb_solve_batch; kind 0..3 as above
  * (kind 3 reads scores_pool[descs[i].offset + v]); td_out[count] and
  * parent_out[pool_len] (graph i's tree at descs[i].offset). Disconnected
