@@ -400,8 +400,9 @@ __device__ __forceinline__ Workspace make_workspace(const DpBatchParams& p, cons
 // shared memory and registers take), a group's time going to unranking and
 // flags (15 %), the gathers (27 %), the classes of the in-tile phase (33 %)
 // and waits at the narrow levels (16 %). 8.5 warp instructions per word of 32
-// subsets; n = 30 takes 0.67 ms, n = 33 4.7 ms (at one byte per subset and one
-// warp per tile, 1.52 warp instructions per subset: 1.92 and 14.9 ms). Tried
+// subsets; the kernel alone takes 0.68 ms at n = 30 and 4.7 ms at n = 33 (whole
+// calls one after another 0.73 and 4.82; at one byte per subset and one warp per
+// tile, 1.52 warp instructions per subset: 1.92 and 14.9 ms). Tried
 // and not kept: a warp per group (0.91 ms), 64 threads per CTA (0.79), the next
 // group unranked by an idle warp beside the in-tile phase (0.72 and 5.2).
 template <int LB>

@@ -307,8 +307,9 @@ unsigned blocks_for(size_t n, unsigned t) { return static_cast<unsigned>((n + t 
 // Training then takes the weight gradients of all layers in a second launch and
 // their sums in a third. Every sum runs in the order of the layer-by-layer
 // kernels above, so results are the same bit for bit (but for the loss, whose
-// order those leave open). Width 64; other widths, graphs larger than a tile
-// and neighbours outside their graph take the layer-by-layer kernels.
+// order those leave open). Width 64; other widths, graphs larger than a tile or
+// without nodes and neighbours outside their graph take the layer-by-layer
+// kernels.
 // ---------------------------------------------------------------------------
 
 constexpr int kWide = 64;            // hidden width
