@@ -65,3 +65,23 @@ def test_adjacency_pool_equals_the_per_graph_masks():
         _lib.adjacency_pool([bad], 1)
     with pytest.raises(ValueError):
         _lib.adjacency_pool([G.path(65)], 1)
+
+
+@pytest.mark.parametrize("words", [1, 2])
+def test_small_batches_are_packed_as_fast_as_graph_by_graph(words):
+    """The native pass costs several times what a few small graphs take; the
+    masks are the same on either side of the rule."""
+    import timeit
+
+    from gisbdw_gb300 import _lib
+
+    def per_graph(gs):
+        return np.concatenate([g.adj64() if words == 1 else g.adj128() for g in gs])
+    for n in range(1, 40):
+        for gs in ([G.path(n)], [G.complete(n)], [G.path(n), G.Graph(1, []), G.cycle(max(n, 3))]):
+            assert np.array_equal(_lib.adjacency_pool(gs, words), per_graph(gs))
+
+    def best(f):
+        return min(timeit.repeat(f, number=200, repeat=9))
+    for gs in ([G.path(5)], [G.Graph(1, []), G.path(4)]):
+        assert best(lambda: _lib.adjacency_pool(gs, words)) < 2.5 * best(lambda: per_graph(gs))
