@@ -226,6 +226,7 @@ struct WarpMem {
   uint8_t order[kBnbMaxN];
   uint8_t mvert[kMiniMax];   // small-component DP: vertex of each local id
   uint16_t madj[kMiniMax];   // ... and its local adjacency
+  uint64_t tag;              // of the memo's slots (not WIDE)
 };
 
 __device__ __forceinline__ bool has(uint64_t lo, uint64_t hi, int v) {
@@ -270,14 +271,25 @@ __device__ __forceinline__ void cas128(uint4* addr, uint64_t clo, uint64_t chi, 
 
 // Memo slot: lo = mask bits 0..63; hi = mask bits 64..103 (bits 0..39) |
 // lb << 40 | ub << 47 | root << 54. An all-zero slot is empty (the empty set
-// is never stored). Graphs of at most 64 vertices have the solve's number (its
-// tag) where bits 64..103 would be: a slot of an earlier solve is empty, and
-// the memo, 256 MB a graph, is not cleared for every call (2.1 ms for 48
-// graphs). Wider graphs (tag 0) use a cleared memo.
+// is never stored). A launch of graphs of at most 64 vertices has the solve's
+// number (its tag) where bits 64..103 would be: a slot of an earlier solve is
+// empty, and the memo, 256 MB a graph, is not cleared for every call (2.1 ms
+// for 48 graphs). A launch with a wider graph (WIDE) uses a cleared memo. Two
+// kernels, the tag in shared memory: one kernel with both tests and the tag in
+// registers searched 3 to 7 % fewer nodes per us (3-regular, 32 vertices: 521 ms
+// against 497 now and without tags; a tree of 48 vertices with 12 more edges 200
+// against 187; the search waits for instructions, so its length counts).
 constexpr uint64_t kKeyHiMask = (1ull << 40) - 1;
 
+template <bool WIDE>
 __device__ __forceinline__ bool memo_empty(uint64_t clo, uint64_t chi, uint64_t tag) {
-  return (clo == 0 && chi == 0) || (tag != 0 && (chi & kKeyHiMask) != tag);
+  return WIDE ? clo == 0 && chi == 0 : (chi & kKeyHiMask) != tag;
+}
+
+// Does a slot that is not empty hold the component (lo, hi)?
+template <bool WIDE>
+__device__ __forceinline__ bool memo_same(uint64_t clo, uint64_t chi, uint64_t lo, uint64_t hi) {
+  return clo == lo && (!WIDE || (chi & kKeyHiMask) == hi);
 }
 
 __device__ __forceinline__ uint64_t memo_hash(uint64_t lo, uint64_t hi) {
@@ -298,26 +310,27 @@ __device__ __forceinline__ MemoHit unpack(uint64_t chi) {
 
 // Lookup (lane 0). Reads are atomic: a CAS that can only write back the
 // value it found.
+template <bool WIDE>
 __device__ MemoHit memo_get(uint4* table, uint32_t mask, uint64_t tag, uint64_t lo, uint64_t hi) {
-  const uint64_t h = memo_hash(lo, hi);
-  hi |= tag;
+  const uint64_t h = memo_hash(lo, WIDE ? hi : 0);
   for (int p = 0; p < kMemoProbes; ++p) {
     uint4* slot = table + ((h + p) & mask);
     uint64_t clo, chi;
     cas128(slot, 0, 0, 0, 0, clo, chi);
-    if (memo_empty(clo, chi, tag))
+    if (memo_empty<WIDE>(clo, chi, tag))
       break;
-    if (clo == lo && (chi & kKeyHiMask) == hi)
+    if (memo_same<WIDE>(clo, chi, lo, hi))
       return unpack(chi);
   }
   return MemoHit{0, kUnknownUb, 0};
 }
 
 // Merges bounds into the memo (lane 0): lb = max, ub = min (with its root).
+template <bool WIDE>
 __device__ void memo_put(uint4* table, uint32_t mask, uint64_t tag, uint64_t lo, uint64_t hi, int lb, int ub,
                          int root) {
-  const uint64_t h = memo_hash(lo, hi);
-  hi |= tag;
+  const uint64_t h = memo_hash(lo, WIDE ? hi : 0);
+  const uint64_t key = WIDE ? hi : tag;
   auto merged = [&](uint64_t chi, bool empty) {
     MemoHit c = empty ? MemoHit{0, kUnknownUb, 0} : unpack(chi);
     const int nlb = max(c.lb, lb);
@@ -326,7 +339,7 @@ __device__ void memo_put(uint4* table, uint32_t mask, uint64_t tag, uint64_t lo,
       nub = ub;
       nroot = root;
     }
-    return hi | (static_cast<uint64_t>(nlb & 0x7F) << 40) | (static_cast<uint64_t>(nub & 0x7F) << 47) |
+    return key | (static_cast<uint64_t>(nlb & 0x7F) << 40) | (static_cast<uint64_t>(nub & 0x7F) << 47) |
            (static_cast<uint64_t>(nroot & 0x7F) << 54);
   };
   int victim = 0, victim_size = 1 << 30;
@@ -335,9 +348,9 @@ __device__ void memo_put(uint4* table, uint32_t mask, uint64_t tag, uint64_t lo,
     uint64_t clo = 0, chi = 0;
     cas128(slot, 0, 0, 0, 0, clo, chi);
     for (int tries = 0; tries < 64; ++tries) {
-      const bool empty = memo_empty(clo, chi, tag);
-      if (!empty && !(clo == lo && (chi & kKeyHiMask) == hi)) {
-        const int sz = __popcll(clo) + (tag ? 0 : __popcll(chi & kKeyHiMask));
+      const bool empty = memo_empty<WIDE>(clo, chi, tag);
+      if (!empty && !memo_same<WIDE>(clo, chi, lo, hi)) {
+        const int sz = __popcll(clo) + (WIDE ? __popcll(chi & kKeyHiMask) : 0);
         if (sz < victim_size) {
           victim_size = sz;
           victim = p;
@@ -383,12 +396,12 @@ struct StopCheck {
   const int32_t* error = nullptr;   // the launch's error word: an abort or an error elsewhere
 };
 
+template <bool WIDE>
 struct Search {
   WarpMem* w;
   int lane, n;
   uint4* memo;
   uint32_t memo_mask;
-  uint64_t tag;  // of the memo's slots
   StopCheck stop;
   unsigned long long nodes;
   bool timed_out, cancelled;
@@ -594,7 +607,7 @@ struct Search {
       if (v < n && has(Clo, Chi, v)) {
         uint64_t lo = Clo, hi = Chi;
         bit_clear(lo, hi, v);
-        const MemoHit m = memo_get(memo, memo_mask, tag, lo, hi);
+        const MemoHit m = memo_get<WIDE>(memo, memo_mask, w->tag, lo, hi);
         best = max(best, m.lb);
         if (m.ub < kUnknownUb)
           ubr = min(ubr, (static_cast<uint32_t>(m.ub) << 8) | static_cast<uint32_t>(v));
@@ -840,7 +853,7 @@ struct Search {
           } else {
             MemoHit hit{0, kUnknownUb, 0};
             if (lane == 0)
-              hit = memo_get(memo, memo_mask, tag, f.lo, f.hi);
+              hit = memo_get<WIDE>(memo, memo_mask, w->tag, f.lo, f.hi);
             hit.lb = __shfl_sync(0xffffffffu, hit.lb, 0);
             hit.ub = __shfl_sync(0xffffffffu, hit.ub, 0);
             hit.root = __shfl_sync(0xffffffffu, hit.root, 0);
@@ -853,7 +866,7 @@ struct Search {
               int r = 0;
               const int td = mini_dp(f.lo, f.hi, csize, &r);
               if (lane == 0)
-                memo_put(memo, memo_mask, tag, f.lo, f.hi, td, td, r);
+                memo_put<WIDE>(memo, memo_mask, w->tag, f.lo, f.hi, td, td, r);
               decision = td <= fk ? 1 : 0;
               vroot = r;
             } else {
@@ -862,7 +875,7 @@ struct Search {
               if (lb <= fk && hit.lb == 0 && csize >= kMmdMin) {
                 lb = max(lb, mmd_lb(f.lo, f.hi));
                 if (lane == 0)
-                  memo_put(memo, memo_mask, tag, f.lo, f.hi, lb, kUnknownUb, 0);
+                  memo_put<WIDE>(memo, memo_mask, w->tag, f.lo, f.hi, lb, kUnknownUb, 0);
               }
               // a path of 2^fk vertices, or a cycle of 2^(fk-1) + 1, would
               // refute td <= fk (a tree, with fewer edges than vertices, has
@@ -872,7 +885,7 @@ struct Search {
                 if (pl > fk) {
                   lb = pl;
                   if (lane == 0)
-                    memo_put(memo, memo_mask, tag, f.lo, f.hi, lb, kUnknownUb, 0);
+                    memo_put<WIDE>(memo, memo_mask, w->tag, f.lo, f.hi, lb, kUnknownUb, 0);
                 }
               }
               // td is monotone under vertex deletion: a memo entry proving
@@ -884,7 +897,7 @@ struct Search {
                 if (sl > fk) {
                   lb = sl;
                   if (lane == 0)
-                    memo_put(memo, memo_mask, tag, f.lo, f.hi, lb, kUnknownUb, 0);
+                    memo_put<WIDE>(memo, memo_mask, w->tag, f.lo, f.hi, lb, kUnknownUb, 0);
                 }
               }
               if (lb > fk) {
@@ -893,7 +906,7 @@ struct Search {
                 decision = 1;
                 vroot = static_cast<int>(ubr & 0xFF);
                 if (lane == 0)
-                  memo_put(memo, memo_mask, tag, f.lo, f.hi, 0, fk, vroot);
+                  memo_put<WIDE>(memo, memo_mask, w->tag, f.lo, f.hi, 0, fk, vroot);
               }
             }
           }
@@ -990,9 +1003,9 @@ struct Search {
       const int fv = f.v;
       if (!f.single && lane == 0) {
         if (ok)
-          memo_put(memo, memo_mask, tag, f.lo, f.hi, 0, fk, fv);
+          memo_put<WIDE>(memo, memo_mask, w->tag, f.lo, f.hi, 0, fk, fv);
         else
-          memo_put(memo, memo_mask, tag, f.lo, f.hi, fk + 1, kUnknownUb, 0);
+          memo_put<WIDE>(memo, memo_mask, w->tag, f.lo, f.hi, fk + 1, kUnknownUb, 0);
       }
       ret = ok;
       ret_root = ok ? fv : -1;
@@ -1155,10 +1168,12 @@ __device__ bool next_pass(const BnbParams& p, uint32_t pass) {
   return __shfl_sync(0xffffffffu, go, 0) != 0;
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(32 * kBnbWarps, 6) bnb_kernel(const __grid_constant__ BnbParams p) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   WarpMem* w = reinterpret_cast<WarpMem*>(smem) + warp;
+  w->tag = p.memo_tag;  // read by the lane that wrote it
   int cur_g = -1;
   for (uint32_t pass = 0;; ++pass) {
   uint32_t split_now = 0;
@@ -1230,7 +1245,7 @@ __global__ void __launch_bounds__(32 * kBnbWarps, 6) bnb_kernel(const __grid_con
     const int v = w->order[r];
     uint64_t fl, fh;
     full_set(G.n, fl, fh);
-    Search s{w, lane, G.n, p.memo + G.memo_off, p.memo_mask, G.n <= 64 ? p.memo_tag : 0ull, StopCheck{}, 0ull, false, false};
+    Search<WIDE> s{w, lane, G.n, p.memo + G.memo_off, p.memo_mask, StopCheck{}, 0ull, false, false};
     s.mini = p.mini ? p.mini + (size_t(blockIdx.x) * kBnbWarps + warp) * (1u << kMiniMax) : nullptr;
     s.stop.best = p.best + g;
     s.stop.lbp = p.lbp + g;
@@ -1662,9 +1677,10 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   p.parent_out = dev(o_parent, static_cast<int32_t*>(nullptr));
 
   const size_t smem = sizeof(WarpMem) * kBnbWarps;
-  GTD_CUDA(h, cudaFuncSetAttribute(bnb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  const auto kernel = max_n > 64 ? bnb_kernel<true> : bnb_kernel<false>;
+  GTD_CUDA(h, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   int occ = 0;
-  GTD_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, bnb_kernel, 32 * kBnbWarps, smem));
+  GTD_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, 32 * kBnbWarps, smem));
   if (opts && opts->ctas_per_sm > 0 && opts->ctas_per_sm < occ)
     occ = opts->ctas_per_sm;
   if (occ < 1)
@@ -1692,7 +1708,7 @@ extern "C" gtd_status gtd_bnb_solve_batch(gtd_handle h, const gtd_graph_desc* de
   GTD_CUDA(h, cudaEventRecord(h->ev[0], h->stream));
   {
     void* args[] = {&p};
-    GTD_CUDA(h, cudaLaunchCooperativeKernel(reinterpret_cast<void*>(bnb_kernel), dim3(static_cast<unsigned>(ctas)),
+    GTD_CUDA(h, cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kernel), dim3(static_cast<unsigned>(ctas)),
                                             dim3(32 * kBnbWarps), args, smem, h->stream));
   }
   const int tree_ctas = std::min(4096, (count + kBnbWarps - 1) / kBnbWarps);
