@@ -1173,7 +1173,8 @@ __global__ void __launch_bounds__(32 * kBnbWarps, 6) bnb_kernel(const __grid_con
   extern __shared__ __align__(16) uint8_t smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   WarpMem* w = reinterpret_cast<WarpMem*>(smem) + warp;
-  w->tag = p.memo_tag;  // read by the lane that wrote it
+  if (!WIDE)
+    w->tag = p.memo_tag;  // read by the lane that wrote it
   int cur_g = -1;
   for (uint32_t pass = 0;; ++pass) {
   uint32_t split_now = 0;
@@ -1263,16 +1264,20 @@ __global__ void __launch_bounds__(32 * kBnbWarps, 6) bnb_kernel(const __grid_con
         b = *reinterpret_cast<volatile uint64_t*>(p.t_begin + g);
       s.stop.deadline = __shfl_sync(0xffffffffu, b, 0) + p.deadline_ns;
     }
-    bool ok = false;
-    int u = -1;  // fixed second root (split items)
+    // What the item decides: td(cl, ch) <= depth under `root` (none: failed).
+    // One call, so that the search, which is inlined, is in the loop once: the
+    // warps wait for instructions, and with a copy for every kind of item (3-regular
+    // graph of 32 vertices 498 ms, a deleted grid of 66 1058) against one (487,
+    // 990) they are in different ones.
+    uint64_t cl = fl, ch = fh;
+    int depth = k, root = -1, u = -1;  // u: fixed second root (split items)
     const bool skip = G.n >= 3 && s.dominated(v, fl, fh);  // another root is at least as good
     if (!skip && !split) {
-      ok = s.decide(fl, fh, k, v, nullptr);
+      root = v;
     } else if (!skip) {
       // Split item (v, order[r2]): when C - v is connected, decide C - v under
       // root u at depth k - 1; else item r2 = 0 decides all of v and the
       // others have nothing to do (they count as failed).
-      uint64_t cl = fl, ch = fh;
       bit_clear(cl, ch, v);
       bool conn = false;
       if (G.n >= 3) {
@@ -1282,16 +1287,19 @@ __global__ void __launch_bounds__(32 * kBnbWarps, 6) bnb_kernel(const __grid_con
       }
       if (!conn) {
         if (r2 == 0)
-          ok = s.decide(fl, fh, k, v, nullptr);
+          root = v;
+        cl = fl;
+        ch = fh;
       } else {
         const int cand = w->order[r2];
         // u = v, or u dominated as a root of C - v: another second root is at least as good
         if (cand != v && !(G.n - 1 >= 3 && s.dominated(cand, cl, ch))) {
-          ok = s.decide(cl, ch, k - 1, cand, nullptr);
-          u = cand;
+          root = u = cand;
+          depth = k - 1;
         }
       }
     }
+    const bool ok = root >= 0 && s.decide(cl, ch, depth, root, nullptr);
     // A success is published only with its tree: the first success of a
     // level claims the level's parent buffer and builds the tree while the
     // memo entries of its search are fresh; later successes of the level
