@@ -341,6 +341,7 @@ struct TileParams {
   int64_t nparams;
   float* part;                 // [kGradRun][nparams]: weight gradients of the chunks of 64 rows of a run
   int first_chunk;             // of the run
+  float* grad_copy;            // the gradient once more next to the flag and the loss, for the one copy back (or null)
 };
 
 // Chunks whose weight gradients are held at a time (51 MB with three layers).
@@ -913,10 +914,13 @@ __global__ void __launch_bounds__(128) gnn_sum_chunks(const __grid_constant__ Ti
 #pragma unroll 8
   for (int c = 0; c < count; ++c)
     acc += from[c * step];
-  if (t == p.nparams)
+  if (t == p.nparams) {
     *loss = acc;
-  else
+  } else {
     grad[t] = 0.f + acc;
+    if (p.grad_copy)
+      p.grad_copy[t] = 0.f + acc;
+  }
 }
 
 }  // namespace
@@ -1192,14 +1196,15 @@ gtd_status run_tiles(gtd_gnn g, const gtd_gnn_batch* b, bool train, float td_wei
     if (a.bytes > kStaged)
       a.at = take(a.bytes);
   const size_t chunks = (std::max(N, G) + 63) / 64, NH = N * size_t(gtd::kWide), L = size_t(g->layers);
-  // results, in one copy back: the flag, the loss or the td estimates, the logits
-  const size_t ores = take(256), otde = take(G * 4), olog = take(N * 4), res_bytes = train ? 8 : off - ores;
+  // results, in one copy back: the flag, and the loss and the gradient or the td estimates and the logits
+  const size_t grad_bytes = train && grad_out ? size_t(g->nparams) * 4 : 0;
+  const size_t ores = take(256), ograd = take(grad_bytes), otde = take(G * 4), olog = take(N * 4);
+  const size_t res_bytes = !train ? off - ores : grad_bytes ? ograd + grad_bytes - ores : 8;
   const size_t ohs = take(train ? (L + 1) * NH * 4 : 0), oas = take(train ? L * NH * 4 : 0),
                odz = take(train ? (L + 1) * NH * 4 : 0), opool = take(train ? G * gtd::kWide * 4 : 0),
                otl2 = take(train ? size_t(tiles) * 4 : 0), opart = take(train ? std::min(chunks, size_t(gtd::kGradRun)) * size_t(g->nparams) * 4 : 0);
   GTD_CUDA(h, gtd::ensure_device(&g->buf, &g->buf_cap, off));
-  const size_t grad_bytes = train && grad_out ? size_t(g->nparams) * 4 : 0;
-  const size_t stage = std::max(staged, res_bytes + grad_bytes);
+  const size_t stage = std::max(staged, res_bytes);
   if (g->stage_cap < stage) {
     if (g->stage)
       cudaFreeHost(g->stage);
@@ -1258,6 +1263,7 @@ gtd_status run_tiles(gtd_gnn g, const gtd_gnn_batch* b, bool train, float td_wei
   p.tile_loss = f(otl2);
   p.nparams = g->nparams;
   p.part = f(opart);
+  p.grad_copy = grad_bytes ? f(ograd) : nullptr;
   if (train) {
     GTD_CUDA(h, (M == 32   ? launch_tile_kernel<32, true>(p, tiles, s)
                  : M == 64 ? launch_tile_kernel<64, true>(p, tiles, s)
@@ -1277,8 +1283,6 @@ gtd_status run_tiles(gtd_gnn g, const gtd_gnn_batch* b, bool train, float td_wei
                            : launch_tile_kernel<128, false>(p, tiles, s)));
   }
   GTD_CUDA(h, cudaMemcpyAsync(pinned, base + ores, res_bytes, cudaMemcpyDeviceToHost, s));
-  if (grad_bytes)
-    GTD_CUDA(h, cudaMemcpyAsync(pinned + res_bytes, g->grad, grad_bytes, cudaMemcpyDeviceToHost, s));
   GTD_CUDA(h, cudaStreamSynchronize(s));
   int32_t outside = 0;
   std::memcpy(&outside, pinned, 4);
@@ -1289,7 +1293,7 @@ gtd_status run_tiles(gtd_gnn g, const gtd_gnn_batch* b, bool train, float td_wei
     if (loss_out)
       std::memcpy(loss_out, pinned + 4, 4);
     if (grad_bytes)
-      std::memcpy(grad_out, pinned + res_bytes, grad_bytes);
+      std::memcpy(grad_out, pinned + (ograd - ores), grad_bytes);
   } else {
     if (td_out)
       std::memcpy(td_out, pinned + (otde - ores), G * 4);
