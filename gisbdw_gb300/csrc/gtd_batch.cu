@@ -3,12 +3,12 @@
 // Planning (host): graphs are put in descending n; those of at most
 // kBatchSmallMaxN vertices are solved one CTA each, with no table; the others
 // go through the level kernel, or where they are many the tile kernel. Of
-// these each gets a table region, a flag range and a descriptor. Tickets run level-major across graphs
-// (level 0 of every graph, then level 1, ...), so the children a tile waits
-// for were issued long before it; the ticket -> (graph, tile) map is filled
-// on the device. The launch sequence (zero the flags and
-// control words, validate, DP, tree) is captured once in a CUDA graph and
-// replayed while the batch keeps its shape and buffers.
+// these each gets a table region, a flag range and a descriptor. Tickets run
+// level-major across graphs (level 0 of every graph, then level 1, ...), so
+// the children a tile waits for were issued long before it; the ticket ->
+// (graph, tile) map is filled on the device. The launch sequence (zero the
+// flags and control words, validate, DP, tree) is captured once in a CUDA
+// graph and replayed while the batch keeps its shape and buffers.
 //
 // The autotuner times the DP kernel per (n, tile bits) on seeded random
 // graphs; where the tile kernel runs, the planner then gives each vertex count
