@@ -330,15 +330,11 @@ def _pack_edges():
     return _PACK or None
 
 
-def _native_pays(graphs, sizes, words: int) -> bool:
-    """Whether the native pass over the edge lists is faster than graph by
-    graph: it has a fixed cost of some 8 us (arrays and the call), as much as
-    100 vertices and edges take in masks of one word, 60 in masks of two (one
-    tree of 20 vertices, two words: 8.3 against 6.4 us; of 64: 8.6 against
-    19.2)."""
-    least = 100 if words == 1 else 60
-    vertices = sum(sizes)
-    return vertices >= least or vertices + sum(len(g.edges) for g in graphs) >= least
+# The native pass over the edge lists has a fixed cost of some 8 us (arrays and
+# the call), what this many vertices and edges take graph by graph, in masks of
+# one and of two words (one tree of 20 vertices, two words: 8.3 against 6.4 us;
+# of 64: 8.6 against 19.2).
+_NATIVE_FROM = {1: 100, 2: 60}
 
 
 def adjacency_pool(graphs, words: int) -> np.ndarray:
@@ -346,14 +342,19 @@ def adjacency_pool(graphs, words: int) -> np.ndarray:
     adj128() (words = 2, lo and hi per vertex) of each, built in one native
     pass over the edge lists where that is to be had and pays."""
     graphs = list(graphs)
-    sizes = [g.n for g in graphs]
-    pack = _pack_edges() if _native_pays(graphs, sizes, words) and max(sizes) <= 64 * words else None
+    least, size = _NATIVE_FROM[words], 0
+    for g in graphs:
+        size += g.n + len(g.edges)
+        if size >= least:
+            break
+    pack = _pack_edges() if size >= least else None
     if pack is not None:
-        ns = np.array(sizes, dtype=np.int64)
+        ns = np.array([g.n for g in graphs], dtype=np.int64)
         offs = np.zeros(len(graphs) + 1, dtype=np.int64)
         np.cumsum(ns, out=offs[1:])
         out = np.zeros(words * int(offs[-1]), dtype=np.uint64)
-        if pack([g.edges for g in graphs], _ptr(ns), _ptr(offs), words, _ptr(out)) == 0:
+        if int(ns.max()) <= 64 * words and \
+                pack([g.edges for g in graphs], _ptr(ns), _ptr(offs), words, _ptr(out)) == 0:
             return out
     parts = [g.adj64() if words == 1 else g.adj128() for g in graphs]
     return np.concatenate(parts).astype(np.uint64) if parts else np.zeros(0, dtype=np.uint64)
